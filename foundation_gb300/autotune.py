@@ -2,7 +2,7 @@
 
 The native tuner (fnd_rt_tune / fnd_rt_batch_tune) times every launch shape
 (block 64/128/256 x shared short stack 4/8/16 x refill threshold
-4/8/16/24 x triangle postponement off/8) on a ray batch, and for single
+4/8/16/24 x waiting-lane threshold default/8) on a ray batch, and for single
 scenes then the best shape with each coherence-order key width (9..21 bits,
 sort time included). This module runs it on representative workloads
 and keeps the winners in a JSON file keyed by

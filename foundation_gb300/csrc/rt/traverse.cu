@@ -11,22 +11,27 @@
 //    lanes hostage);
 //  * one thread per ray; the traversal state is a "node group" (base index of
 //    a node's internal children + the ordered bit mask of children still to
-//    visit) and a "triangle group" (base + bit mask of triangles to test);
-//  * a node's hit mask goes to the ray's traversal order (bit i: slot
-//    i ^ oct) through a shared 8 x 256-byte table in the single-scene and
-//    batched kernels (one load in place of three conditional bit swaps:
-//    +1.6% on the issue-bound kernel; the two-level kernel, whose shared
-//    memory already holds the world rays, keeps the swaps);
-//  * the stack holds node groups; its top kShort entries live in shared
-//    memory (one column per thread, bank-conflict free), deeper entries spill
-//    to a thread-local array; the depth bound kMaxStack is checked on the
-//    host at scene upload and again on every push (a failed push latches
+//    visit), the triangles of hit leaves wait in a ring of the warp (below);
+//  * a node's hit mask goes to the ray's traversal order through a shared
+//    8 x 256-byte table in the single-scene and batched kernels (one load in
+//    place of three conditional bit swaps); the two-level kernel, whose
+//    shared memory already holds the world rays, keeps the swaps;
+//  * the stack holds node groups; its first kShort entries live in shared
+//    memory (one column per thread, bank-conflict free), deeper entries in a
+//    thread-local array; the depth bound kMaxStack is checked on the host at
+//    scene upload and again on every push (a failed push latches
 //    kStatusStackOverflow and ends the ray instead of writing out of bounds).
-// Block size, short-stack depth and the refill threshold are launch
-// parameters chosen by the autotuner (capi/capi_batch.cpp); every
-// combination below is compiled. Two-level scenes (instances) run the same
-// loop with kTwoLevel: a lane descending into an instance pushes a return
-// marker and swaps its ray and node arrays to the instance's object space.
+// Block size, short-stack depth and the thresholds are launch parameters
+// chosen by the autotuner (capi/capi_batch.cpp); every combination below is
+// compiled. Two-level scenes (instances) run the same loop with kTwoLevel: a
+// lane descending into an instance pushes a return marker and swaps its ray
+// and node arrays to the instance's object space.
+//
+// What bounds it: instruction issue (about 80% of the slots busy, the rest
+// short waits; DRAM moves rays and hits only while the tree fits L2). 64
+// registers a thread and 32 warps per SM: at 56 registers (36 warps) the loop
+// spills about ten words a node step (8.4M incoherent Cornell rays 1.92 ms
+// against 1.77), at 72 (28 warps) it lacks warps (1.81 ms).
 #include <cfloat>
 
 #include "traverse.cuh"
@@ -40,13 +45,16 @@ namespace {
 
 constexpr uint32_t kFull = 0xFFFFFFFFu;
 constexpr uint32_t kTriGroupFlag = 0x80000000u;
+// Lanes that only wait for their triangles before a part-filled round runs. Any
+// value from 2 to 16 is within 1% on incoherent and camera rays; 1 costs 1%.
+constexpr uint32_t kWaitMin = 4;
 
 struct Common {
     uint32_t* counter;
     uint32_t* status;
     unsigned long long* stats;
     uint32_t refill_min;
-    uint32_t postpone_min;  // postpone a triangle group when fewer lanes than this have one (0: never)
+    uint32_t wait_min;  // flush the ring once this many lanes only wait for their pairs
 };
 
 // ---- work sources -----------------------------------------------------------
@@ -149,423 +157,462 @@ struct InstancedSource {
 
 constexpr uint32_t kInstanceMarker = 0xFFFFFFFFu;  // stack entry: return to the top level
 
-// ---- warp-cooperative triangle tests ----------------------------------------
-// After a node step each lane holds a triangle group (base + bit mask); lane
-// by lane the groups are uneven (most lanes have none, a few have a whole
-// leaf set), so a loop over its own group leaves most of the warp idle. Here
-// the warp lays its (ray, triangle) pairs out in lane order and tests up to
-// 32 of them per round, one per lane: a round takes the owners (lanes with a
-// group) in ascending lane order while their groups fit, each owner's
-// triangles in ascending order. A pair lane finds its owner from the mask of
-// group start positions (an OR over the warp) and its triangle as the k-th
-// set bit of the owner's mask; the owner's ray constants come from its slot
-// in shared memory, written when the ray was fetched. Each owner merges the
-// hits of its pairs with the sequential rule (smaller t, on equal t the lower
-// id), so the result is the one of a loop over its own group. A round tests
-// against the owner's best t at its start; a later round sees the improved
-// bound.
-
-// Position of the k-th set bit (k from 0) of m; k < popc(m).
-__device__ __forceinline__ uint32_t select_bit(uint32_t m, uint32_t k) {
-    uint32_t pos = 0, c;
-    c = (uint32_t)__popc(m & 0xFFFFu);
-    if (k >= c) { k -= c; m >>= 16; pos += 16; }
-    c = (uint32_t)__popc(m & 0xFFu);
-    if (k >= c) { k -= c; m >>= 8; pos += 8; }
-    c = (uint32_t)__popc(m & 0xFu);
-    if (k >= c) { k -= c; m >>= 4; pos += 4; }
-    c = (uint32_t)__popc(m & 0x3u);
-    if (k >= c) { k -= c; m >>= 2; pos += 2; }
-    return pos + (k >= (m & 1u) ? 1u : 0u);
+// ---- shared memory by 32-bit address ------------------------------------------
+// One address per warp region, kept in a register: through generic pointers
+// the compiler forms the shared window's base anew at nearly every access.
+__device__ __forceinline__ uint32_t shared_addr(const void* p) {
+    uint32_t a = (uint32_t)__cvta_generic_to_shared(p), r;
+    asm volatile("mov.u32 %0, %1;" : "=r"(r) : "r"(a));
+    return r;
+}
+__device__ __forceinline__ uint32_t lds8(uint32_t a) {
+    uint32_t v;
+    asm volatile("ld.shared.u8 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ uint32_t lds32(uint32_t a) {
+    uint32_t v;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ uint2 lds64(uint32_t a) {
+    uint2 v;
+    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ float4 lds128(uint32_t a) {
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                 : "r"(a)
+                 : "memory");
+    return v;
+}
+__device__ __forceinline__ void sts32(uint32_t a, uint32_t v) {
+    asm volatile("st.shared.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+__device__ __forceinline__ void sts64(uint32_t a, uint32_t x, uint32_t y) {
+    asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(a), "r"(x), "r"(y) : "memory");
+}
+__device__ __forceinline__ void sts128(uint32_t a, float x, float y, float z, float w) {
+    asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(a), "f"(x), "f"(y), "f"(z), "f"(w) : "memory");
 }
 
-// Per-thread shared slots of the cooperative stage (kBlock threads); with
-// kMulti (lanes of one warp in different scenes) also the triangle planes of
-// each lane's scene.
-template <int kBlock, bool kMulti>
-struct CoopShared {
-    float4 ray[2 * kBlock];  // [tid]: ox, oy, oz, tmin; [kBlock + tid]: -Sx, -Sy, Sz, kz bits
-    uint32_t owner[kBlock];  // per warp: lane of the group starting at a position
-    float t[kBlock];         // per warp: hit t of the pair at a position
-    uint32_t pid[kBlock];    // per warp: hit id of the pair at a position
-    const float4* planes[kMulti ? 3 * kBlock : 1];  // [a * kBlock + tid]: vertex plane a of the lane's scene
-    uint32_t prim_off[kMulti ? kBlock : 1];         // [tid]: hit-id offset of the lane's scene (instances)
+// Inclusive prefix sum over the warp. The shuffle's own in-range predicate
+// takes the place of a lane compare per step.
+__device__ __forceinline__ uint32_t warp_inclusive_sum(uint32_t v) {
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1)
+        asm volatile(
+            "{\n\t.reg .u32 t;\n\t.reg .pred p;\n\t"
+            "shfl.sync.up.b32 t|p, %0, %1, 0, 0xFFFFFFFF;\n\t"
+            "@p add.u32 %0, %0, t;\n\t}"
+            : "+r"(v)
+            : "r"(o));
+    return v;
+}
+
+// ---- the warp's queue of triangle tests ---------------------------------------
+// After a node step each lane holds the hit leaf slots of its node; lane by
+// lane they are uneven (most lanes have none, a few have several). The lanes
+// append one range (the node's first triangle, the slot's meta byte, the
+// owner lane) per hit leaf to a ring of the warp in shared memory, and the
+// warp tests the ranges' triangles 32 at a time, one per lane, whatever lanes
+// and node steps they came from: an owner's traversal goes on while its
+// ranges wait, against the best t known so far, so every round but a flush is
+// nearly full. The ray constants come from the owner's slot, written when the
+// ray was fetched, and a hit is merged into the owner's best (smaller t, on
+// equal t the lower id). The result does not depend on the order of the
+// tests: a triangle tested late can only have been worth a few node visits
+// more. A ray is finished once its traversal is and the ring has passed its
+// last range.
+constexpr uint32_t kRing = 64;  // ranges
+
+// Shared memory of one warp (byte offsets): per lane the ray's constants
+// (origin and tmin; -Sx, -Sy, Sz and kz; inverse direction and octx), its
+// best hit (t bits, id) and the merge slot, then the ring, with kMulti (lanes
+// of one warp in different scenes) the triangle planes of each lane's scene
+// and its hit-id offset, and the lanes' stacks. The origin and the inverse
+// direction are read back for each node: they are dead before the node
+// test's widest point, where registers are scarce.
+template <int kShort, bool kMulti>
+struct WarpShared {
+    static constexpr uint32_t kRayA = 0, kRayB = 512, kRayC = 1024, kBest = 1536, kWin = 1792, kRanges = 2048;
+    static constexpr uint32_t kPlanes = kRanges + 8 * kRing, kPrimOff = kPlanes + (kMulti ? 3 * 256 : 0);
+    static constexpr uint32_t kStack = kPrimOff + (kMulti ? 128 : 0), kBytes = kStack + 256 * kShort;
 };
 
-template <int kBlock, bool kMulti>
-__device__ __forceinline__ void coop_store_ray(CoopShared<kBlock, kMulti>* cs, const RayState& r,
-                                               const DeviceScene& sc, uint32_t prim_off = 0u) {
-    cs->ray[threadIdx.x] = make_float4(r.ox, r.oy, r.oz, r.tmin);
-    cs->ray[kBlock + threadIdx.x] = make_float4(r.nSx, r.nSy, r.Sz, __int_as_float(r.kz));
-    if constexpr (kMulti) {
-        cs->planes[threadIdx.x] = sc.v0;
-        cs->planes[kBlock + threadIdx.x] = sc.v1;
-        cs->planes[2 * kBlock + threadIdx.x] = sc.v2;
-        cs->prim_off[threadIdx.x] = prim_off;
-    }
-}
+// Group bit <-> slot (see persistent_trace).
+__device__ __forceinline__ uint32_t octx_of(const RayState& r) { return (r.oct ^ 7u) | 24u; }
 
-// All 32 lanes of the warp call this; lanes without a ray pass mine_ok = false.
-template <int kKind, bool kStats, int kBlock, bool kMulti, bool kOffsets = false>
-__device__ __forceinline__ void coop_triangles(const DeviceScene& sc, bool mine_ok, bool any_hit, uint32_t tg_base,
-                                               uint32_t& tg_mask, float& best_t, uint32_t& best_p,
-                                               uint32_t& ng_group, int& sp, CoopShared<kBlock, kMulti>* cs,
-                                               unsigned long long& st_tris, uint32_t& st_wtri) {
-    if (__ballot_sync(kFull, mine_ok && tg_mask != 0u) == 0u) return;
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t wbase = threadIdx.x & ~31u;
-    for (int round = 0; round < 33; ++round) {  // every round empties at least one group
-        const uint32_t mine = mine_ok ? tg_mask : 0u;
-        const uint32_t cnt = (uint32_t)__popc(mine);
-        uint32_t inc = cnt;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t v = __shfl_up_sync(kFull, inc, o);
-            if (lane >= (uint32_t)o) inc += v;
-        }
-        if (__shfl_sync(kFull, inc, 31) == 0u) break;
-        const uint32_t off = inc - cnt;
-        // this round: the owners whose whole group fits in positions 0..31
-        // (the first owner always does, at position 0)
-        const bool part = cnt != 0u && inc <= 32u;
-        const uint32_t starts = __reduce_or_sync(kFull, part ? 1u << off : 0u);
-        const uint32_t np = __reduce_max_sync(kFull, part ? inc : 0u);
-        if (part) cs->owner[wbase + off] = lane;
-        __syncwarp();
-        const uint32_t q = 31u - (uint32_t)__clz(starts & ((2u << lane) - 1u));  // start of this lane's group
-        const uint32_t owner = lane < np ? cs->owner[wbase + q] : 0u;
-        const uint32_t omask = __shfl_sync(kFull, mine, owner);
-        const uint32_t obase = __shfl_sync(kFull, tg_base, owner);
-        const float qt = __shfl_sync(kFull, best_t, owner);
-        bool hit = false;
-        float t = 0.0f;
-        uint32_t pid = 0;
-        if (lane < np) {
-            const uint32_t ti = obase + select_bit(omask, lane - q);
-            const float4 a = cs->ray[wbase + owner];
-            const float4 b = cs->ray[kBlock + wbase + owner];
-            RayState rq;
-            rq.ox = a.x;
-            rq.oy = a.y;
-            rq.oz = a.z;
-            rq.tmin = a.w;
-            rq.nSx = b.x;
-            rq.nSy = b.y;
-            rq.Sz = b.z;
-            rq.kz = __float_as_int(b.w);
-            const float4 *p0 = sc.v0, *p1 = sc.v1, *p2 = sc.v2;
-            if constexpr (kMulti) {
-                p0 = cs->planes[wbase + owner];
-                p1 = cs->planes[kBlock + wbase + owner];
-                p2 = cs->planes[2 * kBlock + wbase + owner];
-            }
-            const float4 v0 = __ldg(p0 + ti);
-            hit = intersect_tri(rq, v0, __ldg(p1 + ti), __ldg(p2 + ti), qt, t);
-            pid = __float_as_uint(v0.w);
-            if constexpr (kOffsets) pid += cs->prim_off[wbase + owner];  // global id of an instance's triangle
-            if (kStats) {
-                st_tris++;
-                if (lane == 0u) st_wtri++;
-            }
-        }
-        if (part && mine_ok) tg_mask = 0u;
-        const uint32_t hm = __ballot_sync(kFull, hit);
-        if (hm) {
-            if (hit) {
-                cs->t[wbase + lane] = t;
-                cs->pid[wbase + lane] = pid;
-            }
-            __syncwarp();
-            uint32_t c = part ? hm & (cnt == 32u ? kFull : ((1u << cnt) - 1u) << off) : 0u;
-            while (c) {
-                const uint32_t j = (uint32_t)__ffs(c) - 1u;
-                c &= c - 1u;
-                const float tj = cs->t[wbase + j];
-                const uint32_t pj = cs->pid[wbase + j];
-                if (kKind == 1 || (kKind == 2 && any_hit)) {
-                    best_t = tj;
-                    best_p = pj;
-                    tg_mask = 0;
-                    ng_group = 0;
-                    sp = 0;
-                    break;
-                }
-                if (best_p == FND_INVALID_ID || tj < best_t || (tj == best_t && pj < best_p)) {
-                    best_t = tj;
-                    best_p = pj;
-                }
-            }
-        }
-        __syncwarp();  // the slots are rewritten by the next round
+template <int kShort, bool kMulti>
+__device__ __forceinline__ void store_ray(uint32_t w, uint32_t lane, const RayState& r) {
+    using W = WarpShared<kShort, kMulti>;
+    sts128(w + 16u * lane + W::kRayA, r.ox, r.oy, r.oz, r.tmin);
+    sts128(w + 16u * lane + W::kRayB, r.nSx, r.nSy, r.Sz, __int_as_float(r.kz));
+    sts128(w + 16u * lane + W::kRayC, r.ix, r.iy, r.iz, __uint_as_float(octx_of(r)));
+}
+// kMulti: the lane's triangle planes and hit-id offset.
+template <int kShort>
+__device__ __forceinline__ void store_scene(uint32_t w, uint32_t lane, const DeviceScene& sc, uint32_t prim_off) {
+    using W = WarpShared<kShort, true>;
+    const float4* p[3] = {sc.v0, sc.v1, sc.v2};
+    for (int a = 0; a < 3; ++a) {
+        const unsigned long long v = (unsigned long long)p[a];
+        sts64(w + 8u * lane + W::kPlanes + 256u * a, (uint32_t)v, (uint32_t)(v >> 32));
     }
+    sts32(w + 4u * lane + W::kPrimOff, prim_off);
+}
+__device__ __forceinline__ const float4* lds_ptr(uint32_t a) {
+    const uint2 v = lds64(a);
+    return (const float4*)((unsigned long long)v.y << 32 | v.x);
 }
 
 // ---- the persistent traversal loop ----------------------------------------
 // kKind: 0 closest, 1 any, 2 per-lane (from the source). kTwoLevel: the
 // source is an InstancedSource (triangle leaves of the top level are
-// instances; per-lane node / triangle arrays).
-template <class Src, int kKind, bool kStats, int kShort, int kBlock, bool kTwoLevel = false, bool kCoop = false,
-          bool kMulti = false>
-__device__ __forceinline__ void persistent_trace(const Src& src, const Common& C, uint2* s_stack,
-                                                 CoopShared<kBlock, kMulti>* s_coop = nullptr,
-                                                 RayState* s_world = nullptr, const uint8_t* s_perm = nullptr) {
-    // two-level cooperative rounds: each lane's planes and hit-id offset
-    // come from its own slot (the lanes of a warp sit in different instances)
-    static_assert(!(kCoop && kTwoLevel) || kMulti, "two-level cooperative rounds need per-lane scenes");
-    static_assert((kShort & (kShort - 1)) == 0, "short stack size must be a power of two");
+// instances; per-lane node / triangle arrays). w: this warp's region of
+// shared memory, tab: the tables of fill_tables.
+//
+// A node group is one word: the internal children still to visit in bits
+// 24..31, the highest bit first (bit 24 + j is slot j ^ 7 ^ oct, so the
+// highest bit is the nearest along the ray's octant), and the node's imask
+// in bits 0..7.
+template <class Src, int kKind, bool kStats, int kShort, bool kTwoLevel = false, bool kMulti = false>
+__device__ __forceinline__ void persistent_trace(const Src& src, const Common& C, uint32_t w, uint32_t tab,
+                                                 float4* s_world = nullptr) {
+    using W = WarpShared<kShort, kMulti>;
+    // two-level: each lane's planes and hit-id offset come from its own slot
+    // (the lanes of a warp sit in different instances)
+    static_assert(!kTwoLevel || kMulti, "two-level traversal needs per-lane scenes");
     uint2 l_stack[kMaxStack - kShort];
-    const int tid = threadIdx.x;
-    const uint32_t lane = tid & 31;
+    uint32_t lane, below;
+    asm volatile("mov.u32 %0, %%laneid;" : "=r"(lane));
+    asm volatile("mov.u32 %0, %%lanemask_lt;" : "=r"(below));
+    const uint32_t wl = w + 8u * lane;  // the lane's 8-byte slots
     const uint32_t n = src.n;
 
     bool active = false, exhausted = false, any_hit = kKind == 1;
     uint32_t ray_id = 0;
     typename Src::Lane ln{};
-    RayState r;
-    float best_t = 0.0f;
-    uint32_t best_p = FND_INVALID_ID;
-    uint32_t ng_base = 0, ng_group = 0, tg_base = 0, tg_mask = 0;
+    float best_t = 0.0f, tmin = 0.0f;
+    uint32_t ng_base = 0, ng_group = 0;
     int sp = 0;
+    // the warp's ring: ranges head .. tail - 1 (modulo 2^32), with `tris` triangles written
+    uint32_t head = 0, tail = 0, tris = 0;
+    uint32_t my_end = 0;  // the ring position after this lane's last range
     unsigned long long st_nodes = 0, st_tris = 0;
     uint32_t st_wnode = 0, st_wtri = 0;  // warp steps, counted by the lowest active lane
-    // two-level state: the arrays the lane traverses now, and its instance
-    bool in_blas = false, moved = false;  // moved: r holds an object-space ray, the world one is in s_world
+    // two-level state: the arrays the lane traverses now, its instance, and
+    // the instances of a top-level leaf still to enter
+    bool in_blas = false, moved = false;  // moved: the lane's ray is an object-space one, the world one is in s_world
     DeviceScene cur{};
-    uint32_t prim_off = 0;
+    uint32_t tl_base = 0, tl_mask = 0;
 
-    auto push = [&](uint2 e) -> bool {
-        if (sp >= kMaxStack) return false;
-        const int s = (sp & (kShort - 1)) * kBlock + tid;
-        if (sp >= kShort) l_stack[sp - kShort] = s_stack[s];
-        s_stack[s] = e;
+    // the first kShort entries in shared memory, deeper ones in local memory
+    auto push = [&](uint32_t x, uint32_t y) -> bool {
+        if (sp < kShort)
+            sts64(wl + W::kStack + 256u * (uint32_t)sp, x, y);
+        else if (sp < kMaxStack)
+            l_stack[sp - kShort] = make_uint2(x, y);
+        else
+            return false;
         sp++;
         return true;
     };
-    // two-level: descend into instance I (from the top level, r the world
-    // ray). Its object-space ray replaces r, and the world ray's set-up
-    // waits in s_world for the return; an identity instance keeps r.
+    // the root as a pseudo group: one internal child in slot 0
+    auto start = [&](uint32_t num_nodes, uint32_t octx) {
+        ng_base = 0;
+        ng_group = num_nodes ? (1u << octx) | 1u : 0u;  // (an empty scene: a miss)
+    };
+    // two-level: descend into instance I (from the top level). Its
+    // object-space ray replaces the lane's ray, and the world ray's constants
+    // wait in s_world for the return; an identity instance keeps them.
     auto enter_instance = [&](const InstanceRec& I) {
         if constexpr (kTwoLevel) {
-            if (!(__ldg(&I.flags) & kInstanceIdentity)) {
+            cur = I.blas;
+            in_blas = true;
+            moved = !(__ldg(&I.flags) & kInstanceIdentity);
+            if (moved) {
+                for (int q = 0; q < 3; ++q) s_world[3 * threadIdx.x + q] = lds128(wl + 8u * lane + W::kRayA + 512u * q);
                 float inv[12];
                 for (int q = 0; q < 12; ++q) inv[q] = __ldg(I.inv + q);
                 float4 r0, r1, o0, o1;
                 src.load(ray_id, r0, r1, ln);
                 instance_ray(inv, r0, r1, o0, o1);
-                s_world[tid] = r;
-                r = setup_ray(o0, o1);
-                moved = true;
+                store_ray<kShort, kMulti>(w, lane, setup_ray(o0, o1));
             }
-            cur = I.blas;
-            prim_off = __ldg(&I.prim_offset);
-            in_blas = true;
-            ng_base = 0;
-            ng_group = cur.num_nodes ? (1u << 8) | (1u << r.oct) : 0u;
-            tg_mask = 0;
+            store_scene<kShort>(w, lane, cur, __ldg(&I.prim_offset));
+            start(cur.num_nodes, lds32(wl + 8u * lane + W::kRayC + 12u));
         }
     };
 
     for (;;) {
-        // ---- dynamic fetch -------------------------------------------------
-        const uint32_t idle = __ballot_sync(kFull, !active);
-        if (!exhausted && idle != 0u && (__popc(idle) >= (int)C.refill_min || idle == kFull)) {
-            const uint32_t cnt = (uint32_t)__popc(idle);
+        // ---- finished rays out, new rays in ----------------------------------
+        // ready: lanes without a ray, or with one whose traversal and ranges
+        // are done. A warp turns to them once there are refill_min (or, when
+        // no rays are left, all).
+        const bool work = ng_group >= (1u << 24) && (!kTwoLevel || tl_mask == 0u);
+        const uint32_t working = __ballot_sync(kFull, work);
+        const uint32_t ready = __ballot_sync(kFull, !work && (!kTwoLevel || tl_mask == 0u) && (int)(my_end - head) <= 0);
+        if (ready == kFull || (!exhausted && (uint32_t)__popc(ready) >= C.refill_min)) {
+            const bool mine = !work && (!kTwoLevel || tl_mask == 0u) && (int)(my_end - head) <= 0;
+            if (mine && active) {
+                const uint2 bst = lds64(wl + W::kBest);
+                src.store(ray_id, ln, any_hit, bst.y, __uint_as_float(bst.x));
+                active = false;
+            }
+            if (exhausted) break;
+            const uint32_t cnt = (uint32_t)__popc(ready);
             uint32_t base = 0;
             if (lane == 0) base = atomicAdd(C.counter, cnt);
             base = __shfl_sync(kFull, base, 0);
-            if (base + cnt >= n) exhausted = true;
-            if (!active) {
-                const uint32_t pos = base + (uint32_t)__popc(idle & ((1u << lane) - 1u));
-                if (pos < n) {
-                    const uint32_t id = src.map(pos);
-                    float4 r0, r1;
-                    src.load(id, r0, r1, ln);
-                    if (kKind == 2) any_hit = src.any_of(ln, false);
-                    r = setup_ray(r0, r1);
-                    if constexpr (kCoop) coop_store_ray<kBlock, kMulti>(s_coop, r, src.scene_of(ln));
-                    ray_id = id;
-                    best_t = r.tmax;
-                    best_p = FND_INVALID_ID;
-                    ng_base = 0;
-                    ng_group = (1u << 8) | (1u << r.oct);  // pseudo group holding the root in slot 0
-                    if (src.scene_of(ln).num_nodes == 0) ng_group = 0;  // empty scene: a miss
-                    tg_mask = 0;
-                    sp = 0;
-                    active = true;
-                    if constexpr (kTwoLevel) {
-                        in_blas = false;
-                        moved = false;
-                        cur = src.scene;
-                        prim_off = 0;
-                    }
+            exhausted = base + cnt >= n;
+            const uint32_t pos = base + (uint32_t)__popc(ready & below);
+            if (mine && pos < n) {
+                const uint32_t id = src.map(pos);
+                float4 r0, r1;
+                src.load(id, r0, r1, ln);
+                if (kKind == 2) any_hit = src.any_of(ln, false);
+                const RayState r = setup_ray(r0, r1);
+                store_ray<kShort, kMulti>(w, lane, r);
+                if constexpr (kMulti) store_scene<kShort>(w, lane, src.scene_of(ln), 0u);
+                tmin = r.tmin;
+                ray_id = id;
+                best_t = r.tmax;
+                sts64(wl + W::kBest, __float_as_uint(r.tmax), FND_INVALID_ID);
+                start(src.scene_of(ln).num_nodes, octx_of(r));
+                active = true;
+                if constexpr (kTwoLevel) {
+                    in_blas = false;
+                    moved = false;
+                    cur = src.scene;
                 }
             }
-        }
-        if (__ballot_sync(kFull, active) == 0u) {
-            if (exhausted) break;
+            my_end = mine ? head : my_end;
             continue;
         }
-        // the cooperative triangle stage needs the whole warp: idle lanes
-        // run the iteration with empty node and triangle groups
-        if (!kCoop && !active) continue;
 
-        const DeviceScene& sc = kTwoLevel ? cur : src.scene_of(ln);
-        bool overflow = false;
         // ---- one node --------------------------------------------------------
-        if ((kCoop ? active : true) && (ng_group & 0xFFu)) {
-            const uint32_t b = (uint32_t)__ffs(ng_group & 0xFFu) - 1u;
+        uint32_t leaves = 0, tri_base = 0, meta0 = 0, meta1 = 0;
+        if (work) {
+            const DeviceScene& sc = kTwoLevel ? cur : src.scene_of(ln);
+            const float4 ra = lds128(wl + 8u * lane + W::kRayA), rc = lds128(wl + 8u * lane + W::kRayC);
+            const uint32_t octx = __float_as_uint(rc.w);
+            const uint32_t b = 31u - (uint32_t)__clz(ng_group);
             ng_group &= ~(1u << b);
-            const uint32_t slot = b ^ r.oct;
-            const uint32_t child = ng_base + (uint32_t)__popc((ng_group >> 8) & ((1u << slot) - 1u));
-            if (ng_group & 0xFFu) overflow = !push(make_uint2(ng_base, ng_group));
-            if (overflow) {
-            } else if (child < sc.num_nodes) {
-                const NodeHits h = intersect_node(r, sc.nodes, child, best_t, s_perm);
+            const uint32_t child = ng_base + (uint32_t)__popc(ng_group & ~(kFull << (b ^ octx)));
+            uint32_t fail = 0;
+            if (ng_group >= (1u << 24) && !push(ng_base, ng_group)) fail = kStatusStackOverflow;
+            if (child >= sc.num_nodes) fail |= kStatusBadIndex;
+            if (!fail) {
+                RayState r;
+                r.ox = ra.x;
+                r.oy = ra.y;
+                r.oz = ra.z;
+                r.tmin = tmin;
+                r.ix = rc.x;
+                r.iy = rc.y;
+                r.iz = rc.z;
+                const SlotHits h = intersect_slots(r, sc.nodes, child, best_t);
                 if (kStats) {
                     st_nodes++;
                     if (lane == (uint32_t)__ffs(__activemask()) - 1u) st_wnode++;
                 }
+                const uint32_t inner = h.hitm & h.imask;
+                const uint32_t order = kTwoLevel ? xor_permute8(inner, octx & 7u) : lds8(tab + ((octx & 7u) << 8) + inner);
                 ng_base = h.child_base;
-                ng_group = h.group;
-                tg_base = h.tri_base;
-                tg_mask = h.tris;
-                // a node's triangles must lie inside the triangle arrays
-                if (tg_mask && (uint64_t)tg_base + (uint64_t)(32 - __clz(tg_mask)) > sc.num_tris) {
-                    atomicOr(C.status, kStatusBadIndex);
-                    tg_mask = 0;
-                    ng_group = 0;
-                    sp = 0;
+                ng_group = order << 24 | h.imask;
+                leaves = h.hitm & leaf_slots(h);
+                tri_base = h.tri_base;
+                meta0 = h.meta[0];
+                meta1 = h.meta[1];
+                // a node's triangles (at most 4 from offset 31 on) must lie
+                // inside the triangle arrays; only near their end each range
+                // is looked at
+                if (leaves && (sc.num_tris < 35u || tri_base > sc.num_tris - 35u)) {
+                    for (uint32_t q = leaves; q; q &= q - 1u) {
+                        const uint32_t m = meta_of(h, (uint32_t)__ffs(q) - 1u);
+                        if ((uint64_t)tri_base + (m & 31u) + (m >> 5 & 3u) >= sc.num_tris) fail = kStatusBadIndex;
+                    }
                 }
-                // triangle postponement (Ylitie et al. 2017): when only a few
-                // lanes of the warp have triangles to test, keep traversing
-                // nodes with the rest and test the triangles later
-                if (!kTwoLevel && !kCoop && C.postpone_min) {
-                    const uint32_t tri_lanes = __ballot_sync(__activemask(), tg_mask != 0u);
-                    if (tg_mask && (ng_group & 0xFFu) && (uint32_t)__popc(tri_lanes) < C.postpone_min &&
-                        push(make_uint2(tg_base | kTriGroupFlag, tg_mask)))
-                        tg_mask = 0;
-                }
-            } else {
-                atomicOr(C.status, kStatusBadIndex);
+            }
+            if (fail) {  // the ray ends with the hits found so far
+                atomicOr(C.status, fail);
                 ng_group = 0;
-                tg_mask = 0;
+                leaves = 0;
                 sp = 0;
             }
         }
-        // ---- its triangles, tested by the whole warp ------------------------
-        if constexpr (kCoop) {
-            if constexpr (kTwoLevel) {
-                // a top-level leaf holds instances: the lane enters the first
-                // valid one by itself (resume order as in the per-lane loop
-                // below) and publishes its object-space ray for the rounds
-                while (active && !overflow && !in_blas && tg_mask) {
-                    const uint32_t k = (uint32_t)__ffs(tg_mask) - 1u;
-                    tg_mask &= tg_mask - 1u;
-                    const uint32_t iid = __float_as_uint(__ldg(cur.v0 + tg_base + k).w);
-                    if (iid >= src.num_inst) {
-                        atomicOr(C.status, kStatusBadIndex);
-                        continue;
-                    }
-                    overflow = ((ng_group & 0xFFu) && !push(make_uint2(ng_base, ng_group))) ||
-                               (tg_mask && !push(make_uint2(tg_base | kTriGroupFlag, tg_mask))) ||
-                               !push(make_uint2(kInstanceMarker, 0u));
-                    if (overflow) break;
-                    const InstanceRec& I = src.inst[iid];
-                    enter_instance(I);
-                    coop_store_ray<kBlock, kMulti>(s_coop, r, cur, prim_off);
+        if constexpr (kTwoLevel) {
+            // a top-level leaf holds instances: its slots become one mask
+            while (!in_blas && leaves) {
+                const uint32_t s = (uint32_t)__ffs(leaves) - 1u;
+                leaves &= leaves - 1u;
+                const uint32_t m = __byte_perm(s < 4u ? meta0 : meta1, 0u, 0x4440u | (s & 3u));
+                tl_base = tri_base;
+                tl_mask |= ((2u << (m >> 5 & 3u)) - 1u) << (m & 31u);
+            }
+            // the lane enters the first valid one and publishes its
+            // object-space ray (the ring is empty here: see flush below)
+            while (!in_blas && tl_mask) {
+                const uint32_t k = (uint32_t)__ffs(tl_mask) - 1u;
+                tl_mask &= tl_mask - 1u;
+                const uint32_t iid = __float_as_uint(__ldg(cur.v0 + tl_base + k).w);
+                if (iid >= src.num_inst) {
+                    atomicOr(C.status, kStatusBadIndex);
+                    continue;
                 }
-            }
-            coop_triangles<kKind, kStats, kBlock, kMulti, kTwoLevel>(sc, active && !overflow, any_hit, tg_base,
-                                                                     tg_mask, best_t, best_p, ng_group, sp, s_coop,
-                                                                     st_tris, st_wtri);
-            if (!active) continue;
-        }
-        // ---- its triangles (or, on the top level, its instances) ------------
-        while (!kCoop && tg_mask && !overflow) {
-            const uint32_t k = (uint32_t)__ffs(tg_mask) - 1u;
-            tg_mask &= tg_mask - 1u;
-            const uint32_t ti = tg_base + k;
-            if constexpr (kTwoLevel) {
-                if (!in_blas) {
-                    const uint32_t iid = __float_as_uint(__ldg(sc.v0 + ti).w);
-                    if (iid >= src.num_inst) {
-                        atomicOr(C.status, kStatusBadIndex);
-                        continue;
-                    }
-                    // resume order after the instance: this leaf's other
-                    // instances, then the node's other children
-                    overflow = ((ng_group & 0xFFu) && !push(make_uint2(ng_base, ng_group))) ||
-                               (tg_mask && !push(make_uint2(tg_base | kTriGroupFlag, tg_mask))) ||
-                               !push(make_uint2(kInstanceMarker, 0u));
-                    if (overflow) break;
-                    const InstanceRec& I = src.inst[iid];
-                    enter_instance(I);
-                    break;
-                }
-            }
-            const float4 v0 = __ldg(sc.v0 + ti);
-            const float4 v1 = __ldg(sc.v1 + ti);
-            const float4 v2 = __ldg(sc.v2 + ti);
-            if (kStats) {
-                st_tris++;
-                if (lane == (uint32_t)__ffs(__activemask()) - 1u) st_wtri++;
-            }
-            float t;
-            if (intersect_tri(r, v0, v1, v2, best_t, t)) {
-                const uint32_t pid = __float_as_uint(v0.w) + (kTwoLevel ? prim_off : 0u);
-                if (any_hit) {
-                    best_t = t;
-                    best_p = pid;
-                    tg_mask = 0;
+                // resume order after the instance: this leaf's other
+                // instances, then the node's other children
+                const bool ok = (ng_group < (1u << 24) || push(ng_base, ng_group)) &&
+                                (!tl_mask || push(tl_base | kTriGroupFlag, tl_mask)) && push(kInstanceMarker, 0u);
+                tl_mask = 0;
+                if (!ok) {
+                    atomicOr(C.status, kStatusStackOverflow);
                     ng_group = 0;
                     sp = 0;
-                } else if (best_p == FND_INVALID_ID || t < best_t || (t == best_t && pid < best_p)) {
-                    best_t = t;
-                    best_p = pid;
+                    break;
                 }
+                const InstanceRec& I = src.inst[iid];
+                enter_instance(I);
             }
         }
-        // ---- next group or done ------------------------------------------
-        if ((ng_group & 0xFFu) == 0u && tg_mask == 0u && !overflow) {
-            if (sp > 0) {
-                sp--;
-                const int s = (sp & (kShort - 1)) * kBlock + tid;
-                const uint2 e = s_stack[s];
-                if (sp >= kShort) s_stack[s] = l_stack[sp - kShort];
-                bool marker = false;
-                if constexpr (kTwoLevel) {
-                    if (e.x == kInstanceMarker) {
-                        // back to the top level: the world ray again
-                        if (moved) r = s_world[tid];
-                        moved = false;
-                        cur = src.scene;
-                        prim_off = 0;
-                        in_blas = false;
-                        ng_group = 0;
-                        tg_mask = 0;
-                        marker = true;
+        // ---- its leaves into the ring ------------------------------------------
+        // positions by the bits of the lanes' range counts (at most 8 each)
+        uint32_t at = 0;
+        bool fresh = __ballot_sync(kFull, leaves != 0u) != 0u;
+        if (fresh) {
+            const uint32_t cnt = (uint32_t)__popc(leaves);
+            const uint32_t b0 = __ballot_sync(kFull, cnt & 1u), b1 = __ballot_sync(kFull, cnt & 2u);
+            at = tail + (uint32_t)__popc(b0 & below) + 2u * (uint32_t)__popc(b1 & below);
+            tail += (uint32_t)__popc(b0) + 2u * (uint32_t)__popc(b1);
+            if (__ballot_sync(kFull, cnt > 3u)) {
+                const uint32_t b2 = __ballot_sync(kFull, cnt & 4u), b3 = __ballot_sync(kFull, cnt & 8u);
+                at += 4u * (uint32_t)__popc(b2 & below) + 8u * (uint32_t)__popc(b3 & below);
+                tail += 4u * (uint32_t)__popc(b2) + 8u * (uint32_t)__popc(b3);
+            }
+            if (cnt) my_end = at + cnt;
+        }
+        // ---- rounds: whenever 32 triangles wait, and all of them when several
+        // lanes only wait for theirs or no lane can go on ---------------------
+        // (two-level: after every step, as a lane's slot changes with its instance)
+        const bool flush = kTwoLevel || working == 0u || 32u - (uint32_t)__popc(working | ready) >= C.wait_min;
+        for (;;) {
+            if (fresh) {
+                // ranges [head, head + kRing) are written; more as rounds make room
+                uint32_t sum = 0;
+                while (leaves && at - head < kRing) {
+                    const uint32_t s = 31u - (uint32_t)__clz(leaves);
+                    leaves &= ~(1u << s);
+                    // (meta byte, owner lane, 0, 0)
+                    const uint32_t y = __byte_perm(s < 4u ? meta0 : meta1, lane, 0x5540u | (s & 3u));
+                    sum += (y >> 5 & 3u) + 1u;
+                    sts64(w + W::kRanges + 8u * (at & (kRing - 1u)), tri_base, y);
+                    at++;
+                }
+                tris += __reduce_add_sync(kFull, sum);
+                fresh = tail - head > kRing;
+                __syncwarp();
+            }
+            if (tris < 32u && !fresh && !(flush && tris)) break;
+            // the ranges that fit 32 lanes, in ring order: one lane per range
+            // finds its first position, then one lane per triangle its range
+            const bool have = lane < tail - head;
+            const uint2 e = lds64(w + W::kRanges + 8u * ((head + lane) & (kRing - 1u)));
+            const uint32_t cnt = have ? (e.y >> 5 & 3u) + 1u : 0u;
+            const uint32_t inc = warp_inclusive_sum(cnt);
+            const uint32_t starts = __reduce_or_sync(kFull, have && inc <= 32u ? 1u << (inc - cnt) : 0u);
+            const uint32_t nr = (uint32_t)__popc(starts);
+            const uint32_t np = __shfl_sync(kFull, inc, nr - 1u);
+            const uint32_t upto = starts & (below * 2u + 1u);
+            const uint32_t from = (uint32_t)__popc(upto) - 1u;
+            const uint32_t first = __shfl_sync(kFull, e.x + (e.y & 31u), from);
+            const uint32_t own = w + 8u * __shfl_sync(kFull, e.y >> 8, from);
+            bool hit = false;
+            float t = 0.0f;
+            uint32_t pid = 0;
+            if (lane < np) {
+                const uint32_t ti = first + (lane - (31u - (uint32_t)__clz(upto)));
+                const float4 a = lds128(2u * own - w + W::kRayA);
+                const float4 b = lds128(2u * own - w + W::kRayB);
+                RayState rq;
+                rq.ox = a.x;
+                rq.oy = a.y;
+                rq.oz = a.z;
+                rq.tmin = a.w;
+                rq.nSx = b.x;
+                rq.nSy = b.y;
+                rq.Sz = b.z;
+                rq.kz = __float_as_int(b.w);
+                const float4 *p0 = src.scene_of(ln).v0, *p1 = src.scene_of(ln).v1, *p2 = src.scene_of(ln).v2;
+                if constexpr (kMulti) {
+                    p0 = lds_ptr(own + W::kPlanes);
+                    p1 = lds_ptr(own + W::kPlanes + 256u);
+                    p2 = lds_ptr(own + W::kPlanes + 512u);
+                }
+                const float4 v0 = __ldg(p0 + ti);
+                hit = intersect_tri(rq, v0, __ldg(p1 + ti), __ldg(p2 + ti), __uint_as_float(lds32(own + W::kBest)), t);
+                pid = __float_as_uint(v0.w);
+                if constexpr (kTwoLevel) pid += lds32(w + (own - w) / 2u + W::kPrimOff);  // global id of an instance's triangle
+                if (kStats) {
+                    st_tris++;
+                    if (lane == 0u) st_wtri++;
+                }
+            }
+            head += nr;
+            tris -= np;
+            if (__ballot_sync(kFull, hit)) {
+                // one hit per owner at a time
+                do {
+                    if (hit) sts32(own + W::kWin, lane);
+                    __syncwarp();
+                    if (hit && lds32(own + W::kWin) == lane) {
+                        const uint2 bst = lds64(own + W::kBest);
+                        const float bt = __uint_as_float(bst.x);
+                        if (t < bt || (t == bt && pid < bst.y)) sts64(own + W::kBest, __float_as_uint(t), pid);
+                        hit = false;
                     }
+                    __syncwarp();
+                } while (__ballot_sync(kFull, hit));
+                const uint2 bst = lds64(wl + W::kBest);
+                best_t = __uint_as_float(bst.x);
+                if ((kKind == 1 || (kKind == 2 && any_hit)) && active && bst.y != FND_INVALID_ID) {
+                    ng_group = 0;  // found: only the ranges already in the ring remain
+                    sp = 0;
+                    if (kTwoLevel) tl_mask = 0;
                 }
-                if (marker) {
-                } else if (e.x & kTriGroupFlag) {
-                    tg_base = e.x & ~kTriGroupFlag;
-                    tg_mask = e.y;
-                    ng_group = 0;
-                } else {
-                    ng_base = e.x;
-                    ng_group = e.y;
-                }
-                continue;
             }
-        } else if (!overflow) {
-            continue;
+            __syncwarp();
         }
-        // ray finished (or aborted on overflow)
-        if (overflow) atomicOr(C.status, kStatusStackOverflow);
-        src.store(ray_id, ln, any_hit, best_p, best_t);
-        active = false;
-        ng_group = 0;
-        tg_mask = 0;
+        // ---- next group ----------------------------------------------------
+        if (ng_group < (1u << 24) && sp > 0 && (!kTwoLevel || tl_mask == 0u)) {
+            auto pop = [&] {
+                sp--;
+                return sp < kShort ? lds64(wl + W::kStack + 256u * (uint32_t)sp) : l_stack[sp - kShort];
+            };
+            uint2 e = pop();
+            if constexpr (kTwoLevel) {
+                if (e.x == kInstanceMarker) {
+                    // back to the top level: the world ray again
+                    if (moved)
+                        for (int q = 0; q < 3; ++q) {
+                            const float4 v = s_world[3 * threadIdx.x + q];
+                            sts128(wl + 8u * lane + W::kRayA + 512u * q, v.x, v.y, v.z, v.w);
+                        }
+                    cur = src.scene;
+                    in_blas = false;
+                    e = sp > 0 ? pop() : make_uint2(0u, 0u);
+                }
+                if (e.x & kTriGroupFlag) {  // a top-level leaf's other instances
+                    tl_base = e.x & ~kTriGroupFlag;
+                    tl_mask = e.y;
+                    e.y = 0;
+                }
+            }
+            ng_base = e.x;
+            ng_group = e.y;
+        }
     }
     if (kStats) {
         for (int o = 16; o > 0; o >>= 1) {
@@ -583,24 +630,21 @@ __device__ __forceinline__ void persistent_trace(const Src& src, const Common& C
     }
 }
 
-// 36 resident warps per SM (9 blocks of 128 threads: at most 56 registers)
-// unless the block is 256 threads wide.
-constexpr int MinBlocks(int block) { return block == 256 ? 4 : 1152 / block; }
+// 32 resident warps per SM (64 registers a thread).
+constexpr int MinBlocks(int block) { return 1024 / block; }
 
 // Fills the 8 x 256 byte table of xor_permute8 (all threads of the block).
-__device__ __forceinline__ void fill_perm(uint8_t* t) {
+constexpr int kTableBytes = 2048;
+__device__ __forceinline__ void fill_tables(uint8_t* t) {
     for (uint32_t i = threadIdx.x; i < 2048u; i += blockDim.x) t[i] = (uint8_t)xor_permute8(i & 255u, i >> 8);
-    uint32_t* m = reinterpret_cast<uint32_t*>(t + 2048);
-    for (uint32_t i = threadIdx.x; i < 256u; i += blockDim.x) m[i] = ((2u << ((i >> 5) & 3u)) - 1u) << (i & 31u);
     __syncthreads();
 }
 
 template <bool kAny, bool kStats, int kShort, int kBlock>
 __global__ void __launch_bounds__(kBlock, MinBlocks(kBlock)) trace_kernel(const TraceLaunch L) {
-    __shared__ uint2 s_stack[kShort * kBlock];
-    __shared__ CoopShared<kBlock, false> s_coop;
-    __shared__ __align__(16) uint8_t s_perm[2048 + 1024];
-    fill_perm(s_perm);
+    using W = WarpShared<kShort, false>;
+    __shared__ __align__(16) uint8_t s_mem[kTableBytes + W::kBytes * (kBlock / 32)];
+    fill_tables(s_mem);
     SingleSource src;
     src.scene = L.scene;
     src.rays = L.rays;
@@ -609,32 +653,31 @@ __global__ void __launch_bounds__(kBlock, MinBlocks(kBlock)) trace_kernel(const 
     src.order = L.order;
     src.n = L.n_dev ? min(*L.n_dev, L.n) : L.n;
     if (L.ray_total && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(L.ray_total, (unsigned long long)src.n);
-    const Common C{L.counter, L.status, L.stats, L.refill_min, L.postpone_min};
-    persistent_trace<SingleSource, kAny ? 1 : 0, kStats, kShort, kBlock, false, true>(src, C, s_stack, &s_coop, nullptr,
-                                                                                     s_perm);
+    const Common C{L.counter, L.status, L.stats, L.refill_min, L.postpone_min ? L.postpone_min : kWaitMin};
+    persistent_trace<SingleSource, kAny ? 1 : 0, kStats, kShort>(
+        src, C, shared_addr(s_mem + kTableBytes + W::kBytes * (threadIdx.x >> 5)), shared_addr(s_mem));
 }
 
 template <int kShort, int kBlock>
 __global__ void __launch_bounds__(kBlock, MinBlocks(kBlock)) batch_kernel(const BatchLaunch B) {
-    __shared__ uint2 s_stack[kShort * kBlock];
-    __shared__ CoopShared<kBlock, true> s_coop;
-    __shared__ __align__(16) uint8_t s_perm[2048 + 1024];
-    fill_perm(s_perm);
+    using W = WarpShared<kShort, true>;
+    __shared__ __align__(16) uint8_t s_mem[kTableBytes + W::kBytes * (kBlock / 32)];
+    fill_tables(s_mem);
     BatchSource src;
     src.jobs = B.jobs;
     src.prefix = B.prefix;
     src.njobs = B.njobs;
     src.n = B.total;
-    const Common C{B.counter, B.status, nullptr, B.refill_min, B.postpone_min};
-    persistent_trace<BatchSource, 2, false, kShort, kBlock, false, true, true>(src, C, s_stack, &s_coop, nullptr,
-                                                                             s_perm);
+    const Common C{B.counter, B.status, nullptr, B.refill_min, B.postpone_min ? B.postpone_min : kWaitMin};
+    persistent_trace<BatchSource, 2, false, kShort, false, true>(
+        src, C, shared_addr(s_mem + kTableBytes + W::kBytes * (threadIdx.x >> 5)), shared_addr(s_mem));
 }
 
 template <bool kAny>
 __global__ void __launch_bounds__(128, 8) instanced_trace_kernel(const InstancedLaunch L) {
-    __shared__ uint2 s_stack[8 * 128];
-    __shared__ CoopShared<128, true> s_coop;
-    __shared__ RayState s_world[128];
+    using W = WarpShared<8, true>;
+    __shared__ __align__(16) uint8_t s_mem[W::kBytes * 4];
+    __shared__ float4 s_world[3 * 128];
     InstancedSource src;
     src.scene = L.tlas;
     src.inst = L.inst;
@@ -644,9 +687,9 @@ __global__ void __launch_bounds__(128, 8) instanced_trace_kernel(const Instanced
     src.occluded = L.occluded;
     src.n = L.n_dev ? min(*L.n_dev, L.n) : L.n;
     if (L.ray_total && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(L.ray_total, (unsigned long long)src.n);
-    const Common C{L.counter, L.status, nullptr, 8u, 0u};
-    persistent_trace<InstancedSource, kAny ? 1 : 0, false, 8, 128, true, true, true>(src, C, s_stack, &s_coop,
-                                                                                     s_world);
+    const Common C{L.counter, L.status, nullptr, 8u, kWaitMin};
+    persistent_trace<InstancedSource, kAny ? 1 : 0, false, 8, true, true>(
+        src, C, shared_addr(s_mem + W::kBytes * (threadIdx.x >> 5)), 0u, s_world);
 }
 
 __global__ void fill_miss_kernel(uint2* hits, uint8_t* occluded, uint32_t cap, const uint32_t* n_dev) {

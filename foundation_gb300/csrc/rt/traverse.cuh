@@ -196,22 +196,18 @@ __device__ __forceinline__ uint32_t xor_permute8(uint32_t m, uint32_t oct) {
     return m;
 }
 
-// Tests the 8 child boxes of one compressed node against the ray.
-// Returns the hit mask of internal children in traversal order (bit i is
-// slot i ^ oct) in bits 0..7 with the node's imask in bits 8..15, and the
-// triangle mask (bit k: triangle tri_base + k) of the hit leaf children.
-struct NodeHits {
+// Tests the 8 child boxes of one compressed node against the ray: which slots
+// were hit, and the node's words that say what the slots hold.
+struct SlotHits {
     uint32_t child_base;
     uint32_t tri_base;
-    uint32_t group;  // imask << 8 | ordered internal hits
-    uint32_t tris;
+    uint32_t imask;    // slots of internal children
+    uint32_t hitm;     // bit s: slot s's box was hit (an empty slot's bit means nothing)
+    uint32_t meta[2];  // the 8 meta bytes
 };
 
-// perm (optional): a table of 8 x 256 bytes, perm[oct * 256 + m] =
-// xor_permute8(m, oct), in place of the bit swaps, followed by 256 words:
-// the triangle mask of a leaf slot by its meta byte.
-__device__ __forceinline__ NodeHits intersect_node(const RayState& r, const uint4* __restrict__ nodes, uint32_t idx,
-                                                   float tfar, const uint8_t* perm = nullptr) {
+__device__ __forceinline__ SlotHits intersect_slots(const RayState& r, const uint4* __restrict__ nodes, uint32_t idx,
+                                                    float tfar) {
     const uint4* n = nodes + 5 * (size_t)idx;
     const uint4 w0 = __ldg(n + 0);
     const uint4 w1 = __ldg(n + 1);
@@ -226,7 +222,7 @@ __device__ __forceinline__ NodeHits intersect_node(const RayState& r, const uint
     const float bz = (__uint_as_float(w0.z) - r.oz) * r.iz;
     const uint32_t imask = w0.w >> 24;
     // near / far plane words per axis, chosen by the direction signs
-    const bool fx = r.oct & 1u, fy = r.oct & 2u, fz = r.oct & 4u;
+    const bool fx = signbit(r.ix), fy = signbit(r.iy), fz = signbit(r.iz);
     const uint32_t nx0 = fx ? w3.z : w2.x, nx1 = fx ? w3.w : w2.y;
     const uint32_t gx0 = fx ? w2.x : w3.z, gx1 = fx ? w2.y : w3.w;
     const uint32_t ny0 = fy ? w4.x : w2.z, ny1 = fy ? w4.y : w2.w;
@@ -240,54 +236,90 @@ __device__ __forceinline__ NodeHits intersect_node(const RayState& r, const uint
     //   far:  ru((1024+q) s + ru(b - 1024 s)) >= ru(q s + b) >= rn(q s + b)
     // so every child box is at least as wide as under round-to-nearest
     // fma(q, s, b), the culling stays conservative and the hits exact.
-    const float bnx = __fmaf_rd(-1024.0f, sx, bx), bfx = __fmaf_ru(-1024.0f, sx, bx);
-    const float bny = __fmaf_rd(-1024.0f, sy, by), bfy = __fmaf_ru(-1024.0f, sy, by);
-    const float bnz = __fmaf_rd(-1024.0f, sz, bz), bfz = __fmaf_ru(-1024.0f, sz, bz);
-    // the boxes alone: bit s of hitm for slot s (empty slots included; the
-    // slot kinds below mask them out); two slots per byte pair, their plane
-    // FMAs as packed pairs
-    const F2 sx2 = pack_f2(sx, sx), sy2 = pack_f2(sy, sy), sz2 = pack_f2(sz, sz);
-    const F2 bnx2 = pack_f2(bnx, bnx), bny2 = pack_f2(bny, bny), bnz2 = pack_f2(bnz, bnz);
-    const F2 bfx2 = pack_f2(bfx, bfx), bfy2 = pack_f2(bfy, bfy), bfz2 = pack_f2(bfz, bfz);
-    uint32_t hitm = 0;
+    // A slot's near and far plane go through one packed FMA, the far one
+    // negated (ru(x) = -rd(-x)), so both round down and one pair of constants
+    // per axis serves both: 12 registers across the eight slots (18 with the
+    // constants duplicated for slot pairs, which at the persistent kernels'
+    // 56 registers cost about 60 register moves per node).
+    const F2 sx2 = pack_f2(sx, -sx), sy2 = pack_f2(sy, -sy), sz2 = pack_f2(sz, -sz);
+    const F2 bx2 = pack_f2(__fmaf_rd(-1024.0f, sx, bx), __fmaf_rd(1024.0f, sx, -bx));
+    const F2 by2 = pack_f2(__fmaf_rd(-1024.0f, sy, by), __fmaf_rd(1024.0f, sy, -by));
+    const F2 bz2 = pack_f2(__fmaf_rd(-1024.0f, sz, bz), __fmaf_rd(1024.0f, sz, -bz));
+    // the boxes alone: bit s of miss for slot s (empty slots included)
+    const float ntfar = -tfar;
+    uint32_t miss = 0;
 #pragma unroll
-    for (int pr = 0; pr < 4; ++pr) {
+    for (int pr = 3; pr >= 0; --pr) {
         const uint32_t sel = (pr & 1) ? 0x4342u : 0x4140u;
-        float q0[6], q1[6];
-        plane_pair(pr < 2 ? nx0 : nx1, sel, q0[0], q1[0]);
-        plane_pair(pr < 2 ? ny0 : ny1, sel, q0[1], q1[1]);
-        plane_pair(pr < 2 ? nz0 : nz1, sel, q0[2], q1[2]);
-        plane_pair(pr < 2 ? gx0 : gx1, sel, q0[3], q1[3]);
-        plane_pair(pr < 2 ? gy0 : gy1, sel, q0[4], q1[4]);
-        plane_pair(pr < 2 ? gz0 : gz1, sel, q0[5], q1[5]);
-        float tnx[2], tny[2], tnz[2], tfx[2], tfy[2], tfz[2];
-        fma_dir_f2<false>(pack_f2(q0[0], q1[0]), sx2, bnx2, tnx);
-        fma_dir_f2<false>(pack_f2(q0[1], q1[1]), sy2, bny2, tny);
-        fma_dir_f2<false>(pack_f2(q0[2], q1[2]), sz2, bnz2, tnz);
-        fma_dir_f2<true>(pack_f2(q0[3], q1[3]), sx2, bfx2, tfx);
-        fma_dir_f2<true>(pack_f2(q0[4], q1[4]), sy2, bfy2, tfy);
-        fma_dir_f2<true>(pack_f2(q0[5], q1[5]), sz2, bfz2, tfz);
+        float nx[2], ny[2], nz[2], gx[2], gy[2], gz[2];
+        plane_pair(pr < 2 ? nx0 : nx1, sel, nx[0], nx[1]);
+        plane_pair(pr < 2 ? gx0 : gx1, sel, gx[0], gx[1]);
+        plane_pair(pr < 2 ? ny0 : ny1, sel, ny[0], ny[1]);
+        plane_pair(pr < 2 ? gy0 : gy1, sel, gy[0], gy[1]);
+        plane_pair(pr < 2 ? nz0 : nz1, sel, nz[0], nz[1]);
+        plane_pair(pr < 2 ? gz0 : gz1, sel, gz[0], gz[1]);
 #pragma unroll
-        for (int e = 0; e < 2; ++e) {
-            const float tn = max3f(tnx[e], tny[e], fmaxf(tnz[e], r.tmin));
-            const float tf = min3f(tfx[e], tfy[e], fminf(tfz[e], tfar));
-            hitm |= tn <= tf ? 1u << (2 * pr + e) : 0u;
+        for (int e = 1; e >= 0; --e) {
+            float tx[2], ty[2], tz[2];  // near t, -(far t)
+            fma_dir_f2<false>(pack_f2(nx[e], gx[e]), sx2, bx2, tx);
+            fma_dir_f2<false>(pack_f2(ny[e], gy[e]), sy2, by2, ty);
+            fma_dir_f2<false>(pack_f2(nz[e], gz[e]), sz2, bz2, tz);
+            const float tn = max3f(tx[0], ty[0], fmaxf(tz[0], r.tmin));
+            const float ntf = max3f(tx[1], ty[1], fmaxf(tz[1], ntfar));
+#if defined(__CUDA_ARCH__)
+            // the sign of tf - tn, shifted in (a difference and a funnel
+            // shift: the compare and select of the plain form both go to the
+            // integer pipe, the busier one). Equal infinities give a NaN of
+            // positive sign, a hit as under tn <= tf.
+            miss = __funnelshift_l(__float_as_uint(__fsub_rn(-ntf, tn)), miss, 1);
+#else
+            miss = miss << 1 | (tn <= -ntf ? 0u : 1u);
+#endif
         }
     }
-    // leaf slots: the 0x80 flag of their meta byte
-    const uint32_t leaves = meta_leaf_bits(w1.z) | meta_leaf_bits(w1.w) << 4;
-    uint32_t lh = hitm & leaves, tris = 0;
+    SlotHits out;
+    out.child_base = w1.x;
+    out.tri_base = w1.y;
+    out.imask = imask;
+    out.hitm = ~miss & 0xFFu;
+    out.meta[0] = w1.z;
+    out.meta[1] = w1.w;
+    return out;
+}
+
+// The leaf slots of a node, by the 0x80 flag of their meta bytes.
+__device__ __forceinline__ uint32_t leaf_slots(const SlotHits& h) {
+    return meta_leaf_bits(h.meta[0]) | meta_leaf_bits(h.meta[1]) << 4;
+}
+// Meta byte of slot s.
+__device__ __forceinline__ uint32_t meta_of(const SlotHits& h, uint32_t s) {
+    return __byte_perm(s < 4u ? h.meta[0] : h.meta[1], 0u, 0x4440u | (s & 3u));
+}
+
+// The same as one group of internal children in traversal order (bit i is
+// slot i ^ oct, in bits 0..7, with the node's imask in bits 8..15) and the
+// triangle mask (bit k: triangle tri_base + k) of the hit leaf children.
+struct NodeHits {
+    uint32_t child_base;
+    uint32_t tri_base;
+    uint32_t group;  // imask << 8 | ordered internal hits
+    uint32_t tris;
+};
+
+__device__ __forceinline__ NodeHits intersect_node(const RayState& r, const uint4* __restrict__ nodes, uint32_t idx,
+                                                   float tfar) {
+    const SlotHits h = intersect_slots(r, nodes, idx, tfar);
+    uint32_t lh = h.hitm & leaf_slots(h), tris = 0;
     while (lh) {  // about one hit leaf per three nodes on incoherent rays
         const uint32_t s = (uint32_t)__ffs(lh) - 1u;
         lh &= lh - 1u;
-        const uint32_t meta = __byte_perm(s < 4u ? w1.z : w1.w, 0u, 0x4440u | (s & 3u));
-        tris |= perm ? reinterpret_cast<const uint32_t*>(perm + 2048)[meta]
-                     : ((2u << ((meta >> 5) & 3u)) - 1u) << (meta & 31u);
+        const uint32_t meta = meta_of(h, s);
+        tris |= ((2u << ((meta >> 5) & 3u)) - 1u) << (meta & 31u);
     }
     NodeHits out;
-    out.child_base = w1.x;
-    out.tri_base = w1.y;
-    out.group = (imask << 8) | (perm ? (uint32_t)perm[(r.oct << 8) | (hitm & imask)] : xor_permute8(hitm & imask, r.oct));
+    out.child_base = h.child_base;
+    out.tri_base = h.tri_base;
+    out.group = (h.imask << 8) | xor_permute8(h.hitm & h.imask, r.oct);
     out.tris = tris;
     return out;
 }

@@ -26,7 +26,7 @@ struct TraceLaunch {
     unsigned long long* stats;  // [0] node fetches, [1] triangle tests, [2] / [3] warp steps of the node /
                                 // triangle tests (stats variants)
     uint32_t refill_min;        // refill a warp once this many lanes are idle
-    uint32_t postpone_min;      // triangle postponement threshold (0: off)
+    uint32_t postpone_min;      // test waiting triangles once this many lanes only wait (0: default)
     const uint32_t* order;      // fetch position -> ray index (ray_sort.hpp), or null: input order
 };
 
@@ -35,7 +35,7 @@ struct TraceConfig {
     int block = kTraceBlock;             // 64, 128 or 256 threads
     int short_stack = kTraceShortStack;  // 4, 8 or 16 shared-memory stack entries per thread
     uint32_t refill_min = 8;             // 1..32 idle lanes before a warp refills
-    uint32_t postpone_min = 0;           // postpone triangles when fewer lanes have them (0: never)
+    uint32_t postpone_min = 0;           // test waiting triangles once this many lanes only wait (0: default)
     int blocks_per_sm = 0;               // 0: as many as fit
     uint32_t sort_bits = 0;              // coherence order key bits (ray_sort.hpp), 0: input order
 };

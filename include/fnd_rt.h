@@ -255,8 +255,8 @@ typedef struct fnd_rt_trace_config {
     uint32_t block;        /* 64, 128 or 256 threads */
     uint32_t short_stack;  /* 4, 8 or 16 entries per thread */
     uint32_t refill_min;   /* 1..32 idle lanes before a warp refills */
-    uint32_t postpone_min; /* postpone a node's triangles while fewer than this many lanes
-                              of the warp have triangles to test (0..32, 0: never) */
+    uint32_t postpone_min; /* triangles wait until 32 of a warp's are there; test fewer once
+                              this many lanes only wait for theirs (0..32, 0: the default, 4) */
     uint32_t sort_bits;    /* 0: rays traced in input order; 6..21 (multiple of 3): rays
                               first bucketed by origin cell (Morton order on a grid over
                               the scene box) and direction octant, a key of this many

@@ -1,0 +1,62 @@
+"""The traversal kernels' per-warp ring of waiting triangles, at the sizes
+where it turns: no triangles at all, leaves of one triangle, nodes whose
+leaves fill the ring many times over in one step (coincident triangles, which
+no box separates), ray counts around one warp, and every threshold of the
+launch shape that decides when a part-filled ring is tested. Exact against
+the oracle: the order of the tests must not show."""
+import numpy as np
+import pytest
+
+import oracle as O
+from foundation_gb300 import scenes as S
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx(built):
+    import foundation_gb300 as fg
+    c = fg.Context(0)
+    yield c
+    c.close()
+
+
+def _geometry(kind):
+    rng = np.random.default_rng(3)
+    if kind == "one":
+        v = np.array([[0.0, 0, 0.5], [1, 0, 0.5], [0, 1, 0.5]], np.float32)
+    elif kind == "stack":  # 300 coincident copies, then 300 shifted along z
+        t = np.array([[0.0, 0, 0], [1, 0, 0], [0, 1, 0]])
+        v = np.concatenate([t + [0, 0, 0.25 if k < 300 else k * 1e-3] for k in range(600)]).astype(np.float32)
+    else:
+        return S.soup_scene(3000, seed=5)
+    return S.Scene(v, np.arange(len(v), dtype=np.uint32).reshape(-1, 3))
+
+
+def _rays(n):
+    rays = S.incoherent_rays(n, (0, 0, 0), (1, 1, 1), seed=9)
+    rays[::5, 4:7] = (0.01, 0.02, 1.0)  # through the stacked triangles
+    rays[::7, 7] = 0.3
+    return rays
+
+
+@pytest.mark.parametrize("kind", ["one", "stack", "soup"])
+@pytest.mark.parametrize("n", [1, 31, 33, 5000])
+def test_ring_matches_oracle(ctx, kind, n):
+    sc, rays = _geometry(kind), _rays(n)
+    b = O.OracleBVH(sc.verts, sc.idx)
+    want, want_any = b.closest(rays), b.any(rays)
+    builds = [{}, {"spatial_splits": True, "sah_collapse": True}]
+    if kind != "stack":  # clustering coincident triangles gives a chain deeper than the stack, which upload refuses
+        builds.append({"gpu_build": True, "cluster": True})
+    for opts in builds:
+        scene = ctx.upload(sc.verts, sc.idx, **opts)
+        for refill in (1, 8, 32):
+            for wait in (0, 1, 32):
+                ctx.set_trace_config(short_stack=4, refill_min=refill, postpone_min=wait)
+                h = scene.closest(rays)
+                assert np.array_equal(h["prim"], want["prim"]), (opts, refill, wait)
+                assert np.array_equal(h["t"].view(np.uint32), want["t"].view(np.uint32))
+                assert np.array_equal(scene.any(rays), want_any)
+        scene.close()
+    ctx.set_trace_config()
