@@ -698,7 +698,7 @@ struct CollapseArgs {
     const float* verts;
     const uint32_t* idx;
     WideNode* nodes;
-    float4 *v0, *v1, *v2;
+    float4* tris;  // three vertices per triangle
     float margin;
     int level;
 };
@@ -886,13 +886,13 @@ __global__ void __launch_bounds__(128) collapse_kernel(const CollapseArgs A) {
                         continue;
                     }
                     const uint32_t t = B.vals[ref & ~kLeafRef];
-                    const size_t d = (size_t)tri_base + tri_off + i;
+                    const size_t d = 3 * ((size_t)tri_base + tri_off + i);
                     float v[9];
                     for (int k = 0; k < 3; ++k)
                         for (int q = 0; q < 3; ++q) v[3 * k + q] = A.verts[3 * (size_t)A.idx[3 * (size_t)t + k] + q];
-                    A.v0[d] = make_float4(v[0], v[1], v[2], __uint_as_float(t));
-                    A.v1[d] = make_float4(v[3], v[4], v[5], 0.0f);
-                    A.v2[d] = make_float4(v[6], v[7], v[8], 0.0f);
+                    A.tris[d + 0] = make_float4(v[0], v[1], v[2], __uint_as_float(t));
+                    A.tris[d + 1] = make_float4(v[3], v[4], v[5], 0.0f);
+                    A.tris[d + 2] = make_float4(v[6], v[7], v[8], 0.0f);
                     i++;
                 }
                 if (i != cnt[c]) bad_tree = true;
@@ -934,6 +934,11 @@ __global__ void instance_shade_kernel(const float* __restrict__ inv, const uint3
     const float l = sqrtf(w[0] * w[0] + w[1] * w[1] + w[2] * w[2]);
     const float k = l > 0.0f ? 1.0f / l : 0.0f;
     out[(size_t)off[lo] + t] = l > 0.0f ? make_float4(w[0] * k, w[1] * k, w[2] * k, 0.0f) : make_float4(0, 0, 1, 0);
+}
+
+__global__ void interleave_kernel(const float4* __restrict__ planes, uint32_t n, float4* __restrict__ tris) {
+    const size_t j = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (j < 3 * (size_t)n) tris[j] = planes[(j % 3) * n + j / 3];
 }
 
 __global__ void write_ids_kernel(float4* shade, const uint32_t* ids, uint32_t nt) {
@@ -1154,9 +1159,7 @@ void BuildWideGpu(const float* d_verts, uint32_t nv, const uint32_t* d_idx, uint
     A.verts = d_verts;
     A.idx = d_idx;
     A.nodes = nodes;
-    A.v0 = reinterpret_cast<float4*>(tris);
-    A.v1 = reinterpret_cast<float4*>(tris + 16ull * n);
-    A.v2 = reinterpret_cast<float4*>(tris + 32ull * n);
+    A.tris = reinterpret_cast<float4*>(tris);
     A.margin = out.margin;
     const int grid = std::max(1, sms * 8);
     for (int level = 0; level < kMaxLevels; ++level) {
@@ -1201,6 +1204,12 @@ cudaError_t InstanceShade(const float* d_inv, const uint32_t* d_prefix, const ui
     if (total == 0 || n_inst == 0) return cudaSuccess;
     instance_shade_kernel<<<(total + 255) / 256, 256, 0, s>>>(d_inv, d_prefix, d_prim_offset, d_blas_shade, n_inst,
                                                                 total, d_out);
+    return cudaGetLastError();
+}
+
+cudaError_t InterleaveTriangles(const float4* d_planes, uint32_t n, float4* d_tris, cudaStream_t s) {
+    if (n == 0) return cudaSuccess;
+    interleave_kernel<<<(uint32_t)((3 * (size_t)n + 255) / 256), 256, 0, s>>>(d_planes, n, d_tris);
     return cudaGetLastError();
 }
 

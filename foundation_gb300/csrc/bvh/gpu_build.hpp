@@ -33,7 +33,7 @@ struct GpuBuildParams {
 
 struct GpuBuildOutput {
     void* d_nodes = nullptr;      // WideNode[num_nodes], exact size
-    void* d_tris = nullptr;       // three float4 planes of num_refs entries
+    void* d_tris = nullptr;       // num_refs records of three float4 vertices
     void* d_tri_shade = nullptr;  // float4 per triangle: unit normal, material 0
     uint32_t num_nodes = 0, num_refs = 0, depth = 0, leaves = 0, num_binary_nodes = 0;
     float lo[3] = {0, 0, 0}, hi[3] = {0, 0, 0};
@@ -48,6 +48,10 @@ struct GpuBuildOutput {
 // deeper than the traversal stack allows. Temporary buffers are freed.
 void BuildWideGpu(const float* d_verts, uint32_t nv, const uint32_t* d_idx, uint32_t nt, const GpuBuildParams& p,
                   GpuBuildOutput& out, cudaStream_t s);
+
+// Three planes of n float4 (vertex 0 of every triangle, then 1, then 2) into
+// records of three.
+cudaError_t InterleaveTriangles(const float4* d_planes, uint32_t n, float4* d_tris, cudaStream_t s);
 
 // tri_shade[t].w = material id bits of triangle t.
 cudaError_t WriteMaterialIds(float4* d_tri_shade, const uint32_t* d_ids, uint32_t nt, cudaStream_t s);

@@ -95,11 +95,8 @@ int fnd_rt_instances_upload(fnd_rt_ctx* ctx, const fnd_rt_instance* instances, u
                 CUDA_CHECK(cudaMalloc(&scene->d_nodes, I.node_bytes));
                 CUDA_CHECK(cudaMalloc(&scene->d_tris, I.tri_bytes));
                 CUDA_CHECK(cudaMalloc(&scene->d_instances, sizeof(RT::InstanceRec) * n));
-                char* tris = static_cast<char*>(scene->d_tris);
                 CUDA_CHECK(cudaMemcpy(scene->d_nodes, wide.nodes.data(), I.node_bytes, cudaMemcpyHostToDevice));
-                CUDA_CHECK(cudaMemcpy(tris, wide.v0.data(), 16ull * n, cudaMemcpyHostToDevice));
-                CUDA_CHECK(cudaMemcpy(tris + 16ull * n, wide.v1.data(), 16ull * n, cudaMemcpyHostToDevice));
-                CUDA_CHECK(cudaMemcpy(tris + 32ull * n, wide.v2.data(), 16ull * n, cudaMemcpyHostToDevice));
+                CApi::UploadTriangles(ctx, wide.v0.data(), wide.v1.data(), wide.v2.data(), n, scene->d_tris);
                 CUDA_CHECK(cudaMemcpy(scene->d_instances, recs.data(), sizeof(RT::InstanceRec) * n,
                                       cudaMemcpyHostToDevice));
             } catch (...) {
@@ -107,13 +104,9 @@ int fnd_rt_instances_upload(fnd_rt_ctx* ctx, const fnd_rt_instance* instances, u
                     if (p) cudaFree(p);
                 throw;
             }
-            char* tris = static_cast<char*>(scene->d_tris);
             scene->view.nodes = static_cast<const uint4*>(scene->d_nodes);
-            scene->view.v0 = reinterpret_cast<const float4*>(tris);
-            scene->view.v1 = reinterpret_cast<const float4*>(tris + 16ull * n);
-            scene->view.v2 = reinterpret_cast<const float4*>(tris + 32ull * n);
             scene->view.num_nodes = I.num_wide_nodes;
-            scene->view.num_tris = n;
+            CApi::ViewTriangles(scene->view, scene->d_tris, n);
         }
         // shading records by global id: world normals of every instance's triangles
         {

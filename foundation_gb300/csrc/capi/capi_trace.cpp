@@ -106,6 +106,37 @@ namespace {
 namespace Foundation {
 namespace CApi {
 
+void UploadTriangles(fnd_rt_ctx* ctx, const float* v0, const float* v1, const float* v2, uint32_t n, void* d_tris) {
+    constexpr uint32_t kChunk = 1u << 20;
+    char* staging = nullptr;
+    CUDA_CHECK(cudaMalloc(&staging, 48ull * std::max(1u, std::min(n, kChunk))));
+    try {
+        for (uint32_t at = 0; at < n; at += kChunk) {
+            const uint32_t cnt = std::min(kChunk, n - at);
+            const float* planes[3] = {v0, v1, v2};
+            for (int a = 0; a < 3; ++a)
+                CUDA_CHECK(cudaMemcpyAsync(staging + 16ull * cnt * a, planes[a] + 4 * (size_t)at, 16ull * cnt,
+                                           cudaMemcpyHostToDevice, ctx->stream));
+            CUDA_CHECK(RT::InterleaveTriangles(reinterpret_cast<const float4*>(staging), cnt,
+                                               static_cast<float4*>(d_tris) + 3 * (size_t)at, ctx->stream));
+        }
+        CUDA_CHECK(cudaStreamSynchronize(ctx->stream));
+    } catch (...) {
+        cudaStreamSynchronize(ctx->stream);
+        cudaFree(staging);
+        throw;
+    }
+    CUDA_CHECK(cudaFree(staging));
+}
+
+void ViewTriangles(RT::DeviceScene& view, const void* d_tris, uint32_t n) {
+    view.v0 = static_cast<const float4*>(d_tris);
+    view.v1 = view.v0 + 1;
+    view.v2 = view.v0 + 2;
+    view.num_tris = n;
+    view.tri_stride = 3;
+}
+
 // One grey Lambertian until fnd_rt_scene_set_materials.
 void DefaultMaterial(fnd_rt_scene* scene) {
     PT::DevMaterial m{};
@@ -180,14 +211,9 @@ void UploadGpuBuilt(fnd_rt_ctx* ctx, fnd_rt_scene* scene, const float* verts, ui
         scene->d_nodes = scene->d_tris = scene->d_tri_shade = scene->d_materials = nullptr;
         throw;
     }
-    char* tris = static_cast<char*>(scene->d_tris);
-    const size_t plane = 16ull * scene->info.num_refs;
     scene->view.nodes = static_cast<const uint4*>(scene->d_nodes);
-    scene->view.v0 = reinterpret_cast<const float4*>(tris);
-    scene->view.v1 = reinterpret_cast<const float4*>(tris + plane);
-    scene->view.v2 = reinterpret_cast<const float4*>(tris + 2 * plane);
     scene->view.num_nodes = scene->info.num_wide_nodes;
-    scene->view.num_tris = scene->info.num_refs;
+    CApi::ViewTriangles(scene->view, scene->d_tris, scene->info.num_refs);
 }
 
 }  // namespace
@@ -451,12 +477,8 @@ int fnd_rt_scene_upload(fnd_rt_ctx* ctx, const float* verts, uint32_t nv, const 
         try {
             CUDA_CHECK(cudaMalloc(&scene->d_nodes, I.node_bytes));
             CUDA_CHECK(cudaMalloc(&scene->d_tris, I.tri_bytes));
-            char* tris = static_cast<char*>(scene->d_tris);
-            const size_t plane = 16ull * I.num_refs;
             CUDA_CHECK(cudaMemcpy(scene->d_nodes, wide.nodes.data(), I.node_bytes, cudaMemcpyHostToDevice));
-            CUDA_CHECK(cudaMemcpy(tris, wide.v0.data(), plane, cudaMemcpyHostToDevice));
-            CUDA_CHECK(cudaMemcpy(tris + plane, wide.v1.data(), plane, cudaMemcpyHostToDevice));
-            CUDA_CHECK(cudaMemcpy(tris + 2 * plane, wide.v2.data(), plane, cudaMemcpyHostToDevice));
+            CApi::UploadTriangles(ctx, wide.v0.data(), wide.v1.data(), wide.v2.data(), I.num_refs, scene->d_tris);
             CUDA_CHECK(cudaMalloc(&scene->d_tri_shade, 16ull * nt));
             CUDA_CHECK(cudaMemcpy(scene->d_tri_shade, scene->tri_shade.data(), 16ull * nt, cudaMemcpyHostToDevice));
             std::vector<float>().swap(scene->tri_shade);  // the device copy is the only one kept
@@ -469,14 +491,9 @@ int fnd_rt_scene_upload(fnd_rt_ctx* ctx, const float* verts, uint32_t nv, const 
             throw;
         }
         I.upload_ms = MsSince(t0);
-        char* tris = static_cast<char*>(scene->d_tris);
-        const size_t plane = 16ull * I.num_refs;
         scene->view.nodes = static_cast<const uint4*>(scene->d_nodes);
-        scene->view.v0 = reinterpret_cast<const float4*>(tris);
-        scene->view.v1 = reinterpret_cast<const float4*>(tris + plane);
-        scene->view.v2 = reinterpret_cast<const float4*>(tris + 2 * plane);
         scene->view.num_nodes = I.num_wide_nodes;
-        scene->view.num_tris = I.num_refs;
+        CApi::ViewTriangles(scene->view, scene->d_tris, I.num_refs);
         *out_scene = scene.release();
         ctx->live_scenes++;
     });

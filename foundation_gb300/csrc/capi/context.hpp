@@ -148,6 +148,12 @@ cudaError_t LaunchTraceOrdered(fnd_rt_ctx* ctx, const fnd_rt_scene* scene, Found
                                bool stats, const Foundation::RT::TraceConfig& cfg, int grid,
                                cudaStream_t stream = nullptr);
 
+// The host's three vertex planes (n float4 each) as device records of three
+// vertices per triangle, through a staging buffer of at most 48 MB.
+void UploadTriangles(fnd_rt_ctx* ctx, const float* v0, const float* v1, const float* v2, uint32_t n, void* d_tris);
+// The device view of a scene's triangle records.
+void ViewTriangles(Foundation::RT::DeviceScene& view, const void* d_tris, uint32_t n);
+
 // One grey Lambertian material table on a new scene (capi_trace.cpp).
 void DefaultMaterial(fnd_rt_scene* scene);
 

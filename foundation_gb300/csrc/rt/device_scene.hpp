@@ -31,14 +31,15 @@ constexpr int kMaxStack = 64;  // node-group + triangle-group entries per ray
 
 struct DeviceScene {
     const uint4* nodes;  // 5 uint4 per WideNode
-    const float4* v0;    // (x, y, z, original index bits)
-    const float4* v1;
+    const float4* v0;    // vertex 0 of triangle i at v0[i * tri_stride]: (x, y, z, original index bits)
+    const float4* v1;    // likewise vertices 1 and 2: (x, y, z, 0)
     const float4* v2;
     uint32_t num_nodes;
     uint32_t num_tris;
+    uint32_t tri_stride = 1;  // 3: one 48-byte record per triangle (every uploaded scene), 1: three planes
 };
 
-// One instance of a two-level scene (104 bytes): its bottom-level scene, the
+// One instance of a two-level scene (112 bytes): its bottom-level scene, the
 // world-to-object transform (row-major 3x4, FP32 rounding of the FP64
 // inverse of the instance transform) and the hit id of its triangle 0.
 struct InstanceRec {
@@ -52,7 +53,7 @@ struct InstanceRec {
 // would change at most the sign of zero components); the oracle's instanced
 // brute force makes the same choice.
 constexpr uint32_t kInstanceIdentity = 1u;
-static_assert(sizeof(InstanceRec) == 104, "instance record layout");
+static_assert(sizeof(InstanceRec) == 112, "instance record layout");
 
 }  // namespace RT
 }  // namespace Foundation

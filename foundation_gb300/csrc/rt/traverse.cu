@@ -231,14 +231,14 @@ constexpr uint32_t kRing = 64;  // ranges
 // Shared memory of one warp (byte offsets): per lane the ray's constants
 // (origin and tmin; -Sx, -Sy, Sz and kz; inverse direction and octx), its
 // best hit (t bits, id) and the merge slot, then the ring, with kMulti (lanes
-// of one warp in different scenes) the triangle planes of each lane's scene
+// of one warp in different scenes) the triangle records of each lane's scene
 // and its hit-id offset, and the lanes' stacks. The origin and the inverse
 // direction are read back for each node: they are dead before the node
 // test's widest point, where registers are scarce.
 template <int kShort, bool kMulti>
 struct WarpShared {
     static constexpr uint32_t kRayA = 0, kRayB = 512, kRayC = 1024, kBest = 1536, kWin = 1792, kRanges = 2048;
-    static constexpr uint32_t kPlanes = kRanges + 8 * kRing, kPrimOff = kPlanes + (kMulti ? 3 * 256 : 0);
+    static constexpr uint32_t kTris = kRanges + 8 * kRing, kPrimOff = kTris + (kMulti ? 256 : 0);
     static constexpr uint32_t kStack = kPrimOff + (kMulti ? 128 : 0), kBytes = kStack + 256 * kShort;
 };
 
@@ -252,15 +252,12 @@ __device__ __forceinline__ void store_ray(uint32_t w, uint32_t lane, const RaySt
     sts128(w + 16u * lane + W::kRayB, r.nSx, r.nSy, r.Sz, __int_as_float(r.kz));
     sts128(w + 16u * lane + W::kRayC, r.ix, r.iy, r.iz, __uint_as_float(octx_of(r)));
 }
-// kMulti: the lane's triangle planes and hit-id offset.
+// kMulti: the lane's triangle records and hit-id offset.
 template <int kShort>
 __device__ __forceinline__ void store_scene(uint32_t w, uint32_t lane, const DeviceScene& sc, uint32_t prim_off) {
     using W = WarpShared<kShort, true>;
-    const float4* p[3] = {sc.v0, sc.v1, sc.v2};
-    for (int a = 0; a < 3; ++a) {
-        const unsigned long long v = (unsigned long long)p[a];
-        sts64(w + 8u * lane + W::kPlanes + 256u * a, (uint32_t)v, (uint32_t)(v >> 32));
-    }
+    const unsigned long long v = (unsigned long long)sc.v0;
+    sts64(w + 8u * lane + W::kTris, (uint32_t)v, (uint32_t)(v >> 32));
     sts32(w + 4u * lane + W::kPrimOff, prim_off);
 }
 __device__ __forceinline__ const float4* lds_ptr(uint32_t a) {
@@ -272,17 +269,19 @@ __device__ __forceinline__ const float4* lds_ptr(uint32_t a) {
 // kKind: 0 closest, 1 any, 2 per-lane (from the source). kTwoLevel: the
 // source is an InstancedSource (triangle leaves of the top level are
 // instances; per-lane node / triangle arrays). w: this warp's region of
-// shared memory, tab: the tables of fill_tables.
+// shared memory, tab: the tables of fill_tables. kPlanes: the scene's
+// triangles are three planes (tri_stride 1), not records.
 //
 // A node group is one word: the internal children still to visit in bits
 // 24..31, the highest bit first (bit 24 + j is slot j ^ 7 ^ oct, so the
 // highest bit is the nearest along the ray's octant), and the node's imask
 // in bits 0..7.
-template <class Src, int kKind, bool kStats, int kShort, bool kTwoLevel = false, bool kMulti = false>
+template <class Src, int kKind, bool kStats, int kShort, bool kTwoLevel = false, bool kMulti = false,
+          bool kPlanes = false>
 __device__ __forceinline__ void persistent_trace(const Src& src, const Common& C, uint32_t w, uint32_t tab,
                                                  float4* s_world = nullptr) {
     using W = WarpShared<kShort, kMulti>;
-    // two-level: each lane's planes and hit-id offset come from its own slot
+    // two-level: each lane's triangles and hit-id offset come from its own slot
     // (the lanes of a warp sit in different instances)
     static_assert(!kTwoLevel || kMulti, "two-level traversal needs per-lane scenes");
     uint2 l_stack[kMaxStack - kShort];
@@ -458,7 +457,7 @@ __device__ __forceinline__ void persistent_trace(const Src& src, const Common& C
             while (!in_blas && tl_mask) {
                 const uint32_t k = (uint32_t)__ffs(tl_mask) - 1u;
                 tl_mask &= tl_mask - 1u;
-                const uint32_t iid = __float_as_uint(__ldg(cur.v0 + tl_base + k).w);
+                const uint32_t iid = __float_as_uint(__ldg(cur.v0 + 3 * (size_t)(tl_base + k)).w);
                 if (iid >= src.num_inst) {
                     atomicOr(C.status, kStatusBadIndex);
                     continue;
@@ -545,14 +544,13 @@ __device__ __forceinline__ void persistent_trace(const Src& src, const Common& C
                 rq.nSy = b.y;
                 rq.Sz = b.z;
                 rq.kz = __float_as_int(b.w);
-                const float4 *p0 = src.scene_of(ln).v0, *p1 = src.scene_of(ln).v1, *p2 = src.scene_of(ln).v2;
-                if constexpr (kMulti) {
-                    p0 = lds_ptr(own + W::kPlanes);
-                    p1 = lds_ptr(own + W::kPlanes + 256u);
-                    p2 = lds_ptr(own + W::kPlanes + 512u);
-                }
-                const float4 v0 = __ldg(p0 + ti);
-                hit = intersect_tri(rq, v0, __ldg(p1 + ti), __ldg(p2 + ti), __uint_as_float(lds32(own + W::kBest)), t);
+                const DeviceScene& sc = src.scene_of(ln);
+                const float4* p0 = kMulti ? lds_ptr(own + W::kTris) : sc.v0;
+                p0 += (kPlanes ? 1u : 3u) * (size_t)ti;
+                const float4* p1 = kPlanes ? sc.v1 + ti : p0 + 1;
+                const float4* p2 = kPlanes ? sc.v2 + ti : p0 + 2;
+                const float4 v0 = __ldg(p0);
+                hit = intersect_tri(rq, v0, __ldg(p1), __ldg(p2), __uint_as_float(lds32(own + W::kBest)), t);
                 pid = __float_as_uint(v0.w);
                 if constexpr (kTwoLevel) pid += lds32(w + (own - w) / 2u + W::kPrimOff);  // global id of an instance's triangle
                 if (kStats) {
@@ -640,7 +638,7 @@ __device__ __forceinline__ void fill_tables(uint8_t* t) {
     __syncthreads();
 }
 
-template <bool kAny, bool kStats, int kShort, int kBlock>
+template <bool kAny, bool kStats, int kShort, int kBlock, bool kPlanes = false>
 __global__ void __launch_bounds__(kBlock, MinBlocks(kBlock)) trace_kernel(const TraceLaunch L) {
     using W = WarpShared<kShort, false>;
     __shared__ __align__(16) uint8_t s_mem[kTableBytes + W::kBytes * (kBlock / 32)];
@@ -654,7 +652,7 @@ __global__ void __launch_bounds__(kBlock, MinBlocks(kBlock)) trace_kernel(const 
     src.n = L.n_dev ? min(*L.n_dev, L.n) : L.n;
     if (L.ray_total && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(L.ray_total, (unsigned long long)src.n);
     const Common C{L.counter, L.status, L.stats, L.refill_min, L.postpone_min ? L.postpone_min : kWaitMin};
-    persistent_trace<SingleSource, kAny ? 1 : 0, kStats, kShort>(
+    persistent_trace<SingleSource, kAny ? 1 : 0, kStats, kShort, false, false, kPlanes>(
         src, C, shared_addr(s_mem + kTableBytes + W::kBytes * (threadIdx.x >> 5)), shared_addr(s_mem));
 }
 
@@ -764,7 +762,12 @@ cudaError_t LaunchTraceConfigured(const TraceLaunch& L, bool any, bool stats, co
     cudaError_t e = cudaMemsetAsync(L.counter, 0, sizeof(uint32_t), stream);
     if (e != cudaSuccess) return e;
     const void* fn = any ? select_trace<true>(c, stats) : select_trace<false>(c, stats);
-    const int block = stats ? 128 : normalized_block(c.block);
+    int block = stats ? 128 : normalized_block(c.block);
+    if (L.scene.tri_stride == 1) {  // triangle planes: the default shape
+        fn = any ? reinterpret_cast<const void*>(&trace_kernel<true, false, 8, 128, true>)
+                 : reinterpret_cast<const void*>(&trace_kernel<false, false, 8, 128, true>);
+        block = 128;
+    }
     TraceLaunch arg = L;
     arg.refill_min = c.refill_min ? c.refill_min : L.refill_min;
     arg.postpone_min = c.postpone_min;

@@ -374,9 +374,10 @@ __device__ __forceinline__ bool trace_single(const DeviceScene& sc, const RaySta
             const uint32_t k = (uint32_t)__ffs(tg_mask) - 1u;
             tg_mask &= tg_mask - 1u;
             const uint32_t ti = tg_base + k;
-            const float4 v0 = __ldg(sc.v0 + ti);
+            const size_t at = (size_t)ti * sc.tri_stride;
+            const float4 v0 = __ldg(sc.v0 + at);
             float t;
-            if (intersect_tri(r, v0, __ldg(sc.v1 + ti), __ldg(sc.v2 + ti), best_t, t)) {
+            if (intersect_tri(r, v0, __ldg(sc.v1 + at), __ldg(sc.v2 + at), best_t, t)) {
                 const uint32_t pid = __float_as_uint(v0.w);
                 if (kAny) {
                     best_t = t;
@@ -457,7 +458,7 @@ __device__ __forceinline__ bool trace_two_level(const DeviceScene& tlas, const I
         while (tg_mask) {
             const uint32_t k = (uint32_t)__ffs(tg_mask) - 1u;
             tg_mask &= tg_mask - 1u;
-            const uint32_t id = __float_as_uint(__ldg(tlas.v0 + tg_base + k).w);
+            const uint32_t id = __float_as_uint(__ldg(tlas.v0 + (size_t)(tg_base + k) * tlas.tri_stride).w);
             if (id >= num_inst) {
                 atomicOr(status, kStatusBadIndex);
                 continue;
