@@ -5,10 +5,8 @@
 //  2. 63-bit Morton code of each centroid on a grid of 2^21 cubic cells per
 //     axis over the centroid box's largest extent (dense scenes keep a
 //     spatial order far below the triangle size);
-//  3. stable LSD radix sort of (code, triangle) in eight 8-bit passes: per
-//     2,048-element warp tile a digit histogram, one exclusive scan over the
-//     digit-major counts, then a scatter in which each warp ranks its
-//     elements in order with __match_any_sync;
+//  3. stable LSD radix sort of (code, triangle) in seven 9-bit passes, tiles
+//     of 4,096 put in digit order in shared memory;
 //  4. Karras (2012): internal node i of the n-1 finds its key range and
 //     split by binary searches on the common-prefix length of the sorted
 //     keys (ties between equal codes broken by sorted position); or
@@ -60,8 +58,7 @@ struct Buffers {
     uint32_t* vals;               // triangle ids
     unsigned long long* keys2;    // radix-sort ping-pong
     uint32_t* vals2;
-    uint32_t* cnt;                // digit-major tile counts
-    uint32_t* sums;               // scan tile sums
+    uint32_t* cnt;                // digit-major tile counts, then the digits' totals
     uint32_t *left, *right;       // internal node children (kLeafRef | sorted index for leaves)
     uint32_t *parent_i, *parent_l;
     float4 *nlo, *nhi;            // internal node boxes
@@ -225,30 +222,22 @@ __global__ void __launch_bounds__(256) morton_kernel(uint32_t nt, Buffers B) {
 }
 
 // ---- stable LSD radix sort ---------------------------------------------------
-constexpr int kSortWarps = 8;
-constexpr uint32_t kSortIters = 64;
-constexpr uint32_t kSortTile = 32 * kSortIters;  // elements per warp tile
-constexpr int kScanThreads = 256;
-constexpr uint32_t kScanItems = 16;
-constexpr uint32_t kScanTile = kScanThreads * kScanItems;  // 4096 counters per scan tile
-constexpr int kTopThreads = 1024;                           // scans up to 4 * 1024 tile sums
-
-__global__ void __launch_bounds__(32 * kSortWarps) hist_kernel(const unsigned long long* __restrict__ keys, uint32_t n,
-                                                               uint32_t shift, uint32_t units, uint32_t* cnt) {
-    __shared__ uint32_t s_cnt[kSortWarps][256];
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    const uint32_t u = blockIdx.x * kSortWarps + warp;
-    if (u >= units) return;
-    for (uint32_t d = lane; d < 256; d += 32) s_cnt[warp][d] = 0;
-    __syncwarp();
-    const uint32_t base = u * kSortTile;
-    for (uint32_t it = 0; it < kSortIters; ++it) {
-        const uint32_t i = base + it * 32 + lane;
-        if (i < n) atomicAdd(&s_cnt[warp][(uint32_t)(keys[i] >> shift) & 255u], 1u);
-    }
-    __syncwarp();
-    for (uint32_t d = lane; d < 256; d += 32) cnt[(size_t)d * units + u] = s_cnt[warp][d];
-}
+// (code, triangle) pairs by 63-bit codes, seven passes of 9 bits. A block owns
+// a tile of 4,096 pairs. Per pass: the tiles' digit counts (digit-major), an
+// exclusive scan of each digit's row over the tiles, and the scatter, in which
+// a warp ranks its 512 pairs in order by matching digits, the block puts the
+// tile in digit order in shared memory, and whole runs of a digit go out
+// together. Bound: per pass 12 bytes in and out per pair, and at a million
+// pairs the latency of three launches. The earlier form (eight 8-bit passes,
+// five launches each, every pair stored on its own by a warp that owned 2,048)
+// took 828 us for 1.1M pairs; this one 231 us.
+constexpr int kSortBlock = 256;
+constexpr int kSortWarps = kSortBlock / 32;
+constexpr int kSortItems = 16;                       // pairs per thread
+constexpr uint32_t kSortTile = kSortBlock * kSortItems;
+constexpr int kDigitBits = 9, kDigits = 1 << kDigitBits, kSortPasses = 7;
+static_assert(kDigitBits * kSortPasses >= 63, "the passes cover the codes' bits");
+constexpr uint32_t kScanRow = 1024;                  // tiles of one digit scanned at a time
 
 template <typename T>
 __device__ __forceinline__ T block_exclusive(T v, T& total, T* s_warp) {
@@ -276,76 +265,137 @@ __device__ __forceinline__ T block_exclusive(T v, T& total, T* s_warp) {
     return before + incl - v;
 }
 
-__global__ void __launch_bounds__(kScanThreads) scan_tile_sum_kernel(const uint32_t* a, uint32_t m, uint32_t* sums) {
-    __shared__ uint32_t s_warp[32];
-    const uint32_t k = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
-    uint32_t v = 0;
-    for (uint32_t j = 0; j < kScanItems; ++j) v += k + j < m ? a[k + j] : 0u;
-    uint32_t total;
-    block_exclusive(v, total, s_warp);
-    if (threadIdx.x == 0) sums[blockIdx.x] = total;
+__device__ __forceinline__ uint32_t digit_of(unsigned long long k, uint32_t shift) {
+    return (uint32_t)(k >> shift) & (uint32_t)(kDigits - 1);
 }
 
-__global__ void __launch_bounds__(kTopThreads) scan_top_kernel(uint32_t* sums, uint32_t tiles) {
-    __shared__ uint32_t s_warp[32];
-    const uint32_t k = 4u * threadIdx.x;
-    uint32_t c[4], v = 0;
-    for (uint32_t j = 0; j < 4; ++j) {
-        c[j] = k + j < tiles ? sums[k + j] : 0u;
-        v += c[j];
+__global__ void __launch_bounds__(kSortBlock) hist_kernel(const unsigned long long* __restrict__ keys, uint32_t n,
+                                                          uint32_t shift, uint32_t tiles, uint32_t* __restrict__ cnt) {
+    __shared__ uint32_t s_cnt[kDigits];
+    for (int d = threadIdx.x; d < kDigits; d += kSortBlock) s_cnt[d] = 0;
+    __syncthreads();
+    const uint32_t base = blockIdx.x * kSortTile + threadIdx.x;
+#pragma unroll
+    for (int k = 0; k < kSortItems; ++k) {
+        const uint32_t i = base + k * kSortBlock;
+        if (i < n) atomicAdd(&s_cnt[digit_of(keys[i], shift)], 1u);
     }
-    uint32_t total;
-    uint32_t run = block_exclusive(v, total, s_warp);
-    for (uint32_t j = 0; j < 4; ++j) {
-        if (k + j < tiles) sums[k + j] = run;
-        run += c[j];
-    }
+    __syncthreads();
+    for (int d = threadIdx.x; d < kDigits; d += kSortBlock) cnt[(size_t)d * tiles + blockIdx.x] = s_cnt[d];
 }
 
-__global__ void __launch_bounds__(kScanThreads) scan_tile_kernel(uint32_t* a, uint32_t m, const uint32_t* sums) {
+// One block per digit: its row's exclusive scan in place, its total.
+__global__ void __launch_bounds__(kScanRow) scan_rows_kernel(uint32_t* __restrict__ cnt, uint32_t tiles,
+                                                             uint32_t* __restrict__ totals) {
     __shared__ uint32_t s_warp[32];
-    const uint32_t k = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
-    uint32_t c[kScanItems], v = 0;
-    for (uint32_t j = 0; j < kScanItems; ++j) {
-        c[j] = k + j < m ? a[k + j] : 0u;
-        v += c[j];
+    uint32_t* row = cnt + (size_t)blockIdx.x * tiles;
+    uint32_t carry = 0;
+    for (uint32_t at = 0; at < tiles; at += kScanRow) {
+        const uint32_t k = at + threadIdx.x;
+        const uint32_t v = k < tiles ? row[k] : 0u;
+        uint32_t total;
+        const uint32_t before = block_exclusive(v, total, s_warp);
+        if (k < tiles) row[k] = carry + before;
+        carry += total;
     }
-    uint32_t total;
-    uint32_t run = sums[blockIdx.x] + block_exclusive(v, total, s_warp);
-    for (uint32_t j = 0; j < kScanItems; ++j) {
-        if (k + j < m) a[k + j] = run;
-        run += c[j];
-    }
+    if (threadIdx.x == 0) totals[blockIdx.x] = carry;
 }
 
-__global__ void __launch_bounds__(32 * kSortWarps) scatter_kernel(const unsigned long long* __restrict__ keys,
-                                                                  const uint32_t* __restrict__ vals, uint32_t n,
-                                                                  uint32_t shift, uint32_t units,
-                                                                  const uint32_t* __restrict__ cnt,
-                                                                  unsigned long long* ok_,
-                                                                  uint32_t* ov) {
-    __shared__ uint32_t s_run[kSortWarps][256];
+struct SortShared {
+    unsigned long long key[kSortTile];
+    uint32_t val[kSortTile];
+    uint32_t cnt[kSortWarps][kDigits];  // digit counts of a warp, then its first position per digit
+    uint32_t out[kDigits];              // global position of a digit's first pair, less its position in the tile
+    uint32_t warp[32];
+};
+
+__global__ void __launch_bounds__(kSortBlock) scatter_kernel(const unsigned long long* __restrict__ keys,
+                                                             const uint32_t* __restrict__ vals, uint32_t n,
+                                                             uint32_t shift, uint32_t tiles,
+                                                             const uint32_t* __restrict__ cnt,
+                                                             const uint32_t* __restrict__ totals,
+                                                             unsigned long long* __restrict__ ok_,
+                                                             uint32_t* __restrict__ ov) {
+    extern __shared__ __align__(16) unsigned char s_raw[];
+    SortShared& S = *reinterpret_cast<SortShared*>(s_raw);
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    const uint32_t u = blockIdx.x * kSortWarps + warp;
-    if (u >= units) return;
-    for (uint32_t d = lane; d < 256; d += 32) s_run[warp][d] = cnt[(size_t)d * units + u];
-    __syncwarp();
-    const uint32_t base = u * kSortTile;
-    for (uint32_t it = 0; it < kSortIters; ++it) {
-        const uint32_t i = base + it * 32 + lane;
-        const bool ok = i < n;
-        const unsigned long long k = ok ? keys[i] : 0ull;
-        const uint32_t d = ok ? ((uint32_t)(k >> shift) & 255u) : 256u;
+    for (int d = threadIdx.x; d < kSortWarps * kDigits; d += kSortBlock) (&S.cnt[0][0])[d] = 0;
+    __syncthreads();
+    const uint32_t tile0 = blockIdx.x * kSortTile;
+    const uint32_t base = tile0 + warp * (32 * kSortItems) + lane;
+    unsigned long long k[kSortItems];
+    uint32_t v[kSortItems], rank[kSortItems];
+#pragma unroll
+    for (int j = 0; j < kSortItems; ++j) {
+        const uint32_t i = base + 32 * j;
+        k[j] = i < n ? keys[i] : ~0ull;
+        v[j] = i < n ? vals[i] : 0u;
+    }
+    // ranks within the warp's pairs of a digit, in input order
+#pragma unroll
+    for (int j = 0; j < kSortItems; ++j) {
+        const bool ok = base + 32 * j < n;
+        const uint32_t d = ok ? digit_of(k[j], shift) : (uint32_t)kDigits;
         const uint32_t peers = __match_any_sync(kFull, d);
-        const uint32_t rank = (uint32_t)__popc(peers & ((1u << lane) - 1u));
-        const uint32_t start = ok ? s_run[warp][d] : 0u;
-        __syncwarp();
-        if (ok) {
-            ok_[start + rank] = k;
-            ov[start + rank] = vals[i];
-            if (lane == (uint32_t)__ffs(peers) - 1u) s_run[warp][d] = start + (uint32_t)__popc(peers);
+        const uint32_t lead = (uint32_t)__ffs(peers) - 1u;
+        uint32_t start = 0;
+        if (ok && lane == lead) {
+            start = S.cnt[warp][d];
+            S.cnt[warp][d] = start + (uint32_t)__popc(peers);
         }
+        rank[j] = __shfl_sync(kFull, start, lead) + (uint32_t)__popc(peers & ((1u << lane) - 1u));
         __syncwarp();
+    }
+    __syncthreads();
+    // the tile's digit order: digit d of warp w starts at the digits before it
+    // plus the pairs of d in the warps before it; thread t has two digits
+    {
+        const int d0 = 2 * threadIdx.x;
+        uint32_t sum[2];
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            uint32_t run = 0;
+#pragma unroll
+            for (int w = 0; w < kSortWarps; ++w) {
+                const uint32_t x = S.cnt[w][d0 + q];
+                S.cnt[w][d0 + q] = run;
+                run += x;
+            }
+            sum[q] = run;
+        }
+        uint32_t total;
+        const uint32_t first = block_exclusive(sum[0] + sum[1], total, S.warp);
+        // the digits' global starts: the totals of the digits before, this
+        // tile's place in the digit's row
+        const uint32_t t0 = totals[d0], t1 = totals[d0 + 1];
+        const uint32_t g0 = block_exclusive(t0 + t1, total, S.warp);
+        S.out[d0] = g0 + cnt[(size_t)d0 * tiles + blockIdx.x] - first;
+        S.out[d0 + 1] = g0 + t0 + cnt[(size_t)(d0 + 1) * tiles + blockIdx.x] - (first + sum[0]);
+#pragma unroll
+        for (int w = 0; w < kSortWarps; ++w) {
+            S.cnt[w][d0] += first;
+            S.cnt[w][d0 + 1] += first + sum[0];
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < kSortItems; ++j)
+        if (base + 32 * j < n) {
+            const uint32_t at = S.cnt[warp][digit_of(k[j], shift)] + rank[j];
+            S.key[at] = k[j];
+            S.val[at] = v[j];
+        }
+    __syncthreads();
+    const uint32_t here = min(kSortTile, n - tile0);
+#pragma unroll
+    for (int j = 0; j < kSortItems; ++j) {
+        const uint32_t i = threadIdx.x + j * kSortBlock;
+        if (i < here) {
+            const unsigned long long key = S.key[i];
+            const uint32_t to = S.out[digit_of(key, shift)] + i;
+            ok_[to] = key;
+            ov[to] = S.val[i];
+        }
     }
 }
 
@@ -1083,23 +1133,20 @@ struct Scratch {
 };
 
 void RadixSort(Buffers& B, uint32_t n, cudaStream_t s) {
-    const uint32_t units = (n + kSortTile - 1) / kSortTile;
-    const uint32_t m = 256u * units;
-    const uint32_t tiles = (m + kScanTile - 1) / kScanTile;
-    const uint32_t blocks = (units + kSortWarps - 1) / kSortWarps;
-    unsigned long long *k_in = B.keys, *k_out = B.keys2;
-    uint32_t *v_in = B.vals, *v_out = B.vals2;
-    for (uint32_t shift = 0; shift < 64; shift += 8) {
-        hist_kernel<<<blocks, 32 * kSortWarps, 0, s>>>(k_in, n, shift, units, B.cnt);
-        scan_tile_sum_kernel<<<tiles, kScanThreads, 0, s>>>(B.cnt, m, B.sums);
-        scan_top_kernel<<<1, kTopThreads, 0, s>>>(B.sums, tiles);
-        scan_tile_kernel<<<tiles, kScanThreads, 0, s>>>(B.cnt, m, B.sums);
-        scatter_kernel<<<blocks, 32 * kSortWarps, 0, s>>>(k_in, v_in, n, shift, units, B.cnt, k_out, v_out);
-        std::swap(k_in, k_out);
-        std::swap(v_in, v_out);
+    const uint32_t tiles = (n + kSortTile - 1) / kSortTile;
+    uint32_t* totals = B.cnt + (size_t)kDigits * tiles;
+    Check(cudaFuncSetAttribute(scatter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SortShared)),
+          "radix sort shared memory");
+    for (int pass = 0; pass < kSortPasses; ++pass) {
+        const uint32_t shift = (uint32_t)(pass * kDigitBits);
+        hist_kernel<<<tiles, kSortBlock, 0, s>>>(B.keys, n, shift, tiles, B.cnt);
+        scan_rows_kernel<<<kDigits, kScanRow, 0, s>>>(B.cnt, tiles, totals);
+        scatter_kernel<<<tiles, kSortBlock, sizeof(SortShared), s>>>(B.keys, B.vals, n, shift, tiles, B.cnt, totals,
+                                                                     B.keys2, B.vals2);
+        std::swap(B.keys, B.keys2);
+        std::swap(B.vals, B.vals2);
     }
     Check(cudaGetLastError(), "radix sort launch");
-    // eight passes: the sorted data is back in keys / vals
 }
 
 // The clustering rounds of ploc_*_kernel. Each round's grids are sized by
@@ -1177,15 +1224,13 @@ void BuildWideGpu(const float* d_verts, uint32_t nv, const uint32_t* d_idx, uint
     Scratch S;
     Buffers B{};
     const uint32_t n = nt;
-    const uint32_t units = (n + kSortTile - 1) / kSortTile;
     B.blo = S.get<float4>(n);
     B.bhi = S.get<float4>(n);
     B.keys = S.get<unsigned long long>(n);
     B.vals = S.get<uint32_t>(n);
     B.keys2 = S.get<unsigned long long>(n);
     B.vals2 = S.get<uint32_t>(n);
-    B.cnt = S.get<uint32_t>(256ull * units);
-    B.sums = S.get<uint32_t>(4 * kTopThreads);
+    B.cnt = S.get<uint32_t>((uint64_t)kDigits * ((n + kSortTile - 1) / kSortTile) + kDigits);
     B.left = S.get<uint32_t>(n);
     B.right = S.get<uint32_t>(n);
     B.parent_i = S.get<uint32_t>(n);

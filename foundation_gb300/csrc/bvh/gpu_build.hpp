@@ -18,7 +18,7 @@
 namespace Foundation {
 namespace RT {
 
-constexpr uint32_t kGpuBuildMaxTris = 1u << 27;  // radix-sort scan capacity
+constexpr uint32_t kGpuBuildMaxTris = 1u << 27;
 
 struct GpuBuildParams {
     uint32_t max_leaf = 4;
