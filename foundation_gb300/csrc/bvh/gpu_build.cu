@@ -458,115 +458,137 @@ __host__ __device__ __forceinline__ float half_area(float4 lo, float4 hi) {
 // least one pair. Internal nodes are numbered down from n - 2 in creation
 // order, so the last merge, the root, is node 0 as in the Karras tree, and
 // the same refit and collapse follow.
+//
+// A round is two launches: one finds the neighbours of a tile and of the r
+// clusters around it (so a tile knows its mutual pairs by itself), counts
+// merges and survivors, and its last block to finish scans the tiles' counts;
+// the other merges and compacts. Once kPlocSmall clusters are left one block
+// runs the remaining rounds in shared memory. Bound: at a million clusters the
+// 32-byte cluster records read twice and written once per round, then launch
+// latency. The earlier form (four launches a round down to one cluster,
+// sixteen consecutive clusters per thread) took 1,110 us for 1.1M triangles.
 constexpr int kPlocBlock = 256;
 constexpr int kPlocMaxRadius = 64;
-constexpr uint32_t kPlocItems = 16;
-constexpr uint32_t kPlocTile = kPlocBlock * kPlocItems;  // clusters per scan tile
+constexpr uint32_t kPlocItems = 2;
+constexpr uint32_t kPlocTile = kPlocBlock * kPlocItems;  // clusters per block
+constexpr uint32_t kPlocSmall = 1024;                    // clusters the last kernel takes
+constexpr uint32_t kPlocGone = 0xFFFFFFFFu;              // merged into a lower position
 
 struct PlocState {
     uint32_t count;      // clusters
     uint32_t next_node;  // internal nodes 0 .. next_node - 1 are still to be made
 };
 
-__global__ void __launch_bounds__(kPlocBlock) ploc_init_kernel(uint32_t n, Buffers B, uint32_t* __restrict__ cref,
-                                                               float4* __restrict__ lo, float4* __restrict__ hi,
-                                                               PlocState* st) {
+// Cluster records: lo.w holds the cluster's reference (bits).
+__global__ void __launch_bounds__(kPlocBlock) ploc_init_kernel(uint32_t n, Buffers B, float4* __restrict__ lo,
+                                                               float4* __restrict__ hi, PlocState* st,
+                                                               uint32_t* ticket) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i == 0) *st = PlocState{n, n - 1u};
+    if (i == 0) {
+        *st = PlocState{n, n - 1u};
+        *ticket = 0;
+    }
     if (i >= n) return;
     const uint32_t t = B.vals[i];
-    cref[i] = kLeafRef | i;
-    lo[i] = B.blo[t];
+    const float4 l = B.blo[t];
+    lo[i] = make_float4(l.x, l.y, l.z, __uint_as_float(kLeafRef | i));
     hi[i] = B.bhi[t];
 }
 
-__global__ void __launch_bounds__(kPlocBlock) ploc_nn_kernel(const PlocState* __restrict__ st,
-                                                             const float4* __restrict__ lo,
-                                                             const float4* __restrict__ hi, uint32_t* __restrict__ nn,
-                                                             int r) {
-    __shared__ float4 s_lo[kPlocBlock + 2 * kPlocMaxRadius], s_hi[kPlocBlock + 2 * kPlocMaxRadius];
-    const int count = (int)st->count;
-    const int b0 = (int)(blockIdx.x * kPlocBlock);
-    if (b0 >= count) return;
-    for (int k = threadIdx.x; k < kPlocBlock + 2 * r; k += kPlocBlock) {
-        const int g = b0 - r + k;
-        if (g >= 0 && g < count) {
-            s_lo[k] = lo[g];
-            s_hi[k] = hi[g];
-        }
-    }
-    __syncthreads();
-    const int i = b0 + (int)threadIdx.x;
-    if (i >= count) return;
-    const int li = (int)threadIdx.x + r;
-    const float4 alo = s_lo[li], ahi = s_hi[li];
+// The nearest of the clusters within r of i (positions 0 .. count - 1; at(j)
+// gives a position's index in lo / hi).
+template <typename At>
+__device__ __forceinline__ int ploc_nearest(const float4* lo, const float4* hi, int i, int count, int r, At at) {
+    const float4 alo = lo[at(i)], ahi = hi[at(i)];
     float best = __int_as_float(0x7F800000);
     int bj = i;
     const int jlo = max(0, i - r), jhi = min(count - 1, i + r);
     for (int j = jlo; j <= jhi; ++j) {
         if (j == i) continue;
-        const int lj = j - b0 + r;
+        const float4 olo = lo[at(j)], ohi = hi[at(j)];
         // the lower position's box first, so both ends compute the same bits
-        const float4 plo = j < i ? s_lo[lj] : alo, phi = j < i ? s_hi[lj] : ahi;
-        const float4 qlo = j < i ? alo : s_lo[lj], qhi = j < i ? ahi : s_hi[lj];
+        const float4 plo = j < i ? olo : alo, phi = j < i ? ohi : ahi;
+        const float4 qlo = j < i ? alo : olo, qhi = j < i ? ahi : ohi;
         const float dx = fmaxf(phi.x, qhi.x) - fminf(plo.x, qlo.x);
         const float dy = fmaxf(phi.y, qhi.y) - fminf(plo.y, qlo.y);
         const float dz = fmaxf(phi.z, qhi.z) - fminf(plo.z, qlo.z);
-        // overflowing extents compare as +inf, so the order stays total
-        const float d = fminf(dx * dy + dy * dz + dz * dx, __int_as_float(0x7F800000));
+        // one rounding order wherever this is inlined, so a pair has one area
+        // in both kernels; overflowing extents compare as +inf, so the order
+        // stays total
+        const float area = __fmaf_rn(dz, dx, __fmaf_rn(dy, dz, __fmul_rn(dx, dy)));
+        const float d = fminf(area, __int_as_float(0x7F800000));
         if (d < best || bj == i) {
             best = d;
             bj = j;
         }
     }
-    nn[i] = (uint32_t)bj;
+    return bj;
 }
 
-// per cluster i with neighbour j: merges here (mutual, i < j), survives
-// (not mutual, or the merge's lower end)
-__device__ __forceinline__ void ploc_flags(const uint32_t* __restrict__ nn, uint32_t i, uint32_t& j, bool& merge,
-                                           bool& survive) {
-    j = nn[i];
-    const bool mutual = j != i && nn[j] == i;
-    merge = mutual && i < j;
-    survive = !mutual || i < j;
+// (merges << 32) | survivors of a cluster: `partner` is its own position when
+// it stays alone, the higher one it merges with, or kPlocGone.
+__device__ __forceinline__ unsigned long long ploc_weight(uint32_t i, uint32_t partner) {
+    return partner == kPlocGone ? 0ull : partner == i ? 1ull : (1ull << 32) + 1ull;
 }
 
-// per tile: (merges << 32) | survivors
-__global__ void __launch_bounds__(kPlocBlock) ploc_count_kernel(const PlocState* __restrict__ st,
-                                                                const uint32_t* __restrict__ nn,
-                                                                unsigned long long* __restrict__ tsum) {
+__global__ void __launch_bounds__(kPlocBlock) ploc_pair_kernel(const PlocState* __restrict__ st,
+                                                               PlocState* __restrict__ next,
+                                                               const float4* __restrict__ lo,
+                                                               const float4* __restrict__ hi,
+                                                               uint32_t* __restrict__ partner,
+                                                               unsigned long long* __restrict__ tsum,
+                                                               uint32_t* ticket, int r) {
+    __shared__ float4 s_lo[kPlocTile + 4 * kPlocMaxRadius], s_hi[kPlocTile + 4 * kPlocMaxRadius];
+    __shared__ int s_nn[kPlocTile + 2 * kPlocMaxRadius];
     __shared__ unsigned long long s_warp[32];
-    const uint32_t count = st->count;
-    if (blockIdx.x * kPlocTile >= count) return;
-    const uint32_t base = blockIdx.x * kPlocTile + threadIdx.x * kPlocItems;
-    unsigned long long v = 0;
-    for (uint32_t k = 0; k < kPlocItems; ++k) {
-        const uint32_t i = base + k;
-        if (i >= count) break;
-        uint32_t j;
-        bool merge, survive;
-        ploc_flags(nn, i, j, merge, survive);
-        v += (merge ? (1ull << 32) : 0ull) + (survive ? 1ull : 0ull);
+    __shared__ bool s_last;
+    const int count = (int)st->count;
+    const int b0 = (int)(blockIdx.x * kPlocTile);
+    if (b0 < count) {
+        for (int k = threadIdx.x; k < (int)kPlocTile + 4 * r; k += kPlocBlock) {
+            const int g = b0 - 2 * r + k;
+            if (g >= 0 && g < count) {
+                s_lo[k] = lo[g];
+                s_hi[k] = hi[g];
+            }
+        }
+        __syncthreads();
+        for (int k = threadIdx.x; k < (int)kPlocTile + 2 * r; k += kPlocBlock) {
+            const int i = b0 - r + k;
+            if (i >= 0 && i < count)
+                s_nn[k] = ploc_nearest(s_lo, s_hi, i, count, r, [&](int j) { return j - b0 + 2 * r; });
+        }
+        __syncthreads();
+        unsigned long long v = 0;
+#pragma unroll
+        for (uint32_t q = 0; q < kPlocItems; ++q) {
+            const int i = b0 + (int)(threadIdx.x * kPlocItems + q);
+            if (i >= count) continue;
+            const int j = s_nn[i - b0 + r];
+            const bool mutual = j != i && s_nn[j - b0 + r] == i;
+            const uint32_t p = !mutual ? (uint32_t)i : i < j ? (uint32_t)j : kPlocGone;
+            partner[i] = p;
+            v += ploc_weight((uint32_t)i, p);
+        }
+        unsigned long long total;
+        block_exclusive(v, total, s_warp);
+        if (threadIdx.x == 0) tsum[blockIdx.x] = total;
     }
-    unsigned long long total;
-    block_exclusive(v, total, s_warp);
-    if (threadIdx.x == 0) tsum[blockIdx.x] = total;
-}
-
-// exclusive scan of the tile sums (one block, 4,096 tiles at a time), and
-// the next round's state
-__global__ void __launch_bounds__(1024) ploc_scan_kernel(const PlocState* __restrict__ st, PlocState* __restrict__ next,
-                                                         unsigned long long* __restrict__ tsum) {
-    __shared__ unsigned long long s_warp[32];
-    const uint32_t count = st->count;
-    const uint32_t tiles = (count + kPlocTile - 1) / kPlocTile;
+    // the last block scans the tiles' sums and writes the next round's state
+    if (threadIdx.x == 0) {
+        __threadfence();
+        s_last = atomicAdd(ticket, 1u) == gridDim.x - 1u;
+    }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    const uint32_t tiles = ((uint32_t)count + kPlocTile - 1) / kPlocTile;
     unsigned long long carry = 0;
-    for (uint32_t c0 = 0; c0 < tiles; c0 += 4 * 1024) {
+    for (uint32_t c0 = 0; c0 < tiles; c0 += 4 * kPlocBlock) {
         const uint32_t k = c0 + 4u * threadIdx.x;
         unsigned long long c[4], v = 0;
         for (uint32_t j = 0; j < 4; ++j) {
-            c[j] = k + j < tiles ? tsum[k + j] : 0ull;
+            c[j] = k + j < tiles ? __ldcg(tsum + k + j) : 0ull;
             v += c[j];
         }
         unsigned long long total;
@@ -577,7 +599,10 @@ __global__ void __launch_bounds__(1024) ploc_scan_kernel(const PlocState* __rest
         }
         carry += total;
     }
-    if (threadIdx.x == 0) *next = PlocState{(uint32_t)carry, st->next_node - (uint32_t)(carry >> 32)};
+    if (threadIdx.x == 0) {
+        *next = PlocState{(uint32_t)carry, st->next_node - (uint32_t)(carry >> 32)};
+        *ticket = 0;
+    }
 }
 
 __device__ __forceinline__ void ploc_set_parent(const Buffers& B, uint32_t ref, uint32_t node) {
@@ -587,50 +612,93 @@ __device__ __forceinline__ void ploc_set_parent(const Buffers& B, uint32_t ref, 
         B.parent_i[ref] = node;
 }
 
-__global__ void __launch_bounds__(kPlocBlock) ploc_merge_kernel(
-    const PlocState* __restrict__ st, const unsigned long long* __restrict__ tsum, const uint32_t* __restrict__ nn,
-    const uint32_t* __restrict__ cin, const float4* __restrict__ lin, const float4* __restrict__ hin,
-    uint32_t* __restrict__ cout, float4* __restrict__ lout, float4* __restrict__ hout, Buffers B) {
+// Clusters a (lower position) and b become internal node `node`.
+__device__ __forceinline__ void ploc_join(const Buffers& B, uint32_t node, float4& alo, float4& ahi, float4 blo,
+                                          float4 bhi) {
+    const uint32_t a = __float_as_uint(alo.w), b = __float_as_uint(blo.w);
+    B.left[node] = a;
+    B.right[node] = b;
+    ploc_set_parent(B, a, node);
+    ploc_set_parent(B, b, node);
+    alo = make_float4(fminf(alo.x, blo.x), fminf(alo.y, blo.y), fminf(alo.z, blo.z), __uint_as_float(node));
+    ahi = make_float4(fmaxf(ahi.x, bhi.x), fmaxf(ahi.y, bhi.y), fmaxf(ahi.z, bhi.z), 0.0f);
+}
+
+__global__ void __launch_bounds__(kPlocBlock) ploc_merge_kernel(const PlocState* __restrict__ st,
+                                                                const unsigned long long* __restrict__ tsum,
+                                                                const uint32_t* __restrict__ partner,
+                                                                const float4* __restrict__ lin,
+                                                                const float4* __restrict__ hin,
+                                                                float4* __restrict__ lout, float4* __restrict__ hout,
+                                                                Buffers B) {
     __shared__ unsigned long long s_warp[32];
     const uint32_t count = st->count, next_node = st->next_node;
     if (blockIdx.x * kPlocTile >= count) return;
     const uint32_t base = blockIdx.x * kPlocTile + threadIdx.x * kPlocItems;
-    uint32_t jj[kPlocItems], merge_bits = 0, survive_bits = 0;
+    uint32_t p[kPlocItems];
     unsigned long long v = 0;
-    for (uint32_t k = 0; k < kPlocItems; ++k) {
-        const uint32_t i = base + k;
-        bool merge = false, survive = false;
-        jj[k] = i;
-        if (i < count) ploc_flags(nn, i, jj[k], merge, survive);
-        merge_bits |= (merge ? 1u : 0u) << k;
-        survive_bits |= (survive ? 1u : 0u) << k;
-        v += (merge ? (1ull << 32) : 0ull) + (survive ? 1ull : 0ull);
+#pragma unroll
+    for (uint32_t q = 0; q < kPlocItems; ++q) {
+        p[q] = base + q < count ? partner[base + q] : kPlocGone;
+        v += ploc_weight(base + q, p[q]);
     }
     unsigned long long total;
     unsigned long long run = tsum[blockIdx.x] + block_exclusive(v, total, s_warp);
-    for (uint32_t k = 0; k < kPlocItems; ++k) {
-        if (!(survive_bits >> k & 1u)) continue;
-        const uint32_t i = base + k, at = (uint32_t)run;
-        if (merge_bits >> k & 1u) {
-            const uint32_t j = jj[k];
-            const uint32_t node = next_node - 1u - (uint32_t)(run >> 32);
-            const uint32_t a = cin[i], b = cin[j];
-            B.left[node] = a;
-            B.right[node] = b;
-            ploc_set_parent(B, a, node);
-            ploc_set_parent(B, b, node);
-            const float4 al = lin[i], ah = hin[i], bl = lin[j], bh = hin[j];
-            cout[at] = node;
-            lout[at] = make_float4(fminf(al.x, bl.x), fminf(al.y, bl.y), fminf(al.z, bl.z), 0.0f);
-            hout[at] = make_float4(fmaxf(ah.x, bh.x), fmaxf(ah.y, bh.y), fmaxf(ah.z, bh.z), 0.0f);
-            run += (1ull << 32) + 1ull;
-        } else {
-            cout[at] = cin[i];
-            lout[at] = lin[i];
-            hout[at] = hin[i];
-            run += 1ull;
-        }
+#pragma unroll
+    for (uint32_t q = 0; q < kPlocItems; ++q) {
+        const uint32_t i = base + q;
+        if (p[q] == kPlocGone) continue;
+        float4 lo = lin[i], hi = hin[i];
+        if (p[q] != i) ploc_join(B, next_node - 1u - (uint32_t)(run >> 32), lo, hi, lin[p[q]], hin[p[q]]);
+        lout[(uint32_t)run] = lo;
+        hout[(uint32_t)run] = hi;
+        run += ploc_weight(i, p[q]);
     }
+}
+
+// The rounds of at most kPlocSmall clusters, by one block. Every round merges
+// a pair, so there are fewer rounds than clusters; the bound only guards.
+__global__ void __launch_bounds__(kPlocSmall) ploc_small_kernel(PlocState* st, const float4* __restrict__ lin,
+                                                                const float4* __restrict__ hin, int r, Buffers B) {
+    __shared__ float4 s_lo[kPlocSmall], s_hi[kPlocSmall];
+    __shared__ int s_nn[kPlocSmall];
+    __shared__ unsigned long long s_warp[32];
+    uint32_t count = st->count, next_node = st->next_node;
+    if (count > kPlocSmall) return;  // the host sees the count and reports it
+    const uint32_t i = threadIdx.x;
+    if (i < count) {
+        s_lo[i] = lin[i];
+        s_hi[i] = hin[i];
+    }
+    __syncthreads();
+    for (uint32_t round = 0; count > 1u && round < kPlocSmall; ++round) {
+        if (i < count) s_nn[i] = ploc_nearest(s_lo, s_hi, (int)i, (int)count, r, [](int j) { return j; });
+        __syncthreads();
+        uint32_t p = kPlocGone;
+        if (i < count) {
+            const int j = s_nn[i];
+            const bool mutual = j != (int)i && s_nn[j] == (int)i;
+            p = !mutual ? i : (int)i < j ? (uint32_t)j : kPlocGone;
+        }
+        unsigned long long total;
+        const unsigned long long run = block_exclusive(ploc_weight(i, p), total, s_warp);
+        float4 lo, hi;
+        if (p != kPlocGone) {
+            lo = s_lo[i];
+            hi = s_hi[i];
+            if (p != i) ploc_join(B, next_node - 1u - (uint32_t)(run >> 32), lo, hi, s_lo[p], s_hi[p]);
+        }
+        __syncthreads();
+        if (p != kPlocGone) {
+            s_lo[(uint32_t)run] = lo;
+            s_hi[(uint32_t)run] = hi;
+        }
+        __syncthreads();
+        if ((uint32_t)(total >> 32) == 0u) break;
+        count = (uint32_t)total;
+        next_node -= (uint32_t)(total >> 32);
+    }
+    if (i == 0) *st = PlocState{count, next_node};
 }
 
 struct RefBox {
@@ -1154,12 +1222,12 @@ void RadixSort(Buffers& B, uint32_t n, cudaStream_t s) {
 // fall), so the host never waits for the round it has just queued.
 void PlocHierarchy(Buffers& B, uint32_t n, int r, cudaStream_t s) {
     Scratch S;
-    uint32_t* cref[2] = {S.get<uint32_t>(n), S.get<uint32_t>(n)};
     float4* lo[2] = {S.get<float4>(n), S.get<float4>(n)};
     float4* hi[2] = {S.get<float4>(n), S.get<float4>(n)};
-    uint32_t* nn = S.get<uint32_t>(n);
+    uint32_t* partner = S.get<uint32_t>(n);
     unsigned long long* tsum = S.get<unsigned long long>((n + kPlocTile - 1) / kPlocTile);
     PlocState* st = S.get<PlocState>(2);
+    uint32_t* ticket = S.get<uint32_t>(1);
     PlocState* h = nullptr;  // one pinned slot per round in flight
     Check(cudaHostAlloc(reinterpret_cast<void**>(&h), 2 * sizeof(PlocState), cudaHostAllocDefault),
           "cudaHostAlloc (cluster counts)");
@@ -1174,19 +1242,16 @@ void PlocHierarchy(Buffers& B, uint32_t n, int r, cudaStream_t s) {
         }
     } release{h, ev};
     for (int k = 0; k < 2; ++k) Check(cudaEventCreateWithFlags(&ev[k], cudaEventDisableTiming), "event");
-    ploc_init_kernel<<<(n + kPlocBlock - 1) / kPlocBlock, kPlocBlock, 0, s>>>(n, B, cref[0], lo[0], hi[0], st);
-    uint32_t bound = n, last = n, launched = 0;
+    ploc_init_kernel<<<(n + kPlocBlock - 1) / kPlocBlock, kPlocBlock, 0, s>>>(n, B, lo[0], hi[0], st, ticket);
+    uint32_t bound = n;  // at least the clusters of the round about to be queued
     int cur = 0;
-    bool done = false, stuck = false;
     // every round of two or more clusters merges a pair: at most n - 1 rounds
-    for (uint32_t round = 0; !done && round <= n; ++round) {
-        launched = round + 1;
+    for (uint32_t round = 0; bound > kPlocSmall && round <= n; ++round) {
         const uint32_t tiles = (bound + kPlocTile - 1) / kPlocTile;
-        ploc_nn_kernel<<<(bound + kPlocBlock - 1) / kPlocBlock, kPlocBlock, 0, s>>>(st + cur, lo[cur], hi[cur], nn, r);
-        ploc_count_kernel<<<tiles, kPlocBlock, 0, s>>>(st + cur, nn, tsum);
-        ploc_scan_kernel<<<1, 1024, 0, s>>>(st + cur, st + (cur ^ 1), tsum);
-        ploc_merge_kernel<<<tiles, kPlocBlock, 0, s>>>(st + cur, tsum, nn, cref[cur], lo[cur], hi[cur],
-                                                       cref[cur ^ 1], lo[cur ^ 1], hi[cur ^ 1], B);
+        ploc_pair_kernel<<<tiles, kPlocBlock, 0, s>>>(st + cur, st + (cur ^ 1), lo[cur], hi[cur], partner, tsum,
+                                                      ticket, r);
+        ploc_merge_kernel<<<tiles, kPlocBlock, 0, s>>>(st + cur, tsum, partner, lo[cur], hi[cur], lo[cur ^ 1],
+                                                       hi[cur ^ 1], B);
         Check(cudaMemcpyAsync(h + (round & 1), st + (cur ^ 1), sizeof(PlocState), cudaMemcpyDeviceToHost, s),
               "cluster count");
         Check(cudaEventRecord(ev[round & 1], s), "event");
@@ -1194,15 +1259,14 @@ void PlocHierarchy(Buffers& B, uint32_t n, int r, cudaStream_t s) {
         if (round == 0) continue;
         Check(cudaEventSynchronize(ev[(round - 1) & 1]), "clustering round");
         const uint32_t c = h[(round - 1) & 1].count;
-        done = c <= 1;
-        stuck = c >= last;  // no merge in a round of two or more clusters
-        if (stuck) break;
-        last = bound = c;
+        if (round > 1 && c >= bound) break;  // a round without a merge
+        bound = c;
     }
+    ploc_small_kernel<<<1, kPlocSmall, 0, s>>>(st + cur, lo[cur], hi[cur], r, B);
+    Check(cudaMemcpyAsync(h, st + cur, sizeof(PlocState), cudaMemcpyDeviceToHost, s), "cluster count");
     Check(cudaStreamSynchronize(s), "clustering");
-    const PlocState fin = h[(launched - 1) & 1];
-    CHECK_CODE(!stuck && done && fin.count == 1 && fin.next_node == 0, FND_ERR_INVALID_SCENE,
-               "GPU build: clustering stopped at %u clusters", fin.count);
+    CHECK_CODE(h->count == 1 && h->next_node == 0, FND_ERR_INVALID_SCENE, "GPU build: clustering stopped at %u clusters",
+               h->count);
 }
 
 }  // namespace
