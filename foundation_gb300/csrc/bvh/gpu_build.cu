@@ -49,6 +49,7 @@ constexpr uint32_t kFull = 0xFFFFFFFFu;
 constexpr uint32_t kLeafRef = 0x80000000u;  // reference to a sorted single-triangle leaf
 constexpr uint32_t kLeafNode = 0x80000000u;  // count word: this subtree is one leaf
 constexpr uint32_t kNone = 0xFFFFFFFFu;
+constexpr uint32_t kDpLeaf = 0x80u;  // decision byte 0: this subtree is one leaf slot
 constexpr int kMaxLevels = kMaxStack / 2;  // wide levels the traversal stack allows
 constexpr uint32_t kPrepBadIndex = 1u, kPrepNonFinite = 2u;
 
@@ -61,9 +62,7 @@ struct Buffers {
     uint32_t* cnt;                // digit-major tile counts, then the digits' totals
     uint32_t *left, *right;       // internal node children (kLeafRef | sorted index for leaves)
     uint32_t *parent_i, *parent_l;
-    float4 *nlo, *nhi;            // internal node boxes
-    uint32_t* ncount;             // triangle count | kLeafNode
-    float* ncost;
+    float4 *nlo, *nhi;            // internal node boxes; nlo.w: triangle count | kLeafNode (bits), nhi.w: SAH cost
     uint32_t* flag;               // refit arrival counters
     float* bounds;                // scene lo[3], hi[3], centroid lo[3], hi[3]
     uint32_t* status;
@@ -71,9 +70,9 @@ struct Buffers {
     uint2 *qa, *qb;               // collapse queues (binary ref, wide node)
     // SAH-optimal collapse (null: greedy), per internal node k:
     float* dpc;                   // [8 k + i - 1]: C(k, i), least cost of k's subtree as at most i roots
-    uint8_t* dpch;                // [8 k + i - 1], i >= 2: 0 = C(k, i - 1), else roots given to the left child
-    uint8_t* dpj;                 // roots given to the left child when k is a wide node
-    uint8_t* dpleaf;              // C(k, 1) is one leaf slot
+    uint2* dpch;                  // byte i - 1, i >= 2: 0 = C(k, i - 1), else roots given to the left child;
+                                  // byte 0: roots given to the left child when k is a wide node, | kDpLeaf when
+                                  // C(k, 1) is one leaf slot
     float c_tri;                  // cost of a triangle test relative to a wide-node visit
     uint32_t width;               // children per wide node (2..8)
 };
@@ -718,18 +717,18 @@ __device__ __forceinline__ RefBox ref_box(const Buffers& B, uint32_t ref) {
     } else {
         r.lo = __ldcg(B.nlo + ref);
         r.hi = __ldcg(B.nhi + ref);
-        r.count = __ldcg(B.ncount + ref);
-        r.cost = __ldcg(B.ncost + ref);
+        r.count = __float_as_uint(r.lo.w);
+        r.cost = r.hi.w;
     }
     return r;
 }
 
 // C(ref, 1..8) of a child: a single-triangle leaf costs c_tri x its half area
 // whatever the number of roots.
-__device__ __forceinline__ void dp_child(const Buffers& B, uint32_t ref, float c[8]) {
+__device__ __forceinline__ void dp_child(const Buffers& B, uint32_t ref, const RefBox& box, float c[8]) {
     if (ref & kLeafRef) {
-        const uint32_t t = B.vals[ref & ~kLeafRef];
-        const float v = B.c_tri * half_area(B.blo[t], B.bhi[t]);
+        const float v = B.c_tri * box.cost;
+#pragma unroll
         for (int i = 0; i < 8; ++i) c[i] = v;
     } else {
         const float4 a = __ldcg(reinterpret_cast<const float4*>(B.dpc + 8 * (size_t)ref));
@@ -738,6 +737,11 @@ __device__ __forceinline__ void dp_child(const Buffers& B, uint32_t ref, float c
     }
 }
 
+// Bound: the memory traffic of the node records near the leaves, then the
+// dependent steps of the walk's upper levels. A node is two vectors (count and
+// cost in their w), its decisions one 8-byte word, the programme's tables stay
+// in registers (loops unrolled): with byte-wise stores, separate count and cost
+// arrays and tables in local memory 1.1M triangles took 343 us.
 __global__ void __launch_bounds__(256) refit_kernel(uint32_t n, Buffers B, uint32_t max_leaf, float trav_cost) {
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n || n < 2) return;
@@ -751,62 +755,85 @@ __global__ void __launch_bounds__(256) refit_kernel(uint32_t n, Buffers B, uint3
         __threadfence();
         if (atomicAdd(B.flag + p, 1u) == 0u) return;  // the sibling subtree is not finished yet
         __threadfence();
-        const RefBox l = ref_box(B, B.left[p]), r = ref_box(B, B.right[p]);
+        const uint32_t left = B.left[p], right = B.right[p], up = B.parent_i[p];
+        const RefBox l = ref_box(B, left), r = ref_box(B, right);
         float4 lo = make_float4(fminf(l.lo.x, r.lo.x), fminf(l.lo.y, r.lo.y), fminf(l.lo.z, r.lo.z), 0.0f);
         float4 hi = make_float4(fmaxf(l.hi.x, r.hi.x), fmaxf(l.hi.y, r.hi.y), fmaxf(l.hi.z, r.hi.z), 0.0f);
         const uint32_t cnt = (l.count & ~kLeafNode) + (r.count & ~kLeafNode);
         const float a = half_area(lo, hi);
         const float split = trav_cost * a + l.cost + r.cost;
         const bool leaf = cnt <= max_leaf && (float)cnt * a <= split;
+        lo.w = __uint_as_float(cnt | (leaf ? kLeafNode : 0u));
+        hi.w = leaf ? (float)cnt * a : split;
         B.nlo[p] = lo;
         B.nhi[p] = hi;
-        B.ncount[p] = cnt | (leaf ? kLeafNode : 0u);
-        B.ncost[p] = leaf ? (float)cnt * a : split;
         if (B.dpc) {
             // SAH-optimal collapse: wide node at cost a, leaf slot at c_tri a cnt
-            float cl[8], cr[8], sp[9];
-            uint8_t sj[9];
-            dp_child(B, B.left[p], cl);
-            dp_child(B, B.right[p], cr);
-            for (int i = 2; i <= 8; ++i) {
+            float cl[8], cr[8], sp[7];  // sp[i - 2]: the subtree as i roots, split between the children
+            uint32_t sj[7];             // and the left child's share
+            dp_child(B, left, l, cl);
+            dp_child(B, right, r, cr);
+#pragma unroll
+            for (int i = 0; i < 7; ++i) {
                 sp[i] = FLT_MAX;
                 sj[i] = 1;
-                for (int j = 1; j < i; ++j) {
-                    const float v = cl[j - 1] + cr[i - j - 1];
-                    if (v < sp[i]) {
-                        sp[i] = v;
-                        sj[i] = (uint8_t)j;
-                    }
-                }
             }
+            // j roots left, k right, in ascending j for every sum
+#pragma unroll
+            for (int j = 1; j <= 7; ++j)
+#pragma unroll
+                for (int k = 1; k <= 7; ++k)
+                    if (j + k <= 8) {
+                        const float v = cl[j - 1] + cr[k - 1];
+                        if (v < sp[j + k - 2]) {
+                            sp[j + k - 2] = v;
+                            sj[j + k - 2] = (uint32_t)j;
+                        }
+                    }
+            // (constant indices: the tables stay in registers)
+            const uint32_t width = B.width;
+            const float at_width = width == 8u   ? sp[6]
+                                   : width == 7u ? sp[5]
+                                   : width == 6u ? sp[4]
+                                   : width == 5u ? sp[3]
+                                   : width == 4u ? sp[2]
+                                   : width == 3u ? sp[1]
+                                                 : sp[0];
+            const uint32_t j_width = width == 8u   ? sj[6]
+                                     : width == 7u ? sj[5]
+                                     : width == 6u ? sj[4]
+                                     : width == 5u ? sj[3]
+                                     : width == 4u ? sj[2]
+                                     : width == 3u ? sj[1]
+                                                   : sj[0];
             float c[8];
-            const float node_cost = a + sp[B.width];
+            const float node_cost = a + at_width;
             c[0] = node_cost;
-            uint8_t as_leaf = 0;
+            uint32_t as_leaf = 0;
             if (cnt <= (uint32_t)kMaxLeafTris) {
                 const float leaf_cost = B.c_tri * a * (float)cnt;
                 if (leaf_cost <= node_cost) {
                     c[0] = leaf_cost;
-                    as_leaf = 1;
+                    as_leaf = kDpLeaf;
                 }
             }
-            uint8_t ch[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+            uint2 ch = make_uint2(j_width | as_leaf, 0u);
+#pragma unroll
             for (int i = 2; i <= 8; ++i) {
-                if (sp[i] < c[i - 2]) {
-                    c[i - 1] = sp[i];
-                    ch[i - 1] = sj[i];
-                } else {
-                    c[i - 1] = c[i - 2];
-                }
+                const bool two = sp[i - 2] < c[i - 2];
+                c[i - 1] = two ? sp[i - 2] : c[i - 2];
+                const uint32_t w = two ? sj[i - 2] : 0u;
+                if (i <= 4)
+                    ch.x |= w << 8 * (i - 1);
+                else
+                    ch.y |= w << 8 * (i - 5);
             }
             float4* dc = reinterpret_cast<float4*>(B.dpc + 8 * (size_t)p);
             dc[0] = make_float4(c[0], c[1], c[2], c[3]);
             dc[1] = make_float4(c[4], c[5], c[6], c[7]);
-            for (int i = 0; i < 8; ++i) B.dpch[8 * (size_t)p + i] = ch[i];
-            B.dpj[p] = sj[B.width];
-            B.dpleaf[p] = as_leaf;
+            B.dpch[p] = ch;
         }
-        p = B.parent_i[p];
+        p = up;
     }
 }
 
@@ -874,7 +901,7 @@ __global__ void __launch_bounds__(kCollapseBlock) collapse_kernel(const Collapse
             // left-to-right order: (subtree, roots it may become)
             uint32_t roots = 0;
             if (inner) {
-                const uint32_t j = B.dpj[item.x];
+                const uint32_t j = B.dpch[item.x].x & (kDpLeaf - 1u);
                 kid = c == 0 ? B.left[item.x] : B.right[item.x];
                 roots = c == 0 ? j : B.width - j;
                 nk = 2;
@@ -882,7 +909,7 @@ __global__ void __launch_bounds__(kCollapseBlock) collapse_kernel(const Collapse
             for (int round = 0; round < kWidth; ++round) {
                 uint32_t split = 0;  // roots of the left part, 0: done
                 if (inner && c < nk && roots >= 2u && !(kid & kLeafRef)) {
-                    const uint2 w = *reinterpret_cast<const uint2*>(B.dpch + 8 * (size_t)kid);
+                    const uint2 w = B.dpch[kid];
                     while (roots >= 2u) {
                         split = (roots > 4u ? w.y >> 8 * (roots - 5u) : w.x >> 8 * (roots - 1u)) & 255u;
                         if (split) break;
@@ -915,14 +942,17 @@ __global__ void __launch_bounds__(kCollapseBlock) collapse_kernel(const Collapse
                 }
                 nk = min(total, kWidth);
             }
-            if (inner && c < nk) dp_leaf = (kid & kLeafRef) || B.dpleaf[kid];
+            if (inner && c < nk) dp_leaf = (kid & kLeafRef) || (B.dpch[kid].x & kDpLeaf);
         } else {
             // greedy: the largest inner child is opened until there are width
             float area = -1.0f;
             auto look = [&] {  // area of an openable child, -1 for the others
                 area = -1.0f;
-                if (node && c < nk && !(kid & kLeafRef) && !(__ldcg(B.ncount + kid) & kLeafNode))
-                    area = fmaxf(half_area(__ldcg(B.nlo + kid), __ldcg(B.nhi + kid)), -1.0f);  // (a NaN: not opened)
+                if (node && c < nk && !(kid & kLeafRef)) {
+                    const float4 lo = __ldcg(B.nlo + kid);
+                    if (!(__float_as_uint(lo.w) & kLeafNode))
+                        area = fmaxf(half_area(lo, __ldcg(B.nhi + kid)), -1.0f);  // (a NaN: not opened)
+                }
             };
             look();
             for (int round = 0; round < kWidth; ++round) {
@@ -964,7 +994,7 @@ __global__ void __launch_bounds__(kCollapseBlock) collapse_kernel(const Collapse
             } else {
                 lo = __ldcg(B.nlo + kid);
                 hi = __ldcg(B.nhi + kid);
-                const uint32_t w = __ldcg(B.ncount + kid);
+                const uint32_t w = __float_as_uint(lo.w);
                 is_leaf = (B.dpc && inner) ? dp_leaf : (w & kLeafNode) != 0u;
                 cnt = w & ~kLeafNode;
             }
@@ -1301,8 +1331,6 @@ void BuildWideGpu(const float* d_verts, uint32_t nv, const uint32_t* d_idx, uint
     B.parent_l = S.get<uint32_t>(n);
     B.nlo = S.get<float4>(n);
     B.nhi = S.get<float4>(n);
-    B.ncount = S.get<uint32_t>(n);
-    B.ncost = S.get<float>(n);
     B.flag = S.get<uint32_t>(n);
     B.bounds = S.get<float>(12);
     B.status = S.get<uint32_t>(1);
@@ -1312,9 +1340,7 @@ void BuildWideGpu(const float* d_verts, uint32_t nv, const uint32_t* d_idx, uint
     B.qb = S.get<uint2>(n);
     if (p.sah_collapse && n >= 2) {
         B.dpc = S.get<float>(8ull * n);
-        B.dpch = S.get<uint8_t>(8ull * n);
-        B.dpj = S.get<uint8_t>(n);
-        B.dpleaf = S.get<uint8_t>(n);
+        B.dpch = S.get<uint2>(n);
         B.c_tri = p.c_tri;
     }
     float4* shade = nullptr;
@@ -1358,7 +1384,6 @@ void BuildWideGpu(const float* d_verts, uint32_t nv, const uint32_t* d_idx, uint
     float root_cost = 0.0f, wide_cost = 0.0f;
     float4 rlo{}, rhi{};
     if (n >= 2) {
-        Check(cudaMemcpyAsync(&root_cost, B.ncost, 4, cudaMemcpyDeviceToHost, s), "cost readback");
         if (B.dpc) Check(cudaMemcpyAsync(&wide_cost, B.dpc, 4, cudaMemcpyDeviceToHost, s), "cost readback");
         Check(cudaMemcpyAsync(&rlo, B.nlo, 16, cudaMemcpyDeviceToHost, s), "root box");
         Check(cudaMemcpyAsync(&rhi, B.nhi, 16, cudaMemcpyDeviceToHost, s), "root box");
@@ -1403,6 +1428,7 @@ void BuildWideGpu(const float* d_verts, uint32_t nv, const uint32_t* d_idx, uint
     for (int l = 0; l < kMaxLevels; ++l)
         if (h_counters[4 + l]) out.depth = (uint32_t)l + 1;
     out.num_binary_nodes = 2 * n - 1;
+    root_cost = rhi.w;
     const float ra = n >= 2 ? half_area(rlo, rhi) : 0.0f;
     out.sah_cost = n >= 2 && ra > 0.0f ? (double)root_cost / (double)ra : 0.0;
     if (B.dpc)
