@@ -33,6 +33,7 @@
 #include <cfloat>
 #include <chrono>
 #include <cmath>
+#include <cstring>
 #include <vector>
 
 #include "../../../include/fnd_rt.h"
@@ -1195,6 +1196,12 @@ __global__ void instance_shade_kernel(const float* __restrict__ inv, const uint3
     out[(size_t)off[lo] + t] = l > 0.0f ? make_float4(w[0] * k, w[1] * k, w[2] * k, 0.0f) : make_float4(0, 0, 1, 0);
 }
 
+// The collapse's first queue entry, level 0 of one node.
+__global__ void root_kernel(Buffers B, uint2 item) {
+    B.qa[0] = item;
+    B.counters[4] = 1u;
+}
+
 __global__ void interleave_kernel(const float4* __restrict__ planes, uint32_t n, float4* __restrict__ tris) {
     const size_t j = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (j < 3 * (size_t)n) tris[j] = planes[(j % 3) * n + j / 3];
@@ -1215,18 +1222,23 @@ void Check(cudaError_t e, const char* what) {
                    cudaGetErrorString(e));
 }
 
-// Owner of the temporary device allocations of one build.
+// Owner of the temporary device allocations of one build (stream order).
 struct Scratch {
+    cudaMemPool_t pool;
+    cudaStream_t s;
     std::vector<void*> ptrs;
+    Scratch(cudaMemPool_t pool, cudaStream_t s) : pool(pool), s(s) {}
+    Scratch(const Scratch&) = delete;
+    Scratch& operator=(const Scratch&) = delete;
     template <typename T>
     T* get(size_t count) {
         void* p = nullptr;
-        Check(cudaMalloc(&p, std::max<size_t>(count, 1) * sizeof(T)), "cudaMalloc (GPU build scratch)");
+        Check(cudaMallocFromPoolAsync(&p, std::max<size_t>(count, 1) * sizeof(T), pool, s), "GPU build scratch");
         ptrs.push_back(p);
         return static_cast<T*>(p);
     }
     ~Scratch() {
-        for (void* p : ptrs) cudaFree(p);
+        for (void* p : ptrs) cudaFreeAsync(p, s);
     }
 };
 
@@ -1250,28 +1262,16 @@ void RadixSort(Buffers& B, uint32_t n, cudaStream_t s) {
 // The clustering rounds of ploc_*_kernel. Each round's grids are sized by
 // the cluster count read back one round late (an upper bound: counts only
 // fall), so the host never waits for the round it has just queued.
-void PlocHierarchy(Buffers& B, uint32_t n, int r, cudaStream_t s) {
-    Scratch S;
+void PlocHierarchy(Buffers& B, uint32_t n, int r, GpuBuildResources& res, cudaStream_t s) {
+    Scratch S(res.pool, s);
     float4* lo[2] = {S.get<float4>(n), S.get<float4>(n)};
     float4* hi[2] = {S.get<float4>(n), S.get<float4>(n)};
     uint32_t* partner = S.get<uint32_t>(n);
     unsigned long long* tsum = S.get<unsigned long long>((n + kPlocTile - 1) / kPlocTile);
     PlocState* st = S.get<PlocState>(2);
     uint32_t* ticket = S.get<uint32_t>(1);
-    PlocState* h = nullptr;  // one pinned slot per round in flight
-    Check(cudaHostAlloc(reinterpret_cast<void**>(&h), 2 * sizeof(PlocState), cudaHostAllocDefault),
-          "cudaHostAlloc (cluster counts)");
-    cudaEvent_t ev[2] = {nullptr, nullptr};
-    struct Release {
-        PlocState* h;
-        cudaEvent_t* ev;
-        ~Release() {
-            for (int k = 0; k < 2; ++k)
-                if (ev[k]) cudaEventDestroy(ev[k]);
-            cudaFreeHost(h);
-        }
-    } release{h, ev};
-    for (int k = 0; k < 2; ++k) Check(cudaEventCreateWithFlags(&ev[k], cudaEventDisableTiming), "event");
+    PlocState* h = reinterpret_cast<PlocState*>(res.pinned);  // one slot per round in flight
+    cudaEvent_t* ev = res.ev;
     ploc_init_kernel<<<(n + kPlocBlock - 1) / kPlocBlock, kPlocBlock, 0, s>>>(n, B, lo[0], hi[0], st, ticket);
     uint32_t bound = n;  // at least the clusters of the round about to be queued
     int cur = 0;
@@ -1302,7 +1302,7 @@ void PlocHierarchy(Buffers& B, uint32_t n, int r, cudaStream_t s) {
 }  // namespace
 
 void BuildWideGpu(const float* d_verts, uint32_t nv, const uint32_t* d_idx, uint32_t nt, const GpuBuildParams& p,
-                  GpuBuildOutput& out, cudaStream_t s) {
+                  GpuBuildResources& res, GpuBuildOutput& out, cudaStream_t s) {
     CHECK_CODE(nt >= 1 && nt <= kGpuBuildMaxTris, FND_ERR_INVALID_ARG, "GPU build takes 1..%u triangles, not %u",
                kGpuBuildMaxTris, nt);
     CHECK_CODE(p.max_leaf >= 1 && p.max_leaf <= (uint32_t)kMaxLeafTris, FND_ERR_INVALID_ARG, "max_leaf %u",
@@ -1315,7 +1315,7 @@ void BuildWideGpu(const float* d_verts, uint32_t nv, const uint32_t* d_idx, uint
     Check(cudaGetDevice(&dev), "cudaGetDevice");
     Check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "SM count");
     const auto t0 = std::chrono::steady_clock::now();
-    Scratch S;
+    Scratch S(res.pool, s);
     Buffers B{};
     const uint32_t n = nt;
     B.blo = S.get<float4>(n);
@@ -1343,9 +1343,11 @@ void BuildWideGpu(const float* d_verts, uint32_t nv, const uint32_t* d_idx, uint
         B.dpch = S.get<uint2>(n);
         B.c_tri = p.c_tri;
     }
-    float4* shade = nullptr;
-    Check(cudaMalloc(&shade, 16ull * n), "cudaMalloc (shading normals)");
-    out.d_tri_shade = shade;
+    auto keep = [&](void** p, size_t bytes, const char* what) {
+        Check(cudaMallocFromPoolAsync(p, bytes, res.pool, s), what);
+    };
+    keep(&out.d_tri_shade, 16ull * n, "shading normals");
+    float4* shade = static_cast<float4*>(out.d_tri_shade);
     Check(cudaMemsetAsync(B.status, 0, 4, s), "memset");
     Check(cudaMemsetAsync(B.flag, 0, 4ull * n, s), "memset");
     Check(cudaMemsetAsync(B.parent_i, 0xFF, 4ull * n, s), "memset");
@@ -1354,11 +1356,13 @@ void BuildWideGpu(const float* d_verts, uint32_t nv, const uint32_t* d_idx, uint
     init_bounds_kernel<<<1, 32, 0, s>>>(B.bounds);
     const uint32_t g256 = (n + 255) / 256;
     prep_kernel<<<std::max(1u, std::min(g256, 8u * (uint32_t)sms)), 256, 0, s>>>(d_verts, nv, d_idx, n, B, shade);
-    uint32_t h_status = 0;
+    uint32_t* pinned = res.pinned;
     float h_bounds[12];
-    Check(cudaMemcpyAsync(&h_status, B.status, 4, cudaMemcpyDeviceToHost, s), "status readback");
-    Check(cudaMemcpyAsync(h_bounds, B.bounds, sizeof(h_bounds), cudaMemcpyDeviceToHost, s), "bounds readback");
+    Check(cudaMemcpyAsync(pinned, B.status, 4, cudaMemcpyDeviceToHost, s), "status readback");
+    Check(cudaMemcpyAsync(pinned + 4, B.bounds, sizeof(h_bounds), cudaMemcpyDeviceToHost, s), "bounds readback");
     Check(cudaStreamSynchronize(s), "prep");
+    uint32_t h_status = pinned[0];
+    std::memcpy(h_bounds, pinned + 4, sizeof(h_bounds));
     CHECK_CODE(!(h_status & kPrepBadIndex), FND_ERR_INVALID_ARG, "vertex index out of range (nv = %u)", nv);
     CHECK_CODE(!(h_status & kPrepNonFinite), FND_ERR_INVALID_ARG, "non-finite vertex coordinate");
     for (int a = 0; a < 3; ++a) {
@@ -1370,51 +1374,58 @@ void BuildWideGpu(const float* d_verts, uint32_t nv, const uint32_t* d_idx, uint
     RadixSort(B, n, s);
     if (n >= 2) {
         if (p.ploc_radius)
-            PlocHierarchy(B, n, (int)p.ploc_radius, s);
+            PlocHierarchy(B, n, (int)p.ploc_radius, res, s);
         else
             hierarchy_kernel<<<(n - 1 + 255) / 256, 256, 0, s>>>((int)n, B);
         refit_kernel<<<g256, 256, 0, s>>>(n, B, p.max_leaf, p.trav_cost);
     }
     Check(cudaGetLastError(), "hierarchy launch");
     // root item: internal node 0, or the single leaf
-    const uint2 root = make_uint2(n >= 2 ? 0u : kLeafRef, 0u);
-    Check(cudaMemcpyAsync(B.qa, &root, sizeof(root), cudaMemcpyHostToDevice, s), "root");
-    const uint32_t one = 1u;  // level-0 queue: the root
-    Check(cudaMemcpyAsync(B.counters + 4, &one, 4, cudaMemcpyHostToDevice, s), "queue count");
+    root_kernel<<<1, 1, 0, s>>>(B, make_uint2(n >= 2 ? 0u : kLeafRef, 0u));
     float root_cost = 0.0f, wide_cost = 0.0f;
     float4 rlo{}, rhi{};
     if (n >= 2) {
-        if (B.dpc) Check(cudaMemcpyAsync(&wide_cost, B.dpc, 4, cudaMemcpyDeviceToHost, s), "cost readback");
-        Check(cudaMemcpyAsync(&rlo, B.nlo, 16, cudaMemcpyDeviceToHost, s), "root box");
-        Check(cudaMemcpyAsync(&rhi, B.nhi, 16, cudaMemcpyDeviceToHost, s), "root box");
+        if (B.dpc) Check(cudaMemcpyAsync(pinned, B.dpc, 4, cudaMemcpyDeviceToHost, s), "cost readback");
+        Check(cudaMemcpyAsync(pinned + 4, B.nlo, 16, cudaMemcpyDeviceToHost, s), "root box");
+        Check(cudaMemcpyAsync(pinned + 8, B.nhi, 16, cudaMemcpyDeviceToHost, s), "root box");
     }
     Check(cudaStreamSynchronize(s), "LBVH");
+    if (n >= 2) {
+        if (B.dpc) std::memcpy(&wide_cost, pinned, 4);
+        std::memcpy(&rlo, pinned + 4, 16);
+        std::memcpy(&rhi, pinned + 8, 16);
+    }
     out.build_ms = Ms(t0);
     const auto t1 = std::chrono::steady_clock::now();
-    WideNode* nodes = nullptr;
-    char* tris = nullptr;
-    Check(cudaMalloc(&nodes, sizeof(WideNode) * (size_t)n), "cudaMalloc (wide nodes)");
-    Scratch S2;
-    S2.ptrs.push_back(nodes);
-    Check(cudaMalloc(&tris, 48ull * n), "cudaMalloc (triangles)");
-    out.d_tris = tris;
+    WideNode* nodes = S.get<WideNode>(n);
+    keep(&out.d_tris, 48ull * n, "triangles");
     CollapseArgs A{};
     A.B = B;
     A.verts = d_verts;
     A.idx = d_idx;
     A.nodes = nodes;
-    A.tris = reinterpret_cast<float4*>(tris);
+    A.tris = static_cast<float4*>(out.d_tris);
     A.margin = out.margin;
     const int grid = std::max(1, sms * 8);
-    for (int level = 0; level < kMaxLevels; ++level) {
-        A.level = level;
-        collapse_kernel<<<grid, kCollapseBlock, 0, s>>>(A);
-    }
-    Check(cudaGetLastError(), "collapse launch");
+    // scenes of ordinary depth end within the first levels; the rest is
+    // queued only when the last of them left nodes
+    constexpr int kFirstLevels = 12;
     uint32_t h_counters[4 + kMaxLevels + 2];
-    Check(cudaMemcpyAsync(h_counters, B.counters, sizeof(h_counters), cudaMemcpyDeviceToHost, s), "counters");
-    Check(cudaMemcpyAsync(&h_status, B.status, 4, cudaMemcpyDeviceToHost, s), "status readback");
-    Check(cudaStreamSynchronize(s), "collapse");
+    static_assert(4 + sizeof(h_counters) / 4 <= kGpuBuildPinnedWords, "the counters fit the page-locked words");
+    for (int level = 0; level < kMaxLevels;) {
+        const int end = level == 0 ? kFirstLevels : kMaxLevels;
+        for (; level < end; ++level) {
+            A.level = level;
+            collapse_kernel<<<grid, kCollapseBlock, 0, s>>>(A);
+        }
+        Check(cudaGetLastError(), "collapse launch");
+        Check(cudaMemcpyAsync(pinned, B.status, 4, cudaMemcpyDeviceToHost, s), "status readback");
+        Check(cudaMemcpyAsync(pinned + 4, B.counters, sizeof(h_counters), cudaMemcpyDeviceToHost, s), "counters");
+        Check(cudaStreamSynchronize(s), "collapse");
+        h_status = pinned[0];
+        std::memcpy(h_counters, pinned + 4, sizeof(h_counters));
+        if (h_counters[4 + level] == 0) break;
+    }
     CHECK_CODE(h_counters[4 + kMaxLevels] == 0, FND_ERR_INVALID_SCENE,
                "wide BVH deeper than the traversal stack bound %d", kMaxLevels);
     CHECK_CODE(!(h_status & 4u), FND_ERR_INVALID_SCENE, "child box quantisation failed (scene extent out of range)");
@@ -1435,13 +1446,41 @@ void BuildWideGpu(const float* d_verts, uint32_t nv, const uint32_t* d_idx, uint
         LOG_RUNTIME(FndRt, INFO, "SAH-optimal collapse: wide-tree cost %.4f (root half-area normalised)",
                     ra > 0.0f ? (double)wide_cost / (double)ra : 0.0);
     // exact-size node array
-    void* exact = nullptr;
-    Check(cudaMalloc(&exact, sizeof(WideNode) * (size_t)out.num_nodes), "cudaMalloc (wide nodes)");
-    Check(cudaMemcpyAsync(exact, nodes, sizeof(WideNode) * (size_t)out.num_nodes, cudaMemcpyDeviceToDevice, s),
+    keep(&out.d_nodes, sizeof(WideNode) * (size_t)out.num_nodes, "wide nodes");
+    Check(cudaMemcpyAsync(out.d_nodes, nodes, sizeof(WideNode) * (size_t)out.num_nodes, cudaMemcpyDeviceToDevice, s),
           "node copy");
     Check(cudaStreamSynchronize(s), "node copy");
-    out.d_nodes = exact;
     out.collapse_ms = Ms(t1);
+}
+
+cudaError_t CreateGpuBuildResources(int device, GpuBuildResources& r) {
+    cudaError_t e = cudaSuccess;
+    if (!r.pool) {
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = device;
+        e = cudaMemPoolCreate(&r.pool, &props);
+        if (e != cudaSuccess) return e;
+        uint64_t bytes = kGpuBuildPoolKeep;
+        e = cudaMemPoolSetAttribute(r.pool, cudaMemPoolAttrReleaseThreshold, &bytes);
+        if (e != cudaSuccess) return e;
+    }
+    if (!r.pinned) {
+        e = cudaHostAlloc(reinterpret_cast<void**>(&r.pinned), 4 * kGpuBuildPinnedWords, cudaHostAllocDefault);
+        if (e != cudaSuccess) return e;
+    }
+    for (cudaEvent_t& ev : r.ev)
+        if (!ev && e == cudaSuccess) e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+    return e;
+}
+
+void FreeGpuBuildResources(GpuBuildResources& r) {
+    for (cudaEvent_t ev : r.ev)
+        if (ev) cudaEventDestroy(ev);
+    if (r.pinned) cudaFreeHost(r.pinned);
+    if (r.pool) cudaMemPoolDestroy(r.pool);
+    r = GpuBuildResources{};
 }
 
 cudaError_t InstanceShade(const float* d_inv, const uint32_t* d_prefix, const uint32_t* d_prim_offset,

@@ -160,10 +160,11 @@ void UploadGpuBuilt(fnd_rt_ctx* ctx, fnd_rt_scene* scene, const float* verts, ui
                     uint32_t cluster_radius) {
     void *d_verts = nullptr, *d_idx = nullptr;
     RT::GpuBuildOutput go;
+    CUDA_CHECK(RT::CreateGpuBuildResources(ctx->device, ctx->build));
     try {
         const auto t0 = std::chrono::steady_clock::now();
-        CUDA_CHECK(cudaMalloc(&d_verts, 12ull * std::max(nv, 1u)));
-        CUDA_CHECK(cudaMalloc(&d_idx, 12ull * nt));
+        CUDA_CHECK(cudaMallocFromPoolAsync(&d_verts, 12ull * std::max(nv, 1u), ctx->build.pool, ctx->stream));
+        CUDA_CHECK(cudaMallocFromPoolAsync(&d_idx, 12ull * nt, ctx->build.pool, ctx->stream));
         if (nv) CUDA_CHECK(cudaMemcpyAsync(d_verts, verts, 12ull * nv, cudaMemcpyHostToDevice, ctx->stream));
         CUDA_CHECK(cudaMemcpyAsync(d_idx, idx, 12ull * nt, cudaMemcpyHostToDevice, ctx->stream));
         CUDA_CHECK(cudaStreamSynchronize(ctx->stream));
@@ -176,11 +177,13 @@ void UploadGpuBuilt(fnd_rt_ctx* ctx, fnd_rt_scene* scene, const float* verts, ui
         gp.c_tri = (float)copt.c_tri;
         gp.ploc_radius = cluster_radius;
         gp.width = copt.width;
-        RT::BuildWideGpu(static_cast<const float*>(d_verts), nv, static_cast<const uint32_t*>(d_idx), nt, gp, go,
-                         ctx->stream);
-        CUDA_CHECK(cudaFree(d_verts));
-        CUDA_CHECK(cudaFree(d_idx));
-        d_verts = d_idx = nullptr;
+        RT::BuildWideGpu(static_cast<const float*>(d_verts), nv, static_cast<const uint32_t*>(d_idx), nt, gp,
+                         ctx->build, go, ctx->stream);
+        CUDA_CHECK(cudaFreeAsync(d_verts, ctx->stream));
+        d_verts = nullptr;
+        CUDA_CHECK(cudaFreeAsync(d_idx, ctx->stream));
+        d_idx = nullptr;
+        scene->pooled = true;
         scene->d_nodes = go.d_nodes;
         scene->d_tris = go.d_tris;
         scene->d_tri_shade = go.d_tri_shade;
@@ -206,8 +209,9 @@ void UploadGpuBuilt(fnd_rt_ctx* ctx, fnd_rt_scene* scene, const float* verts, ui
         I.upload_ms = upload_ms;
     } catch (...) {
         for (void* p : {go.d_nodes, go.d_tris, go.d_tri_shade, d_verts, d_idx, scene->d_nodes, scene->d_tris,
-                        scene->d_tri_shade, scene->d_materials})
-            if (p) cudaFree(p);
+                        scene->d_tri_shade})
+            if (p) cudaFreeAsync(p, ctx->stream);
+        if (scene->d_materials) cudaFree(scene->d_materials);
         scene->d_nodes = scene->d_tris = scene->d_tri_shade = scene->d_materials = nullptr;
         throw;
     }
@@ -290,6 +294,7 @@ int fnd_rt_destroy(fnd_rt_ctx* ctx) {
     if (ctx->d_fb) cudaFree(ctx->d_fb);
     if (ctx->d_rgb) cudaFree(ctx->d_rgb);
     if (ctx->d_sort) cudaFree(ctx->d_sort);
+    RT::FreeGpuBuildResources(ctx->build);
     if (ctx->h_status) cudaFreeHost(ctx->h_status);
     for (cudaEvent_t e : ctx->pipe_ev)
         if (e) cudaEventDestroy(e);
@@ -518,9 +523,12 @@ int fnd_rt_scene_destroy(fnd_rt_scene* scene) {
         for (fnd_rt_scene* b : scene->blas) b->users--;
         scene->blas.clear();
         if (scene->d_instances) CUDA_CHECK(cudaFree(scene->d_instances));
-        if (scene->d_nodes) CUDA_CHECK(cudaFree(scene->d_nodes));
-        if (scene->d_tris) CUDA_CHECK(cudaFree(scene->d_tris));
-        if (scene->d_tri_shade) CUDA_CHECK(cudaFree(scene->d_tri_shade));
+        // the pool takes its arrays back in stream order; the training stream
+        // may still read them (cudaFree waits for the device by itself)
+        if (scene->pooled && ctx->cache && ctx->cache->train_stream)
+            CUDA_CHECK(cudaStreamSynchronize(ctx->cache->train_stream));
+        for (void* p : {scene->d_nodes, scene->d_tris, scene->d_tri_shade})
+            if (p) CUDA_CHECK(scene->pooled ? cudaFreeAsync(p, ctx->stream) : cudaFree(p));
         if (scene->d_materials) CUDA_CHECK(cudaFree(scene->d_materials));
         if (scene->d_lights) CUDA_CHECK(cudaFree(scene->d_lights));
     });

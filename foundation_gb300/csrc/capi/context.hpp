@@ -8,6 +8,7 @@
 #include <string>
 
 #include "../../../include/fnd_rt.h"
+#include "../bvh/gpu_build.hpp"
 #include "../core/core.hpp"
 #include "../pt/integrator.hpp"
 #include "../rt/ray_sort.hpp"
@@ -57,6 +58,7 @@ struct fnd_rt_ctx {
     cudaStream_t copy_in = nullptr, copy_out = nullptr, compute2 = nullptr;
     cudaEvent_t pipe_ev[2 + 2 * 17] = {};
     int live_scenes = 0;
+    Foundation::RT::GpuBuildResources build;  // created by the first FND_BVH_GPU_BUILD upload
     Foundation::RT::TraceConfig trace_cfg{};  // launch shape of the traversal kernels
     // path-tracing state: path buffers (capacity paths) and the frame buffer
     Foundation::PT::PathBuffers paths{};
@@ -81,6 +83,7 @@ struct fnd_rt_scene {
     fnd_rt_ctx* ctx = nullptr;
     void* d_nodes = nullptr;
     void* d_tris = nullptr;
+    bool pooled = false;  // d_nodes, d_tris and d_tri_shade come from the context's build pool
     Foundation::RT::DeviceScene view{};
     fnd_rt_scene_info info{};
     // shading data (original triangle order)

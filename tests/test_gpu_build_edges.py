@@ -58,3 +58,30 @@ def test_equal_codes(ctx):
     h, want = s.closest(rays), O.OracleBVH(v.reshape(-1, 3), idx).closest(rays)
     assert np.array_equal(h["prim"], want["prim"]) and np.array_equal(h["t"].view(np.uint32), want["t"].view(np.uint32))
     s.close()
+
+
+def test_pool_reuse_and_return(built):
+    """Builds share a context's pool: a live scene keeps its arrays while others
+    come and go (also while the cache trains on one), and closing the context
+    gives the memory back."""
+    import torch
+    import foundation_gb300 as fg
+    torch.cuda.synchronize()
+    a, b = S.soup_scene(40000, seed=1), S.soup_scene(150000, seed=2)
+    rays = S.incoherent_rays(2000, (0, 0, 0), (1, 1, 1), seed=4)
+    want = O.OracleBVH(a.verts, a.idx).closest(rays)
+    free = []
+    for _ in range(2):  # the first pass also pays for what the process keeps (modules, local memory)
+        with fg.Context(0) as c:
+            keep = c.upload(a.verts, a.idx, gpu_build=True, cluster=True, sah_collapse=True)
+            for k in range(3):
+                other = c.upload(b.verts, b.idx, gpu_build=True, cluster=bool(k & 1), sah_collapse=True)
+                if k == 1:
+                    c.cache_create(other, train_paths=2000, train_steps=1, batch=512)
+                    cam = dict(eye=(0.5, 0.5, 2.5), target=(0.5, 0.5, 0.5))
+                    c.render(other, 64, 64, 1, cam, cache=True, train_only=True, sky=(1.0, 1.0, 1.0))
+                other.close()
+                h = keep.closest(rays)
+                assert np.array_equal(h["prim"], want["prim"]) and np.array_equal(h["t"], want["t"])
+        free.append(torch.cuda.mem_get_info()[0])
+    assert free[0] - free[1] < 16 << 20
