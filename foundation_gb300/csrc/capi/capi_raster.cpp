@@ -98,7 +98,7 @@ int fnd_rt_raster_draw(fnd_rt_ctx* ctx, const fnd_raster_desc* desc, const fnd_r
         const size_t vb = sizeof(fnd_raster_vertex) * nv, ib = 2ull * ni, tb = 4ull * tex_w * tex_h;
         const size_t npix = (size_t)desc->width * desc->height;
         const size_t off_i = (vb + 255) & ~size_t(255), off_t = (off_i + ib + 255) & ~size_t(255);
-        const size_t off_c = (off_t + tb + 255) & ~size_t(255), off_s = off_c + 32ull * nv;
+        const size_t off_c = (off_t + tb + 255) & ~size_t(255), off_s = (off_c + Raster::TriBytes(ni / 3) + 255) & ~size_t(255);
         const size_t off_o = (off_s + 256 + 255) & ~size_t(255);
         const size_t total = off_o + (mem == FND_MEM_HOST ? 4 * npix : 0);
         CApi::EnsureDevice(ctx->d_in, ctx->d_in_cap, total);
@@ -113,7 +113,11 @@ int fnd_rt_raster_draw(fnd_rt_ctx* ctx, const fnd_raster_desc* desc, const fnd_r
         std::memcpy(A.u.model, desc->model, 64);
         std::memcpy(A.u.view, desc->view, 64);
         std::memcpy(A.u.proj, desc->proj, 64);
-        std::memcpy(A.clear, desc->clear, 16);
+        for (int c = 0; c < 4; ++c) {  // round(clamp(c, 0, 1) * 255), as the pixels
+            double v = desc->clear[c];
+            v = v < 0.0 ? 0.0 : (v > 1.0 ? 1.0 : v);
+            A.clear_rgba |= (v == v ? (uint32_t)std::floor(v * 255.0 + 0.5) : 0u) << (8 * c);
+        }
         A.cull_back = desc->cull_back;
         A.verts = reinterpret_cast<const Raster::Vertex*>(base);
         A.nv = nv;
@@ -122,7 +126,7 @@ int fnd_rt_raster_draw(fnd_rt_ctx* ctx, const fnd_raster_desc* desc, const fnd_r
         A.texture = reinterpret_cast<const uint32_t*>(base + off_t);
         A.tex_w = tex_w;
         A.tex_h = tex_h;
-        A.clip = reinterpret_cast<double4*>(base + off_c);
+        A.tris = base + off_c;
         A.status = reinterpret_cast<uint32_t*>(base + off_s);
         A.target = mem == FND_MEM_HOST ? reinterpret_cast<uint32_t*>(base + off_o) : reinterpret_cast<uint32_t*>(rgba);
         CUDA_CHECK(Raster::LaunchDraw(A, ctx->stream));

@@ -30,7 +30,7 @@ struct Uniforms {
 struct DrawArgs {
     uint32_t width, height;
     Uniforms u;
-    float clear[4];
+    uint32_t clear_rgba;      // the encoded clear colour
     uint32_t cull_back;
     const Vertex* verts;
     uint32_t nv;
@@ -39,10 +39,11 @@ struct DrawArgs {
     const uint32_t* texture;  // RGBA8 texels, row-major
     uint32_t tex_w, tex_h;
     uint32_t* target;         // RGBA8 pixels, row-major from the top row
-    double4* clip;            // scratch: nv clip-space positions
+    void* tris;               // scratch: TriBytes(ntri), 16-byte aligned
     uint32_t* status;
 };
 
+size_t TriBytes(uint32_t ntri);
 cudaError_t LaunchDraw(const DrawArgs& a, cudaStream_t s);
 
 }  // namespace Raster
