@@ -143,22 +143,10 @@ __device__ __forceinline__ void fma_dir_f2(F2 a, F2 b, F2 c, float out[2]) {
 #endif
 }
 
-// Two quantised planes as floats 1024 + q, exactly: one PRMT builds the
-// half2 (0x64 | q) pair (a half with exponent 2^10 and q in its low mantissa
-// bits), and the two halves widen to float off the integer pipe. sel picks
-// the byte pair: 0x4140 for bytes 0 and 1, 0x4342 for bytes 2 and 3.
-__device__ __forceinline__ void plane_pair(uint32_t word, uint32_t sel, float& a, float& b) {
-#if defined(__CUDA_ARCH__)
-    const uint32_t h2 = __byte_perm(word, 0x64u, sel);
-    __half2 h;
-    memcpy(&h, &h2, sizeof(h));
-    a = __low2float(h);
-    b = __high2float(h);
-#else
-    const uint32_t k = (sel & 0xFu) * 8u;
-    a = 1024.0f + (float)((word >> k) & 0xFFu);
-    b = 1024.0f + (float)((word >> (k + 8u)) & 0xFFu);
-#endif
+// A quantised plane (byte k of word) as the float 1 + q 2^-15, exactly: one
+// PRMT puts the byte into bits 8..15 of 1.0f's mantissa.
+__device__ __forceinline__ float plane_value(uint32_t word, uint32_t k) {
+    return __uint_as_float(__byte_perm(word, 0x3F800000u, 0x7604u | k << 4));
 }
 
 // max / min of three (one instruction on the sm_100 family; NaN operands
@@ -214,9 +202,9 @@ __device__ __forceinline__ SlotHits intersect_slots(const RayState& r, const uin
     const uint4 w2 = __ldg(n + 2);
     const uint4 w3 = __ldg(n + 3);
     const uint4 w4 = __ldg(n + 4);
-    const float sx = __uint_as_float((w0.w & 0xFFu) << 23) * r.ix;
-    const float sy = __uint_as_float(((w0.w >> 8) & 0xFFu) << 23) * r.iy;
-    const float sz = __uint_as_float(((w0.w >> 16) & 0xFFu) << 23) * r.iz;
+    const float sx = __uint_as_float((w0.w & 0xFFu) << 23) * (32768.0f * r.ix);
+    const float sy = __uint_as_float(((w0.w >> 8) & 0xFFu) << 23) * (32768.0f * r.iy);
+    const float sz = __uint_as_float(((w0.w >> 16) & 0xFFu) << 23) * (32768.0f * r.iz);
     const float bx = (__uint_as_float(w0.x) - r.ox) * r.ix;
     const float by = (__uint_as_float(w0.y) - r.oy) * r.iy;
     const float bz = (__uint_as_float(w0.z) - r.oz) * r.iz;
@@ -230,10 +218,10 @@ __device__ __forceinline__ SlotHits intersect_slots(const RayState& r, const uin
     const uint32_t nz0 = fz ? w4.z : w3.x, nz1 = fz ? w4.w : w3.y;
     const uint32_t gz0 = fz ? w3.x : w4.z, gz1 = fz ? w3.y : w4.w;
     // A plane's t is q * s + b with q the quantised byte. The byte is read
-    // as the float 1024 + q (plane_pair) and the 1024 * s is folded into the
-    // offset, near planes rounded down and far planes up:
-    //   near: rd((1024+q) s + rd(b - 1024 s)) <= rd(q s + b) <= rn(q s + b)
-    //   far:  ru((1024+q) s + ru(b - 1024 s)) >= ru(q s + b) >= rn(q s + b)
+    // as the float v = 1 + q 2^-15 (plane_value) and the step taken as
+    // S = 2^15 s (exact), near planes rounded down and far planes up:
+    //   near: rd(v S + rd(b - S)) <= rd(q s + b) <= rn(q s + b)
+    //   far:  ru(v S + ru(b - S)) >= ru(q s + b) >= rn(q s + b)
     // so every child box is at least as wide as under round-to-nearest
     // fma(q, s, b), the culling stays conservative and the hits exact.
     // A slot's near and far plane go through one packed FMA, the far one
@@ -242,22 +230,25 @@ __device__ __forceinline__ SlotHits intersect_slots(const RayState& r, const uin
     // constants duplicated for slot pairs, which at the persistent kernels'
     // 56 registers cost about 60 register moves per node).
     const F2 sx2 = pack_f2(sx, -sx), sy2 = pack_f2(sy, -sy), sz2 = pack_f2(sz, -sz);
-    const F2 bx2 = pack_f2(__fmaf_rd(-1024.0f, sx, bx), __fmaf_rd(1024.0f, sx, -bx));
-    const F2 by2 = pack_f2(__fmaf_rd(-1024.0f, sy, by), __fmaf_rd(1024.0f, sy, -by));
-    const F2 bz2 = pack_f2(__fmaf_rd(-1024.0f, sz, bz), __fmaf_rd(1024.0f, sz, -bz));
+    const F2 bx2 = pack_f2(__fmaf_rd(-1.0f, sx, bx), __fmaf_rd(1.0f, sx, -bx));
+    const F2 by2 = pack_f2(__fmaf_rd(-1.0f, sy, by), __fmaf_rd(1.0f, sy, -by));
+    const F2 bz2 = pack_f2(__fmaf_rd(-1.0f, sz, bz), __fmaf_rd(1.0f, sz, -bz));
     // the boxes alone: bit s of miss for slot s (empty slots included)
     const float ntfar = -tfar;
     uint32_t miss = 0;
 #pragma unroll
     for (int pr = 3; pr >= 0; --pr) {
-        const uint32_t sel = (pr & 1) ? 0x4342u : 0x4140u;
+        const uint32_t k = 2u * (pr & 1);
         float nx[2], ny[2], nz[2], gx[2], gy[2], gz[2];
-        plane_pair(pr < 2 ? nx0 : nx1, sel, nx[0], nx[1]);
-        plane_pair(pr < 2 ? gx0 : gx1, sel, gx[0], gx[1]);
-        plane_pair(pr < 2 ? ny0 : ny1, sel, ny[0], ny[1]);
-        plane_pair(pr < 2 ? gy0 : gy1, sel, gy[0], gy[1]);
-        plane_pair(pr < 2 ? nz0 : nz1, sel, nz[0], nz[1]);
-        plane_pair(pr < 2 ? gz0 : gz1, sel, gz[0], gz[1]);
+#pragma unroll
+        for (uint32_t e = 0; e < 2; ++e) {
+            nx[e] = plane_value(pr < 2 ? nx0 : nx1, k + e);
+            gx[e] = plane_value(pr < 2 ? gx0 : gx1, k + e);
+            ny[e] = plane_value(pr < 2 ? ny0 : ny1, k + e);
+            gy[e] = plane_value(pr < 2 ? gy0 : gy1, k + e);
+            nz[e] = plane_value(pr < 2 ? nz0 : nz1, k + e);
+            gz[e] = plane_value(pr < 2 ? gz0 : gz1, k + e);
+        }
 #pragma unroll
         for (int e = 1; e >= 0; --e) {
             float tx[2], ty[2], tz[2];  // near t, -(far t)
