@@ -32,6 +32,7 @@
 // registers a thread and 32 warps per SM: at 56 registers (36 warps) the loop
 // spills about ten words a node step (8.4M incoherent Cornell rays 1.92 ms
 // against 1.77), at 72 (28 warps) it lacks warps (1.81 ms).
+#include <algorithm>
 #include <cfloat>
 
 #include "traverse.cuh"
@@ -54,6 +55,7 @@ struct Common {
     uint32_t* status;
     unsigned long long* stats;
     uint32_t refill_min;
+    uint32_t lanes;     // kFew: lanes of a warp that take rays
     uint32_t wait_min;  // flush the ring once this many lanes only wait for their pairs
 };
 
@@ -270,14 +272,16 @@ __device__ __forceinline__ const float4* lds_ptr(uint32_t a) {
 // source is an InstancedSource (triangle leaves of the top level are
 // instances; per-lane node / triangle arrays). w: this warp's region of
 // shared memory, tab: the tables of fill_tables. kPlanes: the scene's
-// triangles are three planes (tri_stride 1), not records.
+// triangles are three planes (tri_stride 1), not records. kFew: only the first
+// C.lanes lanes of a warp take rays (LanesPerWarp); compiled apart, because the
+// three values it keeps cost the full kernels 1-3%.
 //
 // A node group is one word: the internal children still to visit in bits
 // 24..31, the highest bit first (bit 24 + j is slot j ^ 7 ^ oct, so the
 // highest bit is the nearest along the ray's octant), and the node's imask
 // in bits 0..7.
 template <class Src, int kKind, bool kStats, int kShort, bool kTwoLevel = false, bool kMulti = false,
-          bool kPlanes = false>
+          bool kPlanes = false, bool kFew = false>
 __device__ __forceinline__ void persistent_trace(const Src& src, const Common& C, uint32_t w, uint32_t tab,
                                                  float4* s_world = nullptr) {
     using W = WarpShared<kShort, kMulti>;
@@ -353,9 +357,12 @@ __device__ __forceinline__ void persistent_trace(const Src& src, const Common& C
         // no rays are left, all).
         const bool work = ng_group >= (1u << 24) && (!kTwoLevel || tl_mask == 0u);
         const uint32_t working = __ballot_sync(kFull, work);
-        const uint32_t ready = __ballot_sync(kFull, !work && (!kTwoLevel || tl_mask == 0u) && (int)(my_end - head) <= 0);
-        if (ready == kFull || (!exhausted && (uint32_t)__popc(ready) >= C.refill_min)) {
-            const bool mine = !work && (!kTwoLevel || tl_mask == 0u) && (int)(my_end - head) <= 0;
+        const uint32_t holders = kFew ? kFull >> (32u - C.lanes) : kFull;
+        const uint32_t ready =
+            __ballot_sync(kFull, !work && (!kTwoLevel || tl_mask == 0u) && (int)(my_end - head) <= 0) & holders;
+        if (ready == holders || (!exhausted && (uint32_t)__popc(ready) >= C.refill_min)) {
+            const bool mine = !work && (!kTwoLevel || tl_mask == 0u) && (int)(my_end - head) <= 0 &&
+                              (!kFew || lane < C.lanes);
             if (mine && active) {
                 const uint2 bst = lds64(wl + W::kBest);
                 src.store(ray_id, ln, any_hit, bst.y, __uint_as_float(bst.x));
@@ -496,7 +503,7 @@ __device__ __forceinline__ void persistent_trace(const Src& src, const Common& C
         // ---- rounds: whenever 32 triangles wait, and all of them when several
         // lanes only wait for theirs or no lane can go on ---------------------
         // (two-level: after every step, as a lane's slot changes with its instance)
-        const bool flush = kTwoLevel || working == 0u || 32u - (uint32_t)__popc(working | ready) >= C.wait_min;
+        const bool flush = kTwoLevel || working == 0u || (kFew ? C.lanes : 32u) - (uint32_t)__popc(working | ready) >= C.wait_min;
         for (;;) {
             if (fresh) {
                 // ranges [head, head + kRing) are written; more as rounds make room
@@ -638,11 +645,30 @@ __device__ __forceinline__ void fill_tables(uint8_t* t) {
     __syncthreads();
 }
 
-template <bool kAny, bool kStats, int kShort, int kBlock, bool kPlanes = false>
+// Lanes of a warp that take rays, for n rays on a grid of `warps` warps. The
+// time of a small batch is the latency of its longest rays, and a warp's
+// triangle rounds serve all its rays in turn, so a batch finishes sooner on
+// few lanes of many warps: a quarter of what the warps could hold is the
+// balance between that and warps in each other's way. us per pass with 32
+// lanes, this rule, and a sixteenth: 1,000 incoherent rays on the sphere scene
+// 368, 163, 151; 4,000 385, 218, 214; 10,000 398, 254, 286; on the 1M soup
+// 167, 112, 109 and 204, 156, 174. Not below two: short rays gain from a
+// neighbour's warm cache (300 segments on Cornell 37 us, 37, 40 with one lane).
+uint32_t LanesPerWarp(uint32_t n, uint32_t warps) {
+    const uint64_t l = (4ull * n + warps - 1) / (warps ? warps : 1u);
+    return l >= 32 ? 32u : l < 2 ? 2u : (uint32_t)l;
+}
+// Blocks for n rays: no more than have rays to take.
+int SmallGrid(uint32_t n, int grid, int block, uint32_t lanes) {
+    const uint64_t per_block = (uint64_t)lanes * ((uint32_t)block / 32u);
+    const uint64_t need = ((uint64_t)n + per_block - 1) / per_block;
+    return need < (uint64_t)grid ? (int)(need > 0 ? need : 1) : grid;
+}
+
+template <bool kAny, bool kStats, int kShort, int kBlock, bool kPlanes = false, bool kFew = false>
 __global__ void __launch_bounds__(kBlock, MinBlocks(kBlock)) trace_kernel(const TraceLaunch L) {
     using W = WarpShared<kShort, false>;
     __shared__ __align__(16) uint8_t s_mem[kTableBytes + W::kBytes * (kBlock / 32)];
-    fill_tables(s_mem);
     SingleSource src;
     src.scene = L.scene;
     src.rays = L.rays;
@@ -650,9 +676,11 @@ __global__ void __launch_bounds__(kBlock, MinBlocks(kBlock)) trace_kernel(const 
     src.occluded = L.occluded;
     src.order = L.order;
     src.n = L.n_dev ? min(*L.n_dev, L.n) : L.n;
+    if (src.n == 0) return;  // an empty queue of the path tracer
     if (L.ray_total && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(L.ray_total, (unsigned long long)src.n);
-    const Common C{L.counter, L.status, L.stats, L.refill_min, L.postpone_min ? L.postpone_min : kWaitMin};
-    persistent_trace<SingleSource, kAny ? 1 : 0, kStats, kShort, false, false, kPlanes>(
+    fill_tables(s_mem);
+    const Common C{L.counter, L.status, L.stats, L.refill_min, L.lanes, L.postpone_min ? L.postpone_min : kWaitMin};
+    persistent_trace<SingleSource, kAny ? 1 : 0, kStats, kShort, false, false, kPlanes, kFew>(
         src, C, shared_addr(s_mem + kTableBytes + W::kBytes * (threadIdx.x >> 5)), shared_addr(s_mem));
 }
 
@@ -666,12 +694,12 @@ __global__ void __launch_bounds__(kBlock, MinBlocks(kBlock)) batch_kernel(const 
     src.prefix = B.prefix;
     src.njobs = B.njobs;
     src.n = B.total;
-    const Common C{B.counter, B.status, nullptr, B.refill_min, B.postpone_min ? B.postpone_min : kWaitMin};
+    const Common C{B.counter, B.status, nullptr, B.refill_min, 32u, B.postpone_min ? B.postpone_min : kWaitMin};
     persistent_trace<BatchSource, 2, false, kShort, false, true>(
         src, C, shared_addr(s_mem + kTableBytes + W::kBytes * (threadIdx.x >> 5)), shared_addr(s_mem));
 }
 
-template <bool kAny>
+template <bool kAny, bool kFew>
 __global__ void __launch_bounds__(128, 8) instanced_trace_kernel(const InstancedLaunch L) {
     using W = WarpShared<8, true>;
     __shared__ __align__(16) uint8_t s_mem[W::kBytes * 4];
@@ -685,8 +713,8 @@ __global__ void __launch_bounds__(128, 8) instanced_trace_kernel(const Instanced
     src.occluded = L.occluded;
     src.n = L.n_dev ? min(*L.n_dev, L.n) : L.n;
     if (L.ray_total && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(L.ray_total, (unsigned long long)src.n);
-    const Common C{L.counter, L.status, nullptr, 8u, kWaitMin};
-    persistent_trace<InstancedSource, kAny ? 1 : 0, false, 8, true, true>(
+    const Common C{L.counter, L.status, nullptr, kFew ? min(8u, L.lanes) : 8u, L.lanes, kWaitMin};
+    persistent_trace<InstancedSource, kAny ? 1 : 0, false, 8, true, true, false, kFew>(
         src, C, shared_addr(s_mem + W::kBytes * (threadIdx.x >> 5)), 0u, s_world);
 }
 
@@ -771,6 +799,17 @@ cudaError_t LaunchTraceConfigured(const TraceLaunch& L, bool any, bool stats, co
     TraceLaunch arg = L;
     arg.refill_min = c.refill_min ? c.refill_min : L.refill_min;
     arg.postpone_min = c.postpone_min;
+    arg.lanes = 32;  // (a device queue's length is not known here)
+    if (!L.n_dev && !stats) {
+        arg.lanes = LanesPerWarp(L.n, (uint32_t)(grid * (block / 32)));
+        if (arg.lanes < 32 && L.scene.tri_stride != 1) {  // a small batch: the default shape on few lanes
+            block = 128;
+            fn = any ? reinterpret_cast<const void*>(&trace_kernel<true, false, 8, 128, false, true>)
+                     : reinterpret_cast<const void*>(&trace_kernel<false, false, 8, 128, false, true>);
+            grid = SmallGrid(L.n, grid, block, arg.lanes);
+            arg.refill_min = std::min(arg.refill_min, arg.lanes);
+        }
+    }
     void* params[] = {&arg};
     return cudaLaunchKernel(fn, dim3(grid), dim3(block), params, 0, stream);
 }
@@ -785,14 +824,24 @@ cudaError_t LaunchInstanced(const InstancedLaunch& L, bool any, int sm_count, cu
     if (L.n == 0) return cudaSuccess;
     cudaError_t e = cudaMemsetAsync(L.counter, 0, sizeof(uint32_t), stream);
     if (e != cudaSuccess) return e;
-    const void* fn = any ? reinterpret_cast<const void*>(&instanced_trace_kernel<true>)
-                         : reinterpret_cast<const void*>(&instanced_trace_kernel<false>);
+    const void* fn = any ? reinterpret_cast<const void*>(&instanced_trace_kernel<true, false>)
+                         : reinterpret_cast<const void*>(&instanced_trace_kernel<false, false>);
     int blocks = 0;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, fn, 128, 0);
     if (e != cudaSuccess) return e;
     InstancedLaunch arg = L;
+    int grid = sm_count * (blocks > 0 ? blocks : 1);
+    arg.lanes = 32;
+    if (!L.n_dev) {
+        arg.lanes = LanesPerWarp(L.n, (uint32_t)(4 * grid));
+        if (arg.lanes < 32) {
+            fn = any ? reinterpret_cast<const void*>(&instanced_trace_kernel<true, true>)
+                     : reinterpret_cast<const void*>(&instanced_trace_kernel<false, true>);
+            grid = SmallGrid(L.n, grid, 128, arg.lanes);
+        }
+    }
     void* params[] = {&arg};
-    return cudaLaunchKernel(fn, dim3(sm_count * (blocks > 0 ? blocks : 1)), dim3(128), params, 0, stream);
+    return cudaLaunchKernel(fn, dim3(grid), dim3(128), params, 0, stream);
 }
 
 cudaError_t LaunchBatch(const BatchLaunch& B, const TraceConfig& c, int grid, cudaStream_t stream) {
@@ -802,8 +851,10 @@ cudaError_t LaunchBatch(const BatchLaunch& B, const TraceConfig& c, int grid, cu
     BatchLaunch arg = B;
     arg.refill_min = c.refill_min ? c.refill_min : B.refill_min;
     arg.postpone_min = c.postpone_min;
+    const int block = normalized_block(c.block);
+    grid = SmallGrid(B.total, grid, block, 32);
     void* params[] = {&arg};
-    return cudaLaunchKernel(select_batch(c), dim3(grid), dim3(normalized_block(c.block)), params, 0, stream);
+    return cudaLaunchKernel(select_batch(c), dim3(grid), dim3(block), params, 0, stream);
 }
 
 }  // namespace RT

@@ -60,3 +60,22 @@ def test_ring_matches_oracle(ctx, kind, n):
                 assert np.array_equal(scene.any(rays), want_any)
         scene.close()
     ctx.set_trace_config()
+
+
+@pytest.mark.parametrize("n", [2, 63, 300, 1217, 2433, 4865, 30000, 38911, 38913])
+def test_small_batches(ctx, n):
+    """Batches on few lanes per warp, around the sizes where the lane count and
+    the grid change (1,216 blocks of four warps on the full chip), one- and
+    two-level."""
+    sc, rays = _geometry("soup"), _rays(n)
+    b = O.OracleBVH(sc.verts, sc.idx)
+    want, want_any = b.closest(rays), b.any(rays)
+    scene = ctx.upload(sc.verts, sc.idx)
+    two = ctx.instances([(scene, np.eye(3, 4, dtype=np.float32), 0)])
+    for s in (scene, two):
+        h = s.closest(rays)
+        assert np.array_equal(h["prim"], want["prim"])
+        assert np.array_equal(h["t"].view(np.uint32), want["t"].view(np.uint32))
+        assert np.array_equal(s.any(rays), want_any)
+    two.close()
+    scene.close()
