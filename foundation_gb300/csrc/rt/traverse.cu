@@ -9,7 +9,9 @@
 //    the new rays to its idle lanes (dynamic fetch: a warp refills once at
 //    least `refill_min` lanes are idle, so long rays do not hold 31 idle
 //    lanes hostage);
-//  * one thread per ray; the traversal state is a "node group" (base index of
+//  * one thread per ray while rays are left to fetch (then, and in small
+//    batches, lanes without work share the others' rays: persistent_trace);
+//    the traversal state is a "node group" (base index of
 //    a node's internal children + the ordered bit mask of children still to
 //    visit), the triangles of hit leaves wait in a ring of the warp (below);
 //  * a node's hit mask goes to the ray's traversal order through a shared
@@ -49,15 +51,40 @@ constexpr uint32_t kTriGroupFlag = 0x80000000u;
 // Lanes that only wait for their triangles before a part-filled round runs. Any
 // value from 2 to 16 is within 1% on incoherent and camera rays; 1 costs 1%.
 constexpr uint32_t kWaitMin = 4;
+// With no rays left to fetch, a warp turns to helping once at most this many of
+// its lanes have work (8.4M / 1M rays on Cornell: 0 (never) 1.70 ms / 263 us,
+// 16 1.66 / 237, 28 1.65 / 237).
+constexpr uint32_t kHelpAt = 28;
 
 struct Common {
     uint32_t* counter;
     uint32_t* status;
     unsigned long long* stats;
     uint32_t refill_min;
-    uint32_t lanes;     // kFew: lanes of a warp that take rays
+    uint32_t few_rays, full_warps;  // (see persistent_trace)
     uint32_t wait_min;  // flush the ring once this many lanes only wait for their pairs
 };
+
+// Lanes of a warp that take rays, for n rays on a grid of `warps` warps. The
+// time of a small batch is the latency of its longest rays, and a warp's
+// triangle rounds serve all its rays in turn, so a batch finishes sooner on
+// few lanes of many warps, where the others help (persistent_trace). Twice the
+// lanes that an even spread asks for, so that warps with short rays fetch more. us per pass, 32 lanes without
+// helping / this rule: 1,000 incoherent rays on the sphere scene 368 / 65, on
+// the 1M soup 167 / 59; 10,000 398 / 111 and 204 / 82; 30,000 417 / 220 and
+// 199 / 145. Factors 8, 4, 2 and 1 in place of two: 10,000 rays 234, 154, 111,
+// 99 on the spheres, 121, 98, 82, 80 on the soup; 30,000 on Cornell 46, 41, 39,
+// 46. Not below two lanes: short rays gain from a neighbour's warm cache (300
+// segments on Cornell 37 us, 40 with one lane).
+__host__ __device__ __forceinline__ uint32_t LanesPerWarp(uint32_t n, uint32_t warps) {
+    const uint64_t l = (2ull * n + warps - 1) / (warps ? warps : 1u);
+    return l >= 32 ? 32u : l < 2 ? 2u : (uint32_t)l;
+}
+// The largest batch for it (117 thousand rays on the full chip): there the two
+// loops of persistent_trace cross. 100,000 / 150,000 incoherent rays, second
+// loop alone against both: 556 / 671 us and 600 / 628 on the sphere scene, 276
+// / 332 and 281 / 292 on the 1M soup, 62 / 72 and 63 / 67 on Cornell.
+uint32_t FewRays(uint32_t warps) { return 24u * warps; }
 
 // ---- work sources -----------------------------------------------------------
 // One scene, one ray array, one query kind for the whole launch.
@@ -272,35 +299,49 @@ __device__ __forceinline__ const float4* lds_ptr(uint32_t a) {
 // source is an InstancedSource (triangle leaves of the top level are
 // instances; per-lane node / triangle arrays). w: this warp's region of
 // shared memory, tab: the tables of fill_tables. kPlanes: the scene's
-// triangles are three planes (tri_stride 1), not records. kFew: only the first
-// C.lanes lanes of a warp take rays (LanesPerWarp); compiled apart, because the
-// three values it keeps cost the full kernels 1-3%.
+// triangles are three planes (tri_stride 1), not records.
 //
 // A node group is one word: the internal children still to visit in bits
 // 24..31, the highest bit first (bit 24 + j is slot j ^ 7 ^ oct, so the
 // highest bit is the nearest along the ray's octant), and the node's imask
 // in bits 0..7.
-template <class Src, int kKind, bool kStats, int kShort, bool kTwoLevel = false, bool kMulti = false,
-          bool kPlanes = false, bool kFew = false>
-__device__ __forceinline__ void persistent_trace(const Src& src, const Common& C, uint32_t w, uint32_t tab,
-                                                 float4* s_world = nullptr) {
+// What the first loop hands to the second: a lane's traversal and its ray, and
+// whether rays are left. (The ring is empty there.)
+struct LaneState {
+    uint32_t ray_id, ng_base, ng_group;
+    float best_t;
+    int sp;
+    bool active, exhausted;
+};
+
+// Helping is not for two-level scenes (a lane's slot changes with its
+// instance), nor for scenes made by hand, whose depth no upload has checked:
+// sharing a stack would hide that it is too deep.
+template <bool kTwoLevel, bool kPlanes>
+constexpr bool kHelps = !kTwoLevel && !kPlanes;
+
+// One of the two loops of persistent_trace (kFew: the second). l_stack: the
+// lane's entries past the shared ones.
+template <class Src, int kKind, bool kStats, int kShort, bool kTwoLevel, bool kMulti, bool kPlanes, bool kFew>
+__device__ __forceinline__ void trace_loop(const Src& src, const Common& C, uint32_t w, uint32_t tab, float4* s_world,
+                                           LaneState& st, typename Src::Lane& lane_src, uint2* l_stack) {
     using W = WarpShared<kShort, kMulti>;
     // two-level: each lane's triangles and hit-id offset come from its own slot
     // (the lanes of a warp sit in different instances)
     static_assert(!kTwoLevel || kMulti, "two-level traversal needs per-lane scenes");
-    uint2 l_stack[kMaxStack - kShort];
     uint32_t lane, below;
     asm volatile("mov.u32 %0, %%laneid;" : "=r"(lane));
     asm volatile("mov.u32 %0, %%lanemask_lt;" : "=r"(below));
     const uint32_t wl = w + 8u * lane;  // the lane's 8-byte slots
     const uint32_t n = src.n;
 
-    bool active = false, exhausted = false, any_hit = kKind == 1;
-    uint32_t ray_id = 0;
-    typename Src::Lane ln{};
-    float best_t = 0.0f, tmin = 0.0f;
-    uint32_t ng_base = 0, ng_group = 0;
-    int sp = 0;
+    uint32_t slot = lane;  // kSteal: the lane whose ray this one follows
+    typename Src::Lane ln = lane_src;
+    bool active = st.active, exhausted = st.exhausted, any_hit = kKind == 1 || (kKind == 2 && st.active && src.any_of(ln, false));
+    uint32_t ray_id = st.ray_id;
+    float best_t = st.best_t, tmin = 0.0f;
+    uint32_t ng_base = st.ng_base, ng_group = st.ng_group;
+    int sp = st.sp;
     // the warp's ring: ranges head .. tail - 1 (modulo 2^32), with `tris` triangles written
     uint32_t head = 0, tail = 0, tris = 0;
     uint32_t my_end = 0;  // the ring position after this lane's last range
@@ -349,7 +390,16 @@ __device__ __forceinline__ void persistent_trace(const Src& src, const Common& C
             start(cur.num_nodes, lds32(wl + 8u * lane + W::kRayC + 12u));
         }
     };
-
+    const uint32_t lanes = kFew && n <= C.few_rays ? LanesPerWarp(n, C.full_warps) : 32u;
+    constexpr bool kHelp = kHelps<kTwoLevel, kPlanes>;
+    constexpr bool kSteal = kFew && kHelp;
+    // kSteal in a batch: the followed ray's scene (cur) and kind
+    constexpr bool kOwnScene = kSteal && kMulti;
+    bool follows_any = any_hit;
+    if constexpr (kOwnScene) {
+        cur = src.scene_of(ln);
+        follows_any = any_hit;
+    }
     for (;;) {
         // ---- finished rays out, new rays in ----------------------------------
         // ready: lanes without a ray, or with one whose traversal and ranges
@@ -357,12 +407,14 @@ __device__ __forceinline__ void persistent_trace(const Src& src, const Common& C
         // no rays are left, all).
         const bool work = ng_group >= (1u << 24) && (!kTwoLevel || tl_mask == 0u);
         const uint32_t working = __ballot_sync(kFull, work);
-        const uint32_t holders = kFew ? kFull >> (32u - C.lanes) : kFull;
-        const uint32_t ready =
-            __ballot_sync(kFull, !work && (!kTwoLevel || tl_mask == 0u) && (int)(my_end - head) <= 0) & holders;
-        if (ready == holders || (!exhausted && (uint32_t)__popc(ready) >= C.refill_min)) {
-            const bool mine = !work && (!kTwoLevel || tl_mask == 0u) && (int)(my_end - head) <= 0 &&
-                              (!kFew || lane < C.lanes);
+        const uint32_t holders = kFew ? kFull >> (32u - lanes) : kFull;
+        // kSteal (the ring is empty here): a ray is done when no lane follows it
+        const uint32_t followed = kSteal ? __reduce_or_sync(kFull, work ? 1u << slot : 0u) : 0u;
+        const bool done = !work && (kSteal ? !(followed >> lane & 1u)
+                                           : (!kTwoLevel || tl_mask == 0u) && (int)(my_end - head) <= 0);
+        const uint32_t ready = __ballot_sync(kFull, done) & holders;
+        if (ready == holders || (!exhausted && (uint32_t)__popc(ready) >= (kFew ? min(C.refill_min, lanes) : C.refill_min))) {
+            const bool mine = done && (!kFew || lane < lanes);
             if (mine && active) {
                 const uint2 bst = lds64(wl + W::kBest);
                 src.store(ray_id, ln, any_hit, bst.y, __uint_as_float(bst.x));
@@ -385,6 +437,11 @@ __device__ __forceinline__ void persistent_trace(const Src& src, const Common& C
                 if constexpr (kMulti) store_scene<kShort>(w, lane, src.scene_of(ln), 0u);
                 tmin = r.tmin;
                 ray_id = id;
+                slot = lane;
+                if constexpr (kOwnScene) {
+                    cur = src.scene_of(ln);
+                    follows_any = any_hit;
+                }
                 best_t = r.tmax;
                 sts64(wl + W::kBest, __float_as_uint(r.tmax), FND_INVALID_ID);
                 start(src.scene_of(ln).num_nodes, octx_of(r));
@@ -399,11 +456,46 @@ __device__ __forceinline__ void persistent_trace(const Src& src, const Common& C
             continue;
         }
 
+        if constexpr (kSteal) {
+            // the k-th lane without work takes the top of the k-th stack
+            const uint32_t from = __ballot_sync(kFull, sp > 0 && sp <= kShort);
+            const uint32_t idle = ~working;
+            if (from && idle) {
+                const uint32_t rank = (uint32_t)__popc(from & below);
+                const bool gives = (from >> lane & 1u) && rank < (uint32_t)__popc(idle);
+                if (gives) {
+                    sp--;
+                    sts32(w + 8u * rank + W::kWin, lane);
+                }
+                __syncwarp();
+                const uint32_t k = (uint32_t)__popc(idle & below);
+                const bool takes = !work && k < (uint32_t)__popc(from);
+                const uint32_t victim = takes ? lds32(w + 8u * k + W::kWin) : lane;
+                const uint32_t top = __shfl_sync(kFull, (uint32_t)sp, victim);
+                const uint32_t whose = __shfl_sync(kFull, slot, victim);
+                if constexpr (kOwnScene) {  // (lanes that take nothing read their own)
+                    cur.nodes = (const uint4*)__shfl_sync(kFull, (unsigned long long)cur.nodes, victim);
+                    cur.num_nodes = __shfl_sync(kFull, cur.num_nodes, victim);
+                    cur.num_tris = __shfl_sync(kFull, cur.num_tris, victim);
+                    follows_any = __shfl_sync(kFull, follows_any ? 1 : 0, victim) != 0;
+                }
+                if (takes) {
+                    const uint2 e = lds64(w + 8u * victim + W::kStack + 256u * top);
+                    ng_base = e.x;
+                    ng_group = e.y;
+                    slot = whose;
+                    best_t = __uint_as_float(lds32(w + 8u * slot + W::kBest));
+                }
+                __syncwarp();
+            }
+        }
+        const uint32_t ws = kSteal ? w + 8u * slot : wl;  // the slots of the followed ray
         // ---- one node --------------------------------------------------------
         uint32_t leaves = 0, tri_base = 0, meta0 = 0, meta1 = 0;
-        if (work) {
-            const DeviceScene& sc = kTwoLevel ? cur : src.scene_of(ln);
-            const float4 ra = lds128(wl + 8u * lane + W::kRayA), rc = lds128(wl + 8u * lane + W::kRayC);
+        if (kSteal ? ng_group >= (1u << 24) : work) {
+            const DeviceScene& sc = kTwoLevel || kOwnScene ? cur : src.scene_of(ln);
+            const uint32_t wr = kSteal ? w + 16u * slot : wl + 8u * lane;
+            const float4 ra = lds128(wr + W::kRayA), rc = lds128(wr + W::kRayC);
             const uint32_t octx = __float_as_uint(rc.w);
             const uint32_t b = 31u - (uint32_t)__clz(ng_group);
             ng_group &= ~(1u << b);
@@ -416,7 +508,7 @@ __device__ __forceinline__ void persistent_trace(const Src& src, const Common& C
                 r.ox = ra.x;
                 r.oy = ra.y;
                 r.oz = ra.z;
-                r.tmin = tmin;
+                r.tmin = kSteal ? ra.w : tmin;
                 r.ix = rc.x;
                 r.iy = rc.y;
                 r.iz = rc.z;
@@ -503,7 +595,9 @@ __device__ __forceinline__ void persistent_trace(const Src& src, const Common& C
         // ---- rounds: whenever 32 triangles wait, and all of them when several
         // lanes only wait for theirs or no lane can go on ---------------------
         // (two-level: after every step, as a lane's slot changes with its instance)
-        const bool flush = kTwoLevel || working == 0u || (kFew ? C.lanes : 32u) - (uint32_t)__popc(working | ready) >= C.wait_min;
+        // (few lanes: likewise, for the latency)
+        const bool leave = !kFew && kHelp && exhausted && (uint32_t)__popc(working) <= kHelpAt;
+        const bool flush = kTwoLevel || kFew || leave || working == 0u || 32u - (uint32_t)__popc(working | ready) >= C.wait_min;
         for (;;) {
             if (fresh) {
                 // ranges [head, head + kRing) are written; more as rounds make room
@@ -512,7 +606,7 @@ __device__ __forceinline__ void persistent_trace(const Src& src, const Common& C
                     const uint32_t s = 31u - (uint32_t)__clz(leaves);
                     leaves &= ~(1u << s);
                     // (meta byte, owner lane, 0, 0)
-                    const uint32_t y = __byte_perm(s < 4u ? meta0 : meta1, lane, 0x5540u | (s & 3u));
+                    const uint32_t y = __byte_perm(s < 4u ? meta0 : meta1, kSteal ? slot : lane, 0x5540u | (s & 3u));
                     sum += (y >> 5 & 3u) + 1u;
                     sts64(w + W::kRanges + 8u * (at & (kRing - 1u)), tri_base, y);
                     at++;
@@ -580,9 +674,9 @@ __device__ __forceinline__ void persistent_trace(const Src& src, const Common& C
                     }
                     __syncwarp();
                 } while (__ballot_sync(kFull, hit));
-                const uint2 bst = lds64(wl + W::kBest);
+                const uint2 bst = lds64(ws + W::kBest);
                 best_t = __uint_as_float(bst.x);
-                if ((kKind == 1 || (kKind == 2 && any_hit)) && active && bst.y != FND_INVALID_ID) {
+                if ((kKind == 1 || (kKind == 2 && (kSteal ? follows_any : any_hit))) && (kSteal || active) && bst.y != FND_INVALID_ID) {
                     ng_group = 0;  // found: only the ranges already in the ring remain
                     sp = 0;
                     if (kTwoLevel) tl_mask = 0;
@@ -618,6 +712,17 @@ __device__ __forceinline__ void persistent_trace(const Src& src, const Common& C
             ng_base = e.x;
             ng_group = e.y;
         }
+        if (leave) break;
+    }
+    if constexpr (kHelp && !kFew) {
+        st.ray_id = ray_id;
+        st.ng_base = ng_base;
+        st.ng_group = ng_group;
+        st.best_t = best_t;
+        st.sp = sp;
+        st.active = active;
+        st.exhausted = exhausted;
+        lane_src = ln;
     }
     if (kStats) {
         for (int o = 16; o > 0; o >>= 1) {
@@ -635,6 +740,34 @@ __device__ __forceinline__ void persistent_trace(const Src& src, const Common& C
     }
 }
 
+// The second loop as a call: its registers are its own, and the first loop is
+// compiled as if it were alone (inlined, the pair cost the first loop 3%).
+template <class Src, int kKind, bool kStats, int kShort, bool kTwoLevel, bool kMulti, bool kPlanes>
+__device__ __noinline__ void help_loop(const Src& src, const Common& C, uint32_t w, uint32_t tab, float4* s_world,
+                                       LaneState& st, typename Src::Lane& ln, uint2* l_stack) {
+    trace_loop<Src, kKind, kStats, kShort, kTwoLevel, kMulti, kPlanes, true>(src, C, w, tab, s_world, st, ln, l_stack);
+}
+
+// A batch of at most few_rays runs the second loop (kFew) only: few lanes of a
+// warp take rays (LanesPerWarp), and the others help. A larger one runs the
+// first until no rays are left to fetch and lanes have nothing to do, and hands
+// what is left to the second. Helping: a lane without work takes the top of
+// another's stack, so a ray is followed by several lanes that share its slot;
+// every step tests all its triangles, so the ring is empty whenever a lane
+// changes rays.
+template <class Src, int kKind, bool kStats, int kShort, bool kTwoLevel = false, bool kMulti = false,
+          bool kPlanes = false>
+__device__ __forceinline__ void persistent_trace(const Src& src, const Common& C, uint32_t w, uint32_t tab,
+                                                 float4* s_world = nullptr) {
+    uint2 l_stack[kMaxStack - kShort];
+    LaneState st{};
+    typename Src::Lane ln{};
+    if (src.n > C.few_rays)
+        trace_loop<Src, kKind, kStats, kShort, kTwoLevel, kMulti, kPlanes, false>(src, C, w, tab, s_world, st, ln, l_stack);
+    if (kHelps<kTwoLevel, kPlanes> || src.n <= C.few_rays)
+        help_loop<Src, kKind, kStats, kShort, kTwoLevel, kMulti, kPlanes>(src, C, w, tab, s_world, st, ln, l_stack);
+}
+
 // 32 resident warps per SM (64 registers a thread).
 constexpr int MinBlocks(int block) { return 1024 / block; }
 
@@ -645,19 +778,6 @@ __device__ __forceinline__ void fill_tables(uint8_t* t) {
     __syncthreads();
 }
 
-// Lanes of a warp that take rays, for n rays on a grid of `warps` warps. The
-// time of a small batch is the latency of its longest rays, and a warp's
-// triangle rounds serve all its rays in turn, so a batch finishes sooner on
-// few lanes of many warps: a quarter of what the warps could hold is the
-// balance between that and warps in each other's way. us per pass with 32
-// lanes, this rule, and a sixteenth: 1,000 incoherent rays on the sphere scene
-// 368, 163, 151; 4,000 385, 218, 214; 10,000 398, 254, 286; on the 1M soup
-// 167, 112, 109 and 204, 156, 174. Not below two: short rays gain from a
-// neighbour's warm cache (300 segments on Cornell 37 us, 37, 40 with one lane).
-uint32_t LanesPerWarp(uint32_t n, uint32_t warps) {
-    const uint64_t l = (4ull * n + warps - 1) / (warps ? warps : 1u);
-    return l >= 32 ? 32u : l < 2 ? 2u : (uint32_t)l;
-}
 // Blocks for n rays: no more than have rays to take.
 int SmallGrid(uint32_t n, int grid, int block, uint32_t lanes) {
     const uint64_t per_block = (uint64_t)lanes * ((uint32_t)block / 32u);
@@ -665,7 +785,7 @@ int SmallGrid(uint32_t n, int grid, int block, uint32_t lanes) {
     return need < (uint64_t)grid ? (int)(need > 0 ? need : 1) : grid;
 }
 
-template <bool kAny, bool kStats, int kShort, int kBlock, bool kPlanes = false, bool kFew = false>
+template <bool kAny, bool kStats, int kShort, int kBlock, bool kPlanes = false>
 __global__ void __launch_bounds__(kBlock, MinBlocks(kBlock)) trace_kernel(const TraceLaunch L) {
     using W = WarpShared<kShort, false>;
     __shared__ __align__(16) uint8_t s_mem[kTableBytes + W::kBytes * (kBlock / 32)];
@@ -679,8 +799,8 @@ __global__ void __launch_bounds__(kBlock, MinBlocks(kBlock)) trace_kernel(const 
     if (src.n == 0) return;  // an empty queue of the path tracer
     if (L.ray_total && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(L.ray_total, (unsigned long long)src.n);
     fill_tables(s_mem);
-    const Common C{L.counter, L.status, L.stats, L.refill_min, L.lanes, L.postpone_min ? L.postpone_min : kWaitMin};
-    persistent_trace<SingleSource, kAny ? 1 : 0, kStats, kShort, false, false, kPlanes, kFew>(
+    const Common C{L.counter, L.status, L.stats, L.refill_min, L.few_rays, L.full_warps, L.postpone_min ? L.postpone_min : kWaitMin};
+    persistent_trace<SingleSource, kAny ? 1 : 0, kStats, kShort, false, false, kPlanes>(
         src, C, shared_addr(s_mem + kTableBytes + W::kBytes * (threadIdx.x >> 5)), shared_addr(s_mem));
 }
 
@@ -694,12 +814,12 @@ __global__ void __launch_bounds__(kBlock, MinBlocks(kBlock)) batch_kernel(const 
     src.prefix = B.prefix;
     src.njobs = B.njobs;
     src.n = B.total;
-    const Common C{B.counter, B.status, nullptr, B.refill_min, 32u, B.postpone_min ? B.postpone_min : kWaitMin};
+    const Common C{B.counter, B.status, nullptr, B.refill_min, B.few_rays, B.full_warps, B.postpone_min ? B.postpone_min : kWaitMin};
     persistent_trace<BatchSource, 2, false, kShort, false, true>(
         src, C, shared_addr(s_mem + kTableBytes + W::kBytes * (threadIdx.x >> 5)), shared_addr(s_mem));
 }
 
-template <bool kAny, bool kFew>
+template <bool kAny>
 __global__ void __launch_bounds__(128, 8) instanced_trace_kernel(const InstancedLaunch L) {
     using W = WarpShared<8, true>;
     __shared__ __align__(16) uint8_t s_mem[W::kBytes * 4];
@@ -713,8 +833,8 @@ __global__ void __launch_bounds__(128, 8) instanced_trace_kernel(const Instanced
     src.occluded = L.occluded;
     src.n = L.n_dev ? min(*L.n_dev, L.n) : L.n;
     if (L.ray_total && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(L.ray_total, (unsigned long long)src.n);
-    const Common C{L.counter, L.status, nullptr, kFew ? min(8u, L.lanes) : 8u, L.lanes, kWaitMin};
-    persistent_trace<InstancedSource, kAny ? 1 : 0, false, 8, true, true, false, kFew>(
+    const Common C{L.counter, L.status, nullptr, 8u, L.few_rays, L.full_warps, kWaitMin};
+    persistent_trace<InstancedSource, kAny ? 1 : 0, false, 8, true, true>(
         src, C, shared_addr(s_mem + W::kBytes * (threadIdx.x >> 5)), 0u, s_world);
 }
 
@@ -799,17 +919,9 @@ cudaError_t LaunchTraceConfigured(const TraceLaunch& L, bool any, bool stats, co
     TraceLaunch arg = L;
     arg.refill_min = c.refill_min ? c.refill_min : L.refill_min;
     arg.postpone_min = c.postpone_min;
-    arg.lanes = 32;  // (a device queue's length is not known here)
-    if (!L.n_dev && !stats) {
-        arg.lanes = LanesPerWarp(L.n, (uint32_t)(grid * (block / 32)));
-        if (arg.lanes < 32 && L.scene.tri_stride != 1) {  // a small batch: the default shape on few lanes
-            block = 128;
-            fn = any ? reinterpret_cast<const void*>(&trace_kernel<true, false, 8, 128, false, true>)
-                     : reinterpret_cast<const void*>(&trace_kernel<false, false, 8, 128, false, true>);
-            grid = SmallGrid(L.n, grid, block, arg.lanes);
-            arg.refill_min = std::min(arg.refill_min, arg.lanes);
-        }
-    }
+    arg.full_warps = (uint32_t)(grid * (block / 32));
+    arg.few_rays = L.scene.tri_stride == 1 ? 0u : FewRays(arg.full_warps);
+    if (!L.n_dev && L.n <= arg.few_rays) grid = SmallGrid(L.n, grid, block, LanesPerWarp(L.n, arg.full_warps));
     void* params[] = {&arg};
     return cudaLaunchKernel(fn, dim3(grid), dim3(block), params, 0, stream);
 }
@@ -824,22 +936,16 @@ cudaError_t LaunchInstanced(const InstancedLaunch& L, bool any, int sm_count, cu
     if (L.n == 0) return cudaSuccess;
     cudaError_t e = cudaMemsetAsync(L.counter, 0, sizeof(uint32_t), stream);
     if (e != cudaSuccess) return e;
-    const void* fn = any ? reinterpret_cast<const void*>(&instanced_trace_kernel<true, false>)
-                         : reinterpret_cast<const void*>(&instanced_trace_kernel<false, false>);
+    const void* fn = any ? reinterpret_cast<const void*>(&instanced_trace_kernel<true>)
+                         : reinterpret_cast<const void*>(&instanced_trace_kernel<false>);
     int blocks = 0;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, fn, 128, 0);
     if (e != cudaSuccess) return e;
     InstancedLaunch arg = L;
     int grid = sm_count * (blocks > 0 ? blocks : 1);
-    arg.lanes = 32;
-    if (!L.n_dev) {
-        arg.lanes = LanesPerWarp(L.n, (uint32_t)(4 * grid));
-        if (arg.lanes < 32) {
-            fn = any ? reinterpret_cast<const void*>(&instanced_trace_kernel<true, true>)
-                     : reinterpret_cast<const void*>(&instanced_trace_kernel<false, true>);
-            grid = SmallGrid(L.n, grid, 128, arg.lanes);
-        }
-    }
+    arg.full_warps = (uint32_t)(4 * grid);
+    arg.few_rays = FewRays(arg.full_warps);
+    if (!L.n_dev && L.n <= arg.few_rays) grid = SmallGrid(L.n, grid, 128, LanesPerWarp(L.n, arg.full_warps));
     void* params[] = {&arg};
     return cudaLaunchKernel(fn, dim3(grid), dim3(128), params, 0, stream);
 }
@@ -852,7 +958,9 @@ cudaError_t LaunchBatch(const BatchLaunch& B, const TraceConfig& c, int grid, cu
     arg.refill_min = c.refill_min ? c.refill_min : B.refill_min;
     arg.postpone_min = c.postpone_min;
     const int block = normalized_block(c.block);
-    grid = SmallGrid(B.total, grid, block, 32);
+    arg.full_warps = (uint32_t)(grid * (block / 32));
+    arg.few_rays = FewRays(arg.full_warps);
+    if (B.total <= arg.few_rays) grid = SmallGrid(B.total, grid, block, LanesPerWarp(B.total, arg.full_warps));
     void* params[] = {&arg};
     return cudaLaunchKernel(select_batch(c), dim3(grid), dim3(block), params, 0, stream);
 }

@@ -27,7 +27,7 @@ struct TraceLaunch {
                                 // triangle tests (stats variants)
     uint32_t refill_min;        // refill a warp once this many lanes are idle
     uint32_t postpone_min;      // test waiting triangles once this many lanes only wait (0: default)
-    uint32_t lanes;             // lanes of a warp that take rays (set at launch)
+    uint32_t few_rays, full_warps;  // set at launch (rt/traverse.cu)
     const uint32_t* order;      // fetch position -> ray index (ray_sort.hpp), or null: input order
 };
 
@@ -60,6 +60,7 @@ struct BatchLaunch {
     uint32_t* status;
     uint32_t refill_min;
     uint32_t postpone_min;
+    uint32_t few_rays, full_warps;  // set at launch (rt/traverse.cu)
 };
 
 // Rays against a two-level scene (instances.cu).
@@ -75,7 +76,7 @@ struct InstancedLaunch {
     uint8_t* occluded;           // uint8[n]   (any)
     uint32_t* counter;
     uint32_t* status;
-    uint32_t lanes;              // lanes of a warp that take rays (set at launch)
+    uint32_t few_rays, full_warps;  // set at launch (rt/traverse.cu)
 };
 cudaError_t LaunchInstanced(const InstancedLaunch& L, bool any, int sm_count, cudaStream_t stream);
 

@@ -62,7 +62,7 @@ def test_ring_matches_oracle(ctx, kind, n):
     ctx.set_trace_config()
 
 
-@pytest.mark.parametrize("n", [2, 63, 300, 1217, 2433, 4865, 30000, 38911, 38913])
+@pytest.mark.parametrize("n", [2, 63, 300, 1217, 2433, 4865, 30000, 116735, 116736, 116737, 300001])
 def test_small_batches(ctx, n):
     """Batches on few lanes per warp, around the sizes where the lane count and
     the grid change (1,216 blocks of four warps on the full chip), one- and
@@ -79,3 +79,36 @@ def test_small_batches(ctx, n):
         assert np.array_equal(s.any(rays), want_any)
     two.close()
     scene.close()
+
+
+@pytest.mark.parametrize("n", [40, 3000, 116735, 116737, 200000])
+def test_batches_of_scenes(ctx, n):
+    """One launch over scenes of different size and both query kinds, on either
+    side of the size from which a warp starts with all its lanes: lanes that
+    help another lane's ray must take its scene and kind with it."""
+    import torch
+    import foundation_gb300 as fg
+    jobs, want = [], []
+    for k, kind in enumerate(("soup", "one", "stack", "soup")):
+        sc, rays = _geometry(kind), _rays(max(1, n // 8))
+        b = O.OracleBVH(sc.verts, sc.idx)
+        scene = ctx.upload(sc.verts, sc.idx)
+        rd = torch.from_numpy(rays).cuda()
+        for q in (0, 1):
+            out = torch.zeros(len(rays) * (1 if q else 2), dtype=torch.uint8 if q else torch.int32, device="cuda")
+            jobs.append((scene, rd, out, q))
+            want.append(b.any(rays) if q else b.closest(rays))
+    torch.cuda.synchronize()
+    batch = fg.Batch(ctx, jobs)
+    batch.launch()
+    ctx.sync()
+    for (scene, rd, out, q), w in zip(jobs, want):
+        got = out.cpu().numpy()
+        if q:
+            assert np.array_equal(got, w)
+        else:
+            got = got.view(np.uint32).reshape(-1, 2)
+            assert np.array_equal(got[:, 0], w["prim"]) and np.array_equal(got[:, 1], w["t"].view(np.uint32))
+    batch.close()
+    for j in jobs[::2]:
+        j[0].close()
