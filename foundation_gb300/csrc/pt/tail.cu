@@ -4,14 +4,15 @@
 // costs a launch plus the latency of its slowest ray; with the radiance
 // cache almost all paths end at their second vertex and the specular
 // chains that remain would otherwise pay that per bounce. Here each lane
-// takes a path from the queue, runs it bounce by bounce (closest hit,
-// shade_vertex, one any-hit ray per light sample) until it ends, then takes
-// the next path, so a warp stays full while paths remain.
+// takes a path from the queue, runs it bounce by bounce (shade_vertex, then
+// its next segment and its shadow rays, traced by the whole warp:
+// path_rays.cuh) until it ends, then takes the next path.
 #include <cuda_runtime.h>
 
 #include "../../../include/fnd_rt.h"
 #include "../rt/traverse.cuh"
 #include "integrator.hpp"
+#include "path_rays.cuh"
 #include "pt_math.cuh"
 #include "shade.cuh"
 
@@ -30,14 +31,6 @@ __device__ __forceinline__ void tl_add(float4* fb, uint32_t pixel, float3 L) {
     atomicAdd(p + 2, L.z);
 }
 
-template <bool kTwoLevel>
-__device__ __forceinline__ bool tl_occluded(const TailArgs& A, float3 o, float3 d, float tmax) {
-    float t = tmax;
-    uint32_t p;
-    return RT::trace_scene<true, kTwoLevel>(A.scene, A.inst, A.num_inst, make_float4(o.x, o.y, o.z, 0.0f),
-                                            make_float4(d.x, d.y, d.z, tmax), t, p, A.status);
-}
-
 template <uint32_t kMode, bool kTwoLevel>
 __global__ void __launch_bounds__(kTailBlock) tail_kernel(const TailArgs A) {
     uint32_t* counts = A.B.counts;
@@ -45,25 +38,30 @@ __global__ void __launch_bounds__(kTailBlock) tail_kernel(const TailArgs A) {
     const bool take = n != 0u && n <= A.threshold;
     const uint32_t lane = threadIdx.x & 31u;
     uint32_t n_ext = 0, n_sh = 0;
+    using M = PathBlock<kTwoLevel, kTailBlock>;
+    __shared__ __align__(16) uint8_t s_mem[M::kBytes];
     if (take) {
+        if (!kTwoLevel) RT::fill_tables(s_mem);
         const PathBuffers& B = A.B;
-        bool have = false, exhausted = false;
+        bool exhausted = false;
         uint32_t pixel = 0, flags = 0, b = 0;
-        float3 o = f3(0.f, 0.f, 0.f), d = o, beta = o;
+        LaneRays r{};  // the path's rays that are still to be traced
+        float3 beta = f3(0.f, 0.f, 0.f), sh_c = beta, sun_c = beta;
+        const float3 sun = f3(A.R.sun_dir[0], A.R.sun_dir[1], A.R.sun_dir[2]);
         float last_pdf = 0.0f;
         Pcg32 rng;
         rng.state = 0;
         rng.inc = 1;
         for (;;) {
             // lanes without a path take the next ones (one atomic per warp)
-            const uint32_t need = __ballot_sync(kFull, !have);
+            const uint32_t need = __ballot_sync(kFull, !(r.next || r.light || r.sun));
             if (need && !exhausted) {
                 const uint32_t leader = (uint32_t)__ffs(need) - 1u;
                 uint32_t base = 0;
                 if (lane == leader) base = atomicAdd(counts + kCountTailFetch, (uint32_t)__popc(need));
                 base = __shfl_sync(kFull, base, leader);
                 exhausted = base + (uint32_t)__popc(need) >= n;
-                if (!have) {
+                if (need >> lane & 1u) {
                     const uint32_t j = base + (uint32_t)__popc(need & ((1u << lane) - 1u));
                     if (j < n) {
                         const uint32_t slot = B.ext_path[A.q][j];
@@ -74,60 +72,59 @@ __global__ void __launch_bounds__(kTailBlock) tail_kernel(const TailArgs A) {
                         rng = unpack_rng(rs);
                         pixel = rs.w & ~kQueryNextFlag;
                         flags = rs.w & kQueryNextFlag;
-                        o = tl_xyz(r0);
-                        d = tl_xyz(r1);
+                        r.o = tl_xyz(r0);
+                        r.d = tl_xyz(r1);
                         beta = tl_xyz(b4);
                         last_pdf = b4.w;
                         b = A.bounce;
-                        have = true;
+                        r.next = true;
                     }
                 }
             }
-            if (!__any_sync(kFull, have)) break;
-            if (!have) continue;
-            // one interaction of this lane's path
-            VertexIn in;
-            float t = __int_as_float(0x7F800000);
-            uint32_t prim;
-            in.hit = RT::trace_scene<false, kTwoLevel>(A.scene, A.inst, A.num_inst, make_float4(o.x, o.y, o.z, 0.0f),
-                                                       make_float4(d.x, d.y, d.z, t), t, prim, A.status);
-            n_ext++;
-            in.o = o;
-            in.d = d;
-            in.prim = prim;
-            in.t = t;
-            in.beta = beta;
-            in.last_pdf = last_pdf;
-            in.query_here = flags != 0u;
-            VertexOut v;
-            shade_vertex<kMode>(A.R, A.S, A.C.specular_alpha, b, A.R.max_depth, in, rng, v);
-            if (max3(v.add) > 0.0f) tl_add(B.fb, pixel, v.add);
-            if (kMode == 1u && v.query) {
-                const uint32_t k = atomicAdd(A.C.query_count, 1u);
-                if (k < A.C.query_cap) {
-                    v.cp.wo_aux.w = __uint_as_float(pixel);
-                    A.C.queries[k] = v.cp;
+            if (!__any_sync(kFull, r.next || r.light || r.sun)) break;
+            LaneHits h{};
+            trace_path_rays<kTwoLevel>(A.scene, A.inst, A.num_inst, A.status, sun, M::region(s_mem), s_mem, r, h);
+            n_sh += (r.light ? 1u : 0u) + (r.sun ? 1u : 0u);
+            if (r.light && !h.light_blocked) tl_add(B.fb, pixel, sh_c);
+            if (r.sun && !h.sun_blocked) tl_add(B.fb, pixel, sun_c);
+            r.light = r.sun = false;
+            if (r.next) {
+                // one interaction of this lane's path
+                n_ext++;
+                VertexIn in;
+                in.hit = h.hit;
+                in.o = r.o;
+                in.d = r.d;
+                in.prim = h.prim;
+                in.t = h.t;
+                in.beta = beta;
+                in.last_pdf = last_pdf;
+                in.query_here = flags != 0u;
+                VertexOut v;
+                shade_vertex<kMode>(A.R, A.S, A.C.specular_alpha, b, A.R.max_depth, in, rng, v);
+                if (max3(v.add) > 0.0f) tl_add(B.fb, pixel, v.add);
+                if (kMode == 1u && v.query) {
+                    const uint32_t k = atomicAdd(A.C.query_count, 1u);
+                    if (k < A.C.query_cap) {
+                        v.cp.wo_aux.w = __uint_as_float(pixel);
+                        A.C.queries[k] = v.cp;
+                    }
                 }
-            }
-            if (v.shadow) {
-                n_sh++;
-                if (!tl_occluded<kTwoLevel>(A, v.surf_o, v.sh_d, v.sh_tmax)) tl_add(B.fb, pixel, v.sh_c);
-            }
-            if (v.sun) {
-                n_sh++;
-                if (!tl_occluded<kTwoLevel>(A, v.surf_o, f3(A.R.sun_dir[0], A.R.sun_dir[1], A.R.sun_dir[2]),
-                                            __int_as_float(0x7F800000)))
-                    tl_add(B.fb, pixel, v.sun_c);
-            }
-            if (v.next) {
-                o = v.surf_o;
-                d = v.next_d;
-                beta = v.beta;
-                last_pdf = v.pdf;
-                if (v.query_next) flags = kQueryNextFlag;
-                b++;
-            } else {
-                have = false;
+                r.o = v.surf_o;
+                r.light = v.shadow;
+                r.ld = v.sh_d;
+                r.lt = v.sh_tmax;
+                sh_c = v.sh_c;
+                r.sun = v.sun;
+                sun_c = v.sun_c;
+                r.next = v.next;
+                if (v.next) {
+                    r.d = v.next_d;
+                    beta = v.beta;
+                    last_pdf = v.pdf;
+                    if (v.query_next) flags = kQueryNextFlag;
+                    b++;
+                }
             }
         }
     }

@@ -17,6 +17,7 @@
 #include "../../../include/fnd_rt.h"
 #include "../rt/traverse.cuh"
 #include "integrator.hpp"
+#include "path_rays.cuh"
 #include "pt_math.cuh"
 #include "shade.cuh"
 
@@ -34,12 +35,6 @@ __device__ __forceinline__ uint32_t hash32(uint32_t v) {
     const uint32_t s = v * 747796405u + 2891336453u;
     const uint32_t w = ((s >> ((s >> 28u) + 4u)) ^ s) * 277803737u;
     return (w >> 22u) ^ w;
-}
-
-template <bool kAny, bool kTwoLevel>
-__device__ __forceinline__ bool trace(const TrainPathsArgs& A, float3 o, float3 d, float& t, uint32_t& p) {
-    return RT::trace_scene<kAny, kTwoLevel>(A.scene, A.inst, A.num_inst, make_float4(o.x, o.y, o.z, 0.0f),
-                                            make_float4(d.x, d.y, d.z, t), t, p, A.status);
 }
 
 // A finished path's samples: slots from one atomic, targets from the
@@ -67,11 +62,11 @@ __device__ __forceinline__ void write_samples(const TrainPathsArgs& A, const NRC
     }
 }
 
-// Persistent: every lane holds one path and, each iteration, runs one
-// interaction of it (closest hit, shade_vertex, its shadow rays); a lane
-// whose path ended takes the next path index at the top of the iteration
-// (one atomic per warp), so the warp stays full until the paths run out and
-// its lanes stay at the same point of the loop.
+// Persistent: every lane holds one path; each iteration the warp traces its
+// lanes' next segments and the shadow rays of their last vertices together
+// (path_rays.cuh), then each lane runs one interaction. A lane whose path
+// ended takes the next path index at the top of the iteration (one atomic per
+// warp), so the warp stays full until the paths run out.
 template <bool kTwoLevel>
 __global__ void __launch_bounds__(kBlock) training_paths_kernel(const TrainPathsArgs A) {
     const RenderParams& R = A.R;
@@ -82,7 +77,11 @@ __global__ void __launch_bounds__(kBlock) training_paths_kernel(const TrainPaths
     NRC::CachePoint pts[kMaxDepthTrain];
     float3 before[kMaxDepthTrain];
     int ns = 0;
-    float3 total = f3(0.f, 0.f, 0.f), o = total, d = total, beta = total;
+    float3 total = f3(0.f, 0.f, 0.f), beta = total, sh_c = total, sun_c = total;
+    LaneRays r{};  // the path's rays that are still to be traced
+    using M = PathBlock<kTwoLevel, kBlock>;
+    __shared__ __align__(16) uint8_t s_mem[M::kBytes];
+    if (!kTwoLevel) RT::fill_tables(s_mem);
     float last_pdf = 0.0f;
     uint32_t bounce = 0;
     Pcg32 rng;
@@ -106,55 +105,56 @@ __global__ void __launch_bounds__(kBlock) training_paths_kernel(const TrainPaths
                     const uint32_t px = pixel % R.width, py = pixel / R.width;
                     const float sx = (2.0f * ((float)px + a) / (float)R.width - 1.0f) * R.tan_half * R.aspect;
                     const float sy = (1.0f - 2.0f * ((float)py + b) / (float)R.height) * R.tan_half;
-                    o = ld3(R.eye);
-                    d = normalize(ld3(R.fwd) + ld3(R.right) * sx + ld3(R.up) * sy);
+                    r.o = ld3(R.eye);
+                    r.d = normalize(ld3(R.fwd) + ld3(R.right) * sx + ld3(R.up) * sy);
                     beta = f3(1.f, 1.f, 1.f);
                     total = f3(0.f, 0.f, 0.f);
                     last_pdf = 0.0f;
                     bounce = 0;
                     ns = 0;
                     have = depth > 0;
+                    r.next = have;
                 }
             }
         }
         if (!__any_sync(kFull, have)) break;
-        if (!have) continue;
-        VertexIn in;
-        float t = __int_as_float(0x7F800000);
-        uint32_t prim;
-        in.hit = trace<false, kTwoLevel>(A, o, d, t, prim);
-        in.o = o;
-        in.d = d;
-        in.prim = prim;
-        in.t = t;
-        in.beta = beta;
-        in.last_pdf = last_pdf;
-        in.query_here = false;
-        VertexOut v;
-        shade_vertex<2u>(R, S, 0.0f, bounce, depth, in, rng, v);
-        total = total + v.add;
-        if (v.sample) {
-            pts[ns] = v.cp;
-            before[ns] = total;
-            ns++;
-        }
-        if (v.shadow) {
-            float ts = v.sh_tmax;
-            uint32_t sp;
-            if (!trace<true, kTwoLevel>(A, v.surf_o, v.sh_d, ts, sp)) total = total + v.sh_c;
-        }
-        if (v.sun) {
-            float ts = __int_as_float(0x7F800000);
-            uint32_t sp;
-            if (!trace<true, kTwoLevel>(A, v.surf_o, ld3(R.sun_dir), ts, sp)) total = total + v.sun_c;
-        }
-        bounce++;
-        if (v.next && bounce < depth) {
-            last_pdf = v.pdf;
+        LaneHits h{};
+        trace_path_rays<kTwoLevel>(A.scene, A.inst, A.num_inst, A.status, ld3(R.sun_dir), M::region(s_mem), s_mem, r, h);
+        if (r.light && !h.light_blocked) total = total + sh_c;
+        if (r.sun && !h.sun_blocked) total = total + sun_c;
+        r.light = r.sun = false;
+        if (r.next) {
+            VertexIn in;
+            in.hit = h.hit;
+            in.o = r.o;
+            in.d = r.d;
+            in.prim = h.prim;
+            in.t = h.t;
+            in.beta = beta;
+            in.last_pdf = last_pdf;
+            in.query_here = false;
+            VertexOut v;
+            shade_vertex<2u>(R, S, 0.0f, bounce, depth, in, rng, v);
+            total = total + v.add;
+            if (v.sample) {
+                pts[ns] = v.cp;
+                before[ns] = total;
+                ns++;
+            }
+            bounce++;
+            r.o = v.surf_o;
+            r.light = v.shadow;
+            r.ld = v.sh_d;
+            r.lt = v.sh_tmax;
+            sh_c = v.sh_c;
+            r.sun = v.sun;
+            sun_c = v.sun_c;
+            r.next = v.next && bounce < depth;
+            r.d = v.next_d;
             beta = v.beta;
-            o = v.surf_o;
-            d = v.next_d;
-        } else {
+            last_pdf = v.pdf;
+        }
+        if (have && !(r.next || r.light || r.sun)) {
             write_samples(A, pts, before, ns, total);
             have = false;
         }

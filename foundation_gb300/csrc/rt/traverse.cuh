@@ -321,10 +321,9 @@ __device__ __forceinline__ NodeHits intersect_node(const RayState& r, const uint
 namespace Foundation {
 namespace RT {
 
-// Single-ray traversal with a thread-local stack and no warp refill, for
-// latency-bound work where each thread follows its own path (the radiance
-// cache's training paths). Same node / triangle tests and tie rule as the
-// persistent kernels. Returns true on a hit (best_t / best_p updated; the
+// Single-ray traversal with a thread-local stack and no warp refill: the plain
+// form that the warp loop (warp_trace.cuh) is tested against, on the host too.
+// Same node / triangle tests and tie rule as the persistent kernels. Returns true on a hit (best_t / best_p updated; the
 // caller initialises best_t to the ray's tmax).
 template <bool kAny>
 __device__ __forceinline__ bool trace_single(const DeviceScene& sc, const RayState& r, float& best_t,
@@ -486,16 +485,6 @@ __device__ __forceinline__ bool trace_two_level(const DeviceScene& tlas, const I
         ng_group = e.y;
     }
     return best_p != FND_INVALID_ID;
-}
-
-// One ray through a one- or two-level scene (per-thread traversal, for the
-// path-tracing megakernels). r0 / r1: the ray in the fnd_ray layout; best_t
-// starts at the ray's tmax.
-template <bool kAny, bool kTwoLevel>
-__device__ __forceinline__ bool trace_scene(const DeviceScene& sc, const InstanceRec* inst, uint32_t num_inst,
-                                            float4 r0, float4 r1, float& best_t, uint32_t& best_p, uint32_t* status) {
-    if constexpr (kTwoLevel) return trace_two_level<kAny>(sc, inst, num_inst, r0, r1, best_t, best_p, status);
-    return trace_single<kAny>(sc, setup_ray(r0, r1), best_t, best_p, status);
 }
 
 }  // namespace RT

@@ -112,3 +112,28 @@ def test_batches_of_scenes(ctx, n):
     batch.close()
     for j in jobs[::2]:
         j[0].close()
+
+
+@pytest.mark.parametrize("width,height", [(1, 1), (31, 1), (33, 1), (65, 3), (200, 7)])
+@pytest.mark.parametrize("sun", [False, True])
+def test_rays_of_a_warps_paths(ctx, width, height, sun):
+    """The tail kernel traces the segments and shadow rays of a warp's paths
+    together (part-filled warps, up to three rays per lane, lanes whose path
+    has ended): the same rays as the wavefront stages, and the same image up to
+    the order of at most 3 x 8 x 3 non-negative FP32 additions (2^-24 each)."""
+    from foundation_gb300 import scenes as S
+    cs = S.cornell_scene()
+    s = ctx.upload(cs.verts, cs.idx)
+    s.set_materials(cs.tri_material, S.material_records(cs))
+    s.set_lights(S.light_records(cs))
+    kw = dict(seed=9, sky=(0.1, 0.2, 0.3), rr_start=2)
+    if sun:
+        kw.update(sun_dir=(0.2, 0.4, 1.0), sun_irradiance=(0.5, 0.25, 0.75))
+    got = []
+    for opts in (dict(wavefront=True), dict(tail_paths=1 << 28)):
+        img = ctx.render(s, width, height, 3, S.CORNELL_CAMERA, **kw, **opts)
+        st = ctx.render_stats()
+        got.append((img, st["extension_rays"], st["shadow_rays"]))
+    assert got[0][1:] == got[1][1:]
+    np.testing.assert_allclose(got[1][0], got[0][0], rtol=72 * 2.0 ** -24, atol=0)
+    s.close()
