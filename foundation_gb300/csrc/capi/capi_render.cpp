@@ -20,7 +20,7 @@ using Foundation::RtCore::Fail;
 
 namespace {
 
-// Paths in flight per wave: 33,554,432 (7.3 GB of path state). Every wave
+// Paths in flight per wave: 33,554,432 (7.9 GB of path state). Every wave
 // pays its bounces' launches and the latency of each bounce's last rays, so
 // fewer, larger waves are faster: 1920x1080 x 64 spp takes 166.7 ms in waves
 // of 2^22 paths, 150.6 ms at 2^23, 142.1 ms at 2^24 and 137.2 ms at 2^25.
@@ -37,15 +37,14 @@ void EnsurePathBuffers(fnd_rt_ctx* ctx, uint32_t capacity) {
     ctx->paths = PT::PathBuffers{};
     const size_t c = capacity;
     const size_t sizes[] = {
-        16 * c,      // rng
-        16 * c,      // beta
+        16 * c,      // rng[0]
+        16 * c,      // rng[1]
+        16 * c,      // beta[0]
+        16 * c,      // beta[1]
         32 * c,      // ext_rays[0]
         32 * c,      // ext_rays[1]
-        4 * c,       // ext_path[0]
-        4 * c,       // ext_path[1]
         8 * c,       // hits
         2 * 32 * c,  // sh_rays (two per path)
-        2 * 4 * c,   // sh_pixel
         2 * 16 * c,  // sh_contrib
         2 * c,       // sh_occluded
         256,         // counts
@@ -64,18 +63,14 @@ void EnsurePathBuffers(fnd_rt_ctx* ctx, uint32_t capacity) {
     };
     PT::PathBuffers& B = ctx->paths;
     B.capacity = capacity;
-    B.rng = reinterpret_cast<uint4*>(take(sizes[0]));
-    B.beta = reinterpret_cast<float4*>(take(sizes[1]));
-    B.ext_rays[0] = reinterpret_cast<float4*>(take(sizes[2]));
-    B.ext_rays[1] = reinterpret_cast<float4*>(take(sizes[3]));
-    B.ext_path[0] = reinterpret_cast<uint32_t*>(take(sizes[4]));
-    B.ext_path[1] = reinterpret_cast<uint32_t*>(take(sizes[5]));
+    for (int q = 0; q < 2; ++q) B.rng[q] = reinterpret_cast<uint4*>(take(sizes[q]));
+    for (int q = 0; q < 2; ++q) B.beta[q] = reinterpret_cast<float4*>(take(sizes[2 + q]));
+    for (int q = 0; q < 2; ++q) B.ext_rays[q] = reinterpret_cast<float4*>(take(sizes[4 + q]));
     B.hits = reinterpret_cast<uint2*>(take(sizes[6]));
     B.sh_rays = reinterpret_cast<float4*>(take(sizes[7]));
-    B.sh_pixel = reinterpret_cast<uint32_t*>(take(sizes[8]));
-    B.sh_contrib = reinterpret_cast<float4*>(take(sizes[9]));
-    B.sh_occluded = reinterpret_cast<uint8_t*>(take(sizes[10]));
-    B.counts = reinterpret_cast<uint32_t*>(take(sizes[11]));
+    B.sh_contrib = reinterpret_cast<float4*>(take(sizes[8]));
+    B.sh_occluded = reinterpret_cast<uint8_t*>(take(sizes[9]));
+    B.counts = reinterpret_cast<uint32_t*>(take(sizes[10]));
     CUDA_CHECK(cudaMemsetAsync(B.counts, 0, 256, ctx->stream));
 }
 
@@ -435,7 +430,9 @@ int fnd_rt_render(fnd_rt_ctx* ctx, const fnd_rt_scene* scene, const fnd_render_d
         for (uint64_t wave_base = 0; wave_base < total; wave_base += cap, ++waves) {
             const uint32_t wave_n = (uint32_t)std::min<uint64_t>(cap, total - wave_base);
             if (use_cache) CUDA_CHECK(cudaMemsetAsync(C.query_count, 0, sizeof(uint32_t), ctx->stream));
-            CUDA_CHECK(PT::LaunchGenerate(B, R, wave_base, wave_n, ctx->stream));
+            B.wave_pixel = (uint32_t)(wave_base % npix);
+            B.wave_sample = (uint32_t)(wave_base / npix);
+            CUDA_CHECK(PT::LaunchGenerate(B, R, wave_n, ctx->stream));
             RunBounces(ctx, scene, B, R, S, C, D.max_depth, grid_shade, tail_paths);
             if (use_cache) {
                 CUDA_CHECK(cudaStreamWaitEvent(ctx->stream, ctx->cache->ev_trained, 0));

@@ -59,14 +59,14 @@ struct RenderParams {
 
 struct PathBuffers {
     uint32_t capacity;
-    uint4* rng;          // x,y = PCG state (lo, hi), z = sequence (sample index), w = pixel
-    float4* beta;        // rgb throughput, w = solid-angle pdf of the last BSDF sample (0 at the camera)
-    float4* ext_rays[2]; // 2 float4 per ray (fnd_ray layout), ping-pong by bounce parity
-    uint32_t* ext_path[2];
+    uint32_t wave_pixel, wave_sample;  // pixel and sample (of this call) of the wave's first path
+    // the extension queues, ping-pong by bounce parity: entry j of every array is one path
+    uint4* rng[2];       // x,y = PCG state (lo, hi), z = sequence (sample index), w = pixel
+    float4* beta[2];     // rgb throughput, w = solid-angle pdf of the last BSDF sample (0 at the camera)
+    float4* ext_rays[2]; // 2 float4 per ray (fnd_ray layout)
     uint2* hits;
     float4* sh_rays;     // 2 float4 per shadow ray; up to 2 per path per bounce
-    uint32_t* sh_pixel;
-    float4* sh_contrib;
+    float4* sh_contrib;  // rgb, w = pixel
     uint8_t* sh_occluded;
     uint32_t* counts;    // [0], [1] extension queues, [2] shadow queue, [3..] statistics
     float4* fb;          // per-pixel radiance sums
@@ -142,8 +142,7 @@ cudaError_t LaunchTail(const TailArgs& A, int grid, cudaStream_t s);
 int TailBlocksPerSm(bool two_level);  // resident tail blocks per SM (occupancy of that variant)
 constexpr int kTailBlock = 128;
 
-cudaError_t LaunchGenerate(const PathBuffers& B, const RenderParams& R, uint64_t wave_base, uint32_t wave_n,
-                           cudaStream_t s);
+cudaError_t LaunchGenerate(const PathBuffers& B, const RenderParams& R, uint32_t wave_n, cudaStream_t s);
 cudaError_t LaunchShade(const PathBuffers& B, const RenderParams& R, const ShadeScene& S, const CacheIO& C, int cur,
                         uint32_t bounce, int grid, cudaStream_t s);
 cudaError_t LaunchResolve(const PathBuffers& B, int grid, cudaStream_t s);

@@ -25,10 +25,7 @@ constexpr uint32_t kFull = 0xFFFFFFFFu;
 __device__ __forceinline__ float3 tl_xyz(float4 v) { return f3(v.x, v.y, v.z); }
 
 __device__ __forceinline__ void tl_add(float4* fb, uint32_t pixel, float3 L) {
-    float* p = reinterpret_cast<float*>(fb + pixel);
-    atomicAdd(p + 0, L.x);
-    atomicAdd(p + 1, L.y);
-    atomicAdd(p + 2, L.z);
+    atomicAdd(fb + pixel, make_float4(L.x, L.y, L.z, 0.0f));
 }
 
 template <uint32_t kMode, bool kTwoLevel>
@@ -64,11 +61,10 @@ __global__ void __launch_bounds__(kTailBlock) tail_kernel(const TailArgs A) {
                 if (need >> lane & 1u) {
                     const uint32_t j = base + (uint32_t)__popc(need & ((1u << lane) - 1u));
                     if (j < n) {
-                        const uint32_t slot = B.ext_path[A.q][j];
                         const float4 r0 = B.ext_rays[A.q][2 * (size_t)j];
                         const float4 r1 = B.ext_rays[A.q][2 * (size_t)j + 1];
-                        const float4 b4 = B.beta[slot];
-                        const uint4 rs = B.rng[slot];
+                        const float4 b4 = B.beta[A.q][j];
+                        const uint4 rs = B.rng[A.q][j];
                         rng = unpack_rng(rs);
                         pixel = rs.w & ~kQueryNextFlag;
                         flags = rs.w & kQueryNextFlag;
