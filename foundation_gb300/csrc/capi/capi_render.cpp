@@ -47,7 +47,7 @@ void EnsurePathBuffers(fnd_rt_ctx* ctx, uint32_t capacity) {
         2 * 32 * c,  // sh_rays (two per path)
         2 * 16 * c,  // sh_contrib
         2 * c,       // sh_occluded
-        256,         // counts
+        sizeof(uint32_t) * PT::kCounts,
     };
     size_t total = 0;
     for (size_t s : sizes) total += Align256(s);
@@ -71,7 +71,6 @@ void EnsurePathBuffers(fnd_rt_ctx* ctx, uint32_t capacity) {
     B.sh_contrib = reinterpret_cast<float4*>(take(sizes[8]));
     B.sh_occluded = reinterpret_cast<uint8_t*>(take(sizes[9]));
     B.counts = reinterpret_cast<uint32_t*>(take(sizes[10]));
-    CUDA_CHECK(cudaMemsetAsync(B.counts, 0, 256, ctx->stream));
 }
 
 void Sub(const double a[3], const double b[3], double o[3]) {
@@ -89,11 +88,12 @@ bool Normalize(double v[3]) {
     return true;
 }
 
-// One wave's bounce loop: extend -> shade -> shadow -> resolve, max_depth
-// times. After each bounce but the last, the tail megakernel finishes the
-// wave when at most `tail_paths` paths continue (tail_paths 0: never).
+// The bounce loop of a wave of wave_n paths: extend -> shade -> shadow ->
+// resolve, max_depth times. After each bounce but the last, the tail megakernel
+// finishes the wave when at most `tail_paths` paths continue (tail_paths 0:
+// never).
 void RunBounces(fnd_rt_ctx* ctx, const fnd_rt_scene* scene, const PT::PathBuffers& B, const PT::RenderParams& R,
-                const PT::ShadeScene& S, const PT::CacheIO& C, uint32_t max_depth, int grid_shade,
+                const PT::ShadeScene& S, const PT::CacheIO& C, uint32_t wave_n, uint32_t max_depth, int grid_shade,
                 uint32_t tail_paths) {
     const int g_closest = CApi::TraceGrid(ctx, ctx->trace_cfg, 0);
     const int g_any = CApi::TraceGrid(ctx, ctx->trace_cfg, 1);
@@ -106,7 +106,8 @@ void RunBounces(fnd_rt_ctx* ctx, const fnd_rt_scene* scene, const PT::PathBuffer
     // cache paths end in queries at the second interaction: what continues
     // after it are specular chains, which the tail megakernel finishes
     // whatever their number, so the later bounces are not enqueued at all
-    // (they would find empty queues)
+    // (they would find empty queues); likewise where the whole wave is no
+    // larger than the tail's threshold
     const bool cache_tail = C.mode == 1 && tail_paths != 0;
     // two-level scenes: the instanced persistent kernel on the device queues
     auto trace = [&](RT::TraceLaunch& L, bool any, const RT::TraceConfig& cfg, int grid) -> cudaError_t {
@@ -128,38 +129,39 @@ void RunBounces(fnd_rt_ctx* ctx, const fnd_rt_scene* scene, const PT::PathBuffer
         I.occluded = L.occluded;
         I.counter = L.counter;
         I.status = L.status;
+        I.counter_ready = L.counter_ready;
         return RT::LaunchInstanced(I, any, ctx->sm_count, ctx->stream);
     };
     for (uint32_t b = 0; b < max_depth; ++b) {
-        const int cur = (int)(b & 1u), nxt = cur ^ 1;
+        const uint32_t cur = b & 1u;
         RT::TraceLaunch L{};
         L.scene = scene->view;
         L.rays = B.ext_rays[cur];
         L.n = B.capacity;
-        L.n_dev = B.counts + cur;
+        L.n_dev = B.counts + PT::kCountExt + b;
         L.ray_total = ctx->d_render_stats + 0;
         L.hits = B.hits;
-        L.counter = ctx->d_counter;
+        L.counter = B.counts + PT::kCountFetch + 2 * b;
+        L.counter_ready = true;
         L.status = ctx->d_status;
         L.refill_min = ctx->refill_min;
         // camera rays keep their (already coherent) order; later bounces and
         // shadow rays take the context's coherence ordering, if any
         CUDA_CHECK(trace(L, false, b == 0 ? cfg0 : ctx->trace_cfg, g_closest));
-        CUDA_CHECK(cudaMemsetAsync(B.counts + nxt, 0, sizeof(uint32_t), ctx->stream));
-        CUDA_CHECK(cudaMemsetAsync(B.counts + PT::kCountShadow, 0, sizeof(uint32_t), ctx->stream));
-        CUDA_CHECK(PT::LaunchShade(B, R, S, C, cur, b, grid_shade, ctx->stream));
+        CUDA_CHECK(PT::LaunchShade(B, R, S, C, b, grid_shade, ctx->stream));
         RT::TraceLaunch A{};
         A.scene = scene->view;
         A.rays = B.sh_rays;
         A.n = 2 * B.capacity;
-        A.n_dev = B.counts + PT::kCountShadow;
+        A.n_dev = B.counts + PT::kCountShadow + b;
         A.ray_total = ctx->d_render_stats + 1;
         A.occluded = B.sh_occluded;
-        A.counter = ctx->d_counter;
+        A.counter = B.counts + PT::kCountFetch + 2 * b + 1;
+        A.counter_ready = true;
         A.status = ctx->d_status;
         A.refill_min = ctx->refill_min;
         CUDA_CHECK(trace(A, true, ctx->trace_cfg, g_any));
-        CUDA_CHECK(PT::LaunchResolve(B, grid_shade, ctx->stream));
+        CUDA_CHECK(PT::LaunchResolve(B, b, grid_shade, ctx->stream));
         if (tail_paths && b + 1 < max_depth) {
             PT::TailArgs T{};
             T.scene = scene->view;
@@ -169,13 +171,12 @@ void RunBounces(fnd_rt_ctx* ctx, const fnd_rt_scene* scene, const PT::PathBuffer
             T.R = R;
             T.S = S;
             T.C = C;
-            T.q = nxt;
             T.bounce = b + 1;
             T.threshold = cache_tail && b == 1 ? 0xFFFFFFFFu : tail_paths;
             T.status = ctx->d_status;
             T.ray_stats = ctx->d_render_stats;
             CUDA_CHECK(PT::LaunchTail(T, g_tail, ctx->stream));
-            if (cache_tail && b == 1) break;
+            if ((cache_tail && b == 1) || wave_n <= T.threshold) break;
         }
     }
 }
@@ -290,7 +291,7 @@ int fnd_rt_render(fnd_rt_ctx* ctx, const fnd_rt_scene* scene, const fnd_render_d
                    "FND_RENDER_TRAIN_ONLY needs FND_RENDER_CACHE");
         CHECK_CODE(D.width > 0 && D.height > 0 && (uint64_t)D.width * D.height <= (1ull << 26), FND_ERR_INVALID_ARG,
                    "image %ux%u out of range", D.width, D.height);
-        CHECK_CODE(D.spp >= 1 && D.max_depth >= 1 && D.max_depth <= 64, FND_ERR_INVALID_ARG,
+        CHECK_CODE(D.spp >= 1 && D.max_depth >= 1 && D.max_depth <= (uint32_t)PT::kMaxBounces, FND_ERR_INVALID_ARG,
                    "spp %u / max_depth %u out of range", D.spp, D.max_depth);
         CHECK_CODE(D.camera.vfov_deg > 0.0f && D.camera.vfov_deg < 180.0f, FND_ERR_INVALID_ARG, "vfov %f",
                    D.camera.vfov_deg);
@@ -433,7 +434,7 @@ int fnd_rt_render(fnd_rt_ctx* ctx, const fnd_rt_scene* scene, const fnd_render_d
             B.wave_pixel = (uint32_t)(wave_base % npix);
             B.wave_sample = (uint32_t)(wave_base / npix);
             CUDA_CHECK(PT::LaunchGenerate(B, R, wave_n, ctx->stream));
-            RunBounces(ctx, scene, B, R, S, C, D.max_depth, grid_shade, tail_paths);
+            RunBounces(ctx, scene, B, R, S, C, wave_n, D.max_depth, grid_shade, tail_paths);
             if (use_cache) {
                 CUDA_CHECK(cudaStreamWaitEvent(ctx->stream, ctx->cache->ev_trained, 0));
                 CUDA_CHECK(NRC::Infer(ctx->cache->net, C.queries, C.query_count, C.query_cap, B.fb,

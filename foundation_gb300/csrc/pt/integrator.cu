@@ -55,13 +55,8 @@ __device__ __forceinline__ Pcg32 camera_path(const PathBuffers& B, const RenderP
 // write and read it (4.1M paths: 36 bytes each way, 45 us).
 __global__ void __launch_bounds__(kBlock) generate_kernel(const PathBuffers B, const RenderParams R, uint32_t wave_n) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i == 0) {
-        B.counts[kCountExt0] = wave_n;
-        B.counts[kCountExt1] = 0;
-        B.counts[kCountShadow] = 0;
-        B.counts[kCountTailDone] = 0;
-        B.counts[kCountTailFetch] = 0;
-    }
+    if (blockIdx.x == 0)
+        for (uint32_t k = threadIdx.x; k < (uint32_t)kCounts; k += blockDim.x) B.counts[k] = k == kCountExt ? wave_n : 0u;
     if (i >= wave_n) return;
     uint32_t pixel, sample;
     float a, b;
@@ -81,9 +76,9 @@ __global__ void __launch_bounds__(kBlock) generate_kernel(const PathBuffers B, c
 // kFirst: the camera rays' hits (see generate_kernel).
 template <uint32_t kMode, bool kFirst>
 __global__ void __launch_bounds__(kShadeBlock, kShadeBlocksPerSm)
-    shade_kernel(const PathBuffers B, const RenderParams R, const ShadeScene S, const CacheIO C, int cur, uint32_t bounce) {
-    const uint32_t n = B.counts[cur];
-    const int nxt = cur ^ 1;
+    shade_kernel(const PathBuffers B, const RenderParams R, const ShadeScene S, const CacheIO C, uint32_t bounce) {
+    const uint32_t n = B.counts[kCountExt + bounce];
+    const uint32_t cur = bounce & 1u, nxt = cur ^ 1u;
     const uint32_t stride = gridDim.x * blockDim.x;
     const uint32_t lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
     for (uint32_t base = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < n; base += stride) {
@@ -125,7 +120,9 @@ __global__ void __launch_bounds__(kShadeBlock, kShadeBlocksPerSm)
         // adds for queue q): each answer is a trip to L2
         const uint32_t ml = __ballot_sync(kFull, v.shadow), ms = __ballot_sync(kFull, v.sun);
         const uint32_t mn = __ballot_sync(kFull, v.next), mq = kMode == 1u ? __ballot_sync(kFull, v.query) : 0u;
-        uint32_t* counter = lane == 0u ? B.counts + kCountShadow : lane == 1u ? B.counts + nxt : C.query_count;
+        uint32_t* counter = lane == 0u   ? B.counts + kCountShadow + bounce
+                            : lane == 1u ? B.counts + kCountExt + bounce + 1u
+                                         : C.query_count;
         const uint32_t count = lane == 0u   ? (uint32_t)__popc(ml) + (uint32_t)__popc(ms)
                                : lane == 1u ? (uint32_t)__popc(mn)
                                : lane == 2u ? (uint32_t)__popc(mq)
@@ -164,8 +161,8 @@ __global__ void __launch_bounds__(kShadeBlock, kShadeBlocksPerSm)
     }
 }
 
-__global__ void __launch_bounds__(kBlock) resolve_kernel(const PathBuffers B) {
-    const uint32_t n = B.counts[kCountShadow];
+__global__ void __launch_bounds__(kBlock) resolve_kernel(const PathBuffers B, uint32_t bounce) {
+    const uint32_t n = B.counts[kCountShadow + bounce];
     const uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += stride) {
         if (B.sh_occluded[k]) continue;
@@ -191,22 +188,22 @@ cudaError_t LaunchGenerate(const PathBuffers& B, const RenderParams& R, uint32_t
     return cudaGetLastError();
 }
 
-cudaError_t LaunchShade(const PathBuffers& B, const RenderParams& R, const ShadeScene& S, const CacheIO& C, int cur,
+cudaError_t LaunchShade(const PathBuffers& B, const RenderParams& R, const ShadeScene& S, const CacheIO& C,
                         uint32_t bounce, int grid, cudaStream_t s) {
     grid *= kBlock / kShadeBlock;
     if (C.mode == 1u && bounce == 0)
-        shade_kernel<1u, true><<<grid, kShadeBlock, 0, s>>>(B, R, S, C, cur, bounce);
+        shade_kernel<1u, true><<<grid, kShadeBlock, 0, s>>>(B, R, S, C, bounce);
     else if (C.mode == 1u)
-        shade_kernel<1u, false><<<grid, kShadeBlock, 0, s>>>(B, R, S, C, cur, bounce);
+        shade_kernel<1u, false><<<grid, kShadeBlock, 0, s>>>(B, R, S, C, bounce);
     else if (bounce == 0)
-        shade_kernel<0u, true><<<grid, kShadeBlock, 0, s>>>(B, R, S, C, cur, bounce);
+        shade_kernel<0u, true><<<grid, kShadeBlock, 0, s>>>(B, R, S, C, bounce);
     else
-        shade_kernel<0u, false><<<grid, kShadeBlock, 0, s>>>(B, R, S, C, cur, bounce);
+        shade_kernel<0u, false><<<grid, kShadeBlock, 0, s>>>(B, R, S, C, bounce);
     return cudaGetLastError();
 }
 
-cudaError_t LaunchResolve(const PathBuffers& B, int grid, cudaStream_t s) {
-    resolve_kernel<<<grid, kBlock, 0, s>>>(B);
+cudaError_t LaunchResolve(const PathBuffers& B, uint32_t bounce, int grid, cudaStream_t s) {
+    resolve_kernel<<<grid, kBlock, 0, s>>>(B, bounce);
     return cudaGetLastError();
 }
 

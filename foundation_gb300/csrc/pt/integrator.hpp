@@ -68,7 +68,7 @@ struct PathBuffers {
     float4* sh_rays;     // 2 float4 per shadow ray; up to 2 per path per bounce
     float4* sh_contrib;  // rgb, w = pixel
     uint8_t* sh_occluded;
-    uint32_t* counts;    // [0], [1] extension queues, [2] shadow queue, [3..] statistics
+    uint32_t* counts;    // kCounts words (below)
     float4* fb;          // per-pixel radiance sums
 };
 
@@ -110,14 +110,18 @@ int TrainingPathsBlocksPerSm(bool two_level);
 
 constexpr uint32_t kQueryNextFlag = 0x80000000u;  // in PathBuffers::rng.w
 
-// Device counters of a wave (PathBuffers::counts): the two extension queue
-// lengths, the shadow queue length, and the tail kernel's block-completion
-// and path-fetch counters (all reset by generate).
-constexpr int kCountExt0 = 0, kCountExt1 = 1, kCountShadow = 2;
-constexpr int kCountTailDone = 8, kCountTailFetch = 9;
+// Device counters of a wave (PathBuffers::counts), all set by generate: every
+// interaction has its own extension and shadow queue length and its own two
+// ray-fetch counters for the trace kernels, so no stage needs a launch that
+// clears one (four a bounce). Then the tail kernel's block-completion and
+// path-fetch counters. A frame of 640x360 took 787 us with those launches and
+// takes 740; 192x108, where one tail launch also ends the sequence, 552 and 355.
+constexpr int kMaxBounces = 64;
+constexpr int kCountExt = 0, kCountShadow = kCountExt + kMaxBounces + 1, kCountFetch = kCountShadow + kMaxBounces;
+constexpr int kCountTailDone = kCountFetch + 2 * kMaxBounces, kCountTailFetch = kCountTailDone + 1;
+constexpr int kCounts = kCountTailFetch + 1;
 
-// The tail of a wave: once the extension queue `q` (the paths that continue
-// to interaction `bounce`) holds at most `threshold` paths, one persistent
+// The tail of a wave: once the extension queue of interaction `bounce` holds at most `threshold` paths, one persistent
 // megakernel finishes every one of them (lanes fetch paths dynamically and
 // run them to the end with single-ray traversal and the shade stage's
 // vertex logic) and empties the queue, so the remaining wavefront stages of
@@ -132,7 +136,6 @@ struct TailArgs {
     RenderParams R;
     ShadeScene S;
     CacheIO C;
-    int q;
     uint32_t bounce;
     uint32_t threshold;
     uint32_t* status;
@@ -143,9 +146,9 @@ int TailBlocksPerSm(bool two_level);  // resident tail blocks per SM (occupancy 
 constexpr int kTailBlock = 128;
 
 cudaError_t LaunchGenerate(const PathBuffers& B, const RenderParams& R, uint32_t wave_n, cudaStream_t s);
-cudaError_t LaunchShade(const PathBuffers& B, const RenderParams& R, const ShadeScene& S, const CacheIO& C, int cur,
+cudaError_t LaunchShade(const PathBuffers& B, const RenderParams& R, const ShadeScene& S, const CacheIO& C,
                         uint32_t bounce, int grid, cudaStream_t s);
-cudaError_t LaunchResolve(const PathBuffers& B, int grid, cudaStream_t s);
+cudaError_t LaunchResolve(const PathBuffers& B, uint32_t bounce, int grid, cudaStream_t s);
 cudaError_t LaunchFinalize(const PathBuffers& B, float* rgb, uint32_t npix, float scale, cudaStream_t s);
 // tonemap.cu: linear RGB floats -> R8G8B8A8_UNORM words (FND_TONEMAP_* mode)
 cudaError_t LaunchTonemap(const float* rgb, uint32_t npix, float exposure, uint32_t mode, uint32_t* rgba,

@@ -31,7 +31,8 @@ __device__ __forceinline__ void tl_add(float4* fb, uint32_t pixel, float3 L) {
 template <uint32_t kMode, bool kTwoLevel>
 __global__ void __launch_bounds__(kTailBlock) tail_kernel(const TailArgs A) {
     uint32_t* counts = A.B.counts;
-    const uint32_t n = counts[A.q];
+    const uint32_t q = A.bounce & 1u;
+    const uint32_t n = counts[kCountExt + A.bounce];
     const bool take = n != 0u && n <= A.threshold;
     const uint32_t lane = threadIdx.x & 31u;
     uint32_t n_ext = 0, n_sh = 0;
@@ -61,10 +62,10 @@ __global__ void __launch_bounds__(kTailBlock) tail_kernel(const TailArgs A) {
                 if (need >> lane & 1u) {
                     const uint32_t j = base + (uint32_t)__popc(need & ((1u << lane) - 1u));
                     if (j < n) {
-                        const float4 r0 = B.ext_rays[A.q][2 * (size_t)j];
-                        const float4 r1 = B.ext_rays[A.q][2 * (size_t)j + 1];
-                        const float4 b4 = B.beta[A.q][j];
-                        const uint4 rs = B.rng[A.q][j];
+                        const float4 r0 = B.ext_rays[q][2 * (size_t)j];
+                        const float4 r1 = B.ext_rays[q][2 * (size_t)j + 1];
+                        const float4 b4 = B.beta[q][j];
+                        const uint4 rs = B.rng[q][j];
                         rng = unpack_rng(rs);
                         pixel = rs.w & ~kQueryNextFlag;
                         flags = rs.w & kQueryNextFlag;
@@ -134,7 +135,7 @@ __global__ void __launch_bounds__(kTailBlock) tail_kernel(const TailArgs A) {
         __threadfence();
         const uint32_t prev = atomicAdd(counts + kCountTailDone, 1u);
         if (prev == gridDim.x - 1u) {
-            if (take) counts[A.q] = 0u;
+            if (take) counts[kCountExt + A.bounce] = 0u;
             counts[kCountTailFetch] = 0u;
             counts[kCountTailDone] = 0u;
             __threadfence();

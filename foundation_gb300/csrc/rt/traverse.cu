@@ -303,8 +303,10 @@ cudaError_t LaunchTraceConfigured(const TraceLaunch& L, bool any, bool stats, co
             any ? nullptr : reinterpret_cast<uint2*>(L.hits), any ? L.occluded : nullptr, L.n, L.n_dev);
         return cudaGetLastError();
     }
-    cudaError_t e = cudaMemsetAsync(L.counter, 0, sizeof(uint32_t), stream);
-    if (e != cudaSuccess) return e;
+    if (!L.counter_ready) {
+        const cudaError_t e = cudaMemsetAsync(L.counter, 0, sizeof(uint32_t), stream);
+        if (e != cudaSuccess) return e;
+    }
     const void* fn = any ? select_trace<true>(c, stats) : select_trace<false>(c, stats);
     int block = stats ? 128 : normalized_block(c.block);
     if (L.scene.tri_stride == 1) {  // triangle planes: the default shape
@@ -330,7 +332,7 @@ cudaError_t LaunchTrace(const TraceLaunch& L, bool any, bool stats, int grid, cu
 
 cudaError_t LaunchInstanced(const InstancedLaunch& L, bool any, int sm_count, cudaStream_t stream) {
     if (L.n == 0) return cudaSuccess;
-    cudaError_t e = cudaMemsetAsync(L.counter, 0, sizeof(uint32_t), stream);
+    cudaError_t e = L.counter_ready ? cudaSuccess : cudaMemsetAsync(L.counter, 0, sizeof(uint32_t), stream);
     if (e != cudaSuccess) return e;
     const void* fn = any ? reinterpret_cast<const void*>(&instanced_trace_kernel<true>)
                          : reinterpret_cast<const void*>(&instanced_trace_kernel<false>);

@@ -21,7 +21,7 @@ struct TraceLaunch {
     unsigned long long* ray_total;  // if set, the launch adds its ray count here
     void* hits;          // fnd_hit[n] (closest)
     uint8_t* occluded;   // uint8[n]   (any)
-    uint32_t* counter;   // work-queue counter (zeroed before each launch)
+    uint32_t* counter;   // work-queue counter (zeroed by the launch, unless counter_ready)
     uint32_t* status;    // latched kStatus* bits
     unsigned long long* stats;  // [0] node fetches, [1] triangle tests, [2] / [3] warp steps of the node /
                                 // triangle tests (stats variants)
@@ -29,6 +29,7 @@ struct TraceLaunch {
     uint32_t postpone_min;      // test waiting triangles once this many lanes only wait (0: default)
     uint32_t few_rays, full_warps;  // set at launch (rt/traverse.cu)
     const uint32_t* order;      // fetch position -> ray index (ray_sort.hpp), or null: input order
+    bool counter_ready;         // *counter is zero on the stream already: no launch to clear it
 };
 
 // Launch shape of a traversal kernel (the autotuner's search space).
@@ -77,6 +78,7 @@ struct InstancedLaunch {
     uint32_t* counter;
     uint32_t* status;
     uint32_t few_rays, full_warps;  // set at launch (rt/traverse.cu)
+    bool counter_ready;             // (see TraceLaunch)
 };
 cudaError_t LaunchInstanced(const InstancedLaunch& L, bool any, int sm_count, cudaStream_t stream);
 
