@@ -85,9 +85,10 @@ cudaError_t LaunchTraceOrdered(fnd_rt_ctx* ctx, const fnd_rt_scene* scene, RT::T
 }
 
 int ReadStatus(fnd_rt_ctx* ctx) {
-    CUDA_CHECK(cudaMemcpyAsync(ctx->h_status, ctx->d_status, sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream));
+    if (ctx->d_status != ctx->h_status)
+        CUDA_CHECK(cudaMemcpyAsync(ctx->h_status, ctx->d_status, sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream));
     CUDA_CHECK(cudaStreamSynchronize(ctx->stream));
-    const uint32_t s = *ctx->h_status;
+    const uint32_t s = *static_cast<volatile uint32_t*>(ctx->h_status);
     if (s == 0) return FND_OK;
     CUDA_CHECK(cudaMemsetAsync(ctx->d_status, 0, sizeof(uint32_t), ctx->stream));
     CUDA_CHECK(cudaStreamSynchronize(ctx->stream));
@@ -242,6 +243,10 @@ int fnd_rt_create(const fnd_rt_desc* desc, fnd_rt_ctx** out_ctx) {
         auto ctx = std::make_unique<fnd_rt_ctx>();
         ctx->device = desc->device;
         ctx->sm_count = prop.multiProcessorCount;
+        int by_host_tables = 0;
+        CUDA_CHECK(cudaDeviceGetAttribute(&by_host_tables, cudaDevAttrPageableMemoryAccessUsesHostPageTables,
+                                          ctx->device));
+        ctx->coherent_host = by_host_tables != 0;
         CUDA_CHECK(cudaSetDevice(ctx->device));
         auto cleanup = [&](fnd_rt_ctx* c) {
             if (c->d_counter) cudaFree(c->d_counter);
@@ -264,6 +269,10 @@ int fnd_rt_create(const fnd_rt_desc* desc, fnd_rt_ctx** out_ctx) {
             ctx->d_render_stats = reinterpret_cast<unsigned long long*>(scratch + 768);
             CUDA_CHECK(cudaMemsetAsync(scratch, 0, 1024, ctx->stream));
             CUDA_CHECK(cudaMallocHost(&ctx->h_status, sizeof(uint32_t)));
+            *ctx->h_status = 0;
+            // kernels only write the status word, and only on a failure: there the
+            // host reads it where it lies (a copy of four bytes takes 8 us)
+            if (ctx->coherent_host) ctx->d_status = ctx->h_status;
             for (int v = 0; v < 4; ++v) CUDA_CHECK(RT::TraceOccupancy(v, &ctx->occupancy[v]));
             CUDA_CHECK(cudaStreamSynchronize(ctx->stream));
         } catch (...) {
@@ -553,8 +562,21 @@ namespace {
 // Per chunk the launch, its tail and the stream waits cost more than the
 // shorter uncovered first copy saves below 2^20 rays per chunk (measured:
 // 8.4M rays in 8 chunks 2.74 ms, in 16 chunks 2.91 ms per call).
+//
+// Where the GPU shares the host's page tables (Grace) the traversal reads the
+// rays in place instead: a ray is read once, at a refill, and those reads hide
+// behind the other warps' work (4.2M Cornell rays: 903 us, 875 from device
+// memory, 1,119 with the pipeline of copies; pageable rays 2,300). Hits are
+// written in place for up to kHitsInPlace rays; past that the 8-byte writes in
+// ray-completion order are slower than a copy (4.2M: 1,218 in place; 262,144:
+// 138 and 143; 1M: 350 and 334). The copy back is covered by one more launch
+// for the last eighth once it takes longer than a launch costs (4.2M: 1,091
+// without, 1,018; a fifth 1,045, a twelfth 1,046; 1M: 333 without, 328).
+constexpr uint32_t kHitsInPlace = 1u << 18;
+constexpr uint32_t kSplitInPlace = 3u << 19;
 constexpr uint32_t kPipeMinChunk = 1u << 19;
 constexpr uint32_t kPipeMaxChunks = 16;
+
 
 uint32_t PipelineChunk(uint32_t n) {
     uint32_t chunk = std::max(kPipeMinChunk, (n + 7u) / 8u);
@@ -628,12 +650,27 @@ int TraceImpl(fnd_rt_ctx* ctx, const fnd_rt_scene* scene, const fnd_ray* rays, u
                        "device rays must be 16-byte aligned and hits 8-byte aligned");
             launch(reinterpret_cast<const float4*>(rays), n, out, ctx->stream, ctx->d_counter);
         } else if (n > 0) {
-            EnsureDevice(ctx->d_in, ctx->d_in_cap, sizeof(fnd_ray) * (size_t)n);
-            EnsureDevice(ctx->d_out, ctx->d_out_cap, hit_bytes * (size_t)n);
+            // rays read in place by the traversal (not where a pass reads them
+            // more than once: coherence order, two levels; nor where hits would
+            // come to lie over rays that are still to be read)
+            const auto* rays_end = reinterpret_cast<const char*>(rays + n);
+            const bool apart = static_cast<char*>(out) >= rays_end ||
+                               static_cast<char*>(out) + hit_bytes * (size_t)n <= reinterpret_cast<const char*>(rays);
+            const bool in_place = ctx->coherent_host && !stats && !scene->two_level && ctx->trace_cfg.sort_bits == 0 &&
+                                  ((uintptr_t)rays & 15u) == 0 && apart;
+            const bool out_in_place =
+                in_place && n <= kHitsInPlace && ((uintptr_t)out & (any ? 0u : 7u)) == 0;
+            if (!in_place) EnsureDevice(ctx->d_in, ctx->d_in_cap, sizeof(fnd_ray) * (size_t)n);
+            if (!out_in_place) EnsureDevice(ctx->d_out, ctx->d_out_cap, hit_bytes * (size_t)n);
             auto* d_in = static_cast<char*>(ctx->d_in);
             auto* d_out = static_cast<char*>(ctx->d_out);
-            const uint32_t chunk = PipelineChunk(n);
-            if (stats || n <= chunk) {
+            const uint32_t chunk = in_place ? (n > kSplitInPlace ? n - n / 8 : n) : PipelineChunk(n);
+            if (out_in_place) {
+                launch(reinterpret_cast<const float4*>(rays), n, out, ctx->stream, ctx->d_counter);
+                copied_back = true;
+            } else if (in_place && n <= chunk) {
+                launch(reinterpret_cast<const float4*>(rays), n, d_out, ctx->stream, ctx->d_counter);
+            } else if (stats || n <= chunk) {
                 CUDA_CHECK(cudaMemcpyAsync(d_in, rays, sizeof(fnd_ray) * (size_t)n, cudaMemcpyHostToDevice,
                                            ctx->stream));
                 launch(reinterpret_cast<const float4*>(d_in), n, d_out, ctx->stream, ctx->d_counter);
@@ -654,30 +691,42 @@ int TraceImpl(fnd_rt_ctx* ctx, const fnd_rt_scene* scene, const fnd_ray* rays, u
                     // the copy and compute streams start after the context
                     // stream's earlier work
                     CUDA_CHECK(cudaEventRecord(ev[0], ctx->stream));
-                    CUDA_CHECK(cudaStreamWaitEvent(ctx->copy_in, ev[0], 0));
+                    if (!in_place) CUDA_CHECK(cudaStreamWaitEvent(ctx->copy_in, ev[0], 0));
                     CUDA_CHECK(cudaStreamWaitEvent(ctx->copy_out, ev[0], 0));
                     if (two) CUDA_CHECK(cudaStreamWaitEvent(ctx->compute2, ev[0], 0));
-                    // chunk 0 is a quarter of the others: its copy in is
-                    // the part of the copies no traversal covers
-                    const uint32_t c0 = chunk / 4;
+                    // with copies in, chunk 0 is a quarter of the others: its
+                    // copy in is the part of the copies no traversal covers
+                    const uint32_t c0 = in_place ? chunk : chunk / 4;
                     const uint32_t chunks = 1 + (n - c0 + chunk - 1) / chunk;
                     CHECK(2 + 2 * (size_t)chunks <= sizeof(ctx->pipe_ev) / sizeof(ctx->pipe_ev[0]));
+                    auto first_of = [&](uint32_t k) -> size_t {
+                        return k == 0 ? 0 : (size_t)c0 + (size_t)(k - 1) * chunk;
+                    };
                     for (uint32_t k = 0; k < chunks; ++k) {
-                        const size_t first = k == 0 ? 0 : (size_t)c0 + (size_t)(k - 1) * chunk;
-                        const uint32_t cnt = (uint32_t)std::min<size_t>(k == 0 ? c0 : chunk, n - first);
+                        const size_t first = first_of(k);
+                        const uint32_t cnt = (uint32_t)((k + 1 < chunks ? first_of(k + 1) : n) - first);
                         cudaEvent_t in_done = ev[2 + 2 * k], traced = ev[3 + 2 * k];
-                        CUDA_CHECK(cudaMemcpyAsync(d_in + sizeof(fnd_ray) * first, rays + first,
-                                                   sizeof(fnd_ray) * cnt, cudaMemcpyHostToDevice, ctx->copy_in));
-                        CUDA_CHECK(cudaEventRecord(in_done, ctx->copy_in));
                         // odd chunks on the second compute stream, with the
                         // counter 32 bytes further in the counter slot
                         const bool odd = two && (k & 1u);
                         cudaStream_t cs = odd ? ctx->compute2 : ctx->stream;
-                        CUDA_CHECK(cudaStreamWaitEvent(cs, in_done, 0));
-                        launch(reinterpret_cast<const float4*>(d_in + sizeof(fnd_ray) * first), cnt,
-                               d_out + hit_bytes * first, cs, ctx->d_counter + (odd ? 8 : 0));
+                        if (!in_place) {
+                            CUDA_CHECK(cudaMemcpyAsync(d_in + sizeof(fnd_ray) * first, rays + first,
+                                                       sizeof(fnd_ray) * cnt, cudaMemcpyHostToDevice, ctx->copy_in));
+                            CUDA_CHECK(cudaEventRecord(in_done, ctx->copy_in));
+                            CUDA_CHECK(cudaStreamWaitEvent(cs, in_done, 0));
+                        }
+                        launch(in_place ? reinterpret_cast<const float4*>(rays + first)
+                                        : reinterpret_cast<const float4*>(d_in + sizeof(fnd_ray) * first),
+                               cnt, d_out + hit_bytes * first, cs, ctx->d_counter + (odd ? 8 : 0));
                         CUDA_CHECK(cudaEventRecord(traced, cs));
-                        CUDA_CHECK(cudaStreamWaitEvent(ctx->copy_out, traced, 0));
+                    }
+                    // (a copy to pageable memory returns only when it is done:
+                    // all launches are queued before the first)
+                    for (uint32_t k = 0; k < chunks; ++k) {
+                        const size_t first = first_of(k);
+                        const size_t cnt = (k + 1 < chunks ? first_of(k + 1) : n) - first;
+                        CUDA_CHECK(cudaStreamWaitEvent(ctx->copy_out, ev[3 + 2 * k], 0));
                         CUDA_CHECK(cudaMemcpyAsync(static_cast<char*>(out) + hit_bytes * first,
                                                    d_out + hit_bytes * first, hit_bytes * cnt,
                                                    cudaMemcpyDeviceToHost, ctx->copy_out));

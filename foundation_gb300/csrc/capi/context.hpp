@@ -40,6 +40,7 @@ struct fnd_rt_ctx {
     cudaStream_t stream = nullptr;
     bool own_stream = false;
     int sm_count = 0;
+    bool coherent_host = false;    // the GPU reads and writes any host memory in place, through the host's page tables
     int occupancy[4] = {0, 0, 0, 0};  // blocks/SM of the trace kernel variants
     uint32_t refill_min = 8;
     // device scratch owned by the context

@@ -137,3 +137,45 @@ def test_rays_of_a_warps_paths(ctx, width, height, sun):
     assert got[0][1:] == got[1][1:]
     np.testing.assert_allclose(got[1][0], got[0][0], rtol=72 * 2.0 ** -24, atol=0)
     s.close()
+
+
+@pytest.mark.parametrize("n", [1, 33, (1 << 18) - 1, 1 << 18, (1 << 18) + 1, 3 << 19, (3 << 19) + 9])
+@pytest.mark.parametrize("kind", ["pageable", "pinned", "rays off by 4 bytes", "hits off by 4 bytes", "overlap"])
+def test_host_rays_in_place(ctx, n, kind):
+    """Host rays are traced where they lie, and small batches' hits written
+    there; past a size the hits are copied back, past another in two parts;
+    unaligned buffers and ones that overlap take copies. All as from the
+    device, to the bit."""
+    import torch
+
+    import foundation_gb300 as fg
+    if kind == "overlap" and n > 1 << 19:
+        pytest.skip("copied in parts: hits may land on rays that are still to be copied")
+    sc = S.soup_scene(3000, seed=5)
+    s = ctx.upload(sc.verts, sc.idx)
+    rays = _rays(n)
+    dev = torch.from_numpy(rays).cuda()
+    want = torch.empty(2 * n, dtype=torch.int32, device="cuda")
+    occ = torch.empty(n, dtype=torch.uint8, device="cuda")
+    s.closest(dev, want)
+    s.any(dev, occ)
+    ctx.sync()
+    want, occ = want.cpu().numpy().view(np.uint32).reshape(n, 2), occ.cpu().numpy()
+    dt = fg.rt.HIT_DTYPE
+    if kind == "pinned":
+        rb, hb = fg.rt.PinnedBuffer(32 * n), fg.rt.PinnedBuffer(8 * n)
+        hr, out = rb.view(np.float32, (n, 8)), hb.view(dt, (n,))
+    else:
+        room = np.zeros(40 * n + 64, np.uint8)
+        at = -room.ctypes.data % 16 + (4 if kind == "rays off by 4 bytes" else 0)
+        hr = room[at:at + 32 * n].view(np.float32).reshape(n, 8)
+        to = at + 32 * n + (-(at + 32 * n + room.ctypes.data)) % 8 + (4 if kind == "hits off by 4 bytes" else 0)
+        out = (room[at:at + 8 * n] if kind == "overlap" else room[to:to + 8 * n]).view(dt)
+    hr[:] = rays
+    if kind != "overlap":
+        got = np.full(n, 7, np.uint8)
+        s.any(hr, got)
+        assert (got == occ).all()
+    s.closest(hr, out)
+    assert (out["prim"] == want[:, 0]).all() and (out["t"].view(np.uint32) == want[:, 1]).all()
+    s.close()
