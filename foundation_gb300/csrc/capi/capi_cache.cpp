@@ -290,16 +290,27 @@ int fnd_rt_cache_gradient(fnd_rt_ctx* ctx, const float* features, const float* t
         CHECK(n >= 1 && features && targets && grad);
         CUDA_CHECK(cudaSetDevice(ctx->device));
         const size_t in_b = 4ull * n * NRC::kIn, t_b = 4ull * n * 3;
-        EnsureDevice(ctx->d_in, ctx->d_in_cap, in_b + t_b);
-        char* d = static_cast<char*>(ctx->d_in);
-        CUDA_CHECK(cudaMemcpyAsync(d, features, in_b, cudaMemcpyHostToDevice, ctx->stream));
-        CUDA_CHECK(cudaMemcpyAsync(d + in_b, targets, t_b, cudaMemcpyHostToDevice, ctx->stream));
-        CUDA_CHECK(NRC::GradRaw(c.net, reinterpret_cast<const float*>(d), reinterpret_cast<const float*>(d + in_b), n,
-                                ctx->d_status, ctx->stream));
-        double l = 0.0;
-        CUDA_CHECK(cudaMemcpyAsync(grad, c.net.grad, 4ull * NRC::kNumParams, cudaMemcpyDeviceToHost, ctx->stream));
-        CUDA_CHECK(cudaMemcpyAsync(&l, c.net.loss, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+        // the kernel reads features and targets once, in place where it can
+        const bool in_place = ctx->coherent_host && ((uintptr_t)features & 15u) == 0 && ((uintptr_t)targets & 3u) == 0;
+        const float *f = features, *t = targets;
+        if (!in_place) {
+            EnsureDevice(ctx->d_in, ctx->d_in_cap, in_b + t_b);
+            char* d = static_cast<char*>(ctx->d_in);
+            f = reinterpret_cast<const float*>(d);
+            t = reinterpret_cast<const float*>(d + in_b);
+            CUDA_CHECK(cudaMemcpyAsync(d, features, in_b, cudaMemcpyHostToDevice, ctx->stream));
+            CUDA_CHECK(cudaMemcpyAsync(d + in_b, targets, t_b, cudaMemcpyHostToDevice, ctx->stream));
+        }
+        try {
+            CUDA_CHECK(NRC::GradRaw(c.net, f, t, n, ctx->d_status, ctx->stream));
+            CUDA_CHECK(cudaMemcpyAsync(ctx->h_loss, c.net.loss, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+            CUDA_CHECK(cudaMemcpyAsync(grad, c.net.grad, 4ull * NRC::kNumParams, cudaMemcpyDeviceToHost, ctx->stream));
+        } catch (...) {
+            cudaStreamSynchronize(ctx->stream);  // the caller's buffers are still read
+            throw;
+        }
         CUDA_CHECK(cudaStreamSynchronize(ctx->stream));
+        const double l = *ctx->h_loss;
         if (loss) *loss = l / (3.0 * n);
     });
 }

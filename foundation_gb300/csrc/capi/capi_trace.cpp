@@ -268,8 +268,9 @@ int fnd_rt_create(const fnd_rt_desc* desc, fnd_rt_ctx** out_ctx) {
             ctx->d_stats = reinterpret_cast<unsigned long long*>(scratch + 512);
             ctx->d_render_stats = reinterpret_cast<unsigned long long*>(scratch + 768);
             CUDA_CHECK(cudaMemsetAsync(scratch, 0, 1024, ctx->stream));
-            CUDA_CHECK(cudaMallocHost(&ctx->h_status, sizeof(uint32_t)));
+            CUDA_CHECK(cudaMallocHost(&ctx->h_status, 16));
             *ctx->h_status = 0;
+            ctx->h_loss = reinterpret_cast<double*>(ctx->h_status + 2);
             // kernels only write the status word, and only on a failure: there the
             // host reads it where it lies (a copy of four bytes takes 8 us)
             if (ctx->coherent_host) ctx->d_status = ctx->h_status;

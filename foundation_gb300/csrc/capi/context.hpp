@@ -48,6 +48,7 @@ struct fnd_rt_ctx {
     uint32_t* d_status = nullptr;
     unsigned long long* d_stats = nullptr;
     uint32_t* h_status = nullptr;  // pinned
+    double* h_loss = nullptr;      // (behind it)
     // staging buffers for FND_MEM_HOST calls
     void* d_in = nullptr;
     size_t d_in_cap = 0;

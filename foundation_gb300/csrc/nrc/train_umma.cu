@@ -21,8 +21,12 @@
 //      dH_l  = dZ_l W_l^T   (M = 128 rows), and the epilogue masks dH_l by
 //                            H_l > 0 into dZ_{l-1} (BF16);
 //  * the weight gradients stay in tensor memory for all of a CTA's tiles and
-//    are added to the global FP32 gradient once, with vector atomics.
-// One elected thread issues every MMA and commits it to one mbarrier; each
+//    are added to the global FP32 gradient once, by the TMA.
+// What bounds it: a chain of twelve GEMMs of a few hundred cycles each, one
+// tile per CTA; so what counts is the latency around them. One elected lane
+// issues every MMA (issued by thread 0 under a plain branch, four took 850
+// cycles: 12 phases of 1,550; elected, unrolled 270: 960 forward, 1,550
+// backward) and commits it to one mbarrier; each
 // wait for it is bounded and, when it runs out, the step latches the
 // timeout bit of the status word, stops, and still releases its tensor
 // memory. Adam (mlp.cu) then applies the gradient.
@@ -62,6 +66,11 @@ static_assert(kSmWb % 1024 == 0 && kSmX % 1024 == 0 && kSmH % 1024 == 0 && kSmDz
 // bytes (into H1) and past H5 by 1024 bytes (into dZ): both stay inside
 static_assert(kSmBytes <= 227 * 1024, "shared memory");
 
+// the gradient as the parts in which the TMA adds it to the global one
+constexpr uint32_t kReduceParts = 20, kReduceFloats = kNumParams / kReduceParts;
+static_assert(kReduceParts * kReduceFloats == kNumParams && kReduceFloats % 4 == 0, "16-byte parts");
+static_assert(4 * kNumParams <= kSmTgt - kSmX, "the gradient fits the activations' space");
+
 struct TrainArgs {
     Net net;
     const TrainSample* samples;  // sampled mode
@@ -93,27 +102,40 @@ __device__ __forceinline__ uint64_t mnmajor(uint32_t saddr, uint32_t cols) {
     return smem_desc(saddr, cols / 8u * 128u, 128u);
 }
 
+// Explicit features (host or device memory): a row's 96 floats are contiguous,
+// so the tile is read as one run of float4.
+__device__ __forceinline__ void stage_raw(const TrainArgs& A, unsigned char* smem, uint32_t tile, uint32_t tid) {
+    const uint32_t rows = min(kRows, A.rows - tile * kRows);
+    const float4* src = reinterpret_cast<const float4*>(A.raw_feats + (size_t)tile * kRows * kIn);
+    float4 v[kRows * kIn / 4 / kThreads];
+#pragma unroll
+    for (uint32_t i = 0; i < kRows * kIn / 4 / kThreads; ++i) {
+        const uint32_t e = tid + kThreads * i;
+        v[i] = e < rows * (kIn / 4) ? __ldcs(src + e) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    float4 tg = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (tid < rows) {
+        const float* t = A.raw_targets + 3 * ((size_t)tile * kRows + tid);
+        tg = make_float4(t[0], t[1], t[2], 1.0f);
+    }
+#pragma unroll
+    for (uint32_t i = 0; i < kRows * kIn / 4 / kThreads; ++i) {
+        const uint32_t e = tid + kThreads * i, r = e / (kIn / 4), c = e % (kIn / 4) * 4;
+        *reinterpret_cast<uint2*>(smem + kSmX + canon_offset(r, c, kIn)) =
+            make_uint2(bf16_bits(v[i].x) | (uint32_t)bf16_bits(v[i].y) << 16,
+                       bf16_bits(v[i].z) | (uint32_t)bf16_bits(v[i].w) << 16);
+    }
+    if (tid < kRows) reinterpret_cast<float4*>(smem + kSmTgt)[tid] = tg;
+}
+
 // Row r's 48 features of one half (tid & 1) into the X array.
-template <bool kRaw>
 __device__ __forceinline__ void stage_inputs(const TrainArgs& A, unsigned char* smem, uint32_t tile, uint32_t count,
                                              uint32_t tid) {
     const uint32_t r = tid >> 1, half = tid & 1;
     const uint32_t b = tile * kRows + r;
     uint16_t f[96];
     float4 tg = make_float4(0.f, 0.f, 0.f, 0.f);
-    const bool valid = b < A.rows && count > 0;
-    if (valid && kRaw) {
-        const float* src = A.raw_feats + (size_t)b * kIn;
-        if (half == 0) {
-#pragma unroll
-            for (int i = 0; i < 48; ++i) f[i] = bf16_bits(src[i]);
-            tg = make_float4(A.raw_targets[3 * (size_t)b], A.raw_targets[3 * (size_t)b + 1],
-                             A.raw_targets[3 * (size_t)b + 2], 1.0f);
-        } else {
-#pragma unroll
-            for (int i = 48; i < 96; ++i) f[i] = bf16_bits(src[i]);
-        }
-    } else if (valid) {
+    if (b < A.rows && count > 0) {
         const uint32_t si = pcg_hash(A.seed ^ pcg_hash(b)) % count;
         const CachePoint pt = A.samples[si].pt;
         encode_half(pt, A.net.lo, A.net.hi, (int)half, f);
@@ -162,7 +184,8 @@ __global__ void __launch_bounds__(kThreads, 1) train_umma_kernel(const TrainArgs
     __shared__ uint64_t s_mbar_w;  // weight images in shared memory
     __shared__ uint32_t s_tmem;
     __shared__ int s_abort;
-    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const uint32_t tid = threadIdx.x, lane = tid & 31;
+    const uint32_t warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0);  // (uniform for the compiler too)
     const uint32_t quarter = warp & 3, chalf = warp >> 2;
     const uint32_t row = 32 * quarter + lane;  // the tile row (tensor-memory lane) of this thread's epilogue
     const uint32_t sbase = smem_u32(smem);
@@ -178,7 +201,7 @@ __global__ void __launch_bounds__(kThreads, 1) train_umma_kernel(const TrainArgs
         bulk_g2s(smem + kSmWb, A.net.ubwd, 2 * kUBwdElems, &s_mbar_w);
     }
     if (warp == 0) tmem_alloc(&s_tmem, kTmemCols);
-    bool weights_ready = false;  // thread 0: the bulk copies have landed
+    bool weights_ready = false;  // warp 0: the bulk copies have landed
     fence_before_sync();
     __syncthreads();
     fence_after_sync();
@@ -201,24 +224,33 @@ __global__ void __launch_bounds__(kThreads, 1) train_umma_kernel(const TrainArgs
     };
 
     for (uint32_t tile = blockIdx.x; tile < ntiles && alive; tile += gridDim.x) {
-        stage_inputs<kRaw>(A, smem, tile, count, tid);
+        if constexpr (kRaw)
+            stage_raw(A, smem, tile, tid);
+        else
+            stage_inputs(A, smem, tile, count, tid);
         publish_smem();
         // ---- forward ----------------------------------------------------
-        for (int l = 0; l < kLayers && alive; ++l) {
+#pragma unroll
+        for (int l = 0; l < kLayers; ++l) {
+            if (!alive) break;
             const uint32_t K = LayerK(l), N = UmmaN(l);
-            if (tid == 0) {
-                if (!weights_ready) weights_ready = mbar_wait(&s_mbar_w, 0, kWaitLimit);
-                if (weights_ready) {
-                    const uint32_t a0 = sbase + (l == 0 ? kSmX : kSmH + (l - 1) * kHBytes);
-                    const uint32_t b0 = sbase + kSmWf + 2 * UFwdOffset(l);
-                    const uint32_t idesc = instr_desc_bf16(128, N, false, false);
-                    for (uint32_t k = 0; k < K / 16; ++k)
-                        mma_bf16(tmem + kColZ, kmajor(a0 + 256 * k, K), kmajor(b0 + 256 * k, K), idesc, k > 0);
-                    mma_commit(&s_mbar);
-                } else {
-                    s_abort = 1;          // the copies never landed: complete the phase
-                    mbar_arrive(&s_mbar);  // without an MMA and stop
+            if (warp == 0) {
+                if (!weights_ready) weights_ready = __all_sync(0xFFFFFFFFu, mbar_wait(&s_mbar_w, 0, kWaitLimit));
+                if (elect_one()) {
+                    if (weights_ready) {
+                        const uint32_t a0 = sbase + (l == 0 ? kSmX : kSmH + (l - 1) * kHBytes);
+                        const uint32_t b0 = sbase + kSmWf + 2 * UFwdOffset(l);
+                        const uint32_t idesc = instr_desc_bf16(128, N, false, false);
+#pragma unroll
+                        for (uint32_t k = 0; k < K / 16; ++k)
+                            mma_bf16(tmem + kColZ, kmajor(a0 + 256 * k, K), kmajor(b0 + 256 * k, K), idesc, k > 0);
+                        mma_commit(&s_mbar);
+                    } else {
+                        s_abort = 1;           // the copies never landed: complete the phase
+                        mbar_arrive(&s_mbar);  // without an MMA and stop
+                    }
                 }
+                __syncwarp();
             }
             alive = wait_mma();
             if (!alive) break;
@@ -263,24 +295,31 @@ __global__ void __launch_bounds__(kThreads, 1) train_umma_kernel(const TrainArgs
             publish_smem();
         }
         // ---- backward ---------------------------------------------------
-        for (int l = kLayers - 1; l >= 0 && alive; --l) {
+#pragma unroll
+        for (int l = kLayers - 1; l >= 0; --l) {
+            if (!alive) break;
             const uint32_t F = LayerK(l), Nb = UmmaN(l);
-            if (tid == 0) {
-                const uint32_t h0 = sbase + (l == 0 ? kSmX : kSmH + (l - 1) * kHBytes);
-                const uint32_t dz0 = sbase + kSmDz;
-                // dW_l (+)= H_l^T dZ_l over this tile's rows
-                const uint32_t idesc_w = instr_desc_bf16(128, Nb, true, true);
-                for (uint32_t k = 0; k < kRows / 16; ++k)
-                    mma_bf16(tmem + kColDW + 64 * l, mnmajor(h0 + 2 * (F / 8 * 128) * k, F),
-                             mnmajor(dz0 + 2 * (Nb / 8 * 128) * k, Nb), idesc_w, !first || k > 0);
-                if (l > 0) {
-                    // dH_l = dZ_l W_l^T
-                    const uint32_t b0 = sbase + kSmWb + 2 * UBwdOffset(l);
-                    const uint32_t idesc_a = instr_desc_bf16(128, kWidth, false, false);
-                    for (uint32_t k = 0; k < Nb / 16; ++k)
-                        mma_bf16(tmem + kColDH, kmajor(dz0 + 256 * k, Nb), kmajor(b0 + 256 * k, Nb), idesc_a, k > 0);
+            if (warp == 0) {
+                if (elect_one()) {
+                    const uint32_t h0 = sbase + (l == 0 ? kSmX : kSmH + (l - 1) * kHBytes);
+                    const uint32_t dz0 = sbase + kSmDz;
+                    if (l > 0) {
+                        // dH_l = dZ_l W_l^T
+                        const uint32_t b0 = sbase + kSmWb + 2 * UBwdOffset(l);
+                        const uint32_t idesc_a = instr_desc_bf16(128, kWidth, false, false);
+#pragma unroll
+                        for (uint32_t k = 0; k < Nb / 16; ++k)
+                            mma_bf16(tmem + kColDH, kmajor(dz0 + 256 * k, Nb), kmajor(b0 + 256 * k, Nb), idesc_a, k > 0);
+                    }
+                    // dW_l (+)= H_l^T dZ_l over this tile's rows
+                    const uint32_t idesc_w = instr_desc_bf16(128, Nb, true, true);
+#pragma unroll
+                    for (uint32_t k = 0; k < kRows / 16; ++k)
+                        mma_bf16(tmem + kColDW + 64 * l, mnmajor(h0 + 2 * (F / 8 * 128) * k, F),
+                                 mnmajor(dz0 + 2 * (Nb / 8 * 128) * k, Nb), idesc_w, !first || k > 0);
+                    mma_commit(&s_mbar);
                 }
-                mma_commit(&s_mbar);
+                __syncwarp();
             }
             alive = wait_mma();
             if (!alive || l == 0) break;
@@ -309,29 +348,55 @@ __global__ void __launch_bounds__(kThreads, 1) train_umma_kernel(const TrainArgs
         }
         first = false;
     }
-    // ---- the CTA's weight gradients -> global (FP32 vector atomics) --------
+    // ---- the CTA's weight gradients -> global -----------------------------
+    // Through shared memory (the activations' space: every MMA is done) as one
+    // array in the order of the parameters, which the TMA adds to the global
+    // one. Each CTA starts elsewhere in it, so they do not queue for the same
+    // lines. (Vector atomics from registers, a row per lane, took 13,500 of the
+    // kernel's 40,600 cycles; this takes 8,500 of 31,000.)
     if (alive && !first) {
+        float* out = reinterpret_cast<float*>(smem + kSmX);
 #pragma unroll 1
         for (int l = 0; l < kLayers; ++l) {
             const uint32_t F = LayerK(l), N = LayerN(l);
             if (32 * quarter >= F) continue;  // whole warp: rows past the layer's inputs are padding
-            float* G = A.net.grad + ParamOffset(l) + (size_t)row * N;
+            float* G = out + ParamOffset(l) + (size_t)row * N;
             if (l + 1 < kLayers) {
                 uint32_t v[32];
                 tmem_ld16(tmem_addr(tmem, 32 * quarter, kColDW + 64 * l + 32 * chalf), v);
                 tmem_ld16(tmem_addr(tmem, 32 * quarter, kColDW + 64 * l + 32 * chalf + 16), v + 16);
                 tmem_ld_wait();
+                // The rows lie 256 bytes apart: lane i writes its eight vectors
+                // in the order j ^ (i & 7), so eight lanes cover all banks.
+#pragma unroll
+                for (int b = 1; b < 8; b <<= 1)
+#pragma unroll
+                    for (int j = 0; j < 8; ++j)
+                        if (!(j & b))
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) {
+                                const uint32_t x = v[4 * j + e], y = v[4 * (j | b) + e];
+                                v[4 * j + e] = lane & b ? y : x;
+                                v[4 * (j | b) + e] = lane & b ? x : y;
+                            }
 #pragma unroll
                 for (int j = 0; j < 8; ++j)
-                    atomicAdd(reinterpret_cast<float4*>(G + 32 * chalf + 4 * j),
-                              make_float4(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]),
-                                          __uint_as_float(v[4 * j + 2]), __uint_as_float(v[4 * j + 3])));
+                    *reinterpret_cast<uint4*>(G + 32 * chalf + 4 * (j ^ (lane & 7u))) =
+                        make_uint4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
             } else if (chalf == 0) {
                 uint32_t v[16];
                 tmem_ld16(tmem_addr(tmem, 32 * quarter, kColDW + 64 * l), v);
                 tmem_ld_wait();
-                for (int c = 0; c < 3; ++c) atomicAdd(G + c, __uint_as_float(v[c]));
+                for (int c = 0; c < 3; ++c) G[c] = __uint_as_float(v[c]);
             }
+        }
+        publish_smem();
+        if (tid == 0) {
+            for (uint32_t i = 0; i < kReduceParts; ++i) {
+                const uint32_t at = (i + blockIdx.x) % kReduceParts * kReduceFloats;
+                bulk_reduce_add(A.net.grad + at, out + at, 4 * kReduceFloats);
+            }
+            bulk_reduce_wait();
         }
     }
     if (!alive) {
@@ -386,8 +451,10 @@ cudaError_t GradRaw(const Net& net, const float* feats, const float* targets, ui
                     cudaStream_t s) {
     cudaError_t e = allow_smem(train_umma_kernel<true>);
     if (e != cudaSuccess) return e;
-    e = cudaMemsetAsync(net.grad, 0, sizeof(float) * kNumParams, s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(net.loss, 0, sizeof(double), s);
+    // (the loss may lie directly behind the gradient: one launch clears both)
+    const bool one = reinterpret_cast<char*>(net.loss) == reinterpret_cast<char*>(net.grad + kNumParams);
+    e = cudaMemsetAsync(net.grad, 0, sizeof(float) * kNumParams + (one ? sizeof(double) : 0), s);
+    if (e == cudaSuccess && !one) e = cudaMemsetAsync(net.loss, 0, sizeof(double), s);
     if (e != cudaSuccess || n == 0) return e;
     TrainArgs A{};
     A.net = net;

@@ -84,6 +84,17 @@ __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t a_desc, uint6
         "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate ? 1u : 0u)
         : "memory");
 }
+// One lane of a converged warp (the same one at every call): MMAs are issued
+// under it, so the compiler keeps their descriptors in uniform registers.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "elect.sync _|p, 0xFFFFFFFF;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}\n"
+        : "=r"(p));
+    return p != 0;
+}
 // The barrier at `mbar` gets one arrival once every MMA this thread issued
 // before has completed.
 __device__ __forceinline__ void mma_commit(uint64_t* mbar) {
@@ -127,6 +138,18 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* mbar) {
 __device__ __forceinline__ void mbar_expect_tx(uint64_t* mbar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(mbar)), "r"(bytes)
                  : "memory");
+}
+
+// ---- bulk reduction (TMA, untiled) -----------------------------------------
+// global[i] += shared[i] over `bytes` of floats, both 16-byte aligned, `bytes`
+// a multiple of 16. bulk_reduce_wait: all that this thread started are done.
+__device__ __forceinline__ void bulk_reduce_add(float* dst, const void* src_smem, uint32_t bytes) {
+    asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;" ::"l"(dst),
+                 "r"(smem_u32(src_smem)), "r"(bytes)
+                 : "memory");
+}
+__device__ __forceinline__ void bulk_reduce_wait() {
+    asm volatile("cp.async.bulk.commit_group;\n\tcp.async.bulk.wait_group 0;" ::: "memory");
 }
 
 // ---- bulk copy (TMA, untiled) ----------------------------------------------
