@@ -302,9 +302,15 @@ int fnd_rt_cache_gradient(fnd_rt_ctx* ctx, const float* features, const float* t
             CUDA_CHECK(cudaMemcpyAsync(d + in_b, targets, t_b, cudaMemcpyHostToDevice, ctx->stream));
         }
         try {
-            CUDA_CHECK(NRC::GradRaw(c.net, f, t, n, ctx->d_status, ctx->stream));
-            CUDA_CHECK(cudaMemcpyAsync(ctx->h_loss, c.net.loss, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-            CUDA_CHECK(cudaMemcpyAsync(grad, c.net.grad, 4ull * NRC::kNumParams, cudaMemcpyDeviceToHost, ctx->stream));
+            const bool out_in_place = ctx->coherent_host && ((uintptr_t)grad & 15u) == 0;
+            CUDA_CHECK(NRC::GradRaw(c.net, f, t, n, out_in_place ? grad : nullptr, ctx->h_loss, ctx->d_status,
+                                    ctx->stream));
+            if (!out_in_place) {
+                CUDA_CHECK(
+                    cudaMemcpyAsync(ctx->h_loss, c.net.loss, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+                CUDA_CHECK(cudaMemcpyAsync(grad, c.net.grad, 4ull * NRC::kNumParams, cudaMemcpyDeviceToHost,
+                                           ctx->stream));
+            }
         } catch (...) {
             cudaStreamSynchronize(ctx->stream);  // the caller's buffers are still read
             throw;

@@ -87,7 +87,7 @@ struct Net {
     float* adam_m;
     float* adam_v;
     float* grad;      // fp32 gradient accumulator (kNumParams)
-    double* loss;     // [0] running sum of the loss of the current step
+    double* loss;     // [0] running sum of the loss of the current step, [1] CTAs done (GradRaw)
     uint32_t step;    // Adam steps taken
     // weight averaging (queries only): fp32 moving average of the iterates
     // and the bf16 forward image of avg / (1 - decay^avg_steps); null: off
@@ -110,9 +110,11 @@ cudaError_t InferRaw(const Net& net, const float* feats, uint32_t n, float* out,
 // *status and ends the step early.
 cudaError_t TrainStep(Net& net, const TrainSample* smp, const float4* targets, const uint32_t* count,
                       uint32_t batch, uint64_t seed, float lr, uint32_t* status, cudaStream_t s);
-// Test hook: gradient of the loss on explicit features / targets (no Adam).
-cudaError_t GradRaw(const Net& net, const float* feats, const float* targets, uint32_t n, uint32_t* status,
-                    cudaStream_t s);
+// Gradient of the loss on explicit features / targets (no Adam), in net.grad and
+// net.loss; with out_grad the last CTA also copies both to out_grad and out_loss.
+// Every pointer may be to host memory that the device reads and writes.
+cudaError_t GradRaw(const Net& net, const float* feats, const float* targets, uint32_t n, float* out_grad,
+                    double* out_loss, uint32_t* status, cudaStream_t s);
 cudaError_t AdamRaw(Net& net, float lr, cudaStream_t s);
 // The step's gradient alone (train_umma.cu): accumulates into net.grad.
 cudaError_t LaunchTrainUmma(const Net& net, const TrainSample* smp, const float4* targets, const uint32_t* count,

@@ -152,6 +152,9 @@ __device__ __forceinline__ void bulk_reduce_wait() {
     asm volatile("cp.async.bulk.commit_group;\n\tcp.async.bulk.wait_group 0;" ::: "memory");
 }
 
+// Orders this thread's generic accesses and completed bulk operations.
+__device__ __forceinline__ void fence_proxies() { asm volatile("fence.proxy.async;" ::: "memory"); }
+
 // ---- bulk copy (TMA, untiled) ----------------------------------------------
 // global -> shared, both 16-byte aligned, `bytes` a multiple of 16; the bytes
 // count towards the barrier's expected transaction bytes.
