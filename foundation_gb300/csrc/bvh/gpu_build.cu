@@ -447,6 +447,133 @@ __host__ __device__ __forceinline__ float half_area(float4 lo, float4 hi) {
     return dx * dy + dy * dz + dz * dx;
 }
 
+// ---- finishing an internal node ------------------------------------------------
+struct RefBox {
+    float4 lo, hi;
+    uint32_t count;  // | kLeafNode when the subtree is one leaf
+    float cost;
+};
+
+__device__ __forceinline__ RefBox ref_box(const Buffers& B, uint32_t ref) {
+    RefBox r;
+    if (ref & kLeafRef) {
+        const uint32_t t = B.vals[ref & ~kLeafRef];
+        r.lo = B.blo[t];
+        r.hi = B.bhi[t];
+        r.count = 1u | kLeafNode;
+        r.cost = half_area(r.lo, r.hi);
+    } else {
+        r.lo = __ldcg(B.nlo + ref);
+        r.hi = __ldcg(B.nhi + ref);
+        r.count = __float_as_uint(r.lo.w);
+        r.cost = r.hi.w;
+    }
+    return r;
+}
+
+// C(ref, 1..8) of a child: a single-triangle leaf costs c_tri x its half area
+// whatever the number of roots.
+__device__ __forceinline__ void dp_child(const Buffers& B, uint32_t ref, const RefBox& box, float c[8]) {
+    if (ref & kLeafRef) {
+        const float v = B.c_tri * box.cost;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) c[i] = v;
+    } else {
+        const float4 a = __ldcg(reinterpret_cast<const float4*>(B.dpc + 8 * (size_t)ref));
+        const float4 b = __ldcg(reinterpret_cast<const float4*>(B.dpc + 8 * (size_t)ref) + 1);
+        c[0] = a.x, c[1] = a.y, c[2] = a.z, c[3] = a.w, c[4] = b.x, c[5] = b.y, c[6] = b.z, c[7] = b.w;
+    }
+}
+
+// Box, count, cost and, for the SAH-optimal collapse, the dynamic programme of
+// internal node p, whose children are finished.
+__device__ __forceinline__ void finish_node(const Buffers& B, uint32_t p, uint32_t left, uint32_t right,
+                                            uint32_t max_leaf, float trav_cost) {
+            const RefBox l = ref_box(B, left), r = ref_box(B, right);
+            float4 lo = make_float4(fminf(l.lo.x, r.lo.x), fminf(l.lo.y, r.lo.y), fminf(l.lo.z, r.lo.z), 0.0f);
+            float4 hi = make_float4(fmaxf(l.hi.x, r.hi.x), fmaxf(l.hi.y, r.hi.y), fmaxf(l.hi.z, r.hi.z), 0.0f);
+            const uint32_t cnt = (l.count & ~kLeafNode) + (r.count & ~kLeafNode);
+            const float a = half_area(lo, hi);
+            const float split = trav_cost * a + l.cost + r.cost;
+            const bool leaf = cnt <= max_leaf && (float)cnt * a <= split;
+            lo.w = __uint_as_float(cnt | (leaf ? kLeafNode : 0u));
+            hi.w = leaf ? (float)cnt * a : split;
+            B.nlo[p] = lo;
+            B.nhi[p] = hi;
+            if (B.dpc) {
+                // SAH-optimal collapse: wide node at cost a, leaf slot at c_tri a cnt
+                float cl[8], cr[8], sp[7];  // sp[i - 2]: the subtree as i roots, split between the children
+                uint32_t sj[7];             // and the left child's share
+                dp_child(B, left, l, cl);
+                dp_child(B, right, r, cr);
+    #pragma unroll
+                for (int i = 0; i < 7; ++i) {
+                    sp[i] = FLT_MAX;
+                    sj[i] = 1;
+                }
+                // j roots left, k right, in ascending j for every sum
+    #pragma unroll
+                for (int j = 1; j <= 7; ++j)
+    #pragma unroll
+                    for (int k = 1; k <= 7; ++k)
+                        if (j + k <= 8) {
+                            const float v = cl[j - 1] + cr[k - 1];
+                            if (v < sp[j + k - 2]) {
+                                sp[j + k - 2] = v;
+                                sj[j + k - 2] = (uint32_t)j;
+                            }
+                        }
+                // (constant indices: the tables stay in registers)
+                const uint32_t width = B.width;
+                const float at_width = width == 8u   ? sp[6]
+                                       : width == 7u ? sp[5]
+                                       : width == 6u ? sp[4]
+                                       : width == 5u ? sp[3]
+                                       : width == 4u ? sp[2]
+                                       : width == 3u ? sp[1]
+                                                     : sp[0];
+                const uint32_t j_width = width == 8u   ? sj[6]
+                                         : width == 7u ? sj[5]
+                                         : width == 6u ? sj[4]
+                                         : width == 5u ? sj[3]
+                                         : width == 4u ? sj[2]
+                                         : width == 3u ? sj[1]
+                                                       : sj[0];
+                float c[8];
+                const float node_cost = a + at_width;
+                c[0] = node_cost;
+                uint32_t as_leaf = 0;
+                if (cnt <= (uint32_t)kMaxLeafTris) {
+                    const float leaf_cost = B.c_tri * a * (float)cnt;
+                    if (leaf_cost <= node_cost) {
+                        c[0] = leaf_cost;
+                        as_leaf = kDpLeaf;
+                    }
+                }
+                uint2 ch = make_uint2(j_width | as_leaf, 0u);
+    #pragma unroll
+                for (int i = 2; i <= 8; ++i) {
+                    const bool two = sp[i - 2] < c[i - 2];
+                    c[i - 1] = two ? sp[i - 2] : c[i - 2];
+                    const uint32_t w = two ? sj[i - 2] : 0u;
+                    if (i <= 4)
+                        ch.x |= w << 8 * (i - 1);
+                    else
+                        ch.y |= w << 8 * (i - 5);
+                }
+                float4* dc = reinterpret_cast<float4*>(B.dpc + 8 * (size_t)p);
+                dc[0] = make_float4(c[0], c[1], c[2], c[3]);
+                dc[1] = make_float4(c[4], c[5], c[6], c[7]);
+                B.dpch[p] = ch;
+            }
+}
+
+// The same as a call, for the clustering kernels, which are there for something
+// else. (In the walk of refit_kernel the call costs 10%.)
+__device__ __noinline__ void finish_made_node(const Buffers& B, uint32_t p, uint32_t max_leaf, float trav_cost) {
+    finish_node(B, p, B.left[p], B.right[p], max_leaf, trav_cost);
+}
+
 // ---- hierarchy by locally-ordered clustering (Meister & Bittner 2018) -----------
 // Clusters start as the sorted single triangles. Each round, every cluster
 // finds the neighbour within r positions of the current cluster array whose
@@ -457,13 +584,17 @@ __host__ __device__ __forceinline__ float half_area(float4 lo, float4 hi) {
 // a round is always mutual, so every round of two or more clusters merges at
 // least one pair. Internal nodes are numbered down from n - 2 in creation
 // order, so the last merge, the root, is node 0 as in the Karras tree, and
-// the same refit and collapse follow.
+// the same collapse follows.
 //
 // A round is two launches: one finds the neighbours of a tile and of the r
 // clusters around it (so a tile knows its mutual pairs by itself), counts
 // merges and survivors, and its last block to finish scans the tiles' counts;
 // the other merges and compacts. Once kPlocSmall clusters are left one block
-// runs the remaining rounds in shared memory. Bound: at a million clusters the
+// runs the remaining rounds in shared memory. The nodes that a round makes are
+// finished (finish_node) by further blocks of the next round's first launch:
+// their children are older, so no bottom-up walk, which took 250 us for 1.05M
+// triangles, follows; the first launches take 34 us more for it, the last
+// kernel 40. Bound: at a million clusters the
 // 32-byte cluster records read twice and written once per round, then launch
 // latency. The earlier form (four launches a round down to one cluster,
 // sixteen consecutive clusters per thread) took 1,110 us for 1.1M triangles.
@@ -477,6 +608,8 @@ constexpr uint32_t kPlocGone = 0xFFFFFFFFu;              // merged into a lower 
 struct PlocState {
     uint32_t count;      // clusters
     uint32_t next_node;  // internal nodes 0 .. next_node - 1 are still to be made
+    uint32_t made_end;   // next_node .. made_end - 1 were made by the round before
+    uint32_t pad;
 };
 
 // Cluster records: lo.w holds the cluster's reference (bits).
@@ -485,7 +618,7 @@ __global__ void __launch_bounds__(kPlocBlock) ploc_init_kernel(uint32_t n, Buffe
                                                                uint32_t* ticket) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i == 0) {
-        *st = PlocState{n, n - 1u};
+        *st = PlocState{n, n - 1u, n - 1u, 0u};
         *ticket = 0;
     }
     if (i >= n) return;
@@ -537,11 +670,20 @@ __global__ void __launch_bounds__(kPlocBlock) ploc_pair_kernel(const PlocState* 
                                                                const float4* __restrict__ hi,
                                                                uint32_t* __restrict__ partner,
                                                                unsigned long long* __restrict__ tsum,
-                                                               uint32_t* ticket, int r) {
+                                                               uint32_t* ticket, int r, uint32_t tile_blocks,
+                                                               Buffers B, uint32_t max_leaf, float trav_cost) {
     __shared__ float4 s_lo[kPlocTile + 4 * kPlocMaxRadius], s_hi[kPlocTile + 4 * kPlocMaxRadius];
     __shared__ int s_nn[kPlocTile + 2 * kPlocMaxRadius];
     __shared__ unsigned long long s_warp[32];
     __shared__ bool s_last;
+    if (blockIdx.x >= tile_blocks) {
+        // beside the tiles: the nodes that the round before has made
+        const uint32_t end = st->made_end;
+        for (uint32_t p = st->next_node + (blockIdx.x - tile_blocks) * kPlocBlock + threadIdx.x; p < end;
+             p += (gridDim.x - tile_blocks) * kPlocBlock)
+            finish_made_node(B, p, max_leaf, trav_cost);
+        return;
+    }
     const int count = (int)st->count;
     const int b0 = (int)(blockIdx.x * kPlocTile);
     if (b0 < count) {
@@ -577,7 +719,7 @@ __global__ void __launch_bounds__(kPlocBlock) ploc_pair_kernel(const PlocState* 
     // the last block scans the tiles' sums and writes the next round's state
     if (threadIdx.x == 0) {
         __threadfence();
-        s_last = atomicAdd(ticket, 1u) == gridDim.x - 1u;
+        s_last = atomicAdd(ticket, 1u) == tile_blocks - 1u;
     }
     __syncthreads();
     if (!s_last) return;
@@ -600,16 +742,9 @@ __global__ void __launch_bounds__(kPlocBlock) ploc_pair_kernel(const PlocState* 
         carry += total;
     }
     if (threadIdx.x == 0) {
-        *next = PlocState{(uint32_t)carry, st->next_node - (uint32_t)(carry >> 32)};
+        *next = PlocState{(uint32_t)carry, st->next_node - (uint32_t)(carry >> 32), st->next_node, 0u};
         *ticket = 0;
     }
-}
-
-__device__ __forceinline__ void ploc_set_parent(const Buffers& B, uint32_t ref, uint32_t node) {
-    if (ref & kLeafRef)
-        B.parent_l[ref & ~kLeafRef] = node;
-    else
-        B.parent_i[ref] = node;
 }
 
 // Clusters a (lower position) and b become internal node `node`.
@@ -618,8 +753,6 @@ __device__ __forceinline__ void ploc_join(const Buffers& B, uint32_t node, float
     const uint32_t a = __float_as_uint(alo.w), b = __float_as_uint(blo.w);
     B.left[node] = a;
     B.right[node] = b;
-    ploc_set_parent(B, a, node);
-    ploc_set_parent(B, b, node);
     alo = make_float4(fminf(alo.x, blo.x), fminf(alo.y, blo.y), fminf(alo.z, blo.z), __uint_as_float(node));
     ahi = make_float4(fmaxf(ahi.x, bhi.x), fmaxf(ahi.y, bhi.y), fmaxf(ahi.z, bhi.z), 0.0f);
 }
@@ -659,10 +792,13 @@ __global__ void __launch_bounds__(kPlocBlock) ploc_merge_kernel(const PlocState*
 // The rounds of at most kPlocSmall clusters, by one block. Every round merges
 // a pair, so there are fewer rounds than clusters; the bound only guards.
 __global__ void __launch_bounds__(kPlocSmall) ploc_small_kernel(PlocState* st, const float4* __restrict__ lin,
-                                                                const float4* __restrict__ hin, int r, Buffers B) {
+                                                                const float4* __restrict__ hin, int r, Buffers B,
+                                                                 uint32_t max_leaf, float trav_cost) {
     __shared__ float4 s_lo[kPlocSmall], s_hi[kPlocSmall];
     __shared__ int s_nn[kPlocSmall];
+    __shared__ uint32_t s_made[kPlocSmall + 1];  // next_node before each round, and after the last
     __shared__ unsigned long long s_warp[32];
+    uint32_t rounds = 0;
     uint32_t count = st->count, next_node = st->next_node;
     if (count > kPlocSmall) return;  // the host sees the count and reports it
     const uint32_t i = threadIdx.x;
@@ -695,47 +831,23 @@ __global__ void __launch_bounds__(kPlocSmall) ploc_small_kernel(PlocState* st, c
         }
         __syncthreads();
         if ((uint32_t)(total >> 32) == 0u) break;
+        if (i == 0) s_made[rounds] = next_node;
+        rounds++;
         count = (uint32_t)total;
         next_node -= (uint32_t)(total >> 32);
     }
-    if (i == 0) *st = PlocState{count, next_node};
-}
-
-struct RefBox {
-    float4 lo, hi;
-    uint32_t count;  // | kLeafNode when the subtree is one leaf
-    float cost;
-};
-
-__device__ __forceinline__ RefBox ref_box(const Buffers& B, uint32_t ref) {
-    RefBox r;
-    if (ref & kLeafRef) {
-        const uint32_t t = B.vals[ref & ~kLeafRef];
-        r.lo = B.blo[t];
-        r.hi = B.bhi[t];
-        r.count = 1u | kLeafNode;
-        r.cost = half_area(r.lo, r.hi);
-    } else {
-        r.lo = __ldcg(B.nlo + ref);
-        r.hi = __ldcg(B.nhi + ref);
-        r.count = __float_as_uint(r.lo.w);
-        r.cost = r.hi.w;
+    // the nodes of the last merge before this kernel, then of each round here
+    const uint32_t first = st->next_node, end = st->made_end;
+    for (uint32_t p = first + i; p < end; p += kPlocSmall) finish_made_node(B, p, max_leaf, trav_cost);
+    if (i == 0) s_made[rounds] = next_node;
+    for (uint32_t k = 0; k < rounds; ++k) {
+        __threadfence_block();
+        __syncthreads();
+        const uint32_t p = s_made[k + 1] + i;
+        if (p < s_made[k]) finish_made_node(B, p, max_leaf, trav_cost);
     }
-    return r;
-}
-
-// C(ref, 1..8) of a child: a single-triangle leaf costs c_tri x its half area
-// whatever the number of roots.
-__device__ __forceinline__ void dp_child(const Buffers& B, uint32_t ref, const RefBox& box, float c[8]) {
-    if (ref & kLeafRef) {
-        const float v = B.c_tri * box.cost;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) c[i] = v;
-    } else {
-        const float4 a = __ldcg(reinterpret_cast<const float4*>(B.dpc + 8 * (size_t)ref));
-        const float4 b = __ldcg(reinterpret_cast<const float4*>(B.dpc + 8 * (size_t)ref) + 1);
-        c[0] = a.x, c[1] = a.y, c[2] = a.z, c[3] = a.w, c[4] = b.x, c[5] = b.y, c[6] = b.z, c[7] = b.w;
-    }
+    __syncthreads();
+    if (i == 0) *st = PlocState{count, next_node, next_node, 0u};
 }
 
 // Bound: the memory traffic of the node records near the leaves, then the
@@ -757,83 +869,7 @@ __global__ void __launch_bounds__(256) refit_kernel(uint32_t n, Buffers B, uint3
         if (atomicAdd(B.flag + p, 1u) == 0u) return;  // the sibling subtree is not finished yet
         __threadfence();
         const uint32_t left = B.left[p], right = B.right[p], up = B.parent_i[p];
-        const RefBox l = ref_box(B, left), r = ref_box(B, right);
-        float4 lo = make_float4(fminf(l.lo.x, r.lo.x), fminf(l.lo.y, r.lo.y), fminf(l.lo.z, r.lo.z), 0.0f);
-        float4 hi = make_float4(fmaxf(l.hi.x, r.hi.x), fmaxf(l.hi.y, r.hi.y), fmaxf(l.hi.z, r.hi.z), 0.0f);
-        const uint32_t cnt = (l.count & ~kLeafNode) + (r.count & ~kLeafNode);
-        const float a = half_area(lo, hi);
-        const float split = trav_cost * a + l.cost + r.cost;
-        const bool leaf = cnt <= max_leaf && (float)cnt * a <= split;
-        lo.w = __uint_as_float(cnt | (leaf ? kLeafNode : 0u));
-        hi.w = leaf ? (float)cnt * a : split;
-        B.nlo[p] = lo;
-        B.nhi[p] = hi;
-        if (B.dpc) {
-            // SAH-optimal collapse: wide node at cost a, leaf slot at c_tri a cnt
-            float cl[8], cr[8], sp[7];  // sp[i - 2]: the subtree as i roots, split between the children
-            uint32_t sj[7];             // and the left child's share
-            dp_child(B, left, l, cl);
-            dp_child(B, right, r, cr);
-#pragma unroll
-            for (int i = 0; i < 7; ++i) {
-                sp[i] = FLT_MAX;
-                sj[i] = 1;
-            }
-            // j roots left, k right, in ascending j for every sum
-#pragma unroll
-            for (int j = 1; j <= 7; ++j)
-#pragma unroll
-                for (int k = 1; k <= 7; ++k)
-                    if (j + k <= 8) {
-                        const float v = cl[j - 1] + cr[k - 1];
-                        if (v < sp[j + k - 2]) {
-                            sp[j + k - 2] = v;
-                            sj[j + k - 2] = (uint32_t)j;
-                        }
-                    }
-            // (constant indices: the tables stay in registers)
-            const uint32_t width = B.width;
-            const float at_width = width == 8u   ? sp[6]
-                                   : width == 7u ? sp[5]
-                                   : width == 6u ? sp[4]
-                                   : width == 5u ? sp[3]
-                                   : width == 4u ? sp[2]
-                                   : width == 3u ? sp[1]
-                                                 : sp[0];
-            const uint32_t j_width = width == 8u   ? sj[6]
-                                     : width == 7u ? sj[5]
-                                     : width == 6u ? sj[4]
-                                     : width == 5u ? sj[3]
-                                     : width == 4u ? sj[2]
-                                     : width == 3u ? sj[1]
-                                                   : sj[0];
-            float c[8];
-            const float node_cost = a + at_width;
-            c[0] = node_cost;
-            uint32_t as_leaf = 0;
-            if (cnt <= (uint32_t)kMaxLeafTris) {
-                const float leaf_cost = B.c_tri * a * (float)cnt;
-                if (leaf_cost <= node_cost) {
-                    c[0] = leaf_cost;
-                    as_leaf = kDpLeaf;
-                }
-            }
-            uint2 ch = make_uint2(j_width | as_leaf, 0u);
-#pragma unroll
-            for (int i = 2; i <= 8; ++i) {
-                const bool two = sp[i - 2] < c[i - 2];
-                c[i - 1] = two ? sp[i - 2] : c[i - 2];
-                const uint32_t w = two ? sj[i - 2] : 0u;
-                if (i <= 4)
-                    ch.x |= w << 8 * (i - 1);
-                else
-                    ch.y |= w << 8 * (i - 5);
-            }
-            float4* dc = reinterpret_cast<float4*>(B.dpc + 8 * (size_t)p);
-            dc[0] = make_float4(c[0], c[1], c[2], c[3]);
-            dc[1] = make_float4(c[4], c[5], c[6], c[7]);
-            B.dpch[p] = ch;
-        }
+        finish_node(B, p, left, right, max_leaf, trav_cost);
         p = up;
     }
 }
@@ -1262,7 +1298,8 @@ void RadixSort(Buffers& B, uint32_t n, cudaStream_t s) {
 // The clustering rounds of ploc_*_kernel. Each round's grids are sized by
 // the cluster count read back one round late (an upper bound: counts only
 // fall), so the host never waits for the round it has just queued.
-void PlocHierarchy(Buffers& B, uint32_t n, int r, GpuBuildResources& res, cudaStream_t s) {
+void PlocHierarchy(Buffers& B, uint32_t n, int r, uint32_t max_leaf, float trav_cost, GpuBuildResources& res,
+                   cudaStream_t s) {
     Scratch S(res.pool, s);
     float4* lo[2] = {S.get<float4>(n), S.get<float4>(n)};
     float4* hi[2] = {S.get<float4>(n), S.get<float4>(n)};
@@ -1278,8 +1315,9 @@ void PlocHierarchy(Buffers& B, uint32_t n, int r, GpuBuildResources& res, cudaSt
     // every round of two or more clusters merges a pair: at most n - 1 rounds
     for (uint32_t round = 0; bound > kPlocSmall && round <= n; ++round) {
         const uint32_t tiles = (bound + kPlocTile - 1) / kPlocTile;
-        ploc_pair_kernel<<<tiles, kPlocBlock, 0, s>>>(st + cur, st + (cur ^ 1), lo[cur], hi[cur], partner, tsum,
-                                                      ticket, r);
+        // as many blocks again for the nodes to finish
+        ploc_pair_kernel<<<2 * tiles, kPlocBlock, 0, s>>>(st + cur, st + (cur ^ 1), lo[cur], hi[cur], partner, tsum,
+                                                          ticket, r, tiles, B, max_leaf, trav_cost);
         ploc_merge_kernel<<<tiles, kPlocBlock, 0, s>>>(st + cur, tsum, partner, lo[cur], hi[cur], lo[cur ^ 1],
                                                        hi[cur ^ 1], B);
         Check(cudaMemcpyAsync(h + (round & 1), st + (cur ^ 1), sizeof(PlocState), cudaMemcpyDeviceToHost, s),
@@ -1292,7 +1330,7 @@ void PlocHierarchy(Buffers& B, uint32_t n, int r, GpuBuildResources& res, cudaSt
         if (round > 1 && c >= bound) break;  // a round without a merge
         bound = c;
     }
-    ploc_small_kernel<<<1, kPlocSmall, 0, s>>>(st + cur, lo[cur], hi[cur], r, B);
+    ploc_small_kernel<<<1, kPlocSmall, 0, s>>>(st + cur, lo[cur], hi[cur], r, B, max_leaf, trav_cost);
     Check(cudaMemcpyAsync(h, st + cur, sizeof(PlocState), cudaMemcpyDeviceToHost, s), "cluster count");
     Check(cudaStreamSynchronize(s), "clustering");
     CHECK_CODE(h->count == 1 && h->next_node == 0, FND_ERR_INVALID_SCENE, "GPU build: clustering stopped at %u clusters",
@@ -1327,11 +1365,14 @@ void BuildWideGpu(const float* d_verts, uint32_t nv, const uint32_t* d_idx, uint
     B.cnt = S.get<uint32_t>((uint64_t)kDigits * ((n + kSortTile - 1) / kSortTile) + kDigits);
     B.left = S.get<uint32_t>(n);
     B.right = S.get<uint32_t>(n);
-    B.parent_i = S.get<uint32_t>(n);
-    B.parent_l = S.get<uint32_t>(n);
+    const bool walk = p.ploc_radius == 0;  // nodes finished by refit_kernel, not by the clustering
+    if (walk) {
+        B.parent_i = S.get<uint32_t>(n);
+        B.parent_l = S.get<uint32_t>(n);
+        B.flag = S.get<uint32_t>(n);
+    }
     B.nlo = S.get<float4>(n);
     B.nhi = S.get<float4>(n);
-    B.flag = S.get<uint32_t>(n);
     B.bounds = S.get<float>(12);
     B.status = S.get<uint32_t>(1);
     B.counters = S.get<uint32_t>(4 + kMaxLevels + 2);
@@ -1349,9 +1390,11 @@ void BuildWideGpu(const float* d_verts, uint32_t nv, const uint32_t* d_idx, uint
     keep(&out.d_tri_shade, 16ull * n, "shading normals");
     float4* shade = static_cast<float4*>(out.d_tri_shade);
     Check(cudaMemsetAsync(B.status, 0, 4, s), "memset");
-    Check(cudaMemsetAsync(B.flag, 0, 4ull * n, s), "memset");
-    Check(cudaMemsetAsync(B.parent_i, 0xFF, 4ull * n, s), "memset");
-    Check(cudaMemsetAsync(B.parent_l, 0xFF, 4ull * n, s), "memset");
+    if (walk) {
+        Check(cudaMemsetAsync(B.flag, 0, 4ull * n, s), "memset");
+        Check(cudaMemsetAsync(B.parent_i, 0xFF, 4ull * n, s), "memset");
+        Check(cudaMemsetAsync(B.parent_l, 0xFF, 4ull * n, s), "memset");
+    }
     Check(cudaMemsetAsync(B.counters, 0, 4ull * (4 + kMaxLevels + 2), s), "memset");
     init_bounds_kernel<<<1, 32, 0, s>>>(B.bounds);
     const uint32_t g256 = (n + 255) / 256;
@@ -1373,11 +1416,12 @@ void BuildWideGpu(const float* d_verts, uint32_t nv, const uint32_t* d_idx, uint
     morton_kernel<<<g256, 256, 0, s>>>(n, B);
     RadixSort(B, n, s);
     if (n >= 2) {
-        if (p.ploc_radius)
-            PlocHierarchy(B, n, (int)p.ploc_radius, res, s);
-        else
+        if (walk) {
             hierarchy_kernel<<<(n - 1 + 255) / 256, 256, 0, s>>>((int)n, B);
-        refit_kernel<<<g256, 256, 0, s>>>(n, B, p.max_leaf, p.trav_cost);
+            refit_kernel<<<g256, 256, 0, s>>>(n, B, p.max_leaf, p.trav_cost);
+        } else {
+            PlocHierarchy(B, n, (int)p.ploc_radius, p.max_leaf, p.trav_cost, res, s);
+        }
     }
     Check(cudaGetLastError(), "hierarchy launch");
     // root item: internal node 0, or the single leaf
