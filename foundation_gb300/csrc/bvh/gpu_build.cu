@@ -604,6 +604,7 @@ constexpr uint32_t kPlocItems = 2;
 constexpr uint32_t kPlocTile = kPlocBlock * kPlocItems;  // clusters per block
 constexpr uint32_t kPlocSmall = 1024;                    // clusters the last kernel takes
 constexpr uint32_t kPlocGone = 0xFFFFFFFFu;              // merged into a lower position
+constexpr uint32_t kTellRoot = 8;                        // page-locked word of the root's RootInfo
 
 struct PlocState {
     uint32_t count;      // clusters
@@ -670,7 +671,7 @@ __global__ void __launch_bounds__(kPlocBlock) ploc_pair_kernel(const PlocState* 
                                                                const float4* __restrict__ hi,
                                                                uint32_t* __restrict__ partner,
                                                                unsigned long long* __restrict__ tsum,
-                                                               uint32_t* ticket, int r, uint32_t tile_blocks,
+                                                               PlocState* seen, uint32_t* ticket, int r, uint32_t tile_blocks,
                                                                Buffers B, uint32_t max_leaf, float trav_cost) {
     __shared__ float4 s_lo[kPlocTile + 4 * kPlocMaxRadius], s_hi[kPlocTile + 4 * kPlocMaxRadius];
     __shared__ int s_nn[kPlocTile + 2 * kPlocMaxRadius];
@@ -743,6 +744,7 @@ __global__ void __launch_bounds__(kPlocBlock) ploc_pair_kernel(const PlocState* 
     }
     if (threadIdx.x == 0) {
         *next = PlocState{(uint32_t)carry, st->next_node - (uint32_t)(carry >> 32), st->next_node, 0u};
+        *seen = *next;  // (page-locked host memory)
         *ticket = 0;
     }
 }
@@ -791,17 +793,21 @@ __global__ void __launch_bounds__(kPlocBlock) ploc_merge_kernel(const PlocState*
 
 // The rounds of at most kPlocSmall clusters, by one block. Every round merges
 // a pair, so there are fewer rounds than clusters; the bound only guards.
-__global__ void __launch_bounds__(kPlocSmall) ploc_small_kernel(PlocState* st, const float4* __restrict__ lin,
+__global__ void __launch_bounds__(kPlocSmall) ploc_small_kernel(const PlocState* __restrict__ st, PlocState* seen,
+                                                                const float4* __restrict__ lin,
                                                                 const float4* __restrict__ hin, int r, Buffers B,
-                                                                 uint32_t max_leaf, float trav_cost) {
+                                                                uint32_t max_leaf, float trav_cost) {
     __shared__ float4 s_lo[kPlocSmall], s_hi[kPlocSmall];
     __shared__ int s_nn[kPlocSmall];
     __shared__ uint32_t s_made[kPlocSmall + 1];  // next_node before each round, and after the last
     __shared__ unsigned long long s_warp[32];
     uint32_t rounds = 0;
     uint32_t count = st->count, next_node = st->next_node;
-    if (count > kPlocSmall) return;  // the host sees the count and reports it
     const uint32_t i = threadIdx.x;
+    if (count > kPlocSmall) {  // the host sees the count and reports it
+        if (i == 0) *seen = *st;
+        return;
+    }
     if (i < count) {
         s_lo[i] = lin[i];
         s_hi[i] = hin[i];
@@ -847,7 +853,7 @@ __global__ void __launch_bounds__(kPlocSmall) ploc_small_kernel(PlocState* st, c
         if (p < s_made[k]) finish_made_node(B, p, max_leaf, trav_cost);
     }
     __syncthreads();
-    if (i == 0) *st = PlocState{count, next_node, next_node, 0u};
+    if (i == 0) *seen = PlocState{count, next_node, next_node, 0u};
 }
 
 // Bound: the memory traffic of the node records near the leaves, then the
@@ -1233,9 +1239,26 @@ __global__ void instance_shade_kernel(const float* __restrict__ inv, const uint3
 }
 
 // The collapse's first queue entry, level 0 of one node.
-__global__ void root_kernel(Buffers B, uint2 item) {
+// The collapse's first item, and what the host asks of the root (`told`).
+struct RootInfo {
+    float4 lo, hi;
+    float wide_cost;
+};
+__global__ void root_kernel(Buffers B, uint2 item, bool internal, RootInfo* told) {
     B.qa[0] = item;
     B.counters[4] = 1u;
+    if (internal) *told = RootInfo{B.nlo[0], B.nhi[0], B.dpc ? B.dpc[0] : 0.0f};
+}
+
+// The status word and `n` words behind `at` into page-locked host memory. The
+// device tells the host its few answers by kernels: a copy of some bytes holds
+// the stream for 8 us, and with one per clustering round (and seven more) an
+// upload of 1.05M triangles, its trace and its end took 1,595 us instead of
+// 1,348.
+__global__ void __launch_bounds__(128) tell_kernel(const uint32_t* __restrict__ status, const uint32_t* __restrict__ at,
+                                                   uint32_t n, uint32_t* told) {
+    if (threadIdx.x == 0) told[0] = *status;
+    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) told[4 + i] = at[i];
 }
 
 __global__ void interleave_kernel(const float4* __restrict__ planes, uint32_t n, float4* __restrict__ tris) {
@@ -1317,12 +1340,10 @@ void PlocHierarchy(Buffers& B, uint32_t n, int r, uint32_t max_leaf, float trav_
         const uint32_t tiles = (bound + kPlocTile - 1) / kPlocTile;
         // as many blocks again for the nodes to finish
         ploc_pair_kernel<<<2 * tiles, kPlocBlock, 0, s>>>(st + cur, st + (cur ^ 1), lo[cur], hi[cur], partner, tsum,
-                                                          ticket, r, tiles, B, max_leaf, trav_cost);
+                                                          h + (round & 1), ticket, r, tiles, B, max_leaf, trav_cost);
+        Check(cudaEventRecord(ev[round & 1], s), "event");
         ploc_merge_kernel<<<tiles, kPlocBlock, 0, s>>>(st + cur, tsum, partner, lo[cur], hi[cur], lo[cur ^ 1],
                                                        hi[cur ^ 1], B);
-        Check(cudaMemcpyAsync(h + (round & 1), st + (cur ^ 1), sizeof(PlocState), cudaMemcpyDeviceToHost, s),
-              "cluster count");
-        Check(cudaEventRecord(ev[round & 1], s), "event");
         cur ^= 1;
         if (round == 0) continue;
         Check(cudaEventSynchronize(ev[(round - 1) & 1]), "clustering round");
@@ -1330,9 +1351,12 @@ void PlocHierarchy(Buffers& B, uint32_t n, int r, uint32_t max_leaf, float trav_
         if (round > 1 && c >= bound) break;  // a round without a merge
         bound = c;
     }
-    ploc_small_kernel<<<1, kPlocSmall, 0, s>>>(st + cur, lo[cur], hi[cur], r, B, max_leaf, trav_cost);
-    Check(cudaMemcpyAsync(h, st + cur, sizeof(PlocState), cudaMemcpyDeviceToHost, s), "cluster count");
-    Check(cudaStreamSynchronize(s), "clustering");
+    ploc_small_kernel<<<1, kPlocSmall, 0, s>>>(st + cur, h, lo[cur], hi[cur], r, B, max_leaf, trav_cost);
+}
+
+// After the stream has passed PlocHierarchy's kernels.
+void CheckClustered(const GpuBuildResources& res) {
+    const PlocState* h = reinterpret_cast<const PlocState*>(res.pinned);
     CHECK_CODE(h->count == 1 && h->next_node == 0, FND_ERR_INVALID_SCENE, "GPU build: clustering stopped at %u clusters",
                h->count);
 }
@@ -1401,8 +1425,8 @@ void BuildWideGpu(const float* d_verts, uint32_t nv, const uint32_t* d_idx, uint
     prep_kernel<<<std::max(1u, std::min(g256, 8u * (uint32_t)sms)), 256, 0, s>>>(d_verts, nv, d_idx, n, B, shade);
     uint32_t* pinned = res.pinned;
     float h_bounds[12];
-    Check(cudaMemcpyAsync(pinned, B.status, 4, cudaMemcpyDeviceToHost, s), "status readback");
-    Check(cudaMemcpyAsync(pinned + 4, B.bounds, sizeof(h_bounds), cudaMemcpyDeviceToHost, s), "bounds readback");
+    tell_kernel<<<1, 128, 0, s>>>(B.status, reinterpret_cast<const uint32_t*>(B.bounds), 12, pinned);
+    Check(cudaGetLastError(), "prep launch");
     Check(cudaStreamSynchronize(s), "prep");
     uint32_t h_status = pinned[0];
     std::memcpy(h_bounds, pinned + 4, sizeof(h_bounds));
@@ -1425,19 +1449,20 @@ void BuildWideGpu(const float* d_verts, uint32_t nv, const uint32_t* d_idx, uint
     }
     Check(cudaGetLastError(), "hierarchy launch");
     // root item: internal node 0, or the single leaf
-    root_kernel<<<1, 1, 0, s>>>(B, make_uint2(n >= 2 ? 0u : kLeafRef, 0u));
+    static_assert(kTellRoot >= 2 * sizeof(PlocState) / 4 && 4 * kTellRoot % alignof(RootInfo) == 0 &&
+                      kTellRoot + sizeof(RootInfo) / 4 <= kGpuBuildPinnedWords,
+                  "behind the clustering's states");
+    RootInfo* told = reinterpret_cast<RootInfo*>(pinned + kTellRoot);
+    root_kernel<<<1, 1, 0, s>>>(B, make_uint2(n >= 2 ? 0u : kLeafRef, 0u), n >= 2, told);
     float root_cost = 0.0f, wide_cost = 0.0f;
     float4 rlo{}, rhi{};
-    if (n >= 2) {
-        if (B.dpc) Check(cudaMemcpyAsync(pinned, B.dpc, 4, cudaMemcpyDeviceToHost, s), "cost readback");
-        Check(cudaMemcpyAsync(pinned + 4, B.nlo, 16, cudaMemcpyDeviceToHost, s), "root box");
-        Check(cudaMemcpyAsync(pinned + 8, B.nhi, 16, cudaMemcpyDeviceToHost, s), "root box");
-    }
+    Check(cudaGetLastError(), "root launch");
     Check(cudaStreamSynchronize(s), "LBVH");
     if (n >= 2) {
-        if (B.dpc) std::memcpy(&wide_cost, pinned, 4);
-        std::memcpy(&rlo, pinned + 4, 16);
-        std::memcpy(&rhi, pinned + 8, 16);
+        if (!walk) CheckClustered(res);
+        wide_cost = told->wide_cost;
+        rlo = told->lo;
+        rhi = told->hi;
     }
     out.build_ms = Ms(t0);
     const auto t1 = std::chrono::steady_clock::now();
@@ -1462,9 +1487,8 @@ void BuildWideGpu(const float* d_verts, uint32_t nv, const uint32_t* d_idx, uint
             A.level = level;
             collapse_kernel<<<grid, kCollapseBlock, 0, s>>>(A);
         }
+        tell_kernel<<<1, 128, 0, s>>>(B.status, B.counters, sizeof(h_counters) / 4, pinned);
         Check(cudaGetLastError(), "collapse launch");
-        Check(cudaMemcpyAsync(pinned, B.status, 4, cudaMemcpyDeviceToHost, s), "status readback");
-        Check(cudaMemcpyAsync(pinned + 4, B.counters, sizeof(h_counters), cudaMemcpyDeviceToHost, s), "counters");
         Check(cudaStreamSynchronize(s), "collapse");
         h_status = pinned[0];
         std::memcpy(h_counters, pinned + 4, sizeof(h_counters));
