@@ -65,7 +65,7 @@ __device__ __forceinline__ long long edge(long long ax, long long ay, long long 
     return (bx - ax) * (py - ay) - (by - ay) * (px - ax);
 }
 
-__global__ void setup_kernel(const DrawArgs A, Tri* tris) {
+__device__ __forceinline__ void setup(const DrawArgs& A, const Vertex* verts, const uint16_t* idx, Tri* tris) {
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= A.ntri) return;
     float vm[16], pvm[16];
@@ -82,13 +82,12 @@ __global__ void setup_kernel(const DrawArgs A, Tri* tris) {
     double w[3];
     uint32_t vid[3];
     for (int k = 0; k < 3; ++k) {
-        vid[k] = A.idx[3 * (size_t)t + k];
-        if (vid[k] >= A.nv) {
-            atomicOr(A.status, 1u);
+        vid[k] = idx[3 * (size_t)t + k];
+        if (vid[k] >= A.nv) {  // (checked on the host)
             ok = false;
             break;
         }
-        const float p[4] = {A.verts[vid[k]].pos[0], A.verts[vid[k]].pos[1], 0.0f, 1.0f};
+        const float p[4] = {verts[vid[k]].pos[0], verts[vid[k]].pos[1], 0.0f, 1.0f};
         double c[4];
         for (int r = 0; r < 4; ++r) {
             float s = __fmul_rn(pvm[0 * 4 + r], p[0]);
@@ -166,7 +165,7 @@ __global__ void setup_kernel(const DrawArgs A, Tri* tris) {
                 T.e0[k] = edge(X[a], Y[a], X[b], Y[b], kSub / 2, kSub / 2);
                 T.sx[k] = -(Y[b] - Y[a]) * kSub;
                 T.sy[k] = (X[b] - X[a]) * kSub;
-                const Vertex& V = A.verts[vid[k]];
+                const Vertex& V = verts[vid[k]];
                 const double iw = 1.0 / w[k];
                 T.iw[k] = iw;
                 T.cu[k] = (double)V.uv[0] * iw * kUvOne;
@@ -182,6 +181,14 @@ __global__ void setup_kernel(const DrawArgs A, Tri* tris) {
         }
     }
     tris[t] = T;
+}
+
+__global__ void setup_kernel(const DrawArgs A, Tri* tris) { setup(A, A.verts, A.idx, tris); }
+// The mesh as a kernel argument; pixel_kernel reads the vertices from memory.
+__global__ void setup_small_kernel(const DrawArgs A, const __grid_constant__ SmallMesh mesh, Tri* tris) {
+    if (blockIdx.x == 0)
+        for (uint32_t i = threadIdx.x; i < A.nv; i += blockDim.x) A.verts[i] = mesh.verts[i];
+    setup(A, mesh.verts, mesh.idx, tris);
 }
 
 __device__ __forceinline__ double unit_frac(double u) {
@@ -366,7 +373,11 @@ size_t TriBytes(uint32_t ntri) { return sizeof(Tri) * (size_t)ntri; }
 
 cudaError_t LaunchDraw(const DrawArgs& a, cudaStream_t s) {
     Tri* tris = static_cast<Tri*>(a.tris);
-    if (a.ntri) setup_kernel<<<(a.ntri + 63) / 64, 64, 0, s>>>(a, tris);
+    const dim3 grid((a.ntri + 63) / 64);
+    if (a.ntri && a.mesh)
+        setup_small_kernel<<<grid, 64, 0, s>>>(a, *a.mesh, tris);
+    else if (a.ntri)
+        setup_kernel<<<grid, 64, 0, s>>>(a, tris);
     const bool wide = a.width % kPixels == 0 && ((uintptr_t)a.target & 15u) == 0;
     const uint32_t per_block = 128 * kPixels;
     pixel_kernel<<<dim3((a.width + per_block - 1) / per_block, a.height), 128, 0, s>>>(a, tris, wide);

@@ -27,12 +27,19 @@ struct Uniforms {
     float model[16], view[16], proj[16];  // column-major (m[c * 4 + r])
 };
 
+// A mesh small enough to travel with the launch.
+struct SmallMesh {
+    static constexpr uint32_t kVertices = 64, kIndices = 128;
+    Vertex verts[kVertices];
+    uint16_t idx[kIndices];
+};
+
 struct DrawArgs {
     uint32_t width, height;
     Uniforms u;
     uint32_t clear_rgba;      // the encoded clear colour
     uint32_t cull_back;
-    const Vertex* verts;
+    Vertex* verts;            // (written by the launch when it gets a SmallMesh)
     uint32_t nv;
     const uint16_t* idx;
     uint32_t ntri;
@@ -40,7 +47,7 @@ struct DrawArgs {
     uint32_t tex_w, tex_h;
     uint32_t* target;         // RGBA8 pixels, row-major from the top row
     void* tris;               // scratch: TriBytes(ntri), 16-byte aligned
-    uint32_t* status;
+    const SmallMesh* mesh;    // host: what verts and idx would hold, or null
 };
 
 size_t TriBytes(uint32_t ntri);

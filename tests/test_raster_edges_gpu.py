@@ -78,3 +78,22 @@ def test_not_finite(built):
     v["uv"][7] = np.nan
     v["uv"][10] = np.inf
     _draw(65, 40, v, np.random.default_rng(1).integers(0, 256, (8, 8, 4), dtype=np.uint8))
+
+
+@pytest.mark.parametrize("nv,ni", [(3, 0), (3, 3), (64, 126), (64, 129), (65, 126), (66, 66), (300, 600)])
+def test_mesh_sizes(built, nv, ni):
+    """Meshes that travel with the launch (up to 64 vertices and 128 indices)
+    and ones that are copied, with shared and unused vertices; bright colours
+    take the paths that read the vertices again."""
+    import foundation_gb300 as fg
+    rng = np.random.default_rng(nv + ni)
+    tex = rng.integers(0, 256, (7, 5, 4), dtype=np.uint8)
+    v = _verts((nv + 2) // 3, 6, 0.8, (-3, 3), (-2, 3))[:nv]
+    idx = rng.integers(0, nv, ni).astype(np.uint16)
+    eye = np.eye(4, dtype=np.float32).ravel(order="F")
+    want = O.raster_draw(97, 41, eye, eye, eye, tex, v.view(np.float32).reshape(-1, 7), idx, clear=(0.2, 0.4, 0.6, 1.0),
+                         cull_back=False)
+    with fg.Context(0) as ctx:
+        for _ in range(2):
+            got = ctx.raster_draw(97, 41, eye, eye, eye, tex, v, idx, clear=(0.2, 0.4, 0.6, 1.0), cull_back=False)
+            assert np.array_equal(got, want)
