@@ -24,7 +24,7 @@ constexpr uint32_t kWaitMin = 4;
 constexpr uint32_t kHelpAt = 28;
 
 struct Common {
-    uint32_t* counter;
+    uint32_t* counter;  // null (few rays): every warp takes its one run of them
     uint32_t* status;
     unsigned long long* stats;
     uint32_t refill_min;
@@ -283,9 +283,14 @@ __device__ __forceinline__ void trace_loop(const Src& src, const Common& C, uint
             if (exhausted) break;
             const uint32_t cnt = (uint32_t)__popc(ready);
             uint32_t base = 0;
-            if (lane == 0) base = atomicAdd(C.counter, cnt);
-            base = __shfl_sync(kFull, base, 0);
-            exhausted = base + cnt >= n;
+            if (kFew && !C.counter) {
+                base = (blockIdx.x * blockDim.x + threadIdx.x) / 32u * lanes;
+                exhausted = true;
+            } else {
+                if (lane == 0) base = atomicAdd(C.counter, cnt);
+                base = __shfl_sync(kFull, base, 0);
+                exhausted = base + cnt >= n;
+            }
             const uint32_t pos = base + (uint32_t)__popc(ready & below);
             if (mine && pos < n) {
                 const uint32_t id = src.map(pos);
