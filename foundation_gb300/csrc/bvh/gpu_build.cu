@@ -13,12 +13,12 @@
 //     locally-ordered clustering of the sorted triangles (Meister & Bittner
 //     2018), rounds of mutual-nearest-neighbour merges within a window of
 //     the cluster array;
-//  5. refit from the leaves upwards (the second thread to reach a node
-//     finishes it): box, triangle count and the SAH decision
+//  5. every node is finished from the leaves upwards (Karras: a walk, the
+//     second thread to reach a node finishes it; clustering: round by round):
+//     box, triangle count and the SAH decision
 //     cost(n) = min(N A, C_trav A + cost(l) + cost(r)), a subtree of at most
 //     max_leaf triangles becoming one leaf when that is not dearer;
-//     With the SAH-optimal collapse the same walk also computes, per node,
-//     the costs C(n, i) of representing its subtree by at most i roots (wide
+//     With the SAH-optimal collapse that also computes, per node, the costs C(n, i) of representing its subtree by at most i roots (wide
 //     nodes or leaf slots of up to 4 triangles) and their decisions, as
 //     collapse.cpp does on the host;
 //  6. collapse to 8-wide nodes, one wide level per launch: the children by

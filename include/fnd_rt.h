@@ -216,8 +216,10 @@ int fnd_rt_scene_destroy(fnd_rt_scene* scene);
  * the watertight ray/triangle test in FP32.
  * mem = FND_MEM_DEVICE: rays / out are device pointers, the call only enqueues
  * work on the context stream (call fnd_rt_sync to wait and read the status);
- * mem = FND_MEM_HOST: host pointers (pinned or pageable), the call copies in,
- * traces, copies out and synchronises. */
+ * mem = FND_MEM_HOST: host pointers (pinned or pageable); the call traces and
+ * synchronises. Where the device shares the host's page tables it reads rays
+ * (16-byte aligned, not overlapping out) in place, and writes small results
+ * there; otherwise it copies in and out. */
 int fnd_rt_trace_closest(fnd_rt_ctx* ctx, const fnd_rt_scene* scene, const fnd_ray* rays, uint32_t n,
                          fnd_hit* out, int mem);
 
