@@ -9,6 +9,7 @@
 #include <chrono>
 #include <cmath>
 #include <cstring>
+#include <exception>
 #include <new>
 #include <thread>
 #include <vector>
@@ -646,6 +647,14 @@ int TraceImpl(fnd_rt_ctx* ctx, const fnd_rt_scene* scene, const fnd_ray* rays, u
         };
         if (stats) CUDA_CHECK(cudaMemsetAsync(ctx->d_stats, 0, 4 * sizeof(unsigned long long), ctx->stream));
         bool copied_back = false;
+        // on a failure after a launch in place: it still reads the caller's
+        // buffers, so the error returns only once it is done
+        struct Drain {
+            cudaStream_t s = nullptr;
+            ~Drain() {
+                if (s && std::uncaught_exceptions()) cudaStreamSynchronize(s);
+            }
+        } drain_in_place;
         if (mem == FND_MEM_DEVICE) {
             CHECK_CODE(((uintptr_t)rays & 15u) == 0 && ((uintptr_t)out & (any ? 0u : 7u)) == 0, FND_ERR_INVALID_ARG,
                        "device rays must be 16-byte aligned and hits 8-byte aligned");
@@ -661,6 +670,7 @@ int TraceImpl(fnd_rt_ctx* ctx, const fnd_rt_scene* scene, const fnd_ray* rays, u
                                   ((uintptr_t)rays & 15u) == 0 && apart;
             const bool out_in_place =
                 in_place && n <= kHitsInPlace && ((uintptr_t)out & (any ? 0u : 7u)) == 0;
+            if (in_place) drain_in_place.s = ctx->stream;
             if (!in_place) EnsureDevice(ctx->d_in, ctx->d_in_cap, sizeof(fnd_ray) * (size_t)n);
             if (!out_in_place) EnsureDevice(ctx->d_out, ctx->d_out_cap, hit_bytes * (size_t)n);
             auto* d_in = static_cast<char*>(ctx->d_in);
