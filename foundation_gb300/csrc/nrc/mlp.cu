@@ -60,61 +60,77 @@ __device__ __forceinline__ uint32_t b_addr(const uint16_t* m, int stride, int n0
     return sptr(m + (size_t)(n0 + 8 * (j >> 1) + r) * stride + k0 + ((j & 1) ? 8 : 0));
 }
 
-// Inference forward of one warp's 16 rows with the activations kept in
-// registers: the FP32 accumulator fragment of one layer, after ReLU and
+// Inference forward of one warp's 32 rows (two tiles of 16) with the activations
+// kept in registers: the FP32 accumulator fragment of one layer, after ReLU and
 // BF16 rounding, is exactly the A fragment of the next (same values as the
 // shared-memory round trip of the tile-wide forward). x: input rows (stride
-// 104).
-__device__ __forceinline__ void forward16_reg(const uint16_t* fwd, const uint16_t* x, int lane, float* y) {
-    uint32_t a[4][4];
-    float acc[8][4];
+// 104). Every weight fragment that is loaded serves both tiles.
+__device__ __forceinline__ void forward32_reg(const uint16_t* fwd, const uint16_t* x, int lane, float y[2][4]) {
+    uint32_t a[2][4][4];
+    float acc[2][8][4];
     // layer 0 from shared memory
 #pragma unroll
-    for (int i = 0; i < 8; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.0f;
+    for (int m = 0; m < 2; ++m)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) acc[m][i][0] = acc[m][i][1] = acc[m][i][2] = acc[m][i][3] = 0.0f;
     {
         const uint16_t* W = fwd + FwdOffset(0);
 #pragma unroll
         for (int kk = 0; kk < kIn / 16; ++kk) {
-            uint32_t af[4];
-            ldsm4(af, a_addr(x, kStrideX, 0, 16 * kk, lane));
+            uint32_t af[2][4];
+#pragma unroll
+            for (int m = 0; m < 2; ++m) ldsm4(af[m], a_addr(x, kStrideX, 16 * m, 16 * kk, lane));
 #pragma unroll
             for (int np = 0; np < 4; ++np) {
                 uint32_t b[4];
                 ldsm4(b, b_addr(W, kIn + kPad, 16 * np, 16 * kk, lane));
-                mma(acc[2 * np], af, b[0], b[1]);
-                mma(acc[2 * np + 1], af, b[2], b[3]);
+#pragma unroll
+                for (int m = 0; m < 2; ++m) {
+                    mma(acc[m][2 * np], af[m], b[0], b[1]);
+                    mma(acc[m][2 * np + 1], af[m], b[2], b[3]);
+                }
             }
         }
     }
 #pragma unroll 1
     for (int l = 1; l < kLayers; ++l) {
 #pragma unroll
-        for (int kk = 0; kk < 4; ++kk) {
-            a[kk][0] = pack2(fmaxf(acc[2 * kk][0], 0.f), fmaxf(acc[2 * kk][1], 0.f));
-            a[kk][1] = pack2(fmaxf(acc[2 * kk][2], 0.f), fmaxf(acc[2 * kk][3], 0.f));
-            a[kk][2] = pack2(fmaxf(acc[2 * kk + 1][0], 0.f), fmaxf(acc[2 * kk + 1][1], 0.f));
-            a[kk][3] = pack2(fmaxf(acc[2 * kk + 1][2], 0.f), fmaxf(acc[2 * kk + 1][3], 0.f));
-        }
+        for (int m = 0; m < 2; ++m)
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk) {
+                const float *c0 = acc[m][2 * kk], *c1 = acc[m][2 * kk + 1];
+                a[m][kk][0] = pack2(fmaxf(c0[0], 0.f), fmaxf(c0[1], 0.f));
+                a[m][kk][1] = pack2(fmaxf(c0[2], 0.f), fmaxf(c0[3], 0.f));
+                a[m][kk][2] = pack2(fmaxf(c1[0], 0.f), fmaxf(c1[1], 0.f));
+                a[m][kk][3] = pack2(fmaxf(c1[2], 0.f), fmaxf(c1[3], 0.f));
+            }
         const uint16_t* W = fwd + FwdOffset(l);
         if (l + 1 < kLayers) {
 #pragma unroll
-            for (int i = 0; i < 8; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.0f;
+            for (int m = 0; m < 2; ++m)
+#pragma unroll
+                for (int i = 0; i < 8; ++i) acc[m][i][0] = acc[m][i][1] = acc[m][i][2] = acc[m][i][3] = 0.0f;
 #pragma unroll
             for (int kk = 0; kk < 4; ++kk)
 #pragma unroll
                 for (int np = 0; np < 4; ++np) {
                     uint32_t b[4];
                     ldsm4(b, b_addr(W, kWidth + kPad, 16 * np, 16 * kk, lane));
-                    mma(acc[2 * np], a[kk], b[0], b[1]);
-                    mma(acc[2 * np + 1], a[kk], b[2], b[3]);
+#pragma unroll
+                    for (int m = 0; m < 2; ++m) {
+                        mma(acc[m][2 * np], a[m][kk], b[0], b[1]);
+                        mma(acc[m][2 * np + 1], a[m][kk], b[2], b[3]);
+                    }
                 }
         } else {
-            y[0] = y[1] = y[2] = y[3] = 0.0f;
+#pragma unroll
+            for (int m = 0; m < 2; ++m) y[m][0] = y[m][1] = y[m][2] = y[m][3] = 0.0f;
 #pragma unroll
             for (int kk = 0; kk < 4; ++kk) {
                 uint32_t b[2];
                 ldsm2(b, b_addr(W, kWidth + kPad, 0, 16 * kk, lane & 15));
-                mma(y, a[kk], b[0], b[1]);
+#pragma unroll
+                for (int m = 0; m < 2; ++m) mma(y[m], a[m][kk], b[0], b[1]);
             }
         }
     }
@@ -122,18 +138,34 @@ __device__ __forceinline__ void forward16_reg(const uint16_t* fwd, const uint16_
 
 
 // ---- inference ----------------------------------------------------------
+// A warp takes 32 queries at a time: a lane encodes one, then the warp runs the
+// network on two tiles of 16 rows. What bounds it: the latency of the chain of
+// warp-level MMAs and of the weight fragments' loads (issue 40%, tensor pipe 44%
+// with one tile of 16 per warp, where moreover the two halves of a row's encoding,
+// a lane each, ran one after the other). 2.07M queries 140 us with that form, 116
+// with this (1080p cache frame 1,333 and 1,316); 12, 16 or 24 warps a block in
+// place of 8 in that form: 0.3% of the frame.
 constexpr int kInferWarps = 8;
+constexpr int kInferRows = 32;  // per warp
+
+// Features first .. first + 47 of a row, as six 16-byte stores.
+__device__ __forceinline__ void store_half(uint16_t* xr, const uint16_t* f, int first) {
+#pragma unroll
+    for (int j = first; j < first + 48; j += 8)
+        *reinterpret_cast<uint4*>(xr + j) =
+            make_uint4((uint32_t)f[j] | (uint32_t)f[j + 1] << 16, (uint32_t)f[j + 2] | (uint32_t)f[j + 3] << 16,
+                       (uint32_t)f[j + 4] | (uint32_t)f[j + 5] << 16, (uint32_t)f[j + 6] | (uint32_t)f[j + 7] << 16);
+}
 
 template <bool kRaw>
-__global__ void __launch_bounds__(32 * kInferWarps) infer_kernel(const Net net, const CachePoint* pts,
-                                                                 const uint32_t* count, uint32_t capacity,
-                                                                 float4* fb, const float* raw_feats, uint32_t raw_n,
-                                                                 float* raw_out) {
+__global__ void __launch_bounds__(32 * kInferWarps, 2)
+    infer_kernel(const Net net, const CachePoint* pts, const uint32_t* count, uint32_t capacity, float4* fb,
+                 const float* raw_feats, uint32_t raw_n, float* raw_out) {
     extern __shared__ __align__(16) uint16_t smem[];
     uint16_t* s_fwd = smem;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, t = lane & 3;
-    uint16_t* xbuf = s_fwd + kFwdElems + warp * (16 * kStrideX);
+    uint16_t* xbuf = s_fwd + kFwdElems + warp * (kInferRows * kStrideX);
     {
         const int4* src = reinterpret_cast<const int4*>(net.fwd_avg ? net.fwd_avg : net.fwd);
         int4* dst = reinterpret_cast<int4*>(s_fwd);
@@ -141,28 +173,39 @@ __global__ void __launch_bounds__(32 * kInferWarps) infer_kernel(const Net net, 
     }
     __syncthreads();
     const uint32_t n = kRaw ? raw_n : min(*count, capacity);
-    const uint32_t tiles = (n + 15) / 16;
+    const uint32_t tiles = (n + kInferRows - 1) / kInferRows;
     for (uint32_t tile = blockIdx.x * kInferWarps + warp; tile < tiles; tile += gridDim.x * kInferWarps) {
-        const int row = lane >> 1, half = lane & 1;
-        const uint32_t q = tile * 16 + row;
-        uint16_t* xr = xbuf + row * kStrideX;
+        const uint32_t q = tile * kInferRows + lane;
+        uint16_t* xr = xbuf + lane * kStrideX;
+        uint16_t f[kIn];
         if (q >= n) {
-            for (int i = half * 48; i < half * 48 + 48; ++i) xr[i] = 0;
+#pragma unroll
+            for (int i = 0; i < kIn; ++i) f[i] = 0;
+            store_half(xr, f, 0);
+            store_half(xr, f, 48);
         } else if (kRaw) {
-            for (int i = half * 48; i < half * 48 + 48; ++i) xr[i] = bf16_bits(raw_feats[(size_t)q * kIn + i]);
+#pragma unroll
+            for (int i = 0; i < kIn; ++i) f[i] = bf16_bits(raw_feats[(size_t)q * kIn + i]);
+            store_half(xr, f, 0);
+            store_half(xr, f, 48);
         } else {
-            encode_half(pts[q], net.lo, net.hi, half, xr);
+            const CachePoint pt = pts[q];
+            encode_half(pt, net.lo, net.hi, 0, f);
+            store_half(xr, f, 0);
+            encode_half(pt, net.lo, net.hi, 1, f);
+            store_half(xr, f, 48);
         }
         __syncwarp();
-        float y[4];
-        forward16_reg(s_fwd, xbuf, lane, y);
+        float y[2][4];
+        forward32_reg(s_fwd, xbuf, lane, y);
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const uint32_t qr = tile * 16 + g + 8 * h;
+        for (int h = 0; h < 4; ++h) {
+            const uint32_t qr = tile * kInferRows + g + 8 * h;
+            const float* out = y[h >> 1] + 2 * (h & 1);
             if (qr >= n) continue;
             if (kRaw) {
                 for (int e = 0; e < 2; ++e)
-                    if (2 * t + e < kOut) raw_out[(size_t)qr * kOut + 2 * t + e] = y[2 * h + e];
+                    if (2 * t + e < kOut) raw_out[(size_t)qr * kOut + 2 * t + e] = out[e];
             } else {
                 const CachePoint& c = pts[qr];
                 const uint32_t pixel = __float_as_uint(c.wo_aux.w);
@@ -171,7 +214,7 @@ __global__ void __launch_bounds__(32 * kInferWarps) infer_kernel(const Net net, 
                 for (int e = 0; e < 2; ++e) {
                     const int ch = 2 * t + e;
                     if (ch < kOut) {
-                        const float v = bt[ch] * fmaxf(y[2 * h + e], 0.0f);
+                        const float v = bt[ch] * fmaxf(out[e], 0.0f);
                         if (v > 0.0f) atomicAdd(dst + ch, v);
                     }
                 }
@@ -268,7 +311,7 @@ __global__ void images_kernel(const Net net) {
     }
 }
 
-size_t infer_smem() { return sizeof(uint16_t) * ((size_t)kFwdElems + (size_t)kInferWarps * 16 * kStrideX); }
+size_t infer_smem() { return sizeof(uint16_t) * ((size_t)kFwdElems + (size_t)kInferWarps * kInferRows * kStrideX); }
 
 template <typename K>
 cudaError_t allow_smem(K kernel, size_t bytes) {
@@ -306,7 +349,7 @@ cudaError_t Infer(const Net& net, const CachePoint* pts, const uint32_t* count, 
 cudaError_t InferRaw(const Net& net, const float* feats, uint32_t n, float* out, cudaStream_t s) {
     cudaError_t e = allow_smem(infer_kernel<true>, infer_smem());
     if (e != cudaSuccess) return e;
-    const uint32_t tiles = (n + 15) / 16;
+    const uint32_t tiles = (n + kInferRows - 1) / kInferRows;
     const int grid = (int)((tiles + kInferWarps - 1) / kInferWarps);
     infer_kernel<true><<<grid > 0 ? grid : 1, 32 * kInferWarps, infer_smem(), s>>>(net, nullptr, nullptr, 0, nullptr,
                                                                                    feats, n, out);

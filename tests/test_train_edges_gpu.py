@@ -51,3 +51,15 @@ def test_gradient_edges(ctx, n):
             off += k
         if n <= 128:
             assert np.array_equal(g, got[0][0]) and loss == got[0][1]
+
+
+@pytest.mark.parametrize("n", [1, 15, 16, 17, 31, 32, 33, 255, 257, 3000])
+def test_inference_edges(ctx, n):
+    """A row's output depends on its own features only, whatever tile of 32 it
+    lies in: the first rows of a large call, to the bit; and rows past the end
+    are not written."""
+    rng = np.random.default_rng(1)
+    x = rng.uniform(-1, 1, (4096, 96)).astype(np.float32)
+    whole = ctx.cache_eval(x)
+    assert np.array_equal(ctx.cache_eval(x[:n]), whole[:n])
+    assert np.array_equal(ctx.cache_eval(x[7:7 + n]), whole[7:7 + n])
