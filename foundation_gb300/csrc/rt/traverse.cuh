@@ -184,8 +184,14 @@ __device__ __forceinline__ uint32_t xor_permute8(uint32_t m, uint32_t oct) {
     return m;
 }
 
+// The culling bound of a best t (or a ray's length) for intersect_slots: the
+// same value, with +0 for -0. A hit at the origin often has t = -0, and against
+// a node's tn = +0 the sign of -0 - (+0) would say that the box is missed, with
+// triangles of equal t and lower id in it. (Once per bound, not per node.)
+__device__ __forceinline__ float bound_of(float t) { return __fadd_rn(t, 0.0f); }
+
 // Tests the 8 child boxes of one compressed node against the ray: which slots
-// were hit, and the node's words that say what the slots hold.
+// were hit, and the node's words that say what the slots hold. tfar: a bound_of.
 struct SlotHits {
     uint32_t child_base;
     uint32_t tri_base;
@@ -251,6 +257,11 @@ __device__ __forceinline__ SlotHits intersect_slots(const RayState& r, const uin
         }
 #pragma unroll
         for (int e = 1; e >= 0; --e) {
+            // miss: the sign of tf - tn, shifted in (a difference and a funnel
+            // shift: the compare and select of the plain form both go to the
+            // integer pipe, the busier one). Equal infinities give a NaN of
+            // positive sign and equal values +0, a hit as under tn <= tf; only
+            // tf = -0 against tn = +0 would differ, hence bound_of.
             float tx[2], ty[2], tz[2];  // near t, -(far t)
             fma_dir_f2<false>(pack_f2(nx[e], gx[e]), sx2, bx2, tx);
             fma_dir_f2<false>(pack_f2(ny[e], gy[e]), sy2, by2, ty);
@@ -258,13 +269,10 @@ __device__ __forceinline__ SlotHits intersect_slots(const RayState& r, const uin
             const float tn = max3f(tx[0], ty[0], fmaxf(tz[0], r.tmin));
             const float ntf = max3f(tx[1], ty[1], fmaxf(tz[1], ntfar));
 #if defined(__CUDA_ARCH__)
-            // the sign of tf - tn, shifted in (a difference and a funnel
-            // shift: the compare and select of the plain form both go to the
-            // integer pipe, the busier one). Equal infinities give a NaN of
-            // positive sign, a hit as under tn <= tf.
             miss = __funnelshift_l(__float_as_uint(__fsub_rn(-ntf, tn)), miss, 1);
 #else
-            miss = miss << 1 | (tn <= -ntf ? 0u : 1u);
+            const float span = -ntf - tn;  // (a host NaN's sign may be set)
+            miss = miss << 1 | (span == span && signbit(span) ? 1u : 0u);
 #endif
         }
     }
@@ -299,7 +307,7 @@ struct NodeHits {
 
 __device__ __forceinline__ NodeHits intersect_node(const RayState& r, const uint4* __restrict__ nodes, uint32_t idx,
                                                    float tfar) {
-    const SlotHits h = intersect_slots(r, nodes, idx, tfar);
+    const SlotHits h = intersect_slots(r, nodes, idx, bound_of(tfar));
     uint32_t lh = h.hitm & leaf_slots(h), tris = 0;
     while (lh) {  // about one hit leaf per three nodes on incoherent rays
         const uint32_t s = (uint32_t)__ffs(lh) - 1u;

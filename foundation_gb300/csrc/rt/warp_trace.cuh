@@ -202,7 +202,7 @@ __device__ __forceinline__ void trace_loop(const Src& src, const Common& C, uint
     typename Src::Lane ln = lane_src;
     bool active = st.active, exhausted = st.exhausted, any_hit = kKind == 1 || (kKind == 2 && st.active && src.any_of(ln, false));
     uint32_t ray_id = st.ray_id;
-    float best_t = st.best_t, tmin = 0.0f;
+    float best_t = st.best_t, tmin = 0.0f;  // best_t: the culling bound (the hit itself is in shared memory)
     uint32_t ng_base = st.ng_base, ng_group = st.ng_group;
     int sp = st.sp;
     // the warp's ring: ranges head .. tail - 1 (modulo 2^32), with `tris` triangles written
@@ -305,7 +305,7 @@ __device__ __forceinline__ void trace_loop(const Src& src, const Common& C, uint
                 slot = lane;
                 if constexpr (kOwnScene) cur = src.scene_of(ln);
                 if constexpr (kOwnKind) follows_any = any_hit;
-                best_t = r.tmax;
+                best_t = bound_of(r.tmax);
                 sts64(wl + W::kBest, __float_as_uint(r.tmax), FND_INVALID_ID);
                 start(src.scene_of(ln).num_nodes, octx_of(r));
                 active = true;
@@ -347,7 +347,7 @@ __device__ __forceinline__ void trace_loop(const Src& src, const Common& C, uint
                     ng_base = e.x;
                     ng_group = e.y;
                     slot = whose;
-                    best_t = __uint_as_float(lds32(w + 8u * slot + W::kBest));
+                    best_t = bound_of(__uint_as_float(lds32(w + 8u * slot + W::kBest)));
                 }
                 __syncwarp();
             }
@@ -538,7 +538,7 @@ __device__ __forceinline__ void trace_loop(const Src& src, const Common& C, uint
                     __syncwarp();
                 } while (__ballot_sync(kFull, hit));
                 const uint2 bst = lds64(ws + W::kBest);
-                best_t = __uint_as_float(bst.x);
+                best_t = bound_of(__uint_as_float(bst.x));
                 if ((kKind == 1 || (kKind == 2 && (kOwnKind ? follows_any : any_hit))) && (kSteal || active) && bst.y != FND_INVALID_ID) {
                     ng_group = 0;  // found: only the ranges already in the ring remain
                     sp = 0;
