@@ -36,13 +36,14 @@ namespace {
 
 constexpr int kSub = 256;  // sub-pixel steps per pixel
 constexpr double kUvOne = 1099511627776.0;  // 2^40: fixed-point texture coordinates
+constexpr double kEps1 = 2.5e-4, kEps2 = 1e-7;  // bounds without the coordinates' errors, per unit of colour (see shade)
 
 struct alignas(16) Tri {
     int x0, y0, x1, y1;    // inclusive pixel bounds; x0 > x1 when the triangle is skipped
     long long e0[3];       // edge functions at the centre of pixel (0, 0), inside >= 0,
     long long sx[3], sy[3];  // and their steps per pixel
     uint32_t topleft;      // bit i: edge opposite vertex i is a top or left edge
-    float cm;              // largest vertex colour (magnitude), at least 1
+    float eps1, eps2;      // error bounds of the two quick evaluations, in codes (see shade)
     // per vertex, over its w: texture coordinates times 2^40, 1, colours
     double cu[3], cv[3], iw[3], cd[3][3];
     float cf[3][3];
@@ -177,7 +178,11 @@ __device__ __forceinline__ void setup(const DrawArgs& A, const Vertex* verts, co
                     cm = V.color[c] == V.color[c] ? fmaxf(cm, fabsf(V.color[c])) : __int_as_float(0x7F800000);
                 }
             }
-            T.cm = cm;
+            // texture coordinates are floored to 2^-40 of a repeat, and a repeat
+            // of n texels takes a channel through n slopes of at most 255 codes
+            const double coords = 255.0 * ((double)A.tex_w + (double)A.tex_h) * (1.0 / kUvOne);
+            T.eps1 = __double2float_ru((double)cm * (kEps1 + coords));
+            T.eps2 = __double2float_ru((double)cm * (kEps2 + coords));
         }
     }
     tris[t] = T;
@@ -264,14 +269,13 @@ __device__ __forceinline__ void wrap(long long c, uint32_t n, uint32_t& i0, uint
     frac = (unsigned long long)t & (one - 1);
 }
 
-// Colour of a covered pixel. Errors of the first try, relative to cm x 255:
-// colours 4.2e-7 (float edge functions, products, sums and reciprocal), two
-// lerps of texels 1.6e-7, their product 1.2e-7, texture coordinates below
-// 1e-9 (|u| <= 1024, at most 16,384 texels): 1.8e-4 of a code, kEps1 2.5e-4.
-// Second try: everything in FP64, below 1e-9.
+// Colour of a covered pixel. Errors of the first try, relative to the largest
+// colour x 255: colours 4.2e-7 (float edge functions, products, sums and
+// reciprocal), two lerps of texels 1.6e-7, their product 1.2e-7: 1.8e-4 of a
+// code, kEps1 2.5e-4. Second try, in FP64: colours and lerps below 1e-11, kEps2
+// 1e-7. To both comes what the error of the texture coordinates can do (setup):
+// 255 (w + h) 2^-40 of a code, 2.4e-7 for 512 texels a side, 7.6e-6 for 16,384.
 __device__ __forceinline__ uint32_t shade(const DrawArgs& A, const Tri& T, const long long E[3]) {
-    constexpr float kEps1 = 2.5e-4f;
-    constexpr double kEps2 = 1e-7;
     const double e[3] = {(double)E[0], (double)E[1], (double)E[2]};
     const double D = fma(e[2], T.iw[2], fma(e[1], T.iw[1], e[0] * T.iw[0]));
     const float Df = (float)D;
@@ -292,7 +296,7 @@ __device__ __forceinline__ uint32_t shade(const DrawArgs& A, const Tri& T, const
                 const float au = (float)(uint32_t)(fu >> 8) * 2.3283064365386963e-10f;  // 2^-32
                 const float av = (float)(uint32_t)(fv >> 8) * 2.3283064365386963e-10f;
                 const float ef[3] = {(float)e[0], (float)e[1], (float)e[2]};
-                const float rf = (float)r, eps = kEps1 * T.cm;
+                const float rf = (float)r, eps = T.eps1;
                 uint32_t out = 0;
                 bool ok = true;
 #pragma unroll
@@ -319,7 +323,7 @@ __device__ __forceinline__ uint32_t shade(const DrawArgs& A, const Tri& T, const
                 double v = fma(av, hi - lo, lo);
                 if (ch < 3) v *= fma(e[2], T.cd[2][ch], fma(e[1], T.cd[1][ch], e[0] * T.cd[0][ch])) * r;
                 uint32_t byte;
-                ok = settle(v, kEps2 * (double)T.cm, byte) && ok;
+                ok = settle(v, (double)T.eps2, byte) && ok;
                 out |= byte << 8 * ch;
             }
             if (ok) return out;
