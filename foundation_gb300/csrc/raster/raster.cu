@@ -36,7 +36,9 @@ namespace {
 
 constexpr int kSub = 256;  // sub-pixel steps per pixel
 constexpr double kUvOne = 1099511627776.0;  // 2^40: fixed-point texture coordinates
-constexpr double kEps1 = 2.5e-4, kEps2 = 1e-7;  // bounds without the coordinates' errors, per unit of colour (see shade)
+// Error bounds (see shade): of a code per unit of colour, without the texture
+// coordinates' errors, and of a coordinate relative to the triangle's largest.
+constexpr double kEps1 = 2.5e-4, kEps2 = 1e-7, kEpsUv = 2.5e-14;
 
 struct alignas(16) Tri {
     int x0, y0, x1, y1;    // inclusive pixel bounds; x0 > x1 when the triangle is skipped
@@ -178,9 +180,15 @@ __device__ __forceinline__ void setup(const DrawArgs& A, const Vertex* verts, co
                     cm = V.color[c] == V.color[c] ? fmaxf(cm, fabsf(V.color[c])) : __int_as_float(0x7F800000);
                 }
             }
-            // texture coordinates are floored to 2^-40 of a repeat, and a repeat
-            // of n texels takes a channel through n slopes of at most 255 codes
-            const double coords = 255.0 * ((double)A.tex_w + (double)A.tex_h) * (1.0 / kUvOne);
+            // texture coordinates are floored to 2^-40 of a repeat and rounded in
+            // proportion to the vertices' (kEpsUv), and a repeat of n texels
+            // takes a channel through n slopes of at most 255 codes
+            double coords = 0.0;
+            for (int c = 0; c < 2; ++c) {
+                const float *a = verts[vid[0]].uv, *b = verts[vid[1]].uv, *d = verts[vid[2]].uv;
+                const double m = fmaxf(fabsf(a[c]), fmaxf(fabsf(b[c]), fabsf(d[c])));  // (a NaN's pixels fail anyway)
+                coords += 255.0 * (double)(c ? A.tex_h : A.tex_w) * (1.0 / kUvOne + kEpsUv * m);
+            }
             T.eps1 = __double2float_ru((double)cm * (kEps1 + coords));
             T.eps2 = __double2float_ru((double)cm * (kEps2 + coords));
         }
@@ -274,13 +282,16 @@ __device__ __forceinline__ void wrap(long long c, uint32_t n, uint32_t& i0, uint
 // reciprocal), two lerps of texels 1.6e-7, their product 1.2e-7: 1.8e-4 of a
 // code, kEps1 2.5e-4. Second try, in FP64: colours and lerps below 1e-11, kEps2
 // 1e-7. To both comes what the error of the texture coordinates can do (setup):
-// 255 (w + h) 2^-40 of a code, 2.4e-7 for 512 texels a side, 7.6e-6 for 16,384.
+// 255 (w + h) 2^-40 of a code, 2.4e-7 for 512 texels a side, 7.6e-6 for 16,384,
+// and their rounding, which scales with the vertices' coordinates where these
+// cancel: 1 / D 128 units of 2^-53 (the square of the float reciprocal's 2^-23),
+// the quick sums and quotients 12, the definition's 12: 1.7e-14, kEpsUv 2.5e-14.
 __device__ __forceinline__ uint32_t shade(const DrawArgs& A, const Tri& T, const long long E[3]) {
     const double e[3] = {(double)E[0], (double)E[1], (double)E[2]};
     const double D = fma(e[2], T.iw[2], fma(e[1], T.iw[1], e[0] * T.iw[0]));
     const float Df = (float)D;
     if (Df > 1e-30f && Df < 1e30f && A.tex_w <= 16384u && A.tex_h <= 16384u) {
-        // 1 / D by one Newton step from the float reciprocal: 4e-15
+        // 1 / D by one Newton step from the float reciprocal: 1.4e-14
         const double r0 = (double)(1.0f / Df);
         const double r = fma(r0, fma(-D, r0, 1.0), r0);
         const double U = fma(e[2], T.cu[2], fma(e[1], T.cu[1], e[0] * T.cu[0])) * r;
