@@ -358,6 +358,7 @@ cudaError_t InferRaw(const Net& net, const float* feats, uint32_t n, float* out,
 
 static cudaError_t launch_adam(Net& net, float lr, cudaStream_t s) {
     net.step += 1;
+    net.grad_left = false;
     const double c1 = 1.0 - std::pow(0.9, (double)net.step), c2 = 1.0 - std::pow(0.99, (double)net.step);
     double c3 = 1.0;
     if (net.avg) {
@@ -370,7 +371,8 @@ static cudaError_t launch_adam(Net& net, float lr, cudaStream_t s) {
 
 cudaError_t TrainStep(Net& net, const TrainSample* smp, const float4* targets, const uint32_t* count, uint32_t batch,
                       uint64_t seed, float lr, uint32_t* status, cudaStream_t s) {
-    cudaError_t e = LaunchTrainUmma(net, smp, targets, count, batch, seed, status, s);
+    cudaError_t e = net.grad_left ? cudaMemsetAsync(net.grad, 0, sizeof(float) * kNumParams, s) : cudaSuccess;
+    if (e == cudaSuccess) e = LaunchTrainUmma(net, smp, targets, count, batch, seed, status, s);
     if (e != cudaSuccess) return e;
     return launch_adam(net, lr, s);
 }

@@ -86,9 +86,10 @@ struct Net {
     float* master;    // fp32 weights, row-major W[K][N] per layer (kNumParams)
     float* adam_m;
     float* adam_v;
-    float* grad;      // fp32 gradient accumulator (kNumParams)
+    float* grad;      // fp32 gradient accumulator (kNumParams): training steps add to it, Adam clears it
     double* loss;     // [0] running sum of the loss of the current step, [1] CTAs done (GradRaw)
     uint32_t step;    // Adam steps taken
+    bool grad_left;   // GradRaw's result is still in grad: the next training step clears it first
     // weight averaging (queries only): fp32 moving average of the iterates
     // and the bf16 forward image of avg / (1 - decay^avg_steps); null: off
     float* avg;
@@ -113,10 +114,10 @@ cudaError_t TrainStep(Net& net, const TrainSample* smp, const float4* targets, c
 // Gradient of the loss on explicit features / targets (no Adam), in net.grad and
 // net.loss; with out_grad the last CTA also copies both to out_grad and out_loss.
 // Every pointer may be to host memory that the device reads and writes.
-cudaError_t GradRaw(const Net& net, const float* feats, const float* targets, uint32_t n, float* out_grad,
+cudaError_t GradRaw(Net& net, const float* feats, const float* targets, uint32_t n, float* out_grad,
                     double* out_loss, uint32_t* status, cudaStream_t s);
 cudaError_t AdamRaw(Net& net, float lr, cudaStream_t s);
-// The step's gradient alone (train_umma.cu): accumulates into net.grad.
+// The step's gradient alone (train_umma.cu), added to net.grad.
 cudaError_t LaunchTrainUmma(const Net& net, const TrainSample* smp, const float4* targets, const uint32_t* count,
                             uint32_t batch, uint64_t seed, uint32_t* status, cudaStream_t s);
 // bf16 images from the fp32 master weights; restarts the weight average

@@ -480,10 +480,11 @@ cudaError_t LaunchTrainUmma(const Net& net, const TrainSample* smp, const float4
     return cudaGetLastError();
 }
 
-cudaError_t GradRaw(const Net& net, const float* feats, const float* targets, uint32_t n, float* out_grad,
+cudaError_t GradRaw(Net& net, const float* feats, const float* targets, uint32_t n, float* out_grad,
                     double* out_loss, uint32_t* status, cudaStream_t s) {
     cudaError_t e = allow_smem(train_umma_kernel<true>);
     if (e != cudaSuccess) return e;
+    net.grad_left = true;
     // (the loss may lie directly behind the gradient: one launch clears both)
     const bool one = reinterpret_cast<char*>(net.loss) == reinterpret_cast<char*>(net.grad + kNumParams);
     const size_t sums = 2 * sizeof(double);  // loss and CTA count
