@@ -315,7 +315,8 @@ int fnd_rt_cache_gradient(fnd_rt_ctx* ctx, const float* features, const float* t
             cudaStreamSynchronize(ctx->stream);  // the caller's buffers are still read
             throw;
         }
-        CUDA_CHECK(cudaStreamSynchronize(ctx->stream));
+        const int st = CApi::ReadStatus(ctx);
+        if (st != FND_OK) Fail(st, "device status after the gradient: %d", st);
         const double l = *ctx->h_loss;
         if (loss) *loss = l / (3.0 * n);
     });

@@ -531,7 +531,8 @@ int fnd_rt_cache_load(fnd_rt_ctx* ctx, const char* path);
 /* Network on explicit features (n x 96 host floats) -> n x 3 host floats. */
 int fnd_rt_cache_eval(fnd_rt_ctx* ctx, const float* features, uint32_t n, float* out);
 /* Gradient of the mean relative-L2 loss on explicit features / targets
- * (n x 3): grad receives FND_CACHE_NUM_PARAMS floats, loss the mean loss. */
+ * (n x 3): grad receives FND_CACHE_NUM_PARAMS floats, loss the mean loss. Reads
+ * and clears the status word, as fnd_rt_sync does. */
 int fnd_rt_cache_gradient(fnd_rt_ctx* ctx, const float* features, const float* targets, uint32_t n, float* grad,
                           double* loss);
 /* The network's input features of n points, each 13 host floats: position,
