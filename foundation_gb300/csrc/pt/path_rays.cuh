@@ -61,6 +61,7 @@ struct LaneHits {
 template <bool kTwoLevel>
 struct PathSource {
     using P = PathShared<kTwoLevel>;
+    static constexpr bool kCounted = true;
     RT::DeviceScene scene;  // two levels: the top one
     const RT::InstanceRec* inst;
     uint32_t num_inst;

@@ -56,6 +56,7 @@ uint32_t FewRays(uint32_t warps) { return 24u * warps; }
 // ---- work sources -----------------------------------------------------------
 // One scene, one ray array, one query kind for the whole launch.
 struct SingleSource {
+    static constexpr bool kCounted = false;
     DeviceScene scene;
     const float4* rays;
     void* hits;
@@ -83,6 +84,7 @@ struct SingleSource {
 // A job table; a global ray id is mapped to its job by binary search over
 // the prefix of ray counts (kept in shared memory when it fits).
 struct BatchSource {
+    static constexpr bool kCounted = false;
     const BatchJob* jobs;
     const uint32_t* prefix;  // njobs + 1 entries
     uint32_t njobs;
@@ -126,6 +128,7 @@ struct BatchSource {
 
 // Rays against a two-level scene: the top level's leaves are instances.
 struct InstancedSource {
+    static constexpr bool kCounted = false;
     DeviceScene scene;  // the top level
     const InstanceRec* inst;
     uint32_t num_inst;

@@ -24,7 +24,7 @@ constexpr uint32_t kWaitMin = 4;
 constexpr uint32_t kHelpAt = 28;
 
 struct Common {
-    uint32_t* counter;  // null (few rays): every warp takes its one run of them
+    uint32_t* counter;  // null (few rays, a source that is not kCounted): every warp takes its one run of them
     uint32_t* status;
     unsigned long long* stats;
     uint32_t refill_min;
@@ -283,7 +283,7 @@ __device__ __forceinline__ void trace_loop(const Src& src, const Common& C, uint
             if (exhausted) break;
             const uint32_t cnt = (uint32_t)__popc(ready);
             uint32_t base = 0;
-            if (kFew && !C.counter) {
+            if (kFew && !Src::kCounted && !C.counter) {
                 base = (blockIdx.x * blockDim.x + threadIdx.x) / 32u * lanes;
                 exhausted = true;
             } else {

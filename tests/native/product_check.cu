@@ -14,3 +14,9 @@ extern "C" int product_latch_status(fnd_rt_ctx* ctx, uint32_t bits) {
                ? 0
                : 1;
 }
+
+// Resident blocks of 128 threads per SM of the path kernels.
+extern "C" int product_tail_blocks(int two_level) { return Foundation::PT::TailBlocksPerSm(two_level != 0); }
+extern "C" int product_training_blocks(int two_level) {
+    return Foundation::PT::TrainingPathsBlocksPerSm(two_level != 0);
+}
