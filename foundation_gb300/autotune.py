@@ -49,12 +49,16 @@ class TuneTable:
         if not os.path.exists(path):
             return cls()
         with open(path) as f:
-            return cls(json.load(f).get("entries", {}))
+            saved = json.load(f)
+        entries = saved.get("entries", {})
+        if saved.get("version", 1) < 2:  # there postpone_min was another threshold: the default in its place
+            entries = {k: dict(e, postpone_min=0) if "postpone_min" in e else e for k, e in entries.items()}
+        return cls(entries)
 
     def save(self, path: str) -> None:
         tmp = path + ".tmp"
         with open(tmp, "w") as f:
-            json.dump({"version": 1, "entries": self.entries}, f, indent=1, sort_keys=True)
+            json.dump({"version": 2, "entries": self.entries}, f, indent=1, sort_keys=True)
         os.replace(tmp, path)
 
     def record(self, num_tris: int, coherence: str, kind: int, best: dict, table: list) -> dict:
