@@ -110,8 +110,12 @@ namespace CApi {
 
 void UploadTriangles(fnd_rt_ctx* ctx, const float* v0, const float* v1, const float* v2, uint32_t n, void* d_tris) {
     constexpr uint32_t kChunk = 1u << 20;
-    char* staging = nullptr;
-    CUDA_CHECK(cudaMalloc(&staging, 48ull * std::max(1u, std::min(n, kChunk))));
+    if (n == 0) return;
+    // staged in the context's input buffer: one that each upload allocates and
+    // frees takes 0.16 ms more (an upload's copies for 20,000 triangles 0.28 and
+    // 0.12 ms, for 1M 1.16 and 1.02)
+    EnsureDevice(ctx->d_in, ctx->d_in_cap, 48ull * std::min(n, kChunk));
+    char* staging = static_cast<char*>(ctx->d_in);
     try {
         for (uint32_t at = 0; at < n; at += kChunk) {
             const uint32_t cnt = std::min(kChunk, n - at);
@@ -122,13 +126,11 @@ void UploadTriangles(fnd_rt_ctx* ctx, const float* v0, const float* v1, const fl
             CUDA_CHECK(RT::InterleaveTriangles(reinterpret_cast<const float4*>(staging), cnt,
                                                static_cast<float4*>(d_tris) + 3 * (size_t)at, ctx->stream));
         }
-        CUDA_CHECK(cudaStreamSynchronize(ctx->stream));
     } catch (...) {
-        cudaStreamSynchronize(ctx->stream);
-        cudaFree(staging);
+        cudaStreamSynchronize(ctx->stream);  // the caller's planes are still read
         throw;
     }
-    CUDA_CHECK(cudaFree(staging));
+    CUDA_CHECK(cudaStreamSynchronize(ctx->stream));
 }
 
 void ViewTriangles(RT::DeviceScene& view, const void* d_tris, uint32_t n) {

@@ -154,7 +154,7 @@ cudaError_t LaunchTraceOrdered(fnd_rt_ctx* ctx, const fnd_rt_scene* scene, Found
                                cudaStream_t stream = nullptr);
 
 // The host's three vertex planes (n float4 each) as device records of three
-// vertices per triangle, through a staging buffer of at most 48 MB.
+// vertices per triangle, staged 1M triangles at a time in ctx->d_in.
 void UploadTriangles(fnd_rt_ctx* ctx, const float* v0, const float* v1, const float* v2, uint32_t n, void* d_tris);
 // The device view of a scene's triangle records.
 void ViewTriangles(Foundation::RT::DeviceScene& view, const void* d_tris, uint32_t n);
