@@ -489,83 +489,83 @@ __device__ __forceinline__ void dp_child(const Buffers& B, uint32_t ref, const R
 // internal node p, whose children are finished.
 __device__ __forceinline__ void finish_node(const Buffers& B, uint32_t p, uint32_t left, uint32_t right,
                                             uint32_t max_leaf, float trav_cost) {
-            const RefBox l = ref_box(B, left), r = ref_box(B, right);
-            float4 lo = make_float4(fminf(l.lo.x, r.lo.x), fminf(l.lo.y, r.lo.y), fminf(l.lo.z, r.lo.z), 0.0f);
-            float4 hi = make_float4(fmaxf(l.hi.x, r.hi.x), fmaxf(l.hi.y, r.hi.y), fmaxf(l.hi.z, r.hi.z), 0.0f);
-            const uint32_t cnt = (l.count & ~kLeafNode) + (r.count & ~kLeafNode);
-            const float a = half_area(lo, hi);
-            const float split = trav_cost * a + l.cost + r.cost;
-            const bool leaf = cnt <= max_leaf && (float)cnt * a <= split;
-            lo.w = __uint_as_float(cnt | (leaf ? kLeafNode : 0u));
-            hi.w = leaf ? (float)cnt * a : split;
-            B.nlo[p] = lo;
-            B.nhi[p] = hi;
-            if (B.dpc) {
-                // SAH-optimal collapse: wide node at cost a, leaf slot at c_tri a cnt
-                float cl[8], cr[8], sp[7];  // sp[i - 2]: the subtree as i roots, split between the children
-                uint32_t sj[7];             // and the left child's share
-                dp_child(B, left, l, cl);
-                dp_child(B, right, r, cr);
-    #pragma unroll
-                for (int i = 0; i < 7; ++i) {
-                    sp[i] = FLT_MAX;
-                    sj[i] = 1;
-                }
-                // j roots left, k right, in ascending j for every sum
-    #pragma unroll
-                for (int j = 1; j <= 7; ++j)
-    #pragma unroll
-                    for (int k = 1; k <= 7; ++k)
-                        if (j + k <= 8) {
-                            const float v = cl[j - 1] + cr[k - 1];
-                            if (v < sp[j + k - 2]) {
-                                sp[j + k - 2] = v;
-                                sj[j + k - 2] = (uint32_t)j;
-                            }
-                        }
-                // (constant indices: the tables stay in registers)
-                const uint32_t width = B.width;
-                const float at_width = width == 8u   ? sp[6]
-                                       : width == 7u ? sp[5]
-                                       : width == 6u ? sp[4]
-                                       : width == 5u ? sp[3]
-                                       : width == 4u ? sp[2]
-                                       : width == 3u ? sp[1]
-                                                     : sp[0];
-                const uint32_t j_width = width == 8u   ? sj[6]
-                                         : width == 7u ? sj[5]
-                                         : width == 6u ? sj[4]
-                                         : width == 5u ? sj[3]
-                                         : width == 4u ? sj[2]
-                                         : width == 3u ? sj[1]
-                                                       : sj[0];
-                float c[8];
-                const float node_cost = a + at_width;
-                c[0] = node_cost;
-                uint32_t as_leaf = 0;
-                if (cnt <= (uint32_t)kMaxLeafTris) {
-                    const float leaf_cost = B.c_tri * a * (float)cnt;
-                    if (leaf_cost <= node_cost) {
-                        c[0] = leaf_cost;
-                        as_leaf = kDpLeaf;
+    const RefBox l = ref_box(B, left), r = ref_box(B, right);
+    float4 lo = make_float4(fminf(l.lo.x, r.lo.x), fminf(l.lo.y, r.lo.y), fminf(l.lo.z, r.lo.z), 0.0f);
+    float4 hi = make_float4(fmaxf(l.hi.x, r.hi.x), fmaxf(l.hi.y, r.hi.y), fmaxf(l.hi.z, r.hi.z), 0.0f);
+    const uint32_t cnt = (l.count & ~kLeafNode) + (r.count & ~kLeafNode);
+    const float a = half_area(lo, hi);
+    const float split = trav_cost * a + l.cost + r.cost;
+    const bool leaf = cnt <= max_leaf && (float)cnt * a <= split;
+    lo.w = __uint_as_float(cnt | (leaf ? kLeafNode : 0u));
+    hi.w = leaf ? (float)cnt * a : split;
+    B.nlo[p] = lo;
+    B.nhi[p] = hi;
+    if (B.dpc) {
+        // SAH-optimal collapse: wide node at cost a, leaf slot at c_tri a cnt
+        float cl[8], cr[8], sp[7];  // sp[i - 2]: the subtree as i roots, split between the children
+        uint32_t sj[7];             // and the left child's share
+        dp_child(B, left, l, cl);
+        dp_child(B, right, r, cr);
+#pragma unroll
+        for (int i = 0; i < 7; ++i) {
+            sp[i] = FLT_MAX;
+            sj[i] = 1;
+        }
+        // j roots left, k right, in ascending j for every sum
+#pragma unroll
+        for (int j = 1; j <= 7; ++j)
+#pragma unroll
+            for (int k = 1; k <= 7; ++k)
+                if (j + k <= 8) {
+                    const float v = cl[j - 1] + cr[k - 1];
+                    if (v < sp[j + k - 2]) {
+                        sp[j + k - 2] = v;
+                        sj[j + k - 2] = (uint32_t)j;
                     }
                 }
-                uint2 ch = make_uint2(j_width | as_leaf, 0u);
-    #pragma unroll
-                for (int i = 2; i <= 8; ++i) {
-                    const bool two = sp[i - 2] < c[i - 2];
-                    c[i - 1] = two ? sp[i - 2] : c[i - 2];
-                    const uint32_t w = two ? sj[i - 2] : 0u;
-                    if (i <= 4)
-                        ch.x |= w << 8 * (i - 1);
-                    else
-                        ch.y |= w << 8 * (i - 5);
-                }
-                float4* dc = reinterpret_cast<float4*>(B.dpc + 8 * (size_t)p);
-                dc[0] = make_float4(c[0], c[1], c[2], c[3]);
-                dc[1] = make_float4(c[4], c[5], c[6], c[7]);
-                B.dpch[p] = ch;
+        // (constant indices: the tables stay in registers)
+        const uint32_t width = B.width;
+        const float at_width = width == 8u   ? sp[6]
+                               : width == 7u ? sp[5]
+                               : width == 6u ? sp[4]
+                               : width == 5u ? sp[3]
+                               : width == 4u ? sp[2]
+                               : width == 3u ? sp[1]
+                                             : sp[0];
+        const uint32_t j_width = width == 8u   ? sj[6]
+                                 : width == 7u ? sj[5]
+                                 : width == 6u ? sj[4]
+                                 : width == 5u ? sj[3]
+                                 : width == 4u ? sj[2]
+                                 : width == 3u ? sj[1]
+                                               : sj[0];
+        float c[8];
+        const float node_cost = a + at_width;
+        c[0] = node_cost;
+        uint32_t as_leaf = 0;
+        if (cnt <= (uint32_t)kMaxLeafTris) {
+            const float leaf_cost = B.c_tri * a * (float)cnt;
+            if (leaf_cost <= node_cost) {
+                c[0] = leaf_cost;
+                as_leaf = kDpLeaf;
             }
+        }
+        uint2 ch = make_uint2(j_width | as_leaf, 0u);
+#pragma unroll
+        for (int i = 2; i <= 8; ++i) {
+            const bool two = sp[i - 2] < c[i - 2];
+            c[i - 1] = two ? sp[i - 2] : c[i - 2];
+            const uint32_t w = two ? sj[i - 2] : 0u;
+            if (i <= 4)
+                ch.x |= w << 8 * (i - 1);
+            else
+                ch.y |= w << 8 * (i - 5);
+        }
+        float4* dc = reinterpret_cast<float4*>(B.dpc + 8 * (size_t)p);
+        dc[0] = make_float4(c[0], c[1], c[2], c[3]);
+        dc[1] = make_float4(c[4], c[5], c[6], c[7]);
+        B.dpch[p] = ch;
+    }
 }
 
 // The same as a call, for the clustering kernels, which are there for something

@@ -101,10 +101,6 @@ int ReadStatus(fnd_rt_ctx* ctx) {
 
 using namespace Foundation::CApi;
 
-namespace {
-
-}  // namespace
-
 namespace Foundation {
 namespace CApi {
 

@@ -71,8 +71,11 @@ __global__ void __launch_bounds__(kBlock) generate_kernel(const PathBuffers B, c
 
 // One interaction of each queued path. What bounds it: the latency of its
 // dependent gathers (queue entry, path state, hit, shading record, material)
-// and of the queue appends, not bytes (DRAM at 11%) nor issue (25%). Hence
-// @CFG@
+// and of the queue appends, not bytes (DRAM at 11%) nor issue (25%). Hence as
+// many warps as registers allow without spills that show: 80 registers, six
+// blocks of 128 (24 warps per SM). Plain 1080p frame of 2 spp with four, five,
+// six and eight such blocks 4,102, 4,090, 4,038 and 4,036 us, with three of 256
+// 4,046; the cache frame 1,366, 1,365, 1,362, 1,367 and 1,365.
 // kFirst: the camera rays' hits (see generate_kernel).
 template <uint32_t kMode, bool kFirst>
 __global__ void __launch_bounds__(kShadeBlock, kShadeBlocksPerSm)

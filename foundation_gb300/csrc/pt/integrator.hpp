@@ -121,11 +121,12 @@ constexpr int kCountExt = 0, kCountShadow = kCountExt + kMaxBounces + 1, kCountF
 constexpr int kCountTailDone = kCountFetch + 2 * kMaxBounces, kCountTailFetch = kCountTailDone + 1;
 constexpr int kCounts = kCountTailFetch + 1;
 
-// The tail of a wave: once the extension queue of interaction `bounce` holds at most `threshold` paths, one persistent
-// megakernel finishes every one of them (lanes fetch paths dynamically and
-// run them to the end with single-ray traversal and the shade stage's
-// vertex logic) and empties the queue, so the remaining wavefront stages of
-// the wave find nothing to do. Above the threshold it returns at once.
+// The tail of a wave: once the extension queue of interaction `bounce` holds at
+// most `threshold` paths, one persistent megakernel finishes every one of them
+// (lanes fetch paths dynamically and run them to the end with the shade stage's
+// vertex logic, their rays traced by the whole warp: path_rays.cuh) and empties
+// the queue, so the remaining wavefront stages of the wave find nothing to do.
+// Above the threshold it returns at once.
 // Results are those of the wavefront stages: same random numbers per path,
 // same hits; only the order of the frame-buffer additions differs.
 struct TailArgs {

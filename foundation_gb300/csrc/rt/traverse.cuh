@@ -106,10 +106,10 @@ __device__ __forceinline__ bool intersect_tri(const RayState& r, float4 v0, floa
     return true;
 }
 
-// Packed FP32 pairs for the child-box test: two slots' plane FMAs in one
-// fma.rm / fma.rp .f32x2 (sm_100 family). Each lane rounds exactly like the
-// scalar __fmaf_rd / __fmaf_ru (tests/test_minmax_gpu.py checks it on the
-// GPU); the host build evaluates the scalar forms.
+// Packed FP32 pairs for the child-box test: a slot's two plane FMAs in one
+// fma.rm.f32x2 (sm_100 family). Each lane rounds exactly like the scalar
+// __fmaf_rd (tests/test_minmax_gpu.py checks it on the GPU); the host build
+// evaluates the scalar form.
 struct F2 {
 #if defined(__CUDA_ARCH__)
     unsigned long long v;
@@ -127,19 +127,15 @@ __device__ __forceinline__ F2 pack_f2(float a, float b) {
 #endif
     return r;
 }
-// out = a * b + c per lane, rounded down (kUp false) or up (kUp true)
-template <bool kUp>
-__device__ __forceinline__ void fma_dir_f2(F2 a, F2 b, F2 c, float out[2]) {
+// out = a * b + c per lane, rounded down
+__device__ __forceinline__ void fma_rd_f2(F2 a, F2 b, F2 c, float out[2]) {
 #if defined(__CUDA_ARCH__)
     unsigned long long d;
-    if (kUp)
-        asm("fma.rp.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a.v), "l"(b.v), "l"(c.v));
-    else
-        asm("fma.rm.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a.v), "l"(b.v), "l"(c.v));
+    asm("fma.rm.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a.v), "l"(b.v), "l"(c.v));
     asm("mov.b64 {%0, %1}, %2;" : "=f"(out[0]), "=f"(out[1]) : "l"(d));
 #else
-    out[0] = kUp ? __fmaf_ru(a.x, b.x, c.x) : __fmaf_rd(a.x, b.x, c.x);
-    out[1] = kUp ? __fmaf_ru(a.y, b.y, c.y) : __fmaf_rd(a.y, b.y, c.y);
+    out[0] = __fmaf_rd(a.x, b.x, c.x);
+    out[1] = __fmaf_rd(a.y, b.y, c.y);
 #endif
 }
 
@@ -232,9 +228,8 @@ __device__ __forceinline__ SlotHits intersect_slots(const RayState& r, const uin
     // fma(q, s, b), the culling stays conservative and the hits exact.
     // A slot's near and far plane go through one packed FMA, the far one
     // negated (ru(x) = -rd(-x)), so both round down and one pair of constants
-    // per axis serves both: 12 registers across the eight slots (18 with the
-    // constants duplicated for slot pairs, which at the persistent kernels'
-    // 56 registers cost about 60 register moves per node).
+    // per axis serves both: 12 registers across the eight slots, 18 with the
+    // constants duplicated for slot pairs.
     const F2 sx2 = pack_f2(sx, -sx), sy2 = pack_f2(sy, -sy), sz2 = pack_f2(sz, -sz);
     const F2 bx2 = pack_f2(__fmaf_rd(-1.0f, sx, bx), __fmaf_rd(1.0f, sx, -bx));
     const F2 by2 = pack_f2(__fmaf_rd(-1.0f, sy, by), __fmaf_rd(1.0f, sy, -by));
@@ -263,9 +258,9 @@ __device__ __forceinline__ SlotHits intersect_slots(const RayState& r, const uin
             // positive sign and equal values +0, a hit as under tn <= tf; only
             // tf = -0 against tn = +0 would differ, hence bound_of.
             float tx[2], ty[2], tz[2];  // near t, -(far t)
-            fma_dir_f2<false>(pack_f2(nx[e], gx[e]), sx2, bx2, tx);
-            fma_dir_f2<false>(pack_f2(ny[e], gy[e]), sy2, by2, ty);
-            fma_dir_f2<false>(pack_f2(nz[e], gz[e]), sz2, bz2, tz);
+            fma_rd_f2(pack_f2(nx[e], gx[e]), sx2, bx2, tx);
+            fma_rd_f2(pack_f2(ny[e], gy[e]), sy2, by2, ty);
+            fma_rd_f2(pack_f2(nz[e], gz[e]), sz2, bz2, tz);
             const float tn = max3f(tx[0], ty[0], fmaxf(tz[0], r.tmin));
             const float ntf = max3f(tx[1], ty[1], fmaxf(tz[1], ntfar));
 #if defined(__CUDA_ARCH__)
@@ -329,10 +324,11 @@ __device__ __forceinline__ NodeHits intersect_node(const RayState& r, const uint
 namespace Foundation {
 namespace RT {
 
-// Single-ray traversal with a thread-local stack and no warp refill: the plain
-// form that the warp loop (warp_trace.cuh) is tested against, on the host too.
-// Same node / triangle tests and tie rule as the persistent kernels. Returns true on a hit (best_t / best_p updated; the
-// caller initialises best_t to the ray's tmax).
+// Reached by tests only, from here on (intersect_node too): the plain form that
+// the warp loop (warp_trace.cuh) is tested against, on the host as well. Single-
+// ray traversal with a thread-local stack and no warp refill; the node and
+// triangle tests and the tie rule are the persistent kernels'. Returns true on a
+// hit (best_t / best_p updated; the caller initialises best_t to the ray's tmax).
 template <bool kAny>
 __device__ __forceinline__ bool trace_single(const DeviceScene& sc, const RayState& r, float& best_t,
                                              uint32_t& best_p, uint32_t* status) {

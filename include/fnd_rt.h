@@ -123,7 +123,9 @@ enum { FND_BVH_SPATIAL_SPLITS = 1u };
  * faster to build (31M triangles in tens of ms), a few per cent slower to
  * trace than the binned-SAH tree on large flat scenes; hits are identical.
  * Up to 2^27 triangles; not combined with spatial splits; build_threads is
- * ignored. */
+ * ignored. From the first such upload on a context keeps up to 1 GB of the
+ * device memory that its builds and their scenes have freed, for the next
+ * build; fnd_rt_destroy gives it back. */
 enum { FND_BVH_GPU_BUILD = 2u };
 /* Collapse the binary tree into 8-wide nodes by the SAH-optimal dynamic
  * programme (Ylitie, Karras & Laine 2017) instead of the greedy rule: fuller
