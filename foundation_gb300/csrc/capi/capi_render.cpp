@@ -369,13 +369,22 @@ int fnd_rt_render(fnd_rt_ctx* ctx, const fnd_rt_scene* scene, const fnd_render_d
         PT::PathBuffers& B = ctx->paths;
         const int grid_shade = std::max(1, std::min<int>((int)((cap + 255) / 256), ctx->sm_count * 8));
         CUDA_CHECK(cudaMemsetAsync(ctx->d_render_stats, 0, 2 * sizeof(unsigned long long), ctx->stream));
-        // tail megakernel threshold: by default two paths per resident tail thread
+        // Tail megakernel threshold: by default 768 paths per SM, and a whole
+        // wave of at most two paths per resident tail thread (1,024 per SM with
+        // one level, 768 with two). The larger threshold for all waves holds the
+        // SMs for the tail's longest paths while frames of other contexts could
+        // use them. us per plain frame, one context / three at once, 768, this
+        // rule, 1,024: 480x270 589 / 370, 435 / 308, 435 / 308; 640x360 728 /
+        // 478, 728 / 478, 714 / 509; 1920x1080 x 2 3,988 / 3,640, 3,988 / 3,640,
+        // 4,000 / 3,690.
         int& tail_occ = ctx->tail_blocks_per_sm[scene->two_level ? 1 : 0];
         if (tail_occ == 0) tail_occ = PT::TailBlocksPerSm(scene->two_level);
-        const uint32_t tail_paths =
-            (D.flags & FND_RENDER_WAVEFRONT)
-                ? 0u
-                : (D.tail_paths ? D.tail_paths : 2u * (uint32_t)ctx->sm_count * (uint32_t)tail_occ * PT::kTailBlock);
+        const uint32_t whole_wave = 2u * (uint32_t)ctx->sm_count * (uint32_t)tail_occ * PT::kTailBlock;
+        auto tail_threshold = [&](uint32_t wave_n) -> uint32_t {
+            if (D.flags & FND_RENDER_WAVEFRONT) return 0u;
+            if (D.tail_paths) return D.tail_paths;
+            return wave_n <= whole_wave ? whole_wave : 768u * (uint32_t)ctx->sm_count;
+        };
         PT::CacheIO C{};
         if (use_cache) {
             // 1) training, on the cache's own stream so it overlaps the render
@@ -434,7 +443,7 @@ int fnd_rt_render(fnd_rt_ctx* ctx, const fnd_rt_scene* scene, const fnd_render_d
             B.wave_pixel = (uint32_t)(wave_base % npix);
             B.wave_sample = (uint32_t)(wave_base / npix);
             CUDA_CHECK(PT::LaunchGenerate(B, R, wave_n, ctx->stream));
-            RunBounces(ctx, scene, B, R, S, C, wave_n, D.max_depth, grid_shade, tail_paths);
+            RunBounces(ctx, scene, B, R, S, C, wave_n, D.max_depth, grid_shade, tail_threshold(wave_n));
             if (use_cache) {
                 CUDA_CHECK(cudaStreamWaitEvent(ctx->stream, ctx->cache->ev_trained, 0));
                 CUDA_CHECK(NRC::Infer(ctx->cache->net, C.queries, C.query_count, C.query_cap, B.fb,

@@ -13,7 +13,8 @@
 // steps 640 and 500 us (with 200 instances 1,440 and 930), a whole frame of
 // 640x360 990 and 790 us (5,020 and 1,820), of 192x108 724 and 560 (2,250 and
 // 1,290), of 1920x1080 x 2 4,130 and 4,025 us. 128 registers and 16 warps per
-// SM: with 80 and 64 registers the training takes 560 and 620 us.
+// SM with one level: with 80 and 64 registers the training took 560 and 620 us
+// against those 500, and with 168 (12 warps) 464 against 455 since (kCounted).
 #pragma once
 
 #include "../rt/warp_trace.cuh"
