@@ -33,13 +33,19 @@ __device__ __forceinline__ float sanitize_dir(float d) {
     return fabsf(d) < 5.421010862427522e-20f ? copysignf(5.421010862427522e-20f, d) : d;
 }
 
+// The culling bound of a best t (or a ray's length) for intersect_slots: the
+// same value, with +0 for -0. A hit at the origin often has t = -0, and against
+// a node's tn = +0 the sign of -0 - (+0) would say that the box is missed, with
+// triangles of equal t and lower id in it. (Once per bound, not per node.)
+__device__ __forceinline__ float bound_of(float t) { return __fadd_rn(t, 0.0f); }
+
 __device__ __forceinline__ RayState setup_ray(float4 r0, float4 r1) {
     RayState s;
     s.ox = r0.x;
     s.oy = r0.y;
     s.oz = r0.z;
     s.tmin = r0.w;
-    s.tmax = r1.w;
+    s.tmax = bound_of(r1.w);
     s.ix = __fdiv_rn(1.0f, sanitize_dir(r1.x));
     s.iy = __fdiv_rn(1.0f, sanitize_dir(r1.y));
     s.iz = __fdiv_rn(1.0f, sanitize_dir(r1.z));
@@ -179,12 +185,6 @@ __device__ __forceinline__ uint32_t xor_permute8(uint32_t m, uint32_t oct) {
     if (oct & 4u) m = ((m & 0x0Fu) << 4) | (m >> 4);
     return m;
 }
-
-// The culling bound of a best t (or a ray's length) for intersect_slots: the
-// same value, with +0 for -0. A hit at the origin often has t = -0, and against
-// a node's tn = +0 the sign of -0 - (+0) would say that the box is missed, with
-// triangles of equal t and lower id in it. (Once per bound, not per node.)
-__device__ __forceinline__ float bound_of(float t) { return __fadd_rn(t, 0.0f); }
 
 // Tests the 8 child boxes of one compressed node against the ray: which slots
 // were hit, and the node's words that say what the slots hold. tfar: a bound_of.

@@ -305,7 +305,7 @@ __device__ __forceinline__ void trace_loop(const Src& src, const Common& C, uint
                 slot = lane;
                 if constexpr (kOwnScene) cur = src.scene_of(ln);
                 if constexpr (kOwnKind) follows_any = any_hit;
-                best_t = bound_of(r.tmax);
+                best_t = r.tmax;
                 sts64(wl + W::kBest, __float_as_uint(r.tmax), FND_INVALID_ID);
                 start(src.scene_of(ln).num_nodes, octx_of(r));
                 active = true;
