@@ -100,7 +100,11 @@ void RunBounces(fnd_rt_ctx* ctx, const fnd_rt_scene* scene, const PT::PathBuffer
     const bool two = scene->two_level;
     int& tail_occ = ctx->tail_blocks_per_sm[two ? 1 : 0];
     if (tail_paths && tail_occ == 0) tail_occ = PT::TailBlocksPerSm(two);
-    const int g_tail = ctx->sm_count * std::max(1, tail_occ);
+    // The tail of a small wave on at most three blocks per SM: its lanes then
+    // take a second path now and then, and other contexts' kernels find room
+    // (167x237 x 2, three frames at once: 324 us with four blocks, 312 with three).
+    const bool small_wave = wave_n <= 768u * (uint32_t)ctx->sm_count;
+    const int g_tail = ctx->sm_count * (small_wave ? std::min(3, std::max(1, tail_occ)) : std::max(1, tail_occ));
     RT::TraceConfig cfg0 = ctx->trace_cfg;
     cfg0.sort_bits = 0;
     // cache paths end in queries at the second interaction: what continues
